@@ -296,6 +296,20 @@ void with_skf(const gfsph_handle* h, F&& f) {
     }
 }
 
+// Calls f with std::integral_constant<int, lanes per particle> of k_density
+// for n particles.  Few particles leave the chip idle and the step waits for
+// the longest chain of one lane: more lanes shorten it (850 particles: 57 us a
+// launch with one, 11 with 8; 23k: 4 and 8 lanes equal, 3.29 and 3.32 ms per 25
+// steps).  From ~100k on the chip is full and the lanes' uneven rows and
+// shuffles count (200k particles, 20 steps with their copies: 6.4, 6.0, 6.4 ms
+// for 1, 2, 4 lanes; 1M, 10 steps: 10.2, 9.7, 10.6 ms).
+template <class F>
+void with_lanes(int n, F&& f) {
+    if (n < 12000) f(std::integral_constant<int, 8>{});
+    else if (n < 100000) f(std::integral_constant<int, 4>{});
+    else f(std::integral_constant<int, 2>{});
+}
+
 // Stage-dependent pressure: the step runs the staged RK45 kernels.
 bool staged(const gfsph_handle* h) { return h->rheo.nor_density || h->rheo.cos_theta || h->rheo.ws; }
 
@@ -334,7 +348,7 @@ Search make_search(gfsph_handle* h) {
     return q;
 }
 
-int big_blocks(const gfsph_handle*) { return 148 * 16; }  // 128 threads: one warp per coarse-level particle
+int big_blocks(const gfsph_handle*) { return 148 * 4; }  // a block of kBigThreads per coarse-level particle
 
 // The cell search: bounds, grid, counting sort, reorder, neighbours+density.
 // Returns the number of kernels enqueued.
@@ -378,17 +392,21 @@ int enqueue_search(gfsph_handle* h, int advance) {
     fork(h, 0);
     with_skf(h, [&](auto sk) {
         constexpr int SKF = decltype(sk)::value;
-        launch(h, K_DENSITY_BIG, [&] { pdl_launch(k_density_big<SKF>, big_blocks(h), 128, sb, h->A, q, S, h->rheo); });
+        launch(h, K_DENSITY_BIG, [&] { pdl_launch(k_density_big<SKF>, big_blocks(h), kBigThreads, sb, h->A, q, S, h->rheo); });
         // the two materials' pair types compiled in only when there are two
-        if (h->rheo.ws) {
-            launch(h, K_DENSITY, [&] { pdl_launch(k_density<false, SKF, true>, pb, kThreads, st, h->A, q, S, h->rheo, n); });
-            launch(h, K_DENSITY_SPARSE,
-                   [&] { pdl_launch(k_density<true, SKF, true>, pb, kThreads, st, h->A, q, S, h->rheo, n); });
-        } else {
-            launch(h, K_DENSITY, [&] { pdl_launch(k_density<false, SKF, false>, pb, kThreads, st, h->A, q, S, h->rheo, n); });
-            launch(h, K_DENSITY_SPARSE,
-                   [&] { pdl_launch(k_density<true, SKF, false>, pb, kThreads, st, h->A, q, S, h->rheo, n); });
-        }
+        with_lanes(n, [&](auto g) {
+            constexpr int G = decltype(g)::value;
+            const int db = std::min(blocks_for((long long)n * G, kDenThreads), 148 * kDenBlocks * 3);
+            if (h->rheo.ws) {
+                launch(h, K_DENSITY, [&] { pdl_launch(k_density<false, SKF, true, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
+                launch(h, K_DENSITY_SPARSE,
+                       [&] { pdl_launch(k_density<true, SKF, true, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
+            } else {
+                launch(h, K_DENSITY, [&] { pdl_launch(k_density<false, SKF, false, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
+                launch(h, K_DENSITY_SPARSE,
+                       [&] { pdl_launch(k_density<true, SKF, false, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
+            }
+        });
     });
     nk += 3;
     join(h, 0);
@@ -420,7 +438,7 @@ int enqueue_norms(gfsph_handle* h, PState As[5]) {
         });
         launch(h, K_NORM_BIG, [&] {
             with_skf(h, [&](auto sk) {
-                pdl_launch(k_norm_big<decltype(sk)::value>, big_blocks(h), 128, st, h->A, q, h->S, c, hp, clamp, As[k].rho);
+                pdl_launch(k_norm_big<decltype(sk)::value>, big_blocks(h), kBigThreads, st, h->A, q, h->S, c, hp, clamp, As[k].rho);
             });
         });
         nk += 2;
@@ -478,7 +496,7 @@ int enqueue_stages(gfsph_handle* h, PState As[5]) {
     if (c.ws) {
         with_skf(h, [&](auto sk) {
             launch(h, K_WIR, [&] {
-                pdl_launch(k_wir_pairs_big<decltype(sk)::value>, big_blocks(h), 128, st, h->A, q, S, c);
+                pdl_launch(k_wir_pairs_big<decltype(sk)::value>, big_blocks(h), kBigThreads, st, h->A, q, S, c);
             });
         });
         nk += 1 + enqueue_wir_stage(h, As, 0);
@@ -487,7 +505,7 @@ int enqueue_stages(gfsph_handle* h, PState As[5]) {
     }
     for (int s = 0; s < 4; s++) {
         launch(h, K_FORCE_BIG, [&] {
-            with_skf(h, [&](auto sk) { pdl_launch(k_force_big<decltype(sk)::value>, big_blocks(h), 128, st, As[s], q, S, c); });
+            with_skf(h, [&](auto sk) { pdl_launch(k_force_big<decltype(sk)::value>, big_blocks(h), kBigThreads, st, As[s], q, S, c); });
         });
         nk++;
         launch(h, K_IFORCE, [&] {
@@ -552,7 +570,7 @@ int enqueue_step(gfsph_handle* h) {
         if (h->rheo.av_vel) {  // av_vel with the final depth
             launch(h, K_XSPH_BIG, [&] {
                 with_skf(h, [&](auto sk) {
-                    pdl_launch(k_xsph_big<decltype(sk)::value>, big_blocks(h), 128, st, As[4], q, S, h->rheo, h->B);
+                    pdl_launch(k_xsph_big<decltype(sk)::value>, big_blocks(h), kBigThreads, st, As[4], q, S, h->rheo, h->B);
                 });
             });
             launch(h, K_XSPH, [&] {
@@ -571,7 +589,7 @@ int enqueue_step(gfsph_handle* h) {
     cudaStream_t sb = side_stream(h);
     fork(h, 1);
     launch(h, K_FORCE_BIG, [&] {
-        with_skf(h, [&](auto sk) { pdl_launch(k_force_big<decltype(sk)::value>, big_blocks(h), 128, sb, h->A, q, S, h->rheo); });
+        with_skf(h, [&](auto sk) { pdl_launch(k_force_big<decltype(sk)::value>, big_blocks(h), kBigThreads, sb, h->A, q, S, h->rheo); });
     });
     nk++;
     launch(h, K_IFORCE, [&] {
@@ -591,7 +609,7 @@ int enqueue_step(gfsph_handle* h) {
         fork(h, 2);
         launch(h, K_XSPH_BIG, [&] {
             with_skf(h, [&](auto sk) {
-                pdl_launch(k_xsph_big<decltype(sk)::value>, big_blocks(h), 128, sb, h->A, q, S, h->rheo, h->B);
+                pdl_launch(k_xsph_big<decltype(sk)::value>, big_blocks(h), kBigThreads, sb, h->A, q, S, h->rheo, h->B);
             });
         });
         nk++;
@@ -1190,7 +1208,7 @@ int gfsph_upload(gfsph_handle* h, int n, const float* x, const float* v, const f
         st |= alloc_pstate(&h->A, n); st |= alloc_pstate(&h->B, n); st |= alloc_pstate(&h->U, n);
         st |= dalloc(&h->cellA, n); st |= dalloc(&h->velfin, n); st |= dalloc(&h->pterm, n);
         st |= dalloc(&h->keyrank, n); st |= dalloc(&h->perm, n); st |= dalloc(&h->ncount, n);
-        st |= dalloc(&h->f2tmp, n); st |= dalloc(&h->xhm, n); st |= dalloc(&h->indv, n); st |= dalloc(&h->rho0, n);
+        st |= dalloc(&h->f2tmp, n); st |= dalloc(&h->xhm, (size_t)n + kScanStep); st |= dalloc(&h->indv, n); st |= dalloc(&h->rho0, n);
         st |= dalloc(&h->xsv, n); st |= dalloc(&h->pr, n);
         if (staged(h)) {
             StageCarry& C = h->carry;
@@ -1436,7 +1454,7 @@ int gfsph_density(gfsph_handle* h, float* rho_out) try {
         });
         launch(h, K_NORM_BIG, [&] {
             with_skf(h, [&](auto sk) {
-                k_norm_big<decltype(sk)::value><<<big_blocks(h), 128, 0, h->stream>>>(h->A, q, h->S, h->rheo, h->rho0, 0,
+                k_norm_big<decltype(sk)::value><<<big_blocks(h), kBigThreads, 0, h->stream>>>(h->A, q, h->S, h->rheo, h->rho0, 0,
                                                                                      h->rhoS);
             });
         });
@@ -1469,7 +1487,7 @@ int gfsph_internal_forces(gfsph_handle* h, float* indvxdt) try {
         with_skf(h, [&](auto sk) { k_iforce<decltype(sk)::value, false><<<blocks_for(n), kThreads, 0, s>>>(As[0], q, h->S, h->rheo, n); });
     });
     launch(h, K_FORCE_BIG, [&] {
-        with_skf(h, [&](auto sk) { k_force_big<decltype(sk)::value><<<big_blocks(h), 128, 0, s>>>(As[0], q, h->S, h->rheo); });
+        with_skf(h, [&](auto sk) { k_force_big<decltype(sk)::value><<<big_blocks(h), kBigThreads, 0, s>>>(As[0], q, h->S, h->rheo); });
     });
     launch(h, K_FORCE_RK, [&] {
         k_force_rk<false, true><<<blocks_for(n), kThreads, 0, s>>>(h->A, q, h->S, h->rheo, h->dem, n, h->B,
@@ -1512,7 +1530,7 @@ int gfsph_neighbours(gfsph_handle* h, int cap, int* offsets, int* idx) try {
             Search q = make_search(h);
             launch(h, K_EXPORT, [&] {
                 with_skf(h, [&](auto sk) {
-                    k_export_big<decltype(sk)::value><<<big_blocks(h), 128, 0, h->stream>>>(q, h->S, dpairs, dcount, pcap);
+                    k_export_big<decltype(sk)::value><<<big_blocks(h), kBigThreads, 0, h->stream>>>(q, h->S, dpairs, dcount, pcap);
                 });
             });
             cudaStreamSynchronize(h->stream);

@@ -19,6 +19,37 @@ __device__ __forceinline__ float ipow5(float x) {
     return (x2 * x) * x2;
 }
 
+// Correctly rounded reciprocal, square root and quotient from the hardware's
+// approximations, for operands that the caller bounds (kQuotMin .. kQuotMax
+// below), so that no range check and no slow path is compiled in:
+// - recip: one Newton-Raphson step in FMA on the approximate reciprocal;
+// - root: Markstein's square root step (P. Markstein, "Computation of
+//   elementary functions on the IBM RISC System/6000 processor", 1990) on the
+//   approximate reciprocal root: g = d y, then g + (d - g g) y/2;
+// - quot: his division step with y = RN(1/b): q = RN(a y), the exact
+//   remainder r = a - q b, RN(q + r y) = RN(a/b); several quotients by one
+//   denominator share the reciprocal.
+// The first two equal the IEEE operators for every mantissa, the third in
+// 1.8e10 random quotients (tests/test_gpu_rounding.py repeats the check).
+__device__ __forceinline__ float recip(float b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return __fmaf_rn(__fmaf_rn(-b, y, 1.f), y, y);
+}
+__device__ __forceinline__ float root(float d) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+    const float g = d * y;
+    return __fmaf_rn(__fmaf_rn(-g, g, d), 0.5f * y, g);
+}
+__device__ __forceinline__ float quot(float a, float b, float y) {
+    const float q = a * y;
+    return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+}
+// Smoothing lengths for which every product and quotient of a pair's kernel
+// stays far from overflow and underflow.
+constexpr float kQuotMin = 1.e-6f, kQuotMax = 1.e9f;
+
 // kernel_TOOLS, My_SPH_Tools_2019.f90:2062-2180 (2-D; skf 1 cubic spline,
 // skf 2 Gaussian, skf 3 quintic, skf 4 Wendland C2).  Returns w and dW/dx
 // for the offset (dx0, dx1) at distance r with smoothing length hs.  The
@@ -81,6 +112,35 @@ __device__ __forceinline__ void sph_kernel(float r, float dx0, float dx1, float 
             d1 = t * (s * dx1);
         }
     }
+}
+
+// The cubic spline (skf 1) of a pair again, from the square of its distance,
+// for smoothing lengths within kQuotMin .. kQuotMax and r < 2 hs: the same
+// values bit for bit, both branches of q in one instruction stream (the lanes
+// of a warp mix them) and the square root and up to six IEEE divisions of a
+// pair as three reciprocals, a root and quot().  r is kept off 0 (coincident
+// particles), where it does not reach a bit of the result.
+__device__ __forceinline__ void sph_kernel_spline(float dr, float dx0, float dx1, float hs, float& w, float& d0,
+                                                  float& d1) {
+    const float r = root(fmaxf(dr, 1.e-36f));
+    const float yh = recip(hs);
+    const float q = quot(r, hs, yh);
+    const float fd = ((7.f * kPi) * hs) * hs;
+    const float factor = quot(15.f, fd, recip(fd));
+    const float f6 = quot(factor, 6.f, 1.f / 6.f);
+    const bool inner = q <= 1.f;
+    const float u = 2.f - q, u2 = u * u;
+    // W
+    const float wi = factor * ((kTwoThirds - q * q) + ((q * q) * q) / 2.f);
+    const float wo = f6 * (u2 * u);
+    // gradient: inner (factor (-2 + 1.5 q)/(hs hs)) dx; outer -(3 f6 u^2/hs) (dx/r)
+    const float h2 = hs * hs;
+    const float yd = recip(inner ? h2 : r);
+    const float num = inner ? factor * (-2.f + 1.5f * q) : -((f6 * 3.f) * u2);
+    const float t = quot(num, inner ? h2 : hs, inner ? yd : yh);
+    w = inner ? wi : wo;
+    d0 = t * (inner ? dx0 : quot(dx0, r, yd));
+    d1 = t * (inner ? dx1 : quot(dx1, r, yd));
 }
 
 template <int SKF>
@@ -147,6 +207,25 @@ __device__ __forceinline__ bool pair_search(float2 xi, float2 xj, float hi, floa
     g.mh = (hi + hj) / 2.f;
     g.r = sqrtf(dr);
     return g.r < (float)SK * g.mh;
+}
+
+// The test alone, for the scan over candidates: lo = 0.99998 (0 takes the
+// exact test always, for smoothing lengths whose squares underflow).  The
+// squares decide away from the edge of the support, with FMA and a margin of
+// 1e-5 on either side, far above their rounding; the pairs in between take
+// the test itself.
+template <int SK>
+__device__ __forceinline__ bool pair_kept(float2 xi, float4 o, float hi, float lo) {
+    const float d0 = xi.x - o.x, d1 = xi.y - o.y;
+    const float dr = __fmaf_rn(d1, d1, d0 * d0);
+    const float t = (SK == 2) ? hi + o.z : 1.5f * (hi + o.z);
+    const float u = t * (t * 1.00001f);
+    bool ok = dr <= u;
+    if (ok && dr >= u * lo) {
+        PairGeom g;
+        ok = pair_search<SK>(xi, make_float2(o.x, o.y), hi, o.z, g);
+    }
+    return ok;
 }
 
 // Float <-> order-preserving uint, for atomicMin/atomicMax reductions.

@@ -9,8 +9,10 @@
 // level (dense mode).  Beyond it (separated releases on a large DEM with
 // small smoothing lengths) the grids are block-sparse: cut into blocks of
 // 32 x 8 cells, a dense block map over the box marks the blocks that hold
-// particles, and only those blocks get cells (slot-major keys: slot * 256 +
-// row * 32 + column), so the cell count follows the area the flow covers.
+// particles, and only those blocks get cells, so the cell count follows the
+// area the flow covers.  The occupied blocks of one block row share their
+// keys row by row (sparse_key), so that a row of cells is one key range in
+// either layout, across block edges too.
 #pragma once
 #include <climits>
 
@@ -21,7 +23,9 @@ namespace gfsph {
 constexpr int kScanTile = 2048;  // cells per scan tile (256 threads x 8)
 constexpr int kScanThreads = 256;
 constexpr float kBigFactor = 1.5f;  // default level-0 bound Hc = kBigFactor * mean(hsml)
-constexpr float kCellDiv = 3.f;     // default cell size of level k: Hc * 2^k / kCellDiv
+constexpr float kCellDiv = 3.f;     // default cell width of level k: Hc * 2^k / kCellDiv
+constexpr float kCellAspect = 1.5f;  // cell height over width: a stencil row is one slot range whatever its width,
+                                     // so fewer, higher rows cost less than the candidates they add
 constexpr int kRegLevels = 2;       // default regular levels: their particles take a thread and the table
 constexpr int kMaxLevels = 24;      // level k cell size Hc * 2^(k-1)
 constexpr int kBlkX = 32;           // cells per block along x
@@ -53,7 +57,7 @@ struct StepScalars {
     int bad;          // non-finite state seen by k_bounds
     float hc;         // regular-hsml bound Hc: level k holds hsml in (Hc*2^(k-1), Hc*2^k], level 0 hsml <= Hc
     int nlev;         // number of grid levels
-    float lev_gx0[kMaxLevels], lev_gy0[kMaxLevels], lev_c[kMaxLevels];  // origin and cell size per level
+    float lev_gx0[kMaxLevels], lev_gy0[kMaxLevels], lev_c[kMaxLevels];  // origin and cell width per level
     int lev_ndx[kMaxLevels], lev_ndy[kMaxLevels];  // cells per level along x and y
     int lev_off[kMaxLevels + 1];  // dense mode: first cell key of each level
     int lev_nbx[kMaxLevels], lev_boff[kMaxLevels + 1];  // sparse mode: blocks per level along x, first block-map entry
@@ -381,7 +385,8 @@ __device__ void grid_setup(const Rheo& c, StepScalars* S, const GridArgs ga) {
     long long off = 0, doff = 0;
     for (int k = 0; k < nlev; k++) {
         float cell = ldexpf(hc, k) / cell_div;
-        float fx = lx / cell + 1.f, fy = ly / cell + 1.f;
+        const float cellh = cell * kCellAspect;
+        float fx = lx / cell + 1.f, fy = ly / cellh + 1.f;
         if (!(fx < 1.0e8f) || !(fy < 1.0e8f) || !(fx * fy < 2.0e9f)) {  // far beyond any capacity
             S->err |= kErrCells;
             S->need_cells = 0x3fffffff;
@@ -389,7 +394,7 @@ __device__ void grid_setup(const Rheo& c, StepScalars* S, const GridArgs ga) {
             return;
         }
         int ndx = (int)fx, ndy = (int)fy;
-        float lxn = (float)ndx * cell, lyn = (float)ndy * cell;
+        float lxn = (float)ndx * cell, lyn = (float)ndy * cellh;
         S->lev_gx0[k] = (xmn - (lxn - lx) / 2.f) - 0.001f * lx;
         S->lev_gy0[k] = (ymn - (lyn - ly) / 2.f) - 0.001f * ly;
         S->lev_c[k] = cell;
@@ -430,7 +435,7 @@ __device__ void grid_setup(const Rheo& c, StepScalars* S, const GridArgs ga) {
 __device__ __forceinline__ void cell_of(float2 p, const StepScalars* S, int k, int& cx, int& cy) {
     float gd = S->lev_c[k];
     int ix = (int)((p.x - S->lev_gx0[k]) / gd + 1.f);
-    int iy = (int)((p.y - S->lev_gy0[k]) / gd + 1.f);
+    int iy = (int)((p.y - S->lev_gy0[k]) / (gd * kCellAspect) + 1.f);
     cx = min(max(ix, 1), S->lev_ndx[k]) - 1;
     cy = min(max(iy, 1), S->lev_ndy[k]) - 1;
 }
@@ -445,6 +450,17 @@ __device__ __forceinline__ int level_of(float hs, const StepScalars* S) {
 // the block sides compile to shifts and masks.
 __device__ __forceinline__ int block_of(const StepScalars* S, int k, int cx, int cy) {
     return S->lev_boff[k] + (int)((unsigned)cy / kBlkY) * S->lev_nbx[k] + (int)((unsigned)cx / kBlkX);
+}
+
+// Sparse layout: the key of cell (cx, cy) of level k, block b.  The occupied
+// blocks of its block row (block-map entries rb .. rb + nbx - 1, slots f ..
+// f + nocc - 1) take 256 nocc keys from 256 f, cell row by cell row, 32 keys a
+// block in each.
+__device__ __forceinline__ int sparse_key(const StepScalars* S, const int* bstart, int k, int cx, int cy, int b) {
+    const int nbx = S->lev_nbx[k], rb = S->lev_boff[k] + (int)((unsigned)cy / kBlkY) * nbx;
+    const int f = bstart[rb], nocc = bstart[rb + nbx] - f;
+    return f * kBlockCells + (int)((unsigned)cy % kBlkY) * (nocc * kBlkX) + (bstart[b] - f) * kBlkX +
+           (int)((unsigned)cx % kBlkX);
 }
 
 // Marks the blocks that hold particles (block map, all levels) and takes the
@@ -482,7 +498,7 @@ __global__ void k_mark(const PState B, int n, DemView dem, StepScalars* S, int* 
         if (lmax[k]) atomicMax(&S->lev_hmax_o[k], lmax[k]);
 }
 
-// Cell key (slot of the particle's block * 256 + cell within the block) and
+// Cell key (row-major in the dense layout, sparse_key in the sparse one) and
 // within-cell arrival rank of each particle (counting sort histogram,
 // grid_find :938-948); out-of-domain particles get key -1.  Clears the block
 // marks for the next step.  If the occupied blocks need more cells than the
@@ -510,7 +526,7 @@ __global__ void k_hist(const PState B, int n, DemView dem, StepScalars* S, int* 
             if (sparse) {
                 int b = block_of(S, k, cx, cy);
                 bmark[b] = 0;
-                key = bstart[b] * kBlockCells + (int)((unsigned)cy % kBlkY) * kBlkX + (int)((unsigned)cx % kBlkX);
+                key = sparse_key(S, bstart, k, cx, cy, b);
             } else {
                 key = S->lev_off[k] + cy * S->lev_ndx[k] + cx;
             }
@@ -746,224 +762,307 @@ __device__ __forceinline__ bool ref_adjacent(const Search& Q, int2 ci, int j) {
     return abs(cj.x - ci.x) <= 1 && abs(cj.y - ci.y) <= 1;
 }
 
-// Stencil of level k around particle i: every j of level k has hsml_j <= Hk
-// (the level's largest smoothing length), so with r < SK/2 (hi + hj) it lies
-// within floor(SK/2 (hi + Hk)/cell + 0.01) + 1 cells of i's cell in that
-// level's grid, whatever the rounding of the cell coordinates.  Returns false
-// for an empty level.
-template <int SK = 2>
-__device__ __forceinline__ bool level_stencil(const StepScalars* S, int k, float2 xi, float hi, int& x0, int& x1,
-                                              int& y0, int& y1) {
-    unsigned int hk = S->lev_hmax_o[k];
-    if (hk == 0u) return false;
-    float rr = support_span<SK>(hi, o2f(hk)) / S->lev_c[k] + 0.01f;
-    int R = (rr < 1.0e8f) ? (int)rr + 1 : 100000000;
-    int cx, cy;
-    cell_of(xi, S, k, cx, cy);
-    x0 = max(cx - R, 0); x1 = min(cx + R, S->lev_ndx[k] - 1);
-    y0 = max(cy - R, 0); y1 = min(cy + R, S->lev_ndy[k] - 1);
-    return true;
-}
-
-// Slot range of the cells x0..x1 of row jy inside block column bx (empty if
-// the block holds no particles).
-__device__ __forceinline__ void block_row_range(const Search& Q, const StepScalars* S, int k, int jy, int bx, int x0,
-                                                int x1, int& ja, int& jb) {
-    if (!S->sparse) {  // dense: the row is one key range (bx is 0)
-        int row = S->lev_off[k] + jy * S->lev_ndx[k];
-        ja = Q.start[row + x0];
-        jb = Q.start[row + x1 + 1];
-        return;
-    }
-    int b = S->lev_boff[k] + (int)((unsigned)jy / kBlkY) * S->lev_nbx[k] + bx;
-    int s0 = Q.bstart[b];
-    if (Q.bstart[b + 1] == s0) { ja = jb = 0; return; }
-    int lo = max(x0, bx * kBlkX) - bx * kBlkX, hi = min(x1, bx * kBlkX + kBlkX - 1) - bx * kBlkX;
-    int key = s0 * kBlockCells + (int)((unsigned)jy % kBlkY) * kBlkX;
-    ja = Q.start[key + lo];
-    jb = Q.start[key + hi + 1];
-}
-
-// Pair test of particle i (reference-grid cell ci) against the slots ja..jb-1.
-template <int SK, class F>
-__device__ __forceinline__ void visit_range(const Search& Q, int i, float2 xi, float hi, int2 ci, int ja, int jb,
-                                            F& f) {
-    for (int j = ja; j < jb; j++) {
-        if (j == i) continue;
-        float4 o = Q.xhm[j];
-        PairGeom g;
-        if (pair_search<SK>(xi, make_float2(o.x, o.y), hi, o.z, g) && ref_adjacent<SK>(Q, ci, j)) f(j, o, g);
-    }
-}
-
-// Visits the particles j != i of level k that are neighbours of particle i
-// (position xi, smoothing length hi), row by row of the stencil, each row in
-// cell order.  Rows further than one cell from i's row are trimmed to the
-// circle: a particle of row jy, d = |jy - cy| >= 2 rows away, is more than
-// (d - 1) cells away in y, so with r < hi + Hk it lies within
-// sqrt(rr^2 - (d - 1)^2) + 1 cells in x (rr and d - 1 carry 0.01-cell
-// margins for the rounding of the cell coordinates).  A dense row is one key
-// range; a sparse row is one range per block column it crosses.
-template <bool SPARSE, int SK, class F>
-__device__ __forceinline__ void level_neighbours(const Search& Q, const StepScalars* S, int k, int i, float2 xi, float hi,
-                                                 int2 ci, F&& f) {
-    const unsigned int hk = S->lev_hmax_o[k];
-    if (hk == 0u) return;
-    const float rr = support_span<SK>(hi, o2f(hk)) / S->lev_c[k] + 0.01f;
-    const int R = (rr < 1.0e8f) ? (int)rr + 1 : 100000000;
-    const float rr2 = rr * rr;
-    int cx, cy;
-    cell_of(xi, S, k, cx, cy);
-    const int ndx = S->lev_ndx[k], nbx = S->lev_nbx[k], boff = S->lev_boff[k];
-    const int y0 = max(cy - R, 0), y1 = min(cy + R, S->lev_ndy[k] - 1);
-    for (int jy = y0; jy <= y1; jy++) {
-        const int d = abs(jy - cy);
-        int rx = R;
-        if (d >= 2) {
-            const float dd = (float)d - 1.01f;
-            const float q = rr2 - dd * dd;
-            if (!(q > 0.f)) continue;
-            rx = min(R, (int)sqrtf(q) + 1);
-        }
-        const int x0 = max(cx - rx, 0), x1 = min(cx + rx, ndx - 1);
-        if (!SPARSE) {
-            const int rowoff = S->lev_off[k] + jy * ndx;
-            visit_range<SK>(Q, i, xi, hi, ci, Q.start[rowoff + x0], Q.start[rowoff + x1 + 1], f);
-            continue;
-        }
-        const int c0 = (int)((unsigned)x0 / kBlkX), c1 = (int)((unsigned)x1 / kBlkX);
-        const int brow = boff + (int)((unsigned)jy / kBlkY) * nbx;
-        const int row = (int)((unsigned)jy % kBlkY) * kBlkX;
-        if (c1 - c0 <= 1) {
-            // one or two block columns: the two slot ranges are walked as one
-            // sequence, so lanes whose rows straddle a block edge and lanes
-            // whose rows do not run the same loop (no divergent second pass)
-            const int s0 = Q.bstart[brow + c0], s1 = Q.bstart[brow + c0 + 1];
-            const int e0 = min(x1, c0 * kBlkX + kBlkX - 1);
-            int ja = 0, na = 0, jb = 0, nb = 0;
-            if (s1 != s0) {
-                const int key = s0 * kBlockCells + row - c0 * kBlkX;
-                ja = Q.start[key + x0];
-                na = Q.start[key + e0 + 1] - ja;
-            }
-            if (c1 > c0) {
-                const int s2 = Q.bstart[brow + c1 + 1];
-                if (s2 != s1) {
-                    const int key = s1 * kBlockCells + row - c1 * kBlkX;
-                    jb = Q.start[key + c1 * kBlkX];
-                    nb = Q.start[key + x1 + 1] - jb;
-                }
-            }
-            for (int t = 0; t < na + nb; t++) {
-                const int j = (t < na) ? ja + t : jb + (t - na);
-                if (j == i) continue;
-                float4 o = Q.xhm[j];
-                PairGeom g;
-                if (pair_search<SK>(xi, make_float2(o.x, o.y), hi, o.z, g) && ref_adjacent<SK>(Q, ci, j)) f(j, o, g);
-            }
-            continue;
-        }
-        int s1 = Q.bstart[brow + c0];
-        for (int bx = c0; bx <= c1; bx++) {
-            const int s0 = s1;
-            s1 = Q.bstart[brow + bx + 1];  // end of this block = start of the next
-            if (s1 == s0) continue;
-            const int key = s0 * kBlockCells + row - bx * kBlkX;
-            visit_range<SK>(Q, i, xi, hi, ci, Q.start[key + max(x0, bx * kBlkX)],
-                        Q.start[key + min(x1, bx * kBlkX + kBlkX - 1) + 1], f);
-        }
-    }
-}
-
 // Neighbour search and summation density of the regular particles, fused:
-// every j with r < 2*(hi+hj)/2 (the pair set of grid_find, :987-1060), on
-// every level, is appended to the neighbour table (tab_base) with the pair's
-// kernel value and gradient, and h_i = W(0,h_i) m_i + sum_j m_j W_ij
-// (sum_density_Tools :1796-1836) is accumulated in FP64.  Also stores the
-// pressure term of IntForces_SW with h clamped to h_inf (:6769, :6797): p/h^2
-// (pa_sph 2) or p (pa_sph 1).
-template <bool SPARSE, int SKF, bool WS>
-__device__ __forceinline__ void density_regular(PState& A, const Search& Q, StepScalars* S, const Rheo& c) {
-    constexpr int SK = SupportScale<SKF>::value;
-    const int nreg = S->nreg, nlev = S->nlev;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nreg; i += gridDim.x * blockDim.x) {
-        float4 me = Q.xhm[i];
-        float2 xi = make_float2(me.x, me.y);
-        float hi = me.z;
-        const int2 ci = (SK == 2) ? make_int2(0, 0) : Q.rcell[i];
-        double acc = (double)(sph_kernel_w<SKF>(0.f, hi) * me.w);
-        int4* tab = Q.nbr + tab_base(i, Q.kcap);
-        int cnt = 0;
-        const unsigned char si = WS ? Q.spec[i] : 0;
-        for (int k = 0; k < nlev; k++)
-            level_neighbours<SPARSE, SK>(Q, S, k, i, xi, hi, ci, [&](int j, float4 o, const PairGeom& g) {
-                // W and grad W of the pair, once per step: the internal force,
-                // av_vel and the normalisation read them from the table
-                float w, d0, d1;
-                sph_kernel<SKF>(g.r, g.dx0, g.dx1, g.mh, w, d0, d1);
-                const bool cross = WS && Q.spec[j] != si;
-                if (cnt < Q.kcap)  // kept in L2 for the internal force (written back to front)
-                    tab[(size_t)cnt * kTabStride] =
-                        make_int4(cross ? (j | kCrossBit) : j, __float_as_int(w), __float_as_int(d0),
-                                  __float_as_int(d1));
-                cnt++;
-                if (!cross) acc += (double)(o.w * w);
-            });
-        Q.ncount[i] = cnt;
-        if (cnt > Q.kcap) {  // table too small: stop this step before any state is written
-            atomicOr(&S->err, kErrNbr);
-            atomicMax(&S->need_nbr, cnt);
-            atomicExch(&S->skip, 1);
+// every j with r < 2*(hi+hj)/2 (the pair set of grid_find, :987-1060) is
+// entered in the neighbour table (tab_base) with the pair's kernel value and
+// gradient, and h_i = W(0,h_i) m_i + sum_j m_j W_ij (sum_density_Tools
+// :1796-1836) is accumulated in FP64.  Also stores the pressure term of
+// IntForces_SW with h clamped to h_inf (:6769, :6797): p/h^2 (pa_sph 2) or p
+// (pa_sph 1).
+//
+// G lanes share a particle.  Two phases: (1) each lane scans every G-th row
+// of the stencil and lists the neighbours it finds in shared memory (the test
+// alone, ~12 instructions a candidate, half of which are kept); (2) the
+// lanes share out the listed pairs evenly and evaluate them, every lane busy,
+// the table entries of a warp in whole sectors.  One pass over the candidates
+// that evaluated a pair wherever one lane of the warp kept it ran the ~130
+// instructions of a pair at a third of its lanes and, with one thread per
+// particle, as one chain of 100 dependent gathers: 57 us even for 850
+// particles.  A lane whose list is full counts on; the scan is then repeated
+// for the next kDenList of each lane.
+constexpr int kDenThreads = 128;
+constexpr int kDenBlocks = 7;  // resident blocks asked for
+constexpr int kScanStep = 2;  // candidates loaded at a time
+template <int G> struct DenList { static constexpr int value = (G == 2) ? 40 : (G == 4 ? 24 : 16); };  // ~1.5x a lane's share of 50
+// The particles of the coarse levels, few, are not searched through their
+// mostly empty grids: each block picks those that reach its particles' box
+// and its lanes test these alone.  Beyond kBigScan of them the grids are
+// walked as well.
+constexpr int kBigScan = 4096;
+
+// The rows of level k's cells that the support of particle i (position xi,
+// smoothing length hi) can touch: every j of the level has hsml_j <= Hk (the
+// level's largest), so |x_i - x_j| < SK/2 (hi + Hk).  In units of the cell
+// width, with i at (u, v): row jy lies dy away from it, and j within
+// sqrt(s^2 - dy^2) of u in that row, taken from i's place inside its cell (the
+// cell numbers alone would cost a cell on each side: 102 candidates for 46
+// neighbours on the lattice, 66 with the place).  ex, ey (cells) cover the
+// rounding of u, v and of j's own cell numbers, 2^-21 of the grid's extent and
+// more.  Either layout keeps a row's cells in order, so each row is one slot
+// range.
+template <bool SPARSE>
+struct LevelRows {
+    float u, v, s2, ex, ey;
+    int y0, nrow, ndx, base, nbx;  // base: the level's first key (dense) or block-map entry (sparse)
+
+    // false for an empty level
+    template <int SK>
+    __device__ __forceinline__ bool open(const StepScalars* S, int k, float2 xi, float hi) {
+        const unsigned int hk = S->lev_hmax_o[k];
+        if (hk == 0u) return false;
+        const float rc = 1.f / S->lev_c[k];
+        ndx = S->lev_ndx[k];
+        const int ndy = S->lev_ndy[k];
+        // clamped as the cell numbers are: that brings no two particles further apart
+        u = fminf(fmaxf((xi.x - S->lev_gx0[k]) * rc, 0.f), (float)ndx);
+        v = fminf(fmaxf((xi.y - S->lev_gy0[k]) * (rc * (1.f / kCellAspect)), 0.f), (float)ndy);
+        const float s = support_span<SK>(hi, o2f(hk)) * rc;
+        s2 = s * s;
+        ex = 0.01f + (float)ndx * 1.e-6f;
+        ey = 0.01f + (float)ndy * 1.e-6f;
+        const float sy = s * (1.f / kCellAspect) + ey;
+        y0 = min(max((int)(v - sy), 0), ndy - 1);
+        nrow = min((int)fminf(v + sy, 1.e9f), ndy - 1) - y0 + 1;
+        base = SPARSE ? S->lev_boff[k] : S->lev_off[k];
+        nbx = SPARSE ? S->lev_nbx[k] : 0;
+        return true;
+    }
+
+    // slots ja .. jb-1 of the row-th row (empty: ja >= jb)
+    __device__ __forceinline__ void range(const Search& Q, int row, int& ja, int& jb) const {
+        ja = jb = 0;
+        const int jy = y0 + row;
+        const float dy = fmaxf(fmaxf((float)jy - v, v - (float)(jy + 1)) - ey, 0.f) * kCellAspect;
+        const float q = s2 - dy * dy;
+        if (!(q > 0.f)) return;
+        const float hw = q * rsqrtf(q) + ex;
+        const int x0 = min(max((int)(u - hw), 0), ndx - 1), x1 = min((int)fminf(u + hw, 1.e9f), ndx - 1);
+        if (!SPARSE) {
+            const int key = base + jy * ndx;
+            ja = Q.start[key + x0];
+            jb = Q.start[key + x1 + 1];
+            return;
         }
-        float h = (float)acc;
-        A.rho[i] = h;
-        float hc = (h < c.h_inf) ? c.h_inf : h;
-        float p = (c.cgra05 * hc) * hc;
-        const float pt = (c.pa_sph == 1) ? p : p / (hc * hc);
-        Q.pterm[i] = pt;
-        Q.pr[i] = make_float4(pt, h, me.w, 0.f);
+        const int rb = base + (int)((unsigned)jy / kBlkY) * nbx;
+        const int f = Q.bstart[rb], nocc = Q.bstart[rb + nbx] - f;
+        if (nocc == 0) return;
+        const int c0 = (int)((unsigned)x0 / kBlkX), c1 = (int)((unsigned)x1 / kBlkX);
+        const int s0 = Q.bstart[rb + c0], s1 = Q.bstart[rb + c1];
+        // an empty block at either end adds no keys
+        const int o0 = (Q.bstart[rb + c0 + 1] != s0) ? (int)((unsigned)x0 % kBlkX) : 0;
+        const int o1 = (Q.bstart[rb + c1 + 1] != s1) ? (int)((unsigned)x1 % kBlkX) + 1 : 0;
+        const int key = f * kBlockCells + (int)((unsigned)jy % kBlkY) * (nocc * kBlkX) - f * kBlkX;
+        ja = Q.start[key + s0 * kBlkX + o0];
+        jb = Q.start[key + s1 * kBlkX + o1];
+    }
+};
+
+// Bound by FP32 issue and the latency of the gathers: 200k particles (release,
+// two lanes) 89 us a launch where one thread per particle, evaluating each
+// pair as it was found, took 115; the flow with coarse levels 106 against 190;
+// 1M particles 390 against 480.  Instantiated for both cell layouts; the
+// launch whose layout this step does not use returns at once.
+template <bool SPARSE, int SKF, bool WS, int G>
+__global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, Search Q, StepScalars* S, Rheo c, int n) {
+    PDL_ENTRY();
+    if ((S->sparse != 0) != SPARSE) return;
+    if (__syncthreads_or(S->skip)) return;  // another block may set it meanwhile: one decision per block
+    constexpr int SK = SupportScale<SKF>::value;
+    constexpr int L = DenList<G>::value, P = kDenThreads / G;
+    constexpr unsigned full = 0xffffffffu;
+    __shared__ int list[L * kDenThreads];  // entry e of thread t at e * kDenThreads + t
+    __shared__ float4 bigs[kDenThreads];
+    __shared__ int bigj[kDenThreads];
+    __shared__ float wbox[kDenThreads / 32][5];
+    __shared__ int wcnt[kDenThreads / 32];
+    const int tid = threadIdx.x, gl = tid % G, lane = tid & 31, wid = tid >> 5;
+    const int nreg = S->nreg, nbig = S->nbig;
+    const bool scan_big = nbig > 0 && nbig <= kBigScan;
+    const int nlev = (nbig > 0 && !scan_big) ? S->nlev : min(S->nlev, S->reg_levels);
+    const float hmax = o2f(S->hmax_o);
+    for (int base = blockIdx.x * P; base < nreg; base += gridDim.x * P) {  // the same trips for the whole block
+        const int i = base + tid / G;
+        const bool act = i < nreg;
+        const float4 me = Q.xhm[act ? i : base];
+        const float2 xi = make_float2(me.x, me.y);
+        const float hi = me.z;
+        const int2 ci = (SK == 2) ? make_int2(0, 0) : Q.rcell[act ? i : base];
+        const unsigned char si = WS ? Q.spec[act ? i : base] : 0;
+        const bool safe = SKF == 1 && hi >= 2.f * kQuotMin && hmax <= kQuotMax;
+        int4* tab = Q.nbr + tab_base(act ? i : base, Q.kcap);
+        float bx0 = 0.f, bx1 = 0.f, by0 = 0.f, by1 = 0.f, bh = 0.f;  // the block's box and largest hsml
+        if (scan_big) {
+            bx0 = warp_min(me.x); bx1 = warp_max(me.x);
+            by0 = warp_min(me.y); by1 = warp_max(me.y);
+            bh = warp_max(hi);
+            if (lane == 0) {
+                wbox[wid][0] = bx0; wbox[wid][1] = bx1; wbox[wid][2] = by0; wbox[wid][3] = by1; wbox[wid][4] = bh;
+            }
+            __syncthreads();
+            for (int w = 0; w < kDenThreads / 32; w++) {
+                bx0 = fminf(bx0, wbox[w][0]); bx1 = fmaxf(bx1, wbox[w][1]);
+                by0 = fminf(by0, wbox[w][2]); by1 = fmaxf(by1, wbox[w][3]);
+                bh = fmaxf(bh, wbox[w][4]);
+            }
+        }
+        const float lo = hi > 1.e-14f ? 0.99998f : 0.f;
+        double acc = 0.0;
+        int found = 0;  // entries of this particle in the table
+        for (int skip = 0;; skip += L) {
+            // phase 1: the neighbours this lane finds, from the skip-th on, go into its list; at points to the next
+            // place, before the list while the first skip ones pass
+            int at = tid - skip * kDenThreads;
+            auto keep = [&](int j) {
+                if ((unsigned)at < (unsigned)(L * kDenThreads)) list[at] = j;
+                at += kDenThreads;
+            };
+            int first = gl;  // this lane's first row of the next level
+            for (int k = 0; k < nlev; k++) {
+                LevelRows<SPARSE> rows;
+                if (!rows.template open<SK>(S, k, xi, hi)) continue;
+                if (act)
+                    for (int s = first; s < rows.nrow; s += G) {
+                        int ja, jb;
+                        rows.range(Q, s, ja, jb);
+                        for (int j = ja; j < jb; j += kScanStep) {
+                            float4 o[kScanStep];  // xhm is padded by kScanStep entries
+#pragma unroll
+                            for (int u = 0; u < kScanStep; u++) o[u] = Q.xhm[j + u];
+#pragma unroll
+                            for (int u = 0; u < kScanStep; u++)
+                                if (pair_kept<SK>(xi, o[u], hi, lo) && j + u < jb && j + u != i &&
+                                    ref_adjacent<SK>(Q, ci, j + u))
+                                    keep(j + u);
+                        }
+                    }
+                first = (first + G - rows.nrow % G) % G;
+            }
+            if (scan_big)
+                for (int b0 = 0; b0 < nbig; b0 += kDenThreads) {
+                    const int b = nreg + b0 + tid;
+                    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+                    bool near = false;
+                    if (b0 + tid < nbig) {
+                        o = Q.xhm[b];
+                        // distance to the box, with a margin for the rounding of both sides
+                        const float dx = fmaxf(0.f, fmaxf(bx0 - o.x, o.x - bx1)), dy = fmaxf(0.f, fmaxf(by0 - o.y, o.y - by1));
+                        const float t = support_span<SK>(bh, o.z);
+                        near = dx * dx + dy * dy <= (t * t) * 1.0001f;
+                    }
+                    const unsigned m = __ballot_sync(full, near);
+                    __syncthreads();  // the last chunk has been read
+                    if (lane == 0) wcnt[wid] = __popc(m);
+                    __syncthreads();
+                    int put = __popc(m & ((1u << lane) - 1u)), tot = 0;
+                    for (int w = 0; w < kDenThreads / 32; w++) {
+                        if (w < wid) put += wcnt[w];
+                        tot += wcnt[w];
+                    }
+                    if (near) { bigs[put] = o; bigj[put] = b; }
+                    __syncthreads();
+                    if (act)
+                        for (int e = gl; e < tot; e += G) {
+                            const int j = bigj[e];
+                            if (pair_kept<SK>(xi, bigs[e], hi, lo) && ref_adjacent<SK>(Q, ci, j)) keep(j);
+                        }
+                }
+            // phase 2: the group's listed pairs in lane order, shared out evenly
+            const int mine = min(max((at - tid) / kDenThreads, 0), L);
+            int pre = mine;  // exclusive prefix over the lanes of the group
+#pragma unroll
+            for (int o = 1; o < G; o <<= 1) {
+                const int t = __shfl_up_sync(full, pre, o, G);
+                if (gl >= o) pre += t;
+            }
+            const int tot = __shfl_sync(full, pre, G - 1, G);
+            pre -= mine;
+            int from[G];  // the lanes' first entries
+#pragma unroll
+            for (int o = 0; o < G; o++) from[o] = __shfl_sync(full, pre, o, G);
+            __syncwarp();
+            auto entry = [&](int t) {  // the neighbour at place t of the group's lists
+                int own = 0, f = 0;
+#pragma unroll
+                for (int o = 1; o < G; o++)
+                    if (t >= from[o]) { own = o; f = from[o]; }
+                return list[(t - f) * kDenThreads + tid - gl + own];
+            };
+            auto pair = [&](int t, int j, const float4& o) {
+                const float dx0 = xi.x - o.x, dx1 = xi.y - o.y;
+                const float dr = dx0 * dx0 + dx1 * dx1;
+                const float mh = (hi + o.z) / 2.f;
+                float w, d0, d1;
+                if (safe) sph_kernel_spline(dr, dx0, dx1, mh, w, d0, d1);
+                else sph_kernel<SKF>(sqrtf(dr), dx0, dx1, mh, w, d0, d1);
+                const bool cross = WS && Q.spec[j] != si;
+                if (found + t < Q.kcap)  // kept in L2 for the internal force (written back to front)
+                    tab[(size_t)(found + t) * kTabStride] = make_int4(cross ? (j | kCrossBit) : j, __float_as_int(w),
+                                                                      __float_as_int(d0), __float_as_int(d1));
+                if (!cross) acc += (double)(o.w * w);
+            };
+            int t = gl;
+            for (; t + G < tot; t += 2 * G) {  // two independent pairs at a time
+                const int ja = entry(t), jb = entry(t + G);
+                const float4 oa = Q.xhm[ja], ob = Q.xhm[jb];
+                pair(t, ja, oa);
+                pair(t + G, jb, ob);
+            }
+            if (t < tot) {
+                const int j = entry(t);
+                pair(t, j, Q.xhm[j]);
+            }
+            found += tot;
+            const bool more = at - tid > L * kDenThreads;
+            if (scan_big ? !__syncthreads_or(more) : !__any_sync(full, more)) break;
+        }
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(full, acc, o);
+        if (act && gl == 0) {
+            Q.ncount[i] = found;
+            if (found > Q.kcap) {  // table too small: stop this step before any state is written
+                atomicOr(&S->err, kErrNbr);
+                atomicMax(&S->need_nbr, found);
+                atomicExch(&S->skip, 1);
+            }
+            const float h = (float)((double)(sph_kernel_w<SKF>(0.f, hi) * me.w) + acc);
+            A.rho[i] = h;
+            const float hc = (h < c.h_inf) ? c.h_inf : h;
+            const float p = (c.cgra05 * hc) * hc;
+            const float pt = (c.pa_sph == 1) ? p : p / (hc * hc);
+            Q.pterm[i] = pt;
+            Q.pr[i] = make_float4(pt, h, me.w, 0.f);
+        }
+        if (scan_big) __syncthreads();  // the box is rewritten
     }
 }
 
-// Instantiated for both cell layouts; the launch whose layout this step does
-// not use returns at once (one kernel with both walks would spill in the
-// dense walk).  Held to 48 registers (10 blocks of 128 per SM): the gathers
-// are latency-bound.
-template <bool SPARSE, int SKF, bool WS>
-__global__ void __launch_bounds__(128, 10) k_density(PState A, Search Q, StepScalars* S, Rheo c, int n) {
-    PDL_ENTRY();
-    if (S->skip || (S->sparse != 0) != SPARSE) return;
-    density_regular<SPARSE, SKF, WS>(A, Q, S, c);
-}
-
-// Visits every neighbour j of particle i cooperatively over one warp: the
-// lanes fetch the slot ranges of up to 32 (row, block column) segments of the
-// stencil at once, then share each segment's candidates.
-template <int SK, class F>
-__device__ __forceinline__ void warp_neighbours(const Search& Q, const StepScalars* S, int i, int lane, F&& f) {
+// A coarse-level particle, few but with up to every particle in its support,
+// takes a block of kBigThreads: its warps share the rows of a level's stencil,
+// the lanes fetch the slot ranges of up to 32 rows at once, then share each
+// row's candidates.  (With one warp each, the one with the longest list took
+// 38 us of the 200k flow's step in each of the three passes.)
+constexpr int kBigThreads = 256;
+template <bool SPARSE, int SK, class F>
+__device__ __forceinline__ void block_rows(const Search& Q, const StepScalars* S, int i, F& f) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    constexpr int W = kBigThreads / 32;
     const float4 me = Q.xhm[i];
     const float2 xi = make_float2(me.x, me.y);
     const float hi = me.z;
     const int2 ci = (SK == 2) ? make_int2(0, 0) : Q.rcell[i];
     for (int k = 0; k < S->nlev; k++) {
-        int x0, x1, y0, y1;
-        if (!level_stencil<SK>(S, k, xi, hi, x0, x1, y0, y1)) continue;
-        const int bx0 = S->sparse ? (int)((unsigned)x0 / kBlkX) : 0;
-        const int ncol = S->sparse ? (int)((unsigned)x1 / kBlkX) - bx0 + 1 : 1;
-        const long long nseg = (long long)(y1 - y0 + 1) * ncol;
-        for (long long sb = 0; sb < nseg; sb += 32) {
-            long long sg = sb + lane;
+        LevelRows<SPARSE> rows;
+        if (!rows.template open<SK>(S, k, xi, hi)) continue;
+        for (int rb = 0; rb < rows.nrow; rb += kBigThreads) {
+            const int row = rb + W * lane + wid;
             int ja = 0, jb = 0;
-            if (sg < nseg) {
-                int jy = y0 + (int)(sg / ncol), bx = bx0 + (int)(sg % ncol);
-                block_row_range(Q, S, k, jy, bx, x0, x1, ja, jb);
-            }
-            int nr = (int)min(32LL, nseg - sb);
+            if (row < rows.nrow) rows.range(Q, row, ja, jb);
+            const int nr = min(32, (rows.nrow - rb - wid + W - 1) / W);
             for (int r = 0; r < nr; r++) {
-                int a = __shfl_sync(0xffffffffu, ja, r), e = __shfl_sync(0xffffffffu, jb, r);
+                const int a = __shfl_sync(0xffffffffu, ja, r), e = __shfl_sync(0xffffffffu, jb, r);
                 for (int j = a + lane; j < e; j += 32) {
                     if (j == i) continue;
-                    float4 o = Q.xhm[j];
+                    const float4 o = Q.xhm[j];
                     PairGeom g;
                     if (pair_search<SK>(xi, make_float2(o.x, o.y), hi, o.z, g) && ref_adjacent<SK>(Q, ci, j))
                         f(j, o, g);
@@ -972,26 +1071,41 @@ __device__ __forceinline__ void warp_neighbours(const Search& Q, const StepScala
         }
     }
 }
+template <int SK, class F>
+__device__ __forceinline__ void block_neighbours(const Search& Q, const StepScalars* S, int i, F&& f) {
+    if (S->sparse) block_rows<true, SK>(Q, S, i, f);
+    else block_rows<false, SK>(Q, S, i, f);
+}
+// Sum over the block in a fixed order, in thread 0; every thread calls it.
+__device__ __forceinline__ double block_sum(double v) {
+    __shared__ double part[kBigThreads / 32];
+    v = warp_sum(v);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < kBigThreads / 32; w++) t += part[w];
+    return t;
+}
 
-// Summation density of the coarse-level particles, one warp per particle.
+// Summation density of the coarse-level particles, one block per particle.
 template <int SKF>
-__global__ void __launch_bounds__(128) k_density_big(PState A, Search Q, StepScalars* S, Rheo c) {
+__global__ void __launch_bounds__(kBigThreads) k_density_big(PState A, Search Q, StepScalars* S, Rheo c) {
     PDL_ENTRY();
     constexpr int SK = SupportScale<SKF>::value;
     if (S->skip) return;
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = warp; b < nbig; b += nwarps) {
+    for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
         int i = nreg + b;
         double acc = 0.0;
         const unsigned char si = c.ws ? Q.spec[i] : 0;
-        warp_neighbours<SK>(Q, S, i, lane, [&](int j, float4 o, const PairGeom& g) {
+        block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
             if (c.ws && Q.spec[j] != si) return;  // type 1: not in the density (:1829)
             acc += (double)(o.w * sph_kernel_w<SKF>(g.r, g.mh));
         });
-        acc = warp_sum(acc);
-        if (lane == 0) {
+        acc = block_sum(acc);
+        if (threadIdx.x == 0) {
             float4 me = Q.xhm[i];
             float h = (float)((double)(sph_kernel_w<SKF>(0.f, me.z) * me.w) + acc);
             A.rho[i] = h;
@@ -1032,28 +1146,26 @@ __device__ __forceinline__ void pressure_pair(const Rheo& c, float pi_, float rh
     pressure_terms(c, pi_, rhoi, pj, rhoj, mj, d0, d1, a0, a1);
 }
 
-// Internal acceleration of the coarse-level particles, one warp per particle.
+// Internal acceleration of the coarse-level particles, one block per particle.
 template <int SKF>
-__global__ void __launch_bounds__(128) k_force_big(PState A, Search Q, StepScalars* S, Rheo c) {
+__global__ void __launch_bounds__(kBigThreads) k_force_big(PState A, Search Q, StepScalars* S, Rheo c) {
     PDL_ENTRY();
     constexpr int SK = SupportScale<SKF>::value;
     if (S->skip) return;
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = warp; b < nbig; b += nwarps) {
+    for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
         int i = nreg + b;
         const float4 pri = Q.pr[i];
         double a0 = 0.0, a1 = 0.0;
         const unsigned char si = c.ws ? Q.spec[i] : 0;
-        warp_neighbours<SK>(Q, S, i, lane, [&](int j, float4 o, const PairGeom& g) {
+        block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
             if (c.ws && Q.spec[j] != si) return;  // type 0 only (:6899)
             const float4 prj = Q.pr[j];
             pressure_pair<SKF>(c, pri.x, pri.y, prj.x, prj.y, o.w, g, a0, a1);
         });
-        a0 = warp_sum(a0);
-        a1 = warp_sum(a1);
-        if (lane == 0) Q.indv[i] = make_float2((float)a0, (float)a1);
+        a0 = block_sum(a0);
+        a1 = block_sum(a1);
+        if (threadIdx.x == 0) Q.indv[i] = make_float2((float)a0, (float)a1);
     }
 }
 
@@ -1460,24 +1572,22 @@ __global__ void __launch_bounds__(128) k_norm(PState A, Search Q, StepScalars* S
     }
 }
 
-// The same for the coarse-level particles, one warp each.
+// The same for the coarse-level particles, one block each.
 template <int SKF>
-__global__ void __launch_bounds__(128) k_norm_big(PState A, Search Q, StepScalars* S, Rheo c, const float* hp,
+__global__ void __launch_bounds__(kBigThreads) k_norm_big(PState A, Search Q, StepScalars* S, Rheo c, const float* hp,
                                                   int clamp_prev, float* hout) {
     PDL_ENTRY();
     constexpr int SK = SupportScale<SKF>::value;
     if (S->skip) return;
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = warp; b < nbig; b += nwarps) {
+    for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
         const int i = nreg + b;
         double den = 0.0;
-        warp_neighbours<SK>(Q, S, i, lane, [&](int j, float4 o, const PairGeom& g) {
+        block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
             den += (double)((o.w / prev_depth(c, hp, j, clamp_prev)) * sph_kernel_w<SKF>(g.r, g.mh));
         });
-        den = warp_sum(den);
-        if (lane == 0) {
+        den = block_sum(den);
+        if (threadIdx.x == 0) {
             const float4 me = Q.xhm[i];
             den = (double)((sph_kernel_w<SKF>(0.f, me.z) * me.w) / prev_depth(c, hp, i, clamp_prev)) + den;
             hout[i] = A.rho[i] / (float)den;
@@ -1642,28 +1752,26 @@ __global__ void __launch_bounds__(128) k_wir_press(PState A, Search Q, StepScala
     }
 }
 
-// The soil-water pair sums of the coarse-level particles, one warp each.
+// The soil-water pair sums of the coarse-level particles, one block each.
 template <int SKF>
-__global__ void __launch_bounds__(128) k_wir_pairs_big(PState A, Search Q, StepScalars* S, Rheo c) {
+__global__ void __launch_bounds__(kBigThreads) k_wir_pairs_big(PState A, Search Q, StepScalars* S, Rheo c) {
     PDL_ENTRY();
     constexpr int SK = SupportScale<SKF>::value;
     if (S->skip) return;
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = warp; b < nbig; b += nwarps) {
+    for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
         const int i = nreg + b;
         const unsigned char si = Q.spec[i];
         double b0 = 0.0, b1 = 0.0;
-        warp_neighbours<SK>(Q, S, i, lane, [&](int j, float4 o, const PairGeom& g) {
+        block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
             if (Q.spec[j] == si) return;
             float w, d0, d1;
             sph_kernel<SKF>(g.r, g.dx0, g.dx1, g.mh, w, d0, d1);
             wir_pair_term(c, si == 2, o.w, d0, d1, b0, b1);
         });
-        b0 = warp_sum(b0);
-        b1 = warp_sum(b1);
-        if (lane == 0) Q.bxy[i] = make_float2((float)b0, (float)b1);
+        b0 = block_sum(b0);
+        b1 = block_sum(b1);
+        if (threadIdx.x == 0) Q.bxy[i] = make_float2((float)b0, (float)b1);
     }
 }
 
@@ -1865,29 +1973,27 @@ __global__ void __launch_bounds__(128) k_xsph(PState A, Search Q, StepScalars* S
 }
 
 template <int SKF>
-__global__ void __launch_bounds__(128) k_xsph_big(PState A, Search Q, StepScalars* S, Rheo c, PState B) {
+__global__ void __launch_bounds__(kBigThreads) k_xsph_big(PState A, Search Q, StepScalars* S, Rheo c, PState B) {
     PDL_ENTRY();
     constexpr int SK = SupportScale<SKF>::value;
     if (S->skip || !c.av_vel) return;
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = warp; b < nbig; b += nwarps) {
+    for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
         int i = nreg + b;
-        if (B.flag[i]) continue;  // uniform over the warp
+        if (B.flag[i]) continue;  // uniform over the block
         const float4 si = Q.xsv[i];
         const float2 vi = make_float2(si.x, si.y);
         const float rhoi = si.z;
         double a0 = 0.0, a1 = 0.0;
         const unsigned char si_ = c.ws ? Q.spec[i] : 0;
-        warp_neighbours<SK>(Q, S, i, lane, [&](int j, float4 o, const PairGeom& g) {
+        block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
             if (c.ws && Q.spec[j] != si_) return;  // type 0 only (SPH_MAIN_2019.f90:3071)
             const float4 sj = Q.xsv[j];
             xsph_pair<SKF>(vi, rhoi, make_float2(sj.x, sj.y), sj.z, sj.w, g, a0, a1);
         });
-        a0 = warp_sum(a0);
-        a1 = warp_sum(a1);
-        if (lane == 0) {
+        a0 = block_sum(a0);
+        a1 = block_sum(a1);
+        if (threadIdx.x == 0) {
             float av0 = 0.3f * (float)a0, av1 = 0.3f * (float)a1;
             B.vel[i] = make_float2(vi.x + av0, vi.y + av1);
         }
@@ -1968,12 +2074,10 @@ __global__ void k_dem_erode(double2* auxv, float* z, float* eroded, float* avail
 template <int SKF>
 __global__ void k_export_big(Search Q, StepScalars* S, int2* pairs, int* npairs, int cap) {
     constexpr int SK = SupportScale<SKF>::value;
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = warp; b < nbig; b += nwarps) {
+    for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
         int i = nreg + b;
-        warp_neighbours<SK>(Q, S, i, lane, [&](int j, float4 o, const PairGeom& g) {
+        block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
             int k = atomicAdd(npairs, 1);
             if (k < cap) pairs[k] = make_int2(i, j);
         });

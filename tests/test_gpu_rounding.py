@@ -1,0 +1,61 @@
+"""recip, root and quot of csrc/gfsph_device.cuh against CUDA's IEEE operators,
+bit for bit: the first two over every mantissa at several exponents of their
+range, the quotient over seeded random operands and over dividends next to
+the midpoints between two floats."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "deslizamientos-y-flujos_b200", "csrc")
+
+SOURCE = r"""
+#include "gfsph_device.cuh"
+using namespace gfsph;
+__global__ void k_check(unsigned long long* bad) {
+    const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    const int ex[6] = {-60, -31, -1, 0, 28, 59};
+    unsigned long long b0 = 0, b1 = 0, b2 = 0;
+    for (unsigned m = tid; m < (1u << 23); m += nt)
+        for (int e = 0; e < 6; e++) {
+            const float b = __uint_as_float(((unsigned)(127 + ex[e]) << 23) | m);
+            if (recip(b) != __fdiv_rn(1.f, b)) b0++;
+            if (root(b) != __fsqrt_rn(b)) b1++;
+        }
+    unsigned long long s = 88172645463325252ULL + tid * 7919000003ULL;
+    for (int i = 0; i < 4000; i++) {
+        s ^= s << 13; s ^= s >> 7; s ^= s << 17;
+        const float b = __uint_as_float(0x3f800000u | (unsigned)((s >> 23) & 0x7fffffu));
+        float a = __uint_as_float(0x3f800000u | (unsigned)(s & 0x7fffffu));
+        if (i & 1) a = (float)(((double)a + ldexp(1.0, -24)) * (double)b);  // a/b next to a midpoint
+        if (quot(a, b, recip(b)) != __fdiv_rn(a, b)) b2++;
+    }
+    if (b0) atomicAdd(bad, b0);
+    if (b1) atomicAdd(bad + 1, b1);
+    if (b2) atomicAdd(bad + 2, b2);
+}
+extern "C" int check(unsigned long long* out) {
+    unsigned long long* d = nullptr;
+    if (cudaMalloc((void**)&d, 24) != cudaSuccess || cudaMemset(d, 0, 24) != cudaSuccess) return 1;
+    k_check<<<148 * 8, 256>>>(d);
+    const int st = cudaMemcpy(out, d, 24, cudaMemcpyDeviceToHost) != cudaSuccess;
+    cudaFree(d);
+    return st;
+}
+"""
+
+
+def test_recip_root_quot_round_correctly(tmp_path):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    src, so = tmp_path / "check.cu", tmp_path / "check.so"
+    src.write_text(SOURCE)
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "--fmad=false", "-I", CSRC,
+                    "-shared", "-Xcompiler", "-fPIC", str(src), "-o", str(so)], check=True, capture_output=True)
+    out = (C.c_ulonglong * 3)()
+    assert C.CDLL(str(so)).check(out) == 0
+    assert list(out) == [0, 0, 0]
