@@ -259,6 +259,19 @@ __global__ void k_adj_seed(const PState A, int n, const float2* lx_o, const floa
     }
 }
 
+// The gradient of table entry `at` (skf 1 and 4, the adjoint's kernels).
+__device__ __forceinline__ void adj_grad(const Search& Q, int skf, size_t at, float2 xk, float4 o, float& d0, float& d1) {
+    if (skf == 1) {
+        TabGrad<1> g;
+        g.load(Q, at);
+        g.grad(xk, o, false, d0, d1);
+    } else {
+        TabGrad<4> g;
+        g.load(Q, at);
+        g.grad(xk, o, false, d0, d1);
+    }
+}
+
 // Adjoint of av_vel: v''_k = v'_k + eps sum_j c_kj (v'_j - v'_k),
 // c_kj = 2 m_j W_kj / (h_k + h_j), W at the start-of-step geometry.
 __global__ void __launch_bounds__(128) k_adj_xsph(PState A, Search Q, Rheo c, int n, const float2* velfin,
@@ -273,10 +286,12 @@ __global__ void __launch_bounds__(128) k_adj_xsph(PState A, Search Q, Rheo c, in
         double s = 0.0, a0 = 0.0, a1 = 0.0, dm = 0.0, dh = 0.0, dx0 = 0.0, dx1 = 0.0, dhs = 0.0;
         for (int q = 0; q < cnt; q++) {
             // the pair's W and grad W as the replayed step's search stored them
-            const int4 e = Q.nbr[tab_base(k, Q.kcap) + (size_t)q * kTabStride];
-            const int j = e.x & ~kCrossBit;
-            const float w = __int_as_float(e.y), d0 = __int_as_float(e.z), d1 = __int_as_float(e.w);
+            const size_t at = tab_base(k, Q.kcap) + (size_t)q * kTabStride;
+            const int j = Q.nj[at];
+            const float w = Q.nw[at];
             const float4 o = Q.xhm[j];
+            float d0, d1;
+            adj_grad(Q, c.skf, at, xk, o, d0, d1);
             // the pair terms in FP64: their sums over the neighbours cancel
             // strongly (antisymmetric in k, j)
             const float2 vj = velfin[j], lj = lv2[j];
@@ -406,10 +421,12 @@ __global__ void __launch_bounds__(128) k_adj_gather(PState A, Search Q, Rheo c, 
         double dhs = lhsacc ? (double)lhk * (double)mk * (-2.0 * (double)w0 / (double)me.z) : 0.0;
         for (int q = 0; q < cnt; q++) {
             // the pair's W and grad W as the replayed step's search stored them
-            const int4 e = Q.nbr[tab_base(k, Q.kcap) + (size_t)q * kTabStride];
-            const int j = e.x & ~kCrossBit;
-            const float w = __int_as_float(e.y), d0 = __int_as_float(e.z), d1 = __int_as_float(e.w);
+            const size_t at = tab_base(k, Q.kcap) + (size_t)q * kTabStride;
+            const int j = Q.nj[at];
+            const float w = Q.nw[at];
             const float4 o = Q.xhm[j];
+            float d0, d1;
+            adj_grad(Q, c.skf, at, xk, o, d0, d1);
             PairGeom g;
             pair_test(xk, make_float2(o.x, o.y), me.z, o.z, g);
             float ca, cb;

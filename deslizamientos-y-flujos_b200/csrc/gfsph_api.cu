@@ -161,12 +161,11 @@ struct gfsph_handle {
     int* cellA = nullptr;
     float2* velfin = nullptr;
     float* pterm = nullptr;
-    float4* pr = nullptr;    // (pterm, h, m, 0) per slot
     int2* keyrank = nullptr;
     int* perm = nullptr;
     float2* f2tmp = nullptr;
     float4* xhm = nullptr;
-    int4* nbr = nullptr;     // neighbour table: {j, W, dW/dx, dW/dy} per entry
+    int* nbr = nullptr;      // neighbour table: the arrays j, W, gradient (Search) in one allocation
     int* ncount = nullptr;
     int kcap = 0;
     float2* indv = nullptr;  // internal acceleration of every active particle
@@ -310,6 +309,18 @@ void with_lanes(int n, F&& f) {
     else f(std::integral_constant<int, 2>{});
 }
 
+// The same for k_iforce and k_xsph, which wait for their gathers: us a launch
+// (k_iforce / k_xsph) for 850 particles 13 / 10 with one lane, 5 / 5 with 4,
+// 4 / 3 with 8; 23k 16 / 13, 7 / 5, 9 / 7; 200k 33 / 30 with one, 33 / 27 with 2,
+// 41 / 32 with 4; 1M 130 / 107 with one, 150 / 120 with 2.
+template <class F>
+void with_pair_lanes(int n, F&& f) {
+    if (n < 12000) f(std::integral_constant<int, 8>{});
+    else if (n < 100000) f(std::integral_constant<int, 4>{});
+    else if (n < 500000) f(std::integral_constant<int, 2>{});
+    else f(std::integral_constant<int, 1>{});
+}
+
 // Stage-dependent pressure: the step runs the staged RK45 kernels.
 bool staged(const gfsph_handle* h) { return h->rheo.nor_density || h->rheo.cos_theta || h->rheo.ws; }
 
@@ -325,16 +336,21 @@ void join(gfsph_handle* h, int k) {
     cudaStreamWaitEvent(h->stream, h->ev_join[k], 0);
 }
 
+// Particles the neighbour table has room for: whole warps (tab_base).
+size_t tab_rows(const gfsph_handle* h) { return ((size_t)std::max(h->n, 1) + 31) / 32 * 32; }
+
 Search make_search(gfsph_handle* h) {
     Search q;
     q.bstart = h->bstart;
     q.start = h->start;
     q.cellA = h->cellA;
     q.xhm = h->xhm;
-    q.nbr = h->nbr;
+    const size_t ents = (size_t)h->kcap * tab_rows(h);
+    q.nj = h->nbr;
+    q.nw = reinterpret_cast<float*>(h->nbr + ents);
+    q.ng = reinterpret_cast<float*>(h->nbr + 2 * ents);
     q.ncount = h->ncount;
     q.pterm = h->pterm;
-    q.pr = h->pr;
     q.indv = h->indv;
     q.rho0 = h->rho0;
     q.rcell = h->rcell;
@@ -477,7 +493,10 @@ int enqueue_wir_stage(gfsph_handle* h, const PState As[5], int s) {
         pdl_launch(k_wir_nodes, blocks_for((long long)np, 256), 256, st, h->wir_acc, h->d_z, h->wir_hsz, np, S);
     });
     launch(h, K_WIR, [&] {
-        pdl_launch(k_wir_press, blocks_for(n), kThreads, st, h->A, q, S, c, h->dem, h->carry, s, As[s].rho, h->wir_hsz);
+        with_skf(h, [&](auto sk) {
+            pdl_launch(k_wir_press<decltype(sk)::value>, blocks_for(n), kThreads, st, h->A, q, S, c, h->dem, h->carry, s,
+                       As[s].rho, h->wir_hsz);
+        });
     });
     return 3;
 }
@@ -510,10 +529,14 @@ int enqueue_stages(gfsph_handle* h, PState As[5]) {
         nk++;
         launch(h, K_IFORCE, [&] {
             with_skf(h, [&](auto sk) {
-                if (c.ws)
-                    pdl_launch(k_iforce<decltype(sk)::value, true>, pb, kThreads, st, As[s], q, S, c, n);
-                else
-                    pdl_launch(k_iforce<decltype(sk)::value, false>, pb, kThreads, st, As[s], q, S, c, n);
+                with_pair_lanes(n, [&](auto g) {
+                    constexpr int G = decltype(g)::value;
+                    const int fb = blocks_for((long long)n * G);
+                    if (c.ws)
+                        pdl_launch(k_iforce<decltype(sk)::value, true, G>, fb, kThreads, st, As[s], q, S, c, n);
+                    else
+                        pdl_launch(k_iforce<decltype(sk)::value, false, G>, fb, kThreads, st, As[s], q, S, c, n);
+                });
             });
         });
         nk++;
@@ -574,11 +597,13 @@ int enqueue_step(gfsph_handle* h) {
                 });
             });
             launch(h, K_XSPH, [&] {
-                with_skf(h, [&](auto sk) {
+                with_pair_lanes(n, [&](auto g) {
+                    constexpr int G = decltype(g)::value;
+                    const int fb = blocks_for((long long)n * G);
                     if (h->rheo.ws)
-                        pdl_launch(k_xsph<decltype(sk)::value, true>, pb, kThreads, st, As[4], q, S, h->rheo, n, h->B);
+                        pdl_launch(k_xsph<true, G>, fb, kThreads, st, As[4], q, S, h->rheo, n, h->B);
                     else
-                        pdl_launch(k_xsph<decltype(sk)::value, false>, pb, kThreads, st, As[4], q, S, h->rheo, n, h->B);
+                        pdl_launch(k_xsph<false, G>, fb, kThreads, st, As[4], q, S, h->rheo, n, h->B);
                 });
             });
             nk += 2;
@@ -593,7 +618,13 @@ int enqueue_step(gfsph_handle* h) {
     });
     nk++;
     launch(h, K_IFORCE, [&] {
-        with_skf(h, [&](auto sk) { pdl_launch(k_iforce<decltype(sk)::value, false>, pb, kThreads, st, h->A, q, S, h->rheo, n); });
+        with_skf(h, [&](auto sk) {
+            with_pair_lanes(n, [&](auto g) {
+                constexpr int G = decltype(g)::value;
+                pdl_launch(k_iforce<decltype(sk)::value, false, G>, blocks_for((long long)n * G), kThreads, st, h->A, q, S,
+                           h->rheo, n);
+            });
+        });
     });
     nk++;
     join(h, 1);
@@ -614,8 +645,9 @@ int enqueue_step(gfsph_handle* h) {
         });
         nk++;
         launch(h, K_XSPH, [&] {
-            with_skf(h, [&](auto sk) {
-                pdl_launch(k_xsph<decltype(sk)::value, false>, pb, kThreads, st, h->A, q, S, h->rheo, n, h->B);
+            with_pair_lanes(n, [&](auto g) {
+                constexpr int G = decltype(g)::value;
+                pdl_launch(k_xsph<false, G>, blocks_for((long long)n * G), kThreads, st, h->A, q, S, h->rheo, n, h->B);
             });
         });
         nk++;
@@ -691,8 +723,8 @@ int alloc_nbr(gfsph_handle* h, int kcap) {
     drop_graphs(h);
     h->kcap = 0;
     dfree(h->nbr);
-    const size_t rows = ((size_t)std::max(h->n, 1) + 31) / 32 * 32;  // whole warps (tab_base)
-    if (dalloc(&h->nbr, (size_t)kcap * rows)) return GFSPH_ERR_CUDA;
+    const size_t words = (h->rheo.skf == 1) ? 3 : 4;  // j, W and the gradient's factor (skf 1) or its components
+    if (dalloc(&h->nbr, words * (size_t)kcap * tab_rows(h))) return GFSPH_ERR_CUDA;
     h->kcap = kcap;
     return 0;
 }
@@ -711,7 +743,7 @@ void free_particles(gfsph_handle* h) {
     dfree(h->cellA); dfree(h->velfin); dfree(h->pterm); dfree(h->keyrank); dfree(h->perm); dfree(h->ncount);
     dfree(h->nbr); dfree(h->f2tmp); dfree(h->xhm); dfree(h->indv); dfree(h->rho0);
     dfree(h->carry.v); dfree(h->carry.acc); dfree(h->carry.dx); dfree(h->carry.dv); dfree(h->carry.xo);
-    dfree(h->carry.out); dfree(h->carry.u); dfree(h->carry.du); dfree(h->carry.Du); dfree(h->rhoS); dfree(h->rcell); dfree(h->xsv); dfree(h->pr);
+    dfree(h->carry.out); dfree(h->carry.u); dfree(h->carry.du); dfree(h->carry.Du); dfree(h->rhoS); dfree(h->rcell); dfree(h->xsv);
     dfree(h->spec_u); dfree(h->spec_a); dfree(h->zpw); dfree(h->gzw); dfree(h->bxy);
     dfree(h->mass0_u);
     h->kcap = 0;
@@ -1209,7 +1241,7 @@ int gfsph_upload(gfsph_handle* h, int n, const float* x, const float* v, const f
         st |= dalloc(&h->cellA, n); st |= dalloc(&h->velfin, n); st |= dalloc(&h->pterm, n);
         st |= dalloc(&h->keyrank, n); st |= dalloc(&h->perm, n); st |= dalloc(&h->ncount, n);
         st |= dalloc(&h->f2tmp, n); st |= dalloc(&h->xhm, (size_t)n + kScanStep); st |= dalloc(&h->indv, n); st |= dalloc(&h->rho0, n);
-        st |= dalloc(&h->xsv, n); st |= dalloc(&h->pr, n);
+        st |= dalloc(&h->xsv, n);
         if (staged(h)) {
             StageCarry& C = h->carry;
             st |= dalloc(&C.v, n); st |= dalloc(&C.acc, n); st |= dalloc(&C.dx, n); st |= dalloc(&C.dv, n);
@@ -1484,7 +1516,12 @@ int gfsph_internal_forces(gfsph_handle* h, float* indvxdt) try {
         As[0] = h->A;
     }
     launch(h, K_IFORCE, [&] {
-        with_skf(h, [&](auto sk) { k_iforce<decltype(sk)::value, false><<<blocks_for(n), kThreads, 0, s>>>(As[0], q, h->S, h->rheo, n); });
+        with_skf(h, [&](auto sk) {
+            if (h->rheo.ws)
+                k_iforce<decltype(sk)::value, true, 1><<<blocks_for(n), kThreads, 0, s>>>(As[0], q, h->S, h->rheo, n);
+            else
+                k_iforce<decltype(sk)::value, false, 1><<<blocks_for(n), kThreads, 0, s>>>(As[0], q, h->S, h->rheo, n);
+        });
     });
     launch(h, K_FORCE_BIG, [&] {
         with_skf(h, [&](auto sk) { k_force_big<decltype(sk)::value><<<big_blocks(h), kBigThreads, 0, s>>>(As[0], q, h->S, h->rheo); });
@@ -1510,15 +1547,15 @@ int gfsph_neighbours(gfsph_handle* h, int cap, int* offsets, int* idx) try {
     if (st) return st;
     int nreg = h->hS->nreg, nbig = h->hS->nbig;
     std::vector<int> cnt(n), id(n);
-    std::vector<int4> tab((size_t)h->kcap * (((size_t)n + 31) / 32 * 32));
+    std::vector<int> tab((size_t)h->kcap * tab_rows(h));
     CK(cudaMemcpy(cnt.data(), h->ncount, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(id.data(), h->A.id, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(tab.data(), h->nbr, tab.size() * sizeof(int4), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(tab.data(), h->nbr, tab.size() * sizeof(int), cudaMemcpyDeviceToHost));
     std::vector<std::vector<int>> lists(n);
     for (int s = 0; s < nreg; s++) {
         auto& L = lists[id[s]];
         for (int k = 0; k < cnt[s] && k < h->kcap; k++)
-            L.push_back(id[tab[tab_base(s, h->kcap) + (size_t)k * kTabStride].x & ~kCrossBit]);
+            L.push_back(id[tab[tab_base(s, h->kcap) + (size_t)k * kTabStride] & ~kCrossBit]);
     }
     if (nbig > 0) {  // pairs of the big particles, found on the device
         int pcap = 1 << 20;

@@ -114,33 +114,63 @@ __device__ __forceinline__ void sph_kernel(float r, float dx0, float dx1, float 
     }
 }
 
-// The cubic spline (skf 1) of a pair again, from the square of its distance,
-// for smoothing lengths within kQuotMin .. kQuotMax and r < 2 hs: the same
-// values bit for bit, both branches of q in one instruction stream (the lanes
-// of a warp mix them) and the square root and up to six IEEE divisions of a
-// pair as three reciprocals, a root and quot().  r is kept off 0 (coincident
-// particles), where it does not reach a bit of the result.
-__device__ __forceinline__ void sph_kernel_spline(float dr, float dx0, float dx1, float hs, float& w, float& d0,
-                                                  float& d1) {
-    const float r = root(fmaxf(dr, 1.e-36f));
-    const float yh = recip(hs);
-    const float q = quot(r, hs, yh);
-    const float fd = ((7.f * kPi) * hs) * hs;
-    const float factor = quot(15.f, fd, recip(fd));
-    const float f6 = quot(factor, 6.f, 1.f / 6.f);
-    const bool inner = q <= 1.f;
-    const float u = 2.f - q, u2 = u * u;
-    // W
-    const float wi = factor * ((kTwoThirds - q * q) + ((q * q) * q) / 2.f);
-    const float wo = f6 * (u2 * u);
-    // gradient: inner (factor (-2 + 1.5 q)/(hs hs)) dx; outer -(3 f6 u^2/hs) (dx/r)
-    const float h2 = hs * hs;
-    const float yd = recip(inner ? h2 : r);
-    const float num = inner ? factor * (-2.f + 1.5f * q) : -((f6 * 3.f) * u2);
-    const float t = quot(num, inner ? h2 : hs, inner ? yd : yh);
-    w = inner ? wi : wo;
-    d0 = t * (inner ? dx0 : quot(dx0, r, yd));
-    d1 = t * (inner ? dx1 : quot(dx1, r, yd));
+// The cubic spline (skf 1) of a pair as the neighbour table keeps it: W and
+// one factor t of its gradient, grad W = t dx where t < 0 (q <= 1) and
+// -t (dx/r) where t >= 0, the operations of sph_kernel<1> split where dx comes
+// in.  safe: smoothing lengths within kQuotMin .. kQuotMax; then both branches
+// of q run in one instruction stream (the lanes of a warp mix them) and the
+// square root and divisions are two reciprocals, a root, a further reciprocal
+// and quot(), the same values bit for bit.  r is kept off 0 there (coincident
+// particles), where it does not reach a bit of the result.  dr = r^2, r < 2 hs.
+__device__ __forceinline__ void spline_pair(float dr, float hs, bool safe, float& w, float& t) {
+    if (safe) {
+        const float r = root(fmaxf(dr, 1.e-36f));
+        const float yh = recip(hs);
+        const float q = quot(r, hs, yh);
+        const float fd = ((7.f * kPi) * hs) * hs;
+        const float factor = quot(15.f, fd, recip(fd));
+        const float f6 = quot(factor, 6.f, 1.f / 6.f);
+        const bool inner = q <= 1.f;
+        const float u = 2.f - q, u2 = u * u, h2 = hs * hs;
+        const float wi = factor * ((kTwoThirds - q * q) + ((q * q) * q) / 2.f);
+        const float wo = f6 * (u2 * u);
+        const float ti = factor * (-2.f + 1.5f * q), to = (f6 * 3.f) * u2;
+        const float yd = recip(h2);
+        w = inner ? wi : wo;
+        t = quot(inner ? ti : to, inner ? h2 : hs, inner ? yd : yh);
+        return;
+    }
+    const float q = sqrtf(dr) / hs;
+    const float factor = 15.f / (((7.f * kPi) * hs) * hs);
+    w = 0.f;
+    t = 0.f;
+    if (q <= 1.f) {
+        w = factor * ((kTwoThirds - q * q) + ((q * q) * q) / 2.f);
+        t = (factor * (-2.f + 1.5f * q)) / (hs * hs);
+    } else if (q <= 2.f) {
+        const float u = 2.f - q;
+        w = ((factor * 1.f) / 6.f) * ((u * u) * u);
+        t = ((((factor * 1.f) / 6.f) * 3.f) * (u * u)) / hs;
+    }
+}
+// grad W from t and the separation dx.
+__device__ __forceinline__ void spline_grad(float t, float dx0, float dx1, bool safe, float& d0, float& d1) {
+    float dr = dx0 * dx0;
+    dr = dr + dx1 * dx1;
+    const bool inner = __float_as_int(t) < 0;
+    if (safe) {
+        const float r = root(fmaxf(dr, 1.e-36f)), y = recip(r);
+        const float ts = inner ? t : -t;
+        d0 = ts * (inner ? dx0 : quot(dx0, r, y));
+        d1 = ts * (inner ? dx1 : quot(dx1, r, y));
+    } else if (inner) {
+        d0 = t * dx0;
+        d1 = t * dx1;
+    } else {
+        const float r = sqrtf(dr);
+        d0 = -(t * (dx0 / r));
+        d1 = -(t * (dx1 / r));
+    }
 }
 
 template <int SKF>

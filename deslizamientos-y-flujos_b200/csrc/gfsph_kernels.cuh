@@ -107,12 +107,18 @@ struct Search {
     const int* start;    // cell key -> first particle slot (exclusive scan), ncells+1
     const int* cellA;    // slot -> cell key (all levels), -1 out of the domain
     const float4* xhm;   // slot -> (x, y, hsml, mass) at the start of the step
-    int4* nbr;           // neighbour table of the regular particles (layout: tab_base); entry
-                         // {j, W_ij, dW_ij/dx, dW_ij/dy} (the FP32 bits of the kernel values,
-                         // computed once per pair by the search, as grid_find stores w and dwdx)
+    // neighbour table of the regular particles (layout: tab_base): per entry
+    // j, W_ij and its gradient, computed once per pair by the search, as
+    // grid_find stores w and dwdx.  Three arrays, since the internal force
+    // reads j and the gradient, av_vel and the normalisation j and W.  With
+    // skf 1 the gradient is spline_pair's one factor (the internal force, which
+    // waits for the table, has the arithmetic for the rest to spare); else a
+    // float2.
+    int* nj;
+    float* nw;
+    float* ng;
     int* ncount;
     float* pterm;        // p/h^2 (pa_sph 2) or p (pa_sph 1)
-    float4* pr;          // (pterm, h, m, 0): what the internal force gathers per neighbour
     float2* indv;        // internal acceleration of every active particle (slot order)
     float* rho0;         // depth at the start of the step, after Adaptive_dt's h_inf clamp (icpwp = 3)
     const int2* rcell;   // slot -> cell of the reference's own grid (skf 2, 3), else null
@@ -166,13 +172,49 @@ __device__ __forceinline__ void scalars_from_smem(StepScalars* S, const StepScal
 
 // Neighbour-table layout, blocked by warps of 32 particles: entry k of
 // particle i is at tab_base(i, kcap) + 32 k.  The lanes of a warp read entry k
-// of their particles as one 512-byte run (16-byte entries), and the entries a
+// of their particles as one 128-byte run, and the entries a
 // warp appends while its lanes are at different k stay within its own
 // 32 kcap entries.
 __host__ __device__ __forceinline__ size_t tab_base(int i, int kcap) {
     return (size_t)(i >> 5) * ((size_t)kcap << 5) + (size_t)(i & 31);
 }
 constexpr int kTabStride = 32;
+
+// Asks for the first rows entries of one table array of a warp's particles
+// (contiguous, tab_base) into L2, one instruction of one lane; at: the
+// warp's first entry.
+__device__ __forceinline__ void prefetch_rows(const void* at, int rows) {
+    if (rows > 0)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(at), "r"(rows * kTabStride * 4) : "memory");
+}
+
+// Whether every pair of a particle with smoothing length hi, in a step whose
+// largest is hmax, has a mean within kQuotMin .. kQuotMax.
+__device__ __forceinline__ bool quot_safe(float hi, float hmax) { return hi >= 2.f * kQuotMin && hmax <= kQuotMax; }
+
+// The gradient of table entry `at` of particle i (at xi) with neighbour j (at
+// xj): load, then grad.
+template <int SKF>
+struct TabGrad {
+    float g0, g1;
+    __device__ __forceinline__ void load(const Search& Q, size_t at) {
+        if (SKF == 1) {
+            g0 = __ldg(Q.ng + at);
+        } else {
+            const float2 g = __ldg(reinterpret_cast<const float2*>(Q.ng) + at);
+            g0 = g.x;
+            g1 = g.y;
+        }
+    }
+    __device__ __forceinline__ void grad(float2 xi, float4 xj, bool safe, float& d0, float& d1) const {
+        if (SKF == 1) {
+            spline_grad(g0, xi.x - xj.x, xi.y - xj.y, safe, d0, d1);
+        } else {
+            d0 = g0;
+            d1 = g1;
+        }
+    }
+};
 
 // ---------------------------------------------------------------- prologue
 // Decides whether the coming step runs and resets its reductions; run at the
@@ -888,8 +930,8 @@ __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, S
         const float hi = me.z;
         const int2 ci = (SK == 2) ? make_int2(0, 0) : Q.rcell[act ? i : base];
         const unsigned char si = WS ? Q.spec[act ? i : base] : 0;
-        const bool safe = SKF == 1 && hi >= 2.f * kQuotMin && hmax <= kQuotMax;
-        int4* tab = Q.nbr + tab_base(act ? i : base, Q.kcap);
+        const bool safe = quot_safe(hi, hmax);
+        const size_t tab = tab_base(act ? i : base, Q.kcap);
         float bx0 = 0.f, bx1 = 0.f, by0 = 0.f, by1 = 0.f, bh = 0.f;  // the block's box and largest hsml
         if (scan_big) {
             bx0 = warp_min(me.x); bx1 = warp_max(me.x);
@@ -992,12 +1034,16 @@ __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, S
                 const float dr = dx0 * dx0 + dx1 * dx1;
                 const float mh = (hi + o.z) / 2.f;
                 float w, d0, d1;
-                if (safe) sph_kernel_spline(dr, dx0, dx1, mh, w, d0, d1);
+                if (SKF == 1) spline_pair(dr, mh, safe, w, d0);
                 else sph_kernel<SKF>(sqrtf(dr), dx0, dx1, mh, w, d0, d1);
                 const bool cross = WS && Q.spec[j] != si;
-                if (found + t < Q.kcap)  // kept in L2 for the internal force (written back to front)
-                    tab[(size_t)(found + t) * kTabStride] = make_int4(cross ? (j | kCrossBit) : j, __float_as_int(w),
-                                                                      __float_as_int(d0), __float_as_int(d1));
+                if (found + t < Q.kcap) {
+                    const size_t to = tab + (size_t)(found + t) * kTabStride;
+                    Q.nj[to] = cross ? (j | kCrossBit) : j;
+                    Q.nw[to] = w;
+                    if (SKF == 1) Q.ng[to] = d0;
+                    else reinterpret_cast<float2*>(Q.ng)[to] = make_float2(d0, d1);
+                }
                 if (!cross) acc += (double)(o.w * w);
             };
             int t = gl;
@@ -1030,7 +1076,6 @@ __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, S
             const float p = (c.cgra05 * hc) * hc;
             const float pt = (c.pa_sph == 1) ? p : p / (hc * hc);
             Q.pterm[i] = pt;
-            Q.pr[i] = make_float4(pt, h, me.w, 0.f);
         }
         if (scan_big) __syncthreads();  // the box is rewritten
     }
@@ -1113,7 +1158,6 @@ __global__ void __launch_bounds__(kBigThreads) k_density_big(PState A, Search Q,
             float p = (c.cgra05 * hc) * hc;
             const float pt = (c.pa_sph == 1) ? p : p / (hc * hc);
             Q.pterm[i] = pt;
-            Q.pr[i] = make_float4(pt, h, me.w, 0.f);
         }
     }
 }
@@ -1155,13 +1199,12 @@ __global__ void __launch_bounds__(kBigThreads) k_force_big(PState A, Search Q, S
     const int nreg = S->nreg, nbig = S->nbig;
     for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
         int i = nreg + b;
-        const float4 pri = Q.pr[i];
+        const float pi_ = Q.pterm[i], rhoi = A.rho[i];
         double a0 = 0.0, a1 = 0.0;
         const unsigned char si = c.ws ? Q.spec[i] : 0;
         block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
             if (c.ws && Q.spec[j] != si) return;  // type 0 only (:6899)
-            const float4 prj = Q.pr[j];
-            pressure_pair<SKF>(c, pri.x, pri.y, prj.x, prj.y, o.w, g, a0, a1);
+            pressure_pair<SKF>(c, pi_, rhoi, Q.pterm[j], A.rho[j], o.w, g, a0, a1);
         });
         a0 = block_sum(a0);
         a1 = block_sum(a1);
@@ -1169,37 +1212,67 @@ __global__ void __launch_bounds__(kBigThreads) k_force_big(PState A, Search Q, S
     }
 }
 
-// Internal acceleration of a regular particle over its neighbour table: per
-// entry the stored kernel gradient and one gather of (p-term, h, m) of the
-// neighbour.  The table is read four entries at a time so that four
-// independent gathers are in flight per thread; the FP64 sum keeps the table
-// order.
-template <bool WS>
-__device__ __forceinline__ void internal_force(const Search& Q, const Rheo& c, int i, float& in0, float& in1) {
-    const float4 pri = __ldg(&Q.pr[i]);
-    const float pi_ = pri.x, rhoi = pri.y;
+// Internal acceleration of a regular particle over its neighbour table, by G
+// lanes: lane gl takes every G-th entry.  Per entry the stored gradient and
+// the gathers of (x, m) and the pressure term of the neighbour (its depth too
+// with pa_sph 1).  The table is read four entries at a time so that the
+// gathers of four pairs are in flight per thread.  The sums over the lanes are
+// valid in all of them.
+template <int SKF, bool WS, int G>
+__device__ __forceinline__ void internal_force(const Search& Q, const Rheo& c, const float* rho, float hmax, int i,
+                                               int gl, float& in0, float& in1) {
+    const float4 me = __ldg(&Q.xhm[i]);
+    const float2 xi = make_float2(me.x, me.y);
+    const bool safe = quot_safe(me.z, hmax);
+    const float pi_ = __ldg(&Q.pterm[i]), rhoi = rho[i];
     double a0 = 0.0, a1 = 0.0;
     const int cnt = Q.ncount[i];
-    const int4* tab = Q.nbr + tab_base(i, Q.kcap);
-    int k = 0;
-    for (; k + 4 <= cnt; k += 4) {
-        int4 e[4];
-        float4 prj[4];
+    const size_t tab = tab_base(i, Q.kcap);
+    auto term = [&](int j, const TabGrad<SKF>& g, const float4& o, float pj) {
+        float d0, d1;
+        g.grad(xi, o, safe, d0, d1);
+        pressure_terms(c, pi_, rhoi, pj, c.pa_sph == 1 ? rho[j] : 0.f, o.w, d0, d1, a0, a1);
+    };
+    // four entries at a time, the next four on their way meanwhile
+    int k = gl;
+    int e[4];
+    TabGrad<SKF> g[4];
+    auto fetch = [&](int k0) {
 #pragma unroll
-        for (int u = 0; u < 4; u++) e[u] = __ldg(tab + (size_t)(k + u) * kTabStride);
+        for (int u = 0; u < 4; u++) {
+            e[u] = __ldg(Q.nj + tab + (size_t)(k0 + u * G) * kTabStride);
+            g[u].load(Q, tab + (size_t)(k0 + u * G) * kTabStride);
+        }
+    };
+    if (k + 3 * G < cnt) fetch(k);
+    for (; k + 3 * G < cnt; k += 4 * G) {
+        int je[4];
+        TabGrad<SKF> gg[4];
+        float4 o[4];
+        float pj[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) prj[u] = __ldg(&Q.pr[WS ? (e[u].x & ~kCrossBit) : e[u].x]);
+        for (int u = 0; u < 4; u++) {
+            je[u] = e[u];
+            gg[u] = g[u];
+            const int j = WS ? (e[u] & ~kCrossBit) : e[u];
+            o[u] = __ldg(&Q.xhm[j]);
+            pj[u] = __ldg(&Q.pterm[j]);
+        }
+        if (k + 7 * G < cnt) fetch(k + 4 * G);
 #pragma unroll
         for (int u = 0; u < 4; u++)
-            if (!WS || e[u].x >= 0)  // type 0 only (:6899)
-                pressure_terms(c, pi_, rhoi, prj[u].x, prj[u].y, prj[u].z, __int_as_float(e[u].z),
-                               __int_as_float(e[u].w), a0, a1);
+            if (!WS || je[u] >= 0) term(je[u], gg[u], o[u], pj[u]);  // type 0 only (:6899)
     }
-    for (; k < cnt; k++) {
-        const int4 e = __ldg(tab + (size_t)k * kTabStride);
-        const float4 prj = __ldg(&Q.pr[WS ? (e.x & ~kCrossBit) : e.x]);
-        if (!WS || e.x >= 0)
-            pressure_terms(c, pi_, rhoi, prj.x, prj.y, prj.z, __int_as_float(e.z), __int_as_float(e.w), a0, a1);
+    for (; k < cnt; k += G) {
+        const int e = __ldg(Q.nj + tab + (size_t)k * kTabStride);
+        TabGrad<SKF> g;
+        g.load(Q, tab + (size_t)k * kTabStride);
+        if (!WS || e >= 0) term(e, g, __ldg(&Q.xhm[e]), __ldg(&Q.pterm[e]));
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
     }
     in0 = (float)a0;
     in1 = (float)a1;
@@ -1369,24 +1442,31 @@ __device__ __forceinline__ void rk_finish(const PState& A, const Search& Q, Step
     }
 }
 
-// Internal acceleration of the regular particles, one thread each.  The
-// warps take the particles from the last to the first warp of the table:
-// the neighbour search has just written the table front to back, so its
-// last-written part (still in L2) is read first, and av_vel, which walks
-// the table front to back after this pass, starts on the part this pass
-// read last.
-template <int SKF, bool WS>
+// Internal acceleration of the regular particles, G lanes each.  The
+// warps take the particles from the last to the first: the neighbour search
+// has just written the table front to back, so its last-written part (still
+// in L2) is read first, and av_vel, which walks the table front to back after
+// this pass, starts on the part this pass read last.
+template <int SKF, bool WS, int G>
 __global__ void __launch_bounds__(128) k_iforce(PState A, Search Q, StepScalars* S, Rheo c, int n) {
     PDL_ENTRY();
     if (S->skip) return;
+    constexpr int P = 32 / G;  // particles per warp
     const int nreg = S->nreg;
-    const int nw = (nreg + 31) >> 5;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nw * 32; t += gridDim.x * blockDim.x) {
-        const int i = (nw - 1 - (t >> 5)) * 32 + (t & 31);
-        if (i >= nreg) continue;
+    const float hmax = o2f(S->hmax_o);
+    const int nw = (nreg + P - 1) / P;
+    const int lane = threadIdx.x & 31;
+    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nw; w += (gridDim.x * blockDim.x) >> 5) {
+        const int i = (nw - 1 - w) * P + lane / G;
+        if (G == 1) {
+            const int rows = __reduce_max_sync(0xffffffffu, Q.ncount[min(i, nreg - 1)]);
+            const size_t at = tab_base(i - lane, Q.kcap);
+            if (lane == 0 && rows <= Q.kcap) prefetch_rows(Q.nj + at, rows);
+            if (lane == 1 && rows <= Q.kcap) prefetch_rows(Q.ng + (SKF == 1 ? at : 2 * at), SKF == 1 ? rows : 2 * rows);
+        }
         float in0, in1;
-        internal_force<WS>(Q, c, i, in0, in1);
-        Q.indv[i] = make_float2(in0, in1);
+        internal_force<SKF, WS, G>(Q, c, A.rho, hmax, min(i, nreg - 1), lane % G, in0, in1);
+        if (i < nreg && lane % G == 0) Q.indv[i] = make_float2(in0, in1);
     }
 }
 
@@ -1562,11 +1642,10 @@ __global__ void __launch_bounds__(128) k_norm(PState A, Search Q, StepScalars* S
         const float hi = me.z;
         double den = (double)((sph_kernel_w<SKF>(0.f, hi) * me.w) / prev_depth(c, hp, i, clamp_prev));
         const int cnt = Q.ncount[i];
-        const int4* tab = Q.nbr + tab_base(i, Q.kcap);
+        const size_t tab = tab_base(i, Q.kcap);
         for (int k = 0; k < cnt; k++) {
-            const int4 e = __ldg(tab + (size_t)k * kTabStride);  // read again by the next calls of the step
-            const int j = e.x;
-            den += (double)((__ldg(&A.mass[j]) / prev_depth(c, hp, j, clamp_prev)) * __int_as_float(e.y));
+            const int j = __ldg(Q.nj + tab + (size_t)k * kTabStride);  // read again by the next calls of the step
+            den += (double)((__ldg(&A.mass[j]) / prev_depth(c, hp, j, clamp_prev)) * __ldg(Q.nw + tab + (size_t)k * kTabStride));
         }
         hout[i] = A.rho[i] / (float)den;
     }
@@ -1620,9 +1699,7 @@ __global__ void __launch_bounds__(128) k_stage_begin(PState A, Search Q, StepSca
     const int nact = S->nactive;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nact; i += gridDim.x * blockDim.x) {
         const float2 p = A.pos[i];
-        const float pt = stage_pterm<COS>(c, dem, h1[i], p.x, p.y);
-        Q.pterm[i] = pt;
-        Q.pr[i] = make_float4(pt, h1[i], A.mass[i], 0.f);
+        Q.pterm[i] = stage_pterm<COS>(c, dem, h1[i], p.x, p.y);
     }
 }
 
@@ -1702,6 +1779,7 @@ __device__ __forceinline__ void wir_pair_term(const Rheo& c, bool water, float m
 // stage (IntForces_SW :6793-6828): g/2 (h^2 - Zp^2) for the water with
 // ic_SWalg = 1, g/2 h^2 otherwise, h clamped to h_inf.  In stage 0 also the
 // soil-water pair sum of every regular particle, from its table.
+template <int SKF>
 __global__ void __launch_bounds__(128) k_wir_press(PState A, Search Q, StepScalars* S, Rheo c, DemView dem,
                                                    StageCarry C, int s, const float* hdep, const float* hsz) {
     PDL_ENTRY();
@@ -1713,19 +1791,23 @@ __global__ void __launch_bounds__(128) k_wir_press(PState A, Search Q, StepScala
         if (s == 0 && i < nreg) {
             double b0 = 0.0, b1 = 0.0;
             const int cnt = Q.ncount[i];
-            const int4* tab = Q.nbr + tab_base(i, Q.kcap);
+            const size_t tab = tab_base(i, Q.kcap);
+            const float4 me = Q.xhm[i];
+            const bool safe = quot_safe(me.z, o2f(S->hmax_o));
             for (int k = 0; k < cnt; k++) {
-                const int4 e = tab[(size_t)k * kTabStride];
-                if (e.x >= 0) continue;
-                wir_pair_term(c, water, Q.xhm[e.x & ~kCrossBit].w, __int_as_float(e.z), __int_as_float(e.w), b0, b1);
+                const int e = Q.nj[tab + (size_t)k * kTabStride];
+                if (e >= 0) continue;
+                const float4 o = Q.xhm[e & ~kCrossBit];
+                TabGrad<SKF> g;
+                g.load(Q, tab + (size_t)k * kTabStride);
+                float d0, d1;
+                g.grad(make_float2(me.x, me.y), o, safe, d0, d1);
+                wir_pair_term(c, water, o.w, d0, d1, b0, b1);
             }
             Q.bxy[i] = make_float2((float)b0, (float)b1);
         }
         float2 p;
-        if (!wir_stage_pos(A, C, s, dt, i, p) || out_of_box(dem, p.x, p.y)) {  // keeps its term
-            Q.pr[i] = make_float4(Q.pterm[i], hdep[i], A.mass[i], 0.f);
-            continue;
-        }
+        if (!wir_stage_pos(A, C, s, dt, i, p) || out_of_box(dem, p.x, p.y)) continue;  // keeps its term
         float zp = 0.f;
         if (water) {
             int ipx = (int)((p.x - dem.xmin) / dem.dx + 1.f), ipy = (int)((p.y - dem.ymin) / dem.dy + 1.f);
@@ -1746,9 +1828,7 @@ __global__ void __launch_bounds__(128) k_wir_press(PState A, Search Q, StepScala
         const float h = hdep[i];
         const float hc = (h < c.h_inf) ? c.h_inf : h;
         const float p_ = (water && c.swalg == 1) ? c.cgra05 * (hc * hc - zp * zp) : (c.cgra05 * hc) * hc;
-        const float pt = (c.pa_sph == 1) ? p_ : p_ / (hc * hc);
-        Q.pterm[i] = pt;
-        Q.pr[i] = make_float4(pt, h, A.mass[i], 0.f);
+        Q.pterm[i] = (c.pa_sph == 1) ? p_ : p_ / (hc * hc);
     }
 }
 
@@ -1793,10 +1873,7 @@ __global__ void __launch_bounds__(128) k_stage(PState A, Search Q, StepScalars* 
     const float f1 = (s == 0) ? 0.f : 0.5f, f2 = (s == 0) ? 1.f : 2.f;
     const float f1n = (s == 2) ? 1.f : 0.5f;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nact; i += gridDim.x * blockDim.x) {
-        if (s > 0 && C.out[i]) {  // frozen: its pressure term stays, its depth is the next call's
-            Q.pr[i] = make_float4(Q.pterm[i], hnext[i], A.mass[i], 0.f);
-            continue;
-        }
+        if (s > 0 && C.out[i]) continue;  // frozen: its pressure term stays
         const float2 x0 = A.pos[i], v0 = A.vel[i];
         float2 vp = v0, ap = make_float2(0.f, 0.f), dx = make_float2(0.f, 0.f), dv = make_float2(0.f, 0.f);
         if (s > 0) { vp = C.v[i]; ap = C.acc[i]; dx = C.dx[i]; dv = C.dv[i]; }
@@ -1808,7 +1885,6 @@ __global__ void __launch_bounds__(128) k_stage(PState A, Search Q, StepScalars* 
             C.out[i] = 1;
             C.xo[i] = make_float2(xx, xy);
             C.v[i] = make_float2(vx, vy);
-            Q.pr[i] = make_float4(Q.pterm[i], hnext[i], A.mass[i], 0.f);
             continue;
         }
         if (s == 0) C.out[i] = 0;
@@ -1835,12 +1911,7 @@ __global__ void __launch_bounds__(128) k_stage(PState A, Search Q, StepScalars* 
         if (c.ws) continue;  // the next stage's pressure needs its soil surface: k_wir_press
         const float fdn = f1n * dt;
         const float nx_ = x0.x + fdn * vx, ny_ = x0.y + fdn * vy;
-        float pt = Q.pterm[i];
-        if (!out_of_box(dem, nx_, ny_)) {
-            pt = stage_pterm<COS>(c, dem, hnext[i], nx_, ny_);
-            Q.pterm[i] = pt;
-        }
-        Q.pr[i] = make_float4(pt, hnext[i], A.mass[i], 0.f);
+        if (!out_of_box(dem, nx_, ny_)) Q.pterm[i] = stage_pterm<COS>(c, dem, hnext[i], nx_, ny_);
     }
 }
 
@@ -1916,14 +1987,23 @@ __global__ void __launch_bounds__(128) k_stage_final(PState A, Search Q, StepSca
 }
 
 // One pair term of av_vel (SPH_MAIN_2019.f90:3072-3080) for particle i with
-// the pair's kernel value w.
+// the pair's kernel value w.  The two quotients share a reciprocal (quot) while
+// the depths are within 1e-18 .. 1e18.
 __device__ __forceinline__ void xsph_terms(float2 vi, float rhoi, float2 vj, float rhoj, float mj, float w, double& a0,
                                            double& a1) {
-    float den = rhoi + rhoj;
-    float t0 = (((2.f * mj) * (vi.x - vj.x)) / den) * w;
-    float t1 = (((2.f * mj) * (vi.y - vj.y)) / den) * w;
-    a0 -= (double)t0;
-    a1 -= (double)t1;
+    const float den = rhoi + rhoj;
+    const float n0 = (2.f * mj) * (vi.x - vj.x), n1 = (2.f * mj) * (vi.y - vj.y);
+    float q0, q1;
+    if (den > 1.e-18f && den < 1.e18f) {
+        const float y = recip(den);
+        q0 = quot(n0, den, y);
+        q1 = quot(n1, den, y);
+    } else {
+        q0 = n0 / den;
+        q1 = n1 / den;
+    }
+    a0 -= (double)(q0 * w);
+    a1 -= (double)(q1 * w);
 }
 
 // The same with the pair geometry: the kernel value evaluated here.
@@ -1934,41 +2014,71 @@ __device__ __forceinline__ void xsph_pair(float2 vi, float rhoi, float2 vj, floa
 }
 
 // av_vel (SPH_MAIN_2019.f90:3042-3099) with the start-of-step W_ij, then
-// v += 0.3*av for particles still inside the domain (:987-993).
-template <int SKF, bool WS>
+// v += 0.3*av for particles still inside the domain (:987-993); G lanes per
+// particle as in k_iforce.
+template <bool WS, int G>
 __global__ void __launch_bounds__(128) k_xsph(PState A, Search Q, StepScalars* S, Rheo c, int n, PState B) {
     PDL_ENTRY();
     if (S->skip || !c.av_vel) return;
+    constexpr int P = 32 / G;  // particles per warp
     const int nreg = S->nreg;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nreg; i += gridDim.x * blockDim.x) {
-        if (B.flag[i]) continue;
+    const int lane = threadIdx.x & 31, gl = lane % G;
+    const int nw = (nreg + P - 1) / P;
+    for (int wp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; wp < nw; wp += (gridDim.x * blockDim.x) >> 5) {
+        const int i0 = wp * P + lane / G, i = min(i0, nreg - 1);
         const float4 si = Q.xsv[i];
         const float2 vi = make_float2(si.x, si.y);
         const float rhoi = si.z;
-        const int cnt = Q.ncount[i];
-        const int4* tab = Q.nbr + tab_base(i, Q.kcap);
+        const bool go = i0 < nreg && !B.flag[i];
+        const int cnt = go ? Q.ncount[i] : 0;
+        const size_t tab = tab_base(i, Q.kcap);
+        if (G == 1) {
+            const int rows = __reduce_max_sync(0xffffffffu, cnt);
+            const size_t at = tab_base(i0 - lane, Q.kcap);
+            if (lane == 0) prefetch_rows(Q.nj + at, rows);
+            if (lane == 1) prefetch_rows(Q.nw + at, rows);
+        }
         double a0 = 0.0, a1 = 0.0;
-        int k = 0;
-        for (; k + 4 <= cnt; k += 4) {
-            int4 e[4];
+        int k = gl;
+        int e[4];
+        float w[4];
+        auto fetch = [&](int k0) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                e[u] = __ldcs(Q.nj + tab + (size_t)(k0 + u * G) * kTabStride);
+                w[u] = __ldcs(Q.nw + tab + (size_t)(k0 + u * G) * kTabStride);
+            }
+        };
+        if (k + 3 * G < cnt) fetch(k);
+        for (; k + 3 * G < cnt; k += 4 * G) {
+            int je[4];
+            float ww[4];
             float4 sj[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) e[u] = __ldcs(tab + (size_t)(k + u) * kTabStride);
-#pragma unroll
-            for (int u = 0; u < 4; u++) sj[u] = Q.xsv[WS ? (e[u].x & ~kCrossBit) : e[u].x];
+            for (int u = 0; u < 4; u++) {
+                je[u] = e[u];
+                ww[u] = w[u];
+                sj[u] = Q.xsv[WS ? (e[u] & ~kCrossBit) : e[u]];
+            }
+            if (k + 7 * G < cnt) fetch(k + 4 * G);
 #pragma unroll
             for (int u = 0; u < 4; u++)
-                if (!WS || e[u].x >= 0)  // type 0 only (SPH_MAIN_2019.f90:3071)
-                    xsph_terms(vi, rhoi, make_float2(sj[u].x, sj[u].y), sj[u].z, sj[u].w, __int_as_float(e[u].y), a0,
-                               a1);
+                if (!WS || je[u] >= 0)  // type 0 only (SPH_MAIN_2019.f90:3071)
+                    xsph_terms(vi, rhoi, make_float2(sj[u].x, sj[u].y), sj[u].z, sj[u].w, ww[u], a0, a1);
         }
-        for (; k < cnt; k++) {
-            const int4 e = __ldcs(tab + (size_t)k * kTabStride);
-            const float4 sj = Q.xsv[WS ? (e.x & ~kCrossBit) : e.x];
-            if (!WS || e.x >= 0) xsph_terms(vi, rhoi, make_float2(sj.x, sj.y), sj.z, sj.w, __int_as_float(e.y), a0, a1);
+        for (; k < cnt; k += G) {
+            const int e = __ldcs(Q.nj + tab + (size_t)k * kTabStride);
+            const float w = __ldcs(Q.nw + tab + (size_t)k * kTabStride);
+            const float4 sj = Q.xsv[WS ? (e & ~kCrossBit) : e];
+            if (!WS || e >= 0) xsph_terms(vi, rhoi, make_float2(sj.x, sj.y), sj.z, sj.w, w, a0, a1);
         }
-        float av0 = 0.3f * (float)a0, av1 = 0.3f * (float)a1;
-        B.vel[i] = make_float2(vi.x + av0, vi.y + av1);
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) {
+            a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+            a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+        }
+        const float av0 = 0.3f * (float)a0, av1 = 0.3f * (float)a1;
+        if (go && gl == 0) B.vel[i] = make_float2(vi.x + av0, vi.y + av1);
     }
 }
 
