@@ -239,23 +239,20 @@ __device__ __forceinline__ bool pair_search(float2 xi, float2 xj, float hi, floa
     return g.r < (float)SK * g.mh;
 }
 
-// The test alone, for the scan over candidates: lo = 0.99998 (0 takes the
-// exact test always, for smoothing lengths whose squares underflow).  The
-// squares decide away from the edge of the support, with FMA and a margin of
-// 1e-5 on either side, far above their rounding; the pairs in between take
-// the test itself.
+// The scan's test of a candidate: v = r^2 - (SK/2 (hi + hj))^2 in FMA, whose
+// sign decides away from the edge of the support.  Within kEdge of the largest
+// square there is, far above the rounding of v, the caller takes pair_search.
+constexpr float kEdge = 1.e-5f;
 template <int SK>
-__device__ __forceinline__ bool pair_kept(float2 xi, float4 o, float hi, float lo) {
+__device__ __forceinline__ float pair_gap(float2 xi, float4 o, float hi) {
     const float d0 = xi.x - o.x, d1 = xi.y - o.y;
-    const float dr = __fmaf_rn(d1, d1, d0 * d0);
     const float t = (SK == 2) ? hi + o.z : 1.5f * (hi + o.z);
-    const float u = t * (t * 1.00001f);
-    bool ok = dr <= u;
-    if (ok && dr >= u * lo) {
-        PairGeom g;
-        ok = pair_search<SK>(xi, make_float2(o.x, o.y), hi, o.z, g);
-    }
-    return ok;
+    return __fmaf_rn(-t, t, __fmaf_rn(d1, d1, d0 * d0));
+}
+template <int SK>
+__device__ __forceinline__ bool pair_exact(float2 xi, float4 o, float hi) {
+    PairGeom g;
+    return pair_search<SK>(xi, make_float2(o.x, o.y), hi, o.z, g);
 }
 
 // Float <-> order-preserving uint, for atomicMin/atomicMax reductions.

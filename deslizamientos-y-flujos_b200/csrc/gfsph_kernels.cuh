@@ -824,7 +824,7 @@ __device__ __forceinline__ bool ref_adjacent(const Search& Q, int2 ci, int j) {
 // for the next kDenList of each lane.
 constexpr int kDenThreads = 128;
 constexpr int kDenBlocks = 7;  // resident blocks asked for
-constexpr int kScanStep = 2;  // candidates loaded at a time
+constexpr int kScanStep = 4;  // candidates loaded at a time
 template <int G> struct DenList { static constexpr int value = (G == 2) ? 40 : (G == 4 ? 24 : 16); };  // ~1.5x a lane's share of 50
 // The particles of the coarse levels, few, are not searched through their
 // mostly empty grids: each block picks those that reach its particles' box
@@ -844,7 +844,7 @@ constexpr int kBigScan = 4096;
 // range.
 template <bool SPARSE>
 struct LevelRows {
-    float u, v, s2, ex, ey;
+    float u, v, s2, ex, ey, reach;  // reach: SK/2 (hi + Hk)
     int y0, nrow, ndx, base, nbx;  // base: the level's first key (dense) or block-map entry (sparse)
 
     // false for an empty level
@@ -858,7 +858,8 @@ struct LevelRows {
         // clamped as the cell numbers are: that brings no two particles further apart
         u = fminf(fmaxf((xi.x - S->lev_gx0[k]) * rc, 0.f), (float)ndx);
         v = fminf(fmaxf((xi.y - S->lev_gy0[k]) * (rc * (1.f / kCellAspect)), 0.f), (float)ndy);
-        const float s = support_span<SK>(hi, o2f(hk)) * rc;
+        reach = support_span<SK>(hi, o2f(hk));
+        const float s = reach * rc;
         s2 = s * s;
         ex = 0.01f + (float)ndx * 1.e-6f;
         ey = 0.01f + (float)ndy * 1.e-6f;
@@ -947,34 +948,44 @@ __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, S
                 bh = fmaxf(bh, wbox[w][4]);
             }
         }
-        const float lo = hi > 1.e-14f ? 0.99998f : 0.f;
         double acc = 0.0;
         int found = 0;  // entries of this particle in the table
         for (int skip = 0;; skip += L) {
-            // phase 1: the neighbours this lane finds, from the skip-th on, go into its list; at points to the next
-            // place, before the list while the first skip ones pass
+            // phase 1: the neighbours this lane finds, from the skip-th on, go into its list; at is the next place,
+            // before the list while the first skip ones pass
             int at = tid - skip * kDenThreads;
-            auto keep = [&](int j) {
-                if ((unsigned)at < (unsigned)(L * kDenThreads)) list[at] = j;
-                at += kDenThreads;
+            auto keep = [&](int j, bool ok) {
+                if (ok && (unsigned)at < (unsigned)(L * kDenThreads)) list[at] = j;
+                at += ok ? kDenThreads : 0;
             };
             int first = gl;  // this lane's first row of the next level
             for (int k = 0; k < nlev; k++) {
                 LevelRows<SPARSE> rows;
                 if (!rows.template open<SK>(S, k, xi, hi)) continue;
+                const float edge = kEdge * rows.reach * rows.reach;
                 if (act)
                     for (int s = first; s < rows.nrow; s += G) {
                         int ja, jb;
                         rows.range(Q, s, ja, jb);
                         for (int j = ja; j < jb; j += kScanStep) {
                             float4 o[kScanStep];  // xhm is padded by kScanStep entries
+                            float v[kScanStep];
+                            bool near = false;
 #pragma unroll
                             for (int u = 0; u < kScanStep; u++) o[u] = Q.xhm[j + u];
 #pragma unroll
+                            for (int u = 0; u < kScanStep; u++) {
+                                v[u] = pair_gap<SK>(xi, o[u], hi);
+                                near |= fabsf(v[u]) <= edge;
+                            }
+                            if (near) {
+#pragma unroll
+                                for (int u = 0; u < kScanStep; u++)
+                                    if (fabsf(v[u]) <= edge) v[u] = pair_exact<SK>(xi, o[u], hi) ? -1.f : 1.f;
+                            }
+#pragma unroll
                             for (int u = 0; u < kScanStep; u++)
-                                if (pair_kept<SK>(xi, o[u], hi, lo) && j + u < jb && j + u != i &&
-                                    ref_adjacent<SK>(Q, ci, j + u))
-                                    keep(j + u);
+                                keep(j + u, (v[u] < 0.f) & (j + u < jb) & (j + u != i) && ref_adjacent<SK>(Q, ci, j + u));
                         }
                     }
                 first = (first + G - rows.nrow % G) % G;
@@ -1005,7 +1016,7 @@ __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, S
                     if (act)
                         for (int e = gl; e < tot; e += G) {
                             const int j = bigj[e];
-                            if (pair_kept<SK>(xi, bigs[e], hi, lo) && ref_adjacent<SK>(Q, ci, j)) keep(j);
+                            keep(j, pair_exact<SK>(xi, bigs[e], hi) && ref_adjacent<SK>(Q, ci, j));
                         }
                 }
             // phase 2: the group's listed pairs in lane order, shared out evenly
