@@ -1067,6 +1067,7 @@ int create_handle(const gfsph_params* p, const gfsph_dem* dem, gfsph_handle* sha
     c.muI = (c.nfric == 8 || c.nfric == 26) ? 1 : (c.nfric == 27 ? 2 : 0);
     c.mu_a = k[2]; c.mu_r = k[5]; c.mu_b = k[6];
     if (c.muI) c.xi = 0.f;  // const(3) is a mu(I) parameter, not xi (:9653)
+    c.rxi = (std::fabs(c.xi) >= 1.e-9f && std::fabs(c.xi) <= 1.e12f) ? 1.f / c.xi : 0.f;
     hb_constants(k, c);
     c.ws = p->ws_interact;
     c.swalg = p->sw_alg;
@@ -1153,6 +1154,8 @@ int create_handle(const gfsph_params* p, const gfsph_dem* dem, gfsph_handle* sha
     d.nx = nx; d.ny = ny; d.xmin = dem->xmin; d.ymin = dem->ymin; d.dx = dem->dx; d.dy = dem->dy;
     d.xmax = d.xmin + (float)(nx - 1) * d.dx;
     d.ymax = d.ymin + (float)(ny - 1) * d.dy;
+    d.rdx = 1.f / d.dx;
+    d.rdy = 1.f / d.dy;
     d.grad = h->d_grad; d.curvA = h->d_curvA; d.curvB = h->d_curvB;
     }
     if (c.ws) {

@@ -46,6 +46,8 @@ __device__ __forceinline__ float quot(float a, float b, float y) {
     const float q = a * y;
     return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
 }
+// The square root of any value: root() within its range, else the operator.
+__device__ __forceinline__ float root_any(float d) { return (d >= 1.e-30f && d <= 1.e37f) ? root(d) : sqrtf(d); }
 // Smoothing lengths for which every product and quotient of a pair's kernel
 // stays far from overflow and underflow.
 constexpr float kQuotMin = 1.e-6f, kQuotMax = 1.e9f;
@@ -279,23 +281,31 @@ struct DemView {
     const float2* __restrict__ grad;  // topol(2:3,:)
     const float4* __restrict__ curvA; // topol(4:7,:)  (nfric 7 only)
     const float2* __restrict__ curvB; // topol(8:9,:)
+    float rdx, rdy;                   // 1/dx, 1/dy (for quot)
 };
+
+// The DEM node (1-based) at or below a point of the box, as
+// int((x - xmin)/dx + 1).
+__device__ __forceinline__ int dem_node_x(const DemView& d, float xx) {
+    return (int)(quot(xx - d.xmin, d.dx, d.rdx) + 1.f);
+}
+__device__ __forceinline__ int dem_node_y(const DemView& d, float yy) {
+    return (int)(quot(yy - d.ymin, d.dy, d.rdy) + 1.f);
+}
 
 // Get_Z_Topo, SPH_FEM_topo_2019.f90:2395-2491: bilinear shape functions on
 // the DEM cell containing (xx, yy).  Returns Zx, Zy and, when want_curv, the
 // six curvature terms topol(4..9).
 __device__ __forceinline__ void dem_lookup(const DemView& d, float xx, float yy, float& zpx, float& zpy,
                                            bool want_curv, float top[6]) {
-    int ipx = (int)((xx - d.xmin) / d.dx + 1.f);
-    int ipy = (int)((yy - d.ymin) / d.dy + 1.f);
-    ipx = min(max(ipx, 1), d.nx - 1);
-    ipy = min(max(ipy, 1), d.ny - 1);
+    int ipx = min(max(dem_node_x(d, xx), 1), d.nx - 1);
+    int ipy = min(max(dem_node_y(d, yy), 1), d.ny - 1);
     int ip = (ipy - 1) * d.nx + (ipx - 1);
     int n1 = ip, n2 = ip + 1, n3 = ip + 1 + d.nx, n4 = n3 - 1;
     float xref = d.xmin + (float)(ipx - 1) * d.dx;
     float yref = d.ymin + (float)(ipy - 1) * d.dy;
-    float xi = (xx - xref) / d.dx;
-    float eta = (yy - yref) / d.dy;
+    float xi = quot(xx - xref, d.dx, d.rdx);
+    float eta = quot(yy - yref, d.dy, d.rdy);
     float sh1 = (1.f - xi) * (1.f - eta);
     float sh2 = xi * (1.f - eta);
     float sh3 = xi * eta;
@@ -319,6 +329,7 @@ __device__ __forceinline__ void dem_lookup(const DemView& d, float xx, float yy,
 struct Rheo {
     float g, dens, xi, tauy0, constK, tanfi, hfrict0, comp, keros, slip, h_inf, cgra05;
     int nfric, erosion, skf, pa_sph, sle, av_vel, ic_adapt;
+    float rxi;  // 1/xi for quot, 0 where xi is too small or large for it
     // stage-dependent pressure: normalised density (nor_density) and the
     // terrain-normal gravity (ic_cosTheta = 1); either runs the staged RK45
     int nor_density, cos_theta;
@@ -357,6 +368,7 @@ __device__ __forceinline__ float powr(float x, float y) { return (float)pow((dou
 // Locals of ExtForces_SW shared with its contained routines.
 struct ExtLocal {
     float h, hu, hv, hinv, vmod, hvmod, hvmodinv, frictx, fricty, totfrict, cf5, gravx, gravy;
+    float hrcp;  // 1/h for quot (also where the clamp to comp leaves hinv 0)
     float hrho;  // rho(ipoin) as ExtForces_SW reads it, before the comp clamp
     // read by erosion law 2: vxx, vyy and tanfi as the friction leaves them,
     // the slopes of Get_Z_Topo
@@ -374,12 +386,14 @@ __device__ __forceinline__ void ext_locals(const Rheo& c, float hdepth, float vx
     L.hv = L.h * vy;
     if (L.h < c.comp) {
         L.h = c.comp;
+        L.hrcp = 1.f / c.comp;
         L.hu = 0.f; L.hv = 0.f; L.hinv = 0.f; L.vmod = 0.f; L.hvmod = 0.f; L.hvmodinv = 0.f;
     } else {
-        L.hinv = 1.f / L.h;
-        L.hvmod = sqrtf(L.hu * L.hu + L.hv * L.hv);
+        L.hinv = recip(L.h);  // comp is above 1e-8
+        L.hrcp = L.hinv;
+        L.hvmod = root_any(L.hu * L.hu + L.hv * L.hv);
         L.vmod = L.hvmod * L.hinv;
-        L.hvmodinv = (L.hvmod >= 1.e-5f) ? 1.f / L.hvmod : 0.f;
+        L.hvmodinv = (L.hvmod >= 1.e-5f) ? recip(L.hvmod) : 0.f;
     }
 }
 
@@ -428,13 +442,13 @@ __device__ __forceinline__ void grav_and_friction(const Rheo& c, const DemView& 
             L.fricty = (cf4b * L.hv) * L.hvmodinv;
         } else {
             float a2 = 48.f, b2 = -(32.f * a_hat) - 114.f, c2 = 65.f;
-            float xh = (-b2 - sqrtf(b2 * b2 - (4.f * a2) * c2)) / (2.f * a2);
+            float xh = quot(-b2 - root_any(b2 * b2 - (4.f * a2) * c2), 96.f, 1.f / 96.f);  // / (2 a2)
             float tau0 = c.tauy0 / xh;
             float cf4b = tau0 / c.dens;
             L.frictx = (cf4b * L.hu) * L.hvmodinv;
             L.fricty = (cf4b * L.hv) * L.hvmodinv;
         }
-        L.totfrict = sqrtf(L.frictx * L.frictx + L.fricty * L.fricty);
+        L.totfrict = root_any(L.frictx * L.frictx + L.fricty * L.fricty);
     } else if (GEN && c.nfric == 3) {  // Bingham of the eroded soil fraction nsoil, :9443-9489
         const float fsoil = 1.f - (float)exp((double)(-(c.xi * nsoil)));  // C3 = const(3)
         const float constKB = c.constK * fsoil, tauy0B = c.tauy0 * fsoil;
@@ -513,9 +527,10 @@ __device__ __forceinline__ void grav_and_friction(const Rheo& c, const DemView& 
             float vxx = L.hu * L.hinv, vyy = L.hv * L.hinv;
             L.vxx = vxx;
             L.vyy = vyy;
-            L.vmod = sqrtf(vxx * vxx + vyy * vyy);
+            L.vmod = root_any(vxx * vxx + vyy * vyy);
             if (L.vmod >= 1e-5f) {
-                float cosa = vxx / L.vmod, sina = vyy / L.vmod;
+                const float vr = recip(L.vmod);
+                float cosa = quot(vxx, L.vmod, vr), sina = quot(vyy, L.vmod, vr);
                 float cos2 = cosa * cosa, sin2 = sina * sina, cbs = sina * cosa;
                 float xnum = (top[3] * cos2 + top[4] * cbs) + top[5] * sin2;
                 float xden = (top[0] * cos2 + top[1] * cbs) + top[2] * sin2;
@@ -552,18 +567,19 @@ __device__ __forceinline__ void grav_and_friction(const Rheo& c, const DemView& 
             L.vxx = vx;  // :9720-9723, 9752-9755
             L.vyy = vy;
             float vm = vx * vx + vy * vy;
-            vm = (vm > 0.f) ? sqrtf(vm) : 0.f;
+            vm = (vm > 0.f) ? root_any(vm) : 0.f;
             L.vmod = vm;
             if (c.xi > 0.f) {
-                L.frictx = L.frictx + ((c.g * L.vmod) * vx) / c.xi;
-                L.fricty = L.fricty + ((c.g * L.vmod) * vy) / c.xi;
+                const float fx = (c.g * L.vmod) * vx, fy = (c.g * L.vmod) * vy;
+                L.frictx = L.frictx + ((c.rxi != 0.f) ? quot(fx, c.xi, c.rxi) : fx / c.xi);
+                L.fricty = L.fricty + ((c.rxi != 0.f) ? quot(fy, c.xi, c.rxi) : fy / c.xi);
             } else {
                 float constMu = -((25.f * c.xi) / 4.f);
                 L.frictx = L.frictx + ((constMu * L.vmod) * vx) / (hfrict * hfrict);
                 L.fricty = L.fricty + ((constMu * L.vmod) * vy) / (hfrict * hfrict);
             }
         }
-        L.totfrict = sqrtf(L.frictx * L.frictx + L.fricty * L.fricty);
+        L.totfrict = root_any(L.frictx * L.frictx + L.fricty * L.fricty);
     }
 }
 
@@ -662,8 +678,8 @@ __device__ __forceinline__ void ext_accel(const Rheo& c, const DemView& d, float
     ex0 = 0.f + L.gravx;
     ex1 = 0.f + L.gravy;
     reversal_filter(c, dt, vx, vy, ex0 + in0, ex1 + in1, L);
-    ex0 = ex0 - L.frictx / L.h;
-    ex1 = ex1 - L.fricty / L.h;
+    ex0 = ex0 - quot(L.frictx, L.h, L.hrcp);
+    ex1 = ex1 - quot(L.fricty, L.h, L.hrcp);
     if (c.erosion) {
         if (GEN && c.eros_law == 3) er = erosion_rate_shear(c, L);
         ex0 = ex0 - ((er * vx) * L.hinv) * c.slip;
@@ -714,8 +730,8 @@ __device__ __forceinline__ void ext_accel_wir(const Rheo& c, const DemView& d, f
         ex1 = b.y + L.gravy;
     }
     reversal_filter(cw, dt, vx, vy, ex0 + in0, ex1 + in1, L);
-    ex0 = ex0 - L.frictx / L.h;
-    ex1 = ex1 - L.fricty / L.h;
+    ex0 = ex0 - quot(L.frictx, L.h, L.hrcp);
+    ex1 = ex1 - quot(L.fricty, L.h, L.hrcp);
 }
 
 // The erosion rate after the RK update (ExtForces_SW(1), :8717-8760) with

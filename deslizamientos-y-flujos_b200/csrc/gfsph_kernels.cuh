@@ -1337,29 +1337,29 @@ __device__ __forceinline__ void erosion_scatter(const DemView& dem, float xx, fl
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int ipx = 0, ipy = 0, key = -1 - lane;  // non-participants: singleton runs with zero terms
     if (part) {
-        ipx = (int)((xx - dem.xmin) / dem.dx + 1.f);
-        ipy = (int)((xy - dem.ymin) / dem.dy + 1.f);
+        ipx = dem_node_x(dem, xx);
+        ipy = dem_node_y(dem, xy);
         key = ipy * (dem.nx + 2) + ipx;
     }
     if (!__any_sync(full, part)) return;
     float(*T)[33] = sterm[wid];
     // the 4x4 nodes (ipx-1..ipx+2) x (ipy-1..ipy+2); nodes outside the DEM add zero
+    float dx2[4], dy2[4];
+#pragma unroll
+    for (int o = 0; o < 4; o++) {
+        const float ddx = xx - (dem.xmin + (float)(ipx + o - 2) * dem.dx), ddy = xy - (dem.ymin + (float)(ipy + o - 2) * dem.dy);
+        dx2[o] = ddx * ddx;
+        dy2[o] = ddy * ddy;
+    }
+#pragma unroll
     for (int o = 0; o < 16; o++) {
         const int ix = ipx + (o >> 2) - 1, iy = ipy + (o & 3) - 1;
         const bool inside = part && ix >= 1 && ix <= dem.nx && iy >= 1 && iy <= dem.ny;
-        float a = 0.f, b = 0.f;
-        if (inside) {
-            float ddx = xx - (dem.xmin + (float)(ix - 1) * dem.dx);
-            ddx = ddx * ddx;
-            float ddy = xy - (dem.ymin + (float)(iy - 1) * dem.dy);
-            ddy = ddy * ddy;
-            float dist = sqrtf(ddx + ddy);
-            dist = (1.e-6f > dist) ? 1.e-6f : dist;
-            a = base / dist;
-            b = 1.f / dist;
-        }
-        T[o][lane] = a;
-        T[16 + o][lane] = b;
+        // max(1e-6, distance); the root is kept off 0
+        const float dist = fmaxf(root(fmaxf(dx2[o >> 2] + dy2[o & 3], 1.e-30f)), 1.e-6f);
+        const float y = recip(dist);
+        T[o][lane] = inside ? quot(base, dist, y) : 0.f;
+        T[16 + o][lane] = inside ? y : 0.f;
     }
     skey[wid][lane] = key;
     if (lane == 0) skey[wid][32] = INT_MIN;  // no key: closes the last run
@@ -1821,12 +1821,11 @@ __global__ void __launch_bounds__(128) k_wir_press(PState A, Search Q, StepScala
         if (!wir_stage_pos(A, C, s, dt, i, p) || out_of_box(dem, p.x, p.y)) continue;  // keeps its term
         float zp = 0.f;
         if (water) {
-            int ipx = (int)((p.x - dem.xmin) / dem.dx + 1.f), ipy = (int)((p.y - dem.ymin) / dem.dy + 1.f);
-            ipx = min(max(ipx, 1), dem.nx - 1);
-            ipy = min(max(ipy, 1), dem.ny - 1);
+            const int ipx = min(max(dem_node_x(dem, p.x), 1), dem.nx - 1);
+            const int ipy = min(max(dem_node_y(dem, p.y), 1), dem.ny - 1);
             const int n1 = (ipy - 1) * dem.nx + (ipx - 1), n2 = n1 + 1, n3 = n1 + 1 + dem.nx, n4 = n3 - 1;
             const float xref = dem.xmin + (float)(ipx - 1) * dem.dx, yref = dem.ymin + (float)(ipy - 1) * dem.dy;
-            const float xi = (p.x - xref) / dem.dx, eta = (p.y - yref) / dem.dy;
+            const float xi = quot(p.x - xref, dem.dx, dem.rdx), eta = quot(p.y - yref, dem.dy, dem.rdy);
             const float sh1 = (1.f - xi) * (1.f - eta), sh2 = xi * (1.f - eta), sh3 = xi * eta, sh4 = (1.f - xi) * eta;
             const float d1x = (-1.f + eta) / dem.dx, d2x = (1.f - eta) / dem.dx, d3x = eta / dem.dx, d4x = (-eta) / dem.dx;
             const float d1y = (-1.f + xi) / dem.dy, d2y = (-xi) / dem.dy, d3y = xi / dem.dy, d4y = (1.f - xi) / dem.dy;
