@@ -382,7 +382,7 @@ int enqueue_search(gfsph_handle* h, int advance) {
     if (!advance) { launch(h, K_PREP, [&] { pdl_launch(k_prep, 1, 32, st, S, advance); }); nk++; }
     const GridArgs ga{h->cap_blocks, h->cap_cells, kMaxCells, h->level_factor, h->cell_div, h->reg_levels};
     launch(h, K_BOUNDS, [&] {
-        pdl_launch(k_bounds, kBoundsBlocks, kThreadsBounds, st, h->B, n, h->rheo, h->dem, S, h->bparts, ga);
+        pdl_launch(k_bounds, std::min(kBoundsBlocks, blocks_for(n, kThreadsBounds)), kThreadsBounds, st, h->B, n, h->rheo, h->dem, S, h->bparts, ga);
     }); nk++;
     launch(h, K_MARK, [&] { pdl_launch(k_mark, pb, kThreads, st, h->B, n, h->dem, S, h->bmark); }); nk++;
     launch(h, K_BSCAN_TILES, [&] {

@@ -32,8 +32,8 @@ constexpr int kBlkX = 32;           // cells per block along x
 constexpr int kBlkY = 8;            // cells per block along y
 constexpr int kBlockCells = kBlkX * kBlkY;
 constexpr long long kDenseCells = 1LL << 22;  // dense-mode budget (or 8 cells per particle)
-constexpr int kThreadsBounds = 128;
-constexpr int kBoundsBlocks = 148 * 8;
+constexpr int kThreadsBounds = 256;
+constexpr int kBoundsBlocks = 148 * 4;  // at most; the last block reduces their partials
 
 // error bits in StepScalars::err
 constexpr int kErrCells = 1;
@@ -363,13 +363,16 @@ __global__ void __launch_bounds__(kThreadsBounds) k_bounds(PState B, int n, Rheo
     if ((threadIdx.x & 31) == 0) wp[threadIdx.x >> 5] = b;
     __syncthreads();
     StepScalars* L = scalars_to_smem(S);
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         BoundsPart t = wp[0];
         for (int k = 1; k < (int)(blockDim.x >> 5); k++) bounds_merge(t, wp[k]);
-        L->xmin_o = f2o(t.xmn); L->xmax_o = f2o(t.xmx); L->ymin_o = f2o(t.ymn); L->ymax_o = f2o(t.ymx);
-        L->hmax_o = f2o(t.hmx); L->dtmin_o = f2o(t.dtm);
-        L->hsum = t.hsum; L->hcount = t.hcnt; L->bad = t.bad;
-        L->bounds_ticket = 0u;
+        if (threadIdx.x == 0) {
+            L->xmin_o = f2o(t.xmn); L->xmax_o = f2o(t.xmx); L->ymin_o = f2o(t.ymn); L->ymax_o = f2o(t.ymx);
+            L->hmax_o = f2o(t.hmx); L->dtmin_o = f2o(t.dtm);
+            L->hsum = t.hsum; L->hcount = t.hcnt; L->bad = t.bad;
+            L->bounds_ticket = 0u;
+        }
+        __syncwarp();
         grid_setup(c, L, ga);
     }
     scalars_from_smem(S, L);
@@ -390,86 +393,95 @@ __global__ void __launch_bounds__(kThreadsBounds) k_bounds(PState B, int n, Rheo
 // level_factor and cell_div are the search's tunables (gfsph_set_search):
 // Hc = min(max, level_factor * mean hsml) and level k's cell size is
 // Hc * 2^k / cell_div; neither changes the neighbour sets.
+// Run by one warp on the shared copy of the scalars: the scalars by all lanes
+// alike (lane 0 writes), level k by lane k.
 __device__ void grid_setup(const Rheo& c, StepScalars* S, const GridArgs ga) {
-    const int cap_blocks = ga.cap_blocks, cap_cells = ga.cap_cells, max_cells = ga.max_cells;
-    const float level_factor = ga.level_factor, cell_div = ga.cell_div;
-    S->reg_levels = ga.reg_levels;
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const bool first = lane == 0;
+    if (first) S->reg_levels = ga.reg_levels;
     if (S->skip) return;
-    if (S->bad) { S->err |= kErrNonFinite; S->skip = 1; return; }
-    float xmn = o2f(S->xmin_o), xmx = o2f(S->xmax_o), ymn = o2f(S->ymin_o), ymx = o2f(S->ymax_o);
-    float hmx = o2f(S->hmax_o);
-    if (S->xmin_o == 0xffffffffu || !(hmx > 0.f) || S->hcount == 0) { S->err |= kErrEmpty; S->skip = 1; return; }
+    auto stop = [&](int bits) {
+        if (first) { S->err |= bits; S->skip = 1; }
+    };
+    if (S->bad) return stop(kErrNonFinite);
+    const float xmn = o2f(S->xmin_o), xmx = o2f(S->xmax_o), ymn = o2f(S->ymin_o), ymx = o2f(S->ymax_o);
+    const float hmx = o2f(S->hmax_o);
+    if (S->xmin_o == 0xffffffffu || !(hmx > 0.f) || S->hcount == 0) return stop(kErrEmpty);
     float dt = S->dt;
     if (S->advance) {
         float dtmin = (c.ic_adapt != 0) ? o2f(S->dtmin_o) : 1.e10f;
         if (dtmin < dt) dt = dtmin;
         else if (c.ic_adapt != 0) dt = fminf(1.1f * dt, dtmin);
     }
-    S->dt_step = dt;
-    {  // the reference's grid: cells of 2*max(hsml) (grid_find_NEW_tools My_SPH_Tools_2019.f90:1168-1181)
+    const float lx = xmx - xmn, ly = ymx - ymn;
+    if (first) {
+        S->dt_step = dt;
+        // the reference's grid: cells of 2*max(hsml) (grid_find_NEW_tools My_SPH_Tools_2019.f90:1168-1181)
         const float delt = hmx * 2.f;
-        float len = xmx - xmn;
-        int nd = (int)(len / delt + 1.f);
+        int nd = (int)(lx / delt + 1.f);
         S->ref_ndx = nd;
-        S->ref_xmin = (xmn - ((float)nd * delt - len) / 2.f) - 0.001f * len;
-        len = ymx - ymn;
-        nd = (int)(len / delt + 1.f);
+        S->ref_xmin = (xmn - ((float)nd * delt - lx) / 2.f) - 0.001f * lx;
+        nd = (int)(ly / delt + 1.f);
         S->ref_ndy = nd;
-        S->ref_ymin = (ymn - ((float)nd * delt - len) / 2.f) - 0.001f * len;
+        S->ref_ymin = (ymn - ((float)nd * delt - ly) / 2.f) - 0.001f * ly;
         S->ref_delt = delt;
     }
-    float mean = (float)(S->hsum / (double)S->hcount);
-    float hc = fminf(hmx, level_factor * mean);
+    const float mean = (float)(S->hsum / (double)S->hcount);
+    const float hc = fminf(hmx, ga.level_factor * mean);
     int nlev = 1;
     while (nlev < kMaxLevels && ldexpf(hc, nlev - 1) < hmx) nlev++;
-    if (ldexpf(hc, nlev - 1) < hmx) { S->err |= kErrCells; S->need_cells = 0x3fffffff; S->skip = 1; return; }
-    float lx = xmx - xmn, ly = ymx - ymn;
-    long long off = 0, doff = 0;
-    for (int k = 0; k < nlev; k++) {
-        float cell = ldexpf(hc, k) / cell_div;
-        const float cellh = cell * kCellAspect;
-        float fx = lx / cell + 1.f, fy = ly / cellh + 1.f;
-        if (!(fx < 1.0e8f) || !(fy < 1.0e8f) || !(fx * fy < 2.0e9f)) {  // far beyond any capacity
-            S->err |= kErrCells;
-            S->need_cells = 0x3fffffff;
-            S->skip = 1;
-            return;
-        }
-        int ndx = (int)fx, ndy = (int)fy;
-        float lxn = (float)ndx * cell, lyn = (float)ndy * cellh;
+    const int k = lane;
+    float cell = 0.f, cellh = 0.f, fx = 1.f, fy = 1.f;
+    if (k < nlev) {
+        cell = ldexpf(hc, k) / ga.cell_div;
+        cellh = cell * kCellAspect;
+        fx = lx / cell + 1.f;
+        fy = ly / cellh + 1.f;
+    }
+    const bool far = !(fx < 1.0e8f) || !(fy < 1.0e8f) || !(fx * fy < 2.0e9f);  // far beyond any capacity
+    if (__any_sync(full, far) || ldexpf(hc, nlev - 1) < hmx) {
+        if (first) S->need_cells = 0x3fffffff;
+        return stop(kErrCells);
+    }
+    const int ndx = (int)fx, ndy = (int)fy;
+    const int nbx = (ndx + kBlkX - 1) / kBlkX, nby = (ndy + kBlkY - 1) / kBlkY;
+    long long off = (k < nlev) ? (long long)nbx * nby : 0, doff = (k < nlev) ? (long long)ndx * ndy : 0;
+    for (int o = 1; o < 32; o <<= 1) {  // the levels' blocks and cells up to and with level k
+        const long long t = __shfl_up_sync(full, off, o), u = __shfl_up_sync(full, doff, o);
+        if (lane >= o) { off += t; doff += u; }
+    }
+    if (k < nlev) {
+        const float lxn = (float)ndx * cell, lyn = (float)ndy * cellh;
         S->lev_gx0[k] = (xmn - (lxn - lx) / 2.f) - 0.001f * lx;
         S->lev_gy0[k] = (ymn - (lyn - ly) / 2.f) - 0.001f * ly;
         S->lev_c[k] = cell;
         S->lev_ndx[k] = ndx;
         S->lev_ndy[k] = ndy;
-        int nbx = (ndx + kBlkX - 1) / kBlkX, nby = (ndy + kBlkY - 1) / kBlkY;
         S->lev_nbx[k] = nbx;
-        S->lev_boff[k] = (int)min(off, 0x7fffffffLL);
-        S->lev_off[k] = (int)min(doff, 0x7fffffffLL);
-        off += (long long)nbx * (long long)nby;
-        doff += (long long)ndx * (long long)ndy;
+        S->lev_boff[k + 1] = (int)min(off, 0x7fffffffLL);
+        S->lev_off[k + 1] = (int)min(doff, 0x7fffffffLL);
     }
-    S->lev_boff[nlev] = (int)min(off, 0x7fffffffLL);
-    S->lev_off[nlev] = (int)min(doff, 0x7fffffffLL);
+    off = __shfl_sync(full, off, nlev - 1);
+    doff = __shfl_sync(full, doff, nlev - 1);
+    if (!first) return;
+    S->lev_boff[0] = 0;
+    S->lev_off[0] = 0;
     S->hc = hc;
     S->nlev = nlev;
-    const long long budget = min((long long)max_cells, max(kDenseCells, 8LL * S->hcount));
+    const long long budget = min((long long)ga.max_cells, max(kDenseCells, 8LL * S->hcount));
     S->sparse = (doff + 1 > budget) ? 1 : 0;
     if (!S->sparse) {
-        if (doff + 1 > (long long)cap_cells) {
-            S->err |= kErrCells;
+        if (doff + 1 > (long long)ga.cap_cells) {
             S->need_cells = (int)(doff + 1);
-            S->skip = 1;
-            return;
+            return stop(kErrCells);
         }
         S->ncells = (int)doff;
         return;
     }
-    if (off + 1 > (long long)cap_blocks) {
-        S->err |= kErrBlocks;
+    if (off + 1 > (long long)ga.cap_blocks) {
         S->need_blocks = (off + 1 > 0x3fffffffLL) ? 0x3fffffff : (int)(off + 1);
-        S->skip = 1;
-        return;
+        return stop(kErrBlocks);
     }
     S->nblocks = (int)off;
 }
