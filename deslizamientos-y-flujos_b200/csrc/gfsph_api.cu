@@ -21,19 +21,17 @@ using namespace gfsph;
 namespace {
 
 enum KernelId {
-    K_PREP, K_BOUNDS, K_HIST, K_SCAN_TILES, K_SCAN_ADD, K_SCATTER, K_CELL_SORT,
-    K_REORDER, K_DENSITY, K_DENSITY_BIG, K_IFORCE, K_FORCE_BIG, K_FORCE_RK, K_XSPH, K_XSPH_BIG, K_DEM_ERODE,
-    K_STEP_END, K_COPY, K_UNSORT, K_RASTER, K_HAZARD, K_EXPORT, K_MARK, K_BSCAN_TILES, K_BSCAN_ADD,
+    K_PREP, K_BOUNDS, K_HIST, K_SCAN_TILES, K_SCATTER, K_REORDER, K_DENSITY, K_DENSITY_BIG, K_IFORCE, K_FORCE_BIG, K_FORCE_RK, K_XSPH, K_XSPH_BIG, K_DEM_ERODE,
+    K_STEP_END, K_COPY, K_UNSORT, K_RASTER, K_HAZARD, K_EXPORT, K_MARK, K_BSCAN_TILES,
     K_DENSITY_SPARSE, K_COUPLE, K_ADJOINT, K_NORM, K_NORM_BIG, K_STAGE, K_WIR,
     K_STEPS,  // not a kernel: device time of whole gfsph_step batches (profile level 2)
     K_COUNT
 };
 const char* kKernelNames[K_COUNT] = {
-    "k_prep", "k_bounds", "k_hist", "k_scan_tiles", "k_scan_add",
-    "k_scatter", "k_cell_sort", "k_reorder", "k_density", "k_density_big", "k_iforce", "k_force_big",
+    "k_prep", "k_bounds", "k_hist", "k_scan_tiles", "k_scatter", "k_reorder", "k_density", "k_density_big", "k_iforce", "k_force_big",
     "k_force_rk", "k_xsph", "k_xsph_big", "k_dem_erode", "k_step_end", "k_copy_state", "k_unsort",
     "k_raster_idw", "k_hazard", "k_export_big", "k_mark", "k_scan_tiles(blocks)",
-    "k_scan_add(blocks)", "k_density(sparse)", "k_couple", "k_adjoint", "k_norm", "k_norm_big", "k_stage", "k_wir", "step_batches"};
+    "k_density(sparse)", "k_couple", "k_adjoint", "k_norm", "k_norm_big", "k_stage", "k_wir", "step_batches"};
 
 constexpr int kThreads = 128;
 static_assert(kThreads <= 32 * kScatterWarps, "erosion_scatter keeps shared terms for kScatterWarps warps");
@@ -158,7 +156,6 @@ struct gfsph_handle {
     // particles
     int n = 0;
     PState A{}, B{}, U{};
-    int* cellA = nullptr;
     float2* velfin = nullptr;
     float* pterm = nullptr;
     int2* keyrank = nullptr;
@@ -188,10 +185,12 @@ struct gfsph_handle {
     float* mass0_u = nullptr;  // mass per caller index at upload (nfric 3's m0)
     // cells
     int* count = nullptr;
-    int* start = nullptr;
+    int* start = nullptr;      // its scan per tile, the scanned tile sums, and the two added
     int* tile_sum = nullptr;
+    int* startF = nullptr;
     int cap_cells = 0;
-    int* bmark = nullptr;   // block map: 1 where a block holds particles (cleared by k_hist)
+    int* bmark = nullptr;   // block map: 1 where a block holds particles (cleared by its scan)
+    int* btile_sum = nullptr;
     int* bstart = nullptr;  // its exclusive scan: slot of each occupied block
     int cap_blocks = 0;
     BoundsPart* bparts = nullptr;  // k_bounds block partials
@@ -213,6 +212,7 @@ struct gfsph_handle {
     long long prof_cnt[K_COUNT]{};
     long long launches = 0;
     bool has_state = false, searched = false;
+    bool sparse_seen = false;  // a step has used the block-sparse layout: its launches get the full grids
     // outputs
     double2* d_racc = nullptr;
     float* d_rout = nullptr;
@@ -342,8 +342,7 @@ size_t tab_rows(const gfsph_handle* h) { return ((size_t)std::max(h->n, 1) + 31)
 Search make_search(gfsph_handle* h) {
     Search q;
     q.bstart = h->bstart;
-    q.start = h->start;
-    q.cellA = h->cellA;
+    q.start = h->startF;
     q.xhm = h->xhm;
     const size_t ents = (size_t)h->kcap * tab_rows(h);
     q.nj = h->nbr;
@@ -364,7 +363,7 @@ Search make_search(gfsph_handle* h) {
     return q;
 }
 
-int big_blocks(const gfsph_handle*) { return 148 * 4; }  // a block of kBigThreads per coarse-level particle
+int big_blocks(const gfsph_handle*) { return 148 * 2; }  // a block of kBigThreads per coarse-level particle; most runs have few
 
 // The cell search: bounds, grid, counting sort, reorder, neighbours+density.
 // Returns the number of kernels enqueued.
@@ -384,43 +383,45 @@ int enqueue_search(gfsph_handle* h, int advance) {
     launch(h, K_BOUNDS, [&] {
         pdl_launch(k_bounds, std::min(kBoundsBlocks, blocks_for(n, kThreadsBounds)), kThreadsBounds, st, h->B, n, h->rheo, h->dem, S, h->bparts, ga);
     }); nk++;
-    launch(h, K_MARK, [&] { pdl_launch(k_mark, pb, kThreads, st, h->B, n, h->dem, S, h->bmark); }); nk++;
+    const TileScan cells{h->start, h->tile_sum}, blocks{h->bstart, h->btile_sum};
+    launch(h, K_MARK, [&] { pdl_launch(k_mark, pb, kThreads, st, h->B, n, h->dem, S, h->bmark); });
     launch(h, K_BSCAN_TILES, [&] {
-        pdl_launch(k_scan_tiles, nbscan, kScanThreads, st, h->bmark, h->bstart, h->tile_sum, nblk, S, 1);
-    }); nk++;
-    launch(h, K_BSCAN_ADD, [&] { pdl_launch(k_scan_add, nbscan, kScanThreads, st, h->bstart, h->tile_sum, nblk, S, 1); }); nk++;
+        pdl_launch(k_scan_tiles, nbscan, kScanThreads, st, h->bmark, h->bstart, h->btile_sum, nblk, S, 1);
+    });
     launch(h, K_HIST, [&] {
-        pdl_launch(k_hist, pb, kThreads, st, h->B, n, h->dem, S, h->bmark, h->bstart, h->count, h->keyrank, h->cap_cells);
-    }); nk++;
+        pdl_launch(k_hist, pb, kThreads, st, h->B, n, h->dem, S, blocks, h->count, h->keyrank, h->cap_cells);
+    });
     launch(h, K_SCAN_TILES, [&] {
         pdl_launch(k_scan_tiles, nscan, kScanThreads, st, h->count, h->start, h->tile_sum, ncel, S, 0);
-    }); nk++;
-    launch(h, K_SCAN_ADD, [&] { pdl_launch(k_scan_add, nscan, kScanThreads, st, h->start, h->tile_sum, ncel, S, 0); }); nk++;
-    launch(h, K_SCATTER, [&] { pdl_launch(k_scatter, pb, kThreads, st, h->keyrank, n, h->start, h->bstart, S, h->perm); }); nk++;
-    launch(h, K_CELL_SORT, [&] { pdl_launch(k_cell_sort, 148 * 4, 128, st, h->perm, h->B.id, h->start, h->count, S); }); nk++;
+    });
+    launch(h, K_SCATTER, [&] { pdl_launch(k_scatter, pb, kThreads, st, h->keyrank, n, cells, blocks, S, h->perm); });
     launch(h, K_REORDER, [&] {
-        pdl_launch(k_reorder, pb, kThreads, st, h->B, n, h->perm, h->keyrank, h->A, h->cellA, h->xhm, S, h->rheo, h->rho0,
-                                           h->rcell, h->spec_u, h->spec_a);
-    }); nk++;
+        pdl_launch(k_reorder, pb, kThreads, st, h->B, n, h->perm, h->keyrank, h->A, h->xhm, S, h->rheo, h->rho0,
+                   h->rcell, h->spec_u, h->spec_a, cells, h->startF, h->bstart, h->btile_sum);
+    });
+    nk += 6;
     // the coarse-level kernels run beside the regular ones when graphs are
     // captured (side stream); serially otherwise
-    cudaStream_t sb = side_stream(h);
+    cudaStream_t side = side_stream(h);
     fork(h, 0);
     with_skf(h, [&](auto sk) {
         constexpr int SKF = decltype(sk)::value;
-        launch(h, K_DENSITY_BIG, [&] { pdl_launch(k_density_big<SKF>, big_blocks(h), kBigThreads, sb, h->A, q, S, h->rheo); });
+        launch(h, K_DENSITY_BIG, [&] { pdl_launch(k_density_big<SKF>, big_blocks(h), kBigThreads, side, h->A, q, S, h->rheo); });
         // the two materials' pair types compiled in only when there are two
         with_lanes(n, [&](auto g) {
             constexpr int G = decltype(g)::value;
-            const int db = std::min(blocks_for((long long)n * G, kDenThreads), 148 * kDenBlocks * 3);
+            // the launch of the layout not in use returns at once: one block per SM, also where it is used after all
+            const int full = std::min(blocks_for((long long)n * G, kDenThreads), 148 * kDenBlocks * 3);
+            const int idle = std::min(full, 148);
+            const int db = h->sparse_seen ? idle : full, sb = h->sparse_seen ? full : idle;
             if (h->rheo.ws) {
                 launch(h, K_DENSITY, [&] { pdl_launch(k_density<false, SKF, true, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
                 launch(h, K_DENSITY_SPARSE,
-                       [&] { pdl_launch(k_density<true, SKF, true, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
+                       [&] { pdl_launch(k_density<true, SKF, true, G>, sb, kDenThreads, st, h->A, q, S, h->rheo, n); });
             } else {
                 launch(h, K_DENSITY, [&] { pdl_launch(k_density<false, SKF, false, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
                 launch(h, K_DENSITY_SPARSE,
-                       [&] { pdl_launch(k_density<true, SKF, false, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
+                       [&] { pdl_launch(k_density<true, SKF, false, G>, sb, kDenThreads, st, h->A, q, S, h->rheo, n); });
             }
         });
     });
@@ -684,7 +685,7 @@ int kernels_per_step(const gfsph_handle* h) {
     // and water: k_wir_pairs_big and per stage k_wir_scatter, k_wir_nodes,
     // k_wir_press), four stages of (k_force_big, k_iforce, k_stage)
     const int body = staged(h) ? (h->rheo.nor_density ? 10 : 0) + (h->rheo.ws ? 13 : 1) + 12 : 3;
-    return 13 + body + (h->rheo.av_vel ? 2 : 0) + 1;
+    return 10 + body + (h->rheo.av_vel ? 2 : 0) + 1;
 }
 
 // The three buffer (re)allocations below drop the graphs (which hold the old
@@ -694,11 +695,12 @@ int alloc_blocks(gfsph_handle* h, int cap) {
     if (cap > kMaxCells) return GFSPH_ERR_CAPACITY;
     drop_graphs(h);
     h->cap_blocks = 0;
-    dfree(h->bmark); dfree(h->bstart);
+    dfree(h->bmark); dfree(h->bstart); dfree(h->btile_sum);
     int st = 0;
     st |= dalloc(&h->bmark, (size_t)cap + 1);
     st |= dalloc(&h->bstart, (size_t)cap + 1);
-    if (st) { dfree(h->bmark); dfree(h->bstart); return GFSPH_ERR_CUDA; }
+    st |= dalloc(&h->btile_sum, 8192 + 1);
+    if (st) { dfree(h->bmark); dfree(h->bstart); dfree(h->btile_sum); return GFSPH_ERR_CUDA; }
     CK(cudaMemsetAsync(h->bmark, 0, ((size_t)cap + 1) * sizeof(int), h->stream));
     h->cap_blocks = cap;
     return 0;
@@ -708,12 +710,13 @@ int alloc_cells(gfsph_handle* h, int cap) {
     if (cap > kMaxCells) return GFSPH_ERR_CAPACITY;
     drop_graphs(h);
     h->cap_cells = 0;
-    dfree(h->count); dfree(h->start); dfree(h->tile_sum);
+    dfree(h->count); dfree(h->start); dfree(h->startF); dfree(h->tile_sum);
     int st = 0;
     st |= dalloc(&h->count, (size_t)cap + 1);
     st |= dalloc(&h->start, (size_t)cap + 1);
-    st |= dalloc(&h->tile_sum, 8192);
-    if (st) { dfree(h->count); dfree(h->start); dfree(h->tile_sum); return GFSPH_ERR_CUDA; }
+    st |= dalloc(&h->startF, (size_t)cap + 1);
+    st |= dalloc(&h->tile_sum, 8192 + 1);
+    if (st) { dfree(h->count); dfree(h->start); dfree(h->startF); dfree(h->tile_sum); return GFSPH_ERR_CUDA; }
     CK(cudaMemsetAsync(h->count, 0, ((size_t)cap + 1) * sizeof(int), h->stream));
     h->cap_cells = cap;
     return 0;
@@ -740,7 +743,7 @@ void free_particles(gfsph_handle* h) {
         dfree(p->pos); dfree(p->vel); dfree(p->rho); dfree(p->mass); dfree(p->hsml); dfree(p->flag); dfree(p->id);
         dfree(p->pwp);
     }
-    dfree(h->cellA); dfree(h->velfin); dfree(h->pterm); dfree(h->keyrank); dfree(h->perm); dfree(h->ncount);
+    dfree(h->velfin); dfree(h->pterm); dfree(h->keyrank); dfree(h->perm); dfree(h->ncount);
     dfree(h->nbr); dfree(h->f2tmp); dfree(h->xhm); dfree(h->indv); dfree(h->rho0);
     dfree(h->carry.v); dfree(h->carry.acc); dfree(h->carry.dx); dfree(h->carry.dv); dfree(h->carry.xo);
     dfree(h->carry.out); dfree(h->carry.u); dfree(h->carry.du); dfree(h->carry.Du); dfree(h->rhoS); dfree(h->rcell); dfree(h->xsv);
@@ -755,7 +758,8 @@ void free_particles(gfsph_handle* h) {
 int drop_state(gfsph_handle* h, int err) {
     drop_graphs(h);
     free_particles(h);
-    dfree(h->count); dfree(h->start); dfree(h->tile_sum); dfree(h->bmark); dfree(h->bstart);
+    dfree(h->count); dfree(h->start); dfree(h->startF); dfree(h->tile_sum); dfree(h->bmark); dfree(h->bstart);
+    dfree(h->btile_sum);
     h->cap_cells = 0;
     h->cap_blocks = 0;
     h->n = 0;
@@ -1186,7 +1190,8 @@ int gfsph_destroy(gfsph_handle* h) try {
     if (h->stream) cudaStreamSynchronize(h->stream);
     drop_graphs(h);
     free_particles(h);
-    dfree(h->count); dfree(h->start); dfree(h->tile_sum); dfree(h->bmark); dfree(h->bstart);
+    dfree(h->count); dfree(h->start); dfree(h->startF); dfree(h->tile_sum); dfree(h->bmark); dfree(h->bstart);
+    dfree(h->btile_sum);
     if (!h->dem_shared) { dfree(h->d_grad); dfree(h->d_curvA); dfree(h->d_curvB); }
     dfree(h->d_z); dfree(h->d_eroded); dfree(h->d_avail);
     dfree(h->d_auxv); dfree(h->S); dfree(h->bparts); dfree(h->d_racc); dfree(h->d_rout); dfree(h->d_lam);
@@ -1241,7 +1246,7 @@ int gfsph_upload(gfsph_handle* h, int n, const float* x, const float* v, const f
         h->n = n;
         int st = 0;
         st |= alloc_pstate(&h->A, n); st |= alloc_pstate(&h->B, n); st |= alloc_pstate(&h->U, n);
-        st |= dalloc(&h->cellA, n); st |= dalloc(&h->velfin, n); st |= dalloc(&h->pterm, n);
+        st |= dalloc(&h->velfin, n); st |= dalloc(&h->pterm, n);
         st |= dalloc(&h->keyrank, n); st |= dalloc(&h->perm, n); st |= dalloc(&h->ncount, n);
         st |= dalloc(&h->f2tmp, n); st |= dalloc(&h->xhm, (size_t)n + kScanStep); st |= dalloc(&h->indv, n); st |= dalloc(&h->rho0, n);
         st |= dalloc(&h->xsv, n);
@@ -1418,6 +1423,10 @@ int finish_chunk(gfsph_handle* h, int chunk, double t_end, int& done, int& guard
     if (st) return st;
     done += h->hS->steps_done;
     h->searched = true;
+    if (h->hS->sparse && !h->sparse_seen) {
+        h->sparse_seen = true;
+        drop_graphs(h);
+    }
     if (h->hS->err) {
         if (++guard > 16) return GFSPH_ERR_CAPACITY;
         st = grow_after_error(h);

@@ -105,7 +105,6 @@ struct PState {
 struct Search {
     const int* bstart;   // block-map entry -> slot of its block (exclusive scan of the marks), nblocks+1
     const int* start;    // cell key -> first particle slot (exclusive scan), ncells+1
-    const int* cellA;    // slot -> cell key (all levels), -1 out of the domain
     const float4* xhm;   // slot -> (x, y, hsml, mass) at the start of the step
     // neighbour table of the regular particles (layout: tab_base): per entry
     // j, W_ij and its gradient, computed once per pair by the search, as
@@ -506,59 +505,51 @@ __device__ __forceinline__ int block_of(const StepScalars* S, int k, int cx, int
     return S->lev_boff[k] + (int)((unsigned)cy / kBlkY) * S->lev_nbx[k] + (int)((unsigned)cx / kBlkX);
 }
 
+// An exclusive scan before its tile offsets are added in (k_scan_tiles leaves
+// the scan of each tile and the scanned tile sums): entry i.
+struct TileScan {
+    const int* part;
+    const int* tile;
+    __device__ __forceinline__ int operator[](int i) const { return part[i] + tile[(unsigned)i / kScanTile]; }
+};
+
 // Sparse layout: the key of cell (cx, cy) of level k, block b.  The occupied
 // blocks of its block row (block-map entries rb .. rb + nbx - 1, slots f ..
 // f + nocc - 1) take 256 nocc keys from 256 f, cell row by cell row, 32 keys a
 // block in each.
-__device__ __forceinline__ int sparse_key(const StepScalars* S, const int* bstart, int k, int cx, int cy, int b) {
+__device__ __forceinline__ int sparse_key(const StepScalars* S, TileScan bstart, int k, int cx, int cy, int b) {
     const int nbx = S->lev_nbx[k], rb = S->lev_boff[k] + (int)((unsigned)cy / kBlkY) * nbx;
     const int f = bstart[rb], nocc = bstart[rb + nbx] - f;
     return f * kBlockCells + (int)((unsigned)cy % kBlkY) * (nocc * kBlkX) + (bstart[b] - f) * kBlkX +
            (int)((unsigned)cx % kBlkX);
 }
 
-// Marks the blocks that hold particles (block map, all levels) and takes the
-// largest smoothing length of every level, which bounds the stencils of the
-// neighbour search more tightly than the level's upper limit.
+// Marks the blocks that hold particles (block map, all levels; block-sparse
+// layout only).
 __global__ void k_mark(const PState B, int n, DemView dem, StepScalars* S, int* bmark) {
     PDL_ENTRY();
-    if (S->skip) return;
-    // per-level largest hsml, reduced in shared memory first: every particle
-    // of a level would otherwise hit the same global word
-    __shared__ unsigned int lmax[kMaxLevels];
-    const int nlev = S->nlev;
-    for (int k = threadIdx.x; k < nlev; k += blockDim.x) lmax[k] = 0u;
-    __syncthreads();
-    unsigned int h0 = 0u;  // largest level-0 hsml seen by this thread
+    if (S->skip || !S->sparse) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (B.flag[i]) continue;
         float2 p = B.pos[i];
         if (out_of_box(dem, p.x, p.y)) continue;
-        float hs = B.hsml[i];
-        int k = level_of(hs, S);
+        int k = level_of(B.hsml[i], S);
         int cx, cy;
         cell_of(p, S, k, cx, cy);
-        if (S->sparse) {
-            int b = block_of(S, k, cx, cy);
-            if (bmark[b] == 0) bmark[b] = 1;
-        }
-        if (k == 0) h0 = max(h0, f2o(hs));
-        else atomicMax(&lmax[k], f2o(hs));
+        int b = block_of(S, k, cx, cy);
+        if (bmark[b] == 0) bmark[b] = 1;
     }
-    h0 = __reduce_max_sync(0xffffffffu, h0);
-    if ((threadIdx.x & 31) == 0 && h0) atomicMax(&lmax[0], h0);
-    __syncthreads();
-    for (int k = threadIdx.x; k < nlev; k += blockDim.x)
-        if (lmax[k]) atomicMax(&S->lev_hmax_o[k], lmax[k]);
 }
 
 // Cell key (row-major in the dense layout, sparse_key in the sparse one) and
 // within-cell arrival rank of each particle (counting sort histogram,
-// grid_find :938-948); out-of-domain particles get key -1.  Clears the block
-// marks for the next step.  If the occupied blocks need more cells than the
-// histogram holds, nothing is counted and the step stops with kErrCells.
-__global__ void k_hist(const PState B, int n, DemView dem, StepScalars* S, int* bmark, const int* bstart, int* count,
-                       int2* keyrank, int cap_cells) {
+// grid_find :938-948); out-of-domain particles get key -1.  Also takes the
+// largest smoothing length of every level, which bounds the stencils of the
+// neighbour search more tightly than the level's upper limit.  If the
+// occupied blocks need more cells than the histogram holds, nothing is
+// counted and the step stops with kErrCells.
+__global__ void k_hist(const PState B, int n, DemView dem, StepScalars* S, TileScan bstart, int* count, int2* keyrank,
+                       int cap_cells) {
     PDL_ENTRY();
     if (S->skip) return;
     const bool sparse = S->sparse != 0;
@@ -569,21 +560,25 @@ __global__ void k_hist(const PState B, int n, DemView dem, StepScalars* S, int* 
         S->need_cells = (ncells + 1 > 0x3fffffffLL) ? 0x3fffffff : (int)(ncells + 1);
     }
     if (sparse && !over && blockIdx.x == 0 && threadIdx.x == 0) S->ncells = (int)ncells;
+    // per-level largest hsml, reduced in shared memory first: every particle
+    // of a level would otherwise hit the same global word
+    __shared__ unsigned int lmax[kMaxLevels];
+    const int nlev = S->nlev;
+    for (int k = threadIdx.x; k < nlev; k += blockDim.x) lmax[k] = 0u;
+    __syncthreads();
+    unsigned int h0 = 0u;  // largest level-0 hsml seen by this thread
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int2 kr = make_int2(-1, 0);
-        float2 p = B.pos[i];
+        const float2 p = B.pos[i];
+        const float hs = B.hsml[i];
         if (!B.flag[i] && !out_of_box(dem, p.x, p.y)) {
-            int k = level_of(B.hsml[i], S);
+            const int k = level_of(hs, S);
+            if (k == 0) h0 = max(h0, f2o(hs));
+            else atomicMax(&lmax[k], f2o(hs));
             int cx, cy;
             cell_of(p, S, k, cx, cy);
-            int key;
-            if (sparse) {
-                int b = block_of(S, k, cx, cy);
-                bmark[b] = 0;
-                key = sparse_key(S, bstart, k, cx, cy, b);
-            } else {
-                key = S->lev_off[k] + cy * S->lev_ndx[k] + cx;
-            }
+            const int key = sparse ? sparse_key(S, bstart, k, cx, cy, block_of(S, k, cx, cy))
+                                   : S->lev_off[k] + cy * S->lev_ndx[k] + cx;
             if (!over) {
                 kr.x = key;
                 kr.y = atomicAdd(&count[key], 1);
@@ -591,6 +586,11 @@ __global__ void k_hist(const PState B, int n, DemView dem, StepScalars* S, int* 
         }
         keyrank[i] = kr;
     }
+    h0 = __reduce_max_sync(0xffffffffu, h0);
+    if ((threadIdx.x & 31) == 0 && h0) atomicMax(&lmax[0], h0);
+    __syncthreads();
+    for (int k = threadIdx.x; k < nlev; k += blockDim.x)
+        if (lmax[k]) atomicMax(&S->lev_hmax_o[k], lmax[k]);
 }
 
 // Exclusive scan of the histogram, tile pass: each block scans kScanTile
@@ -638,10 +638,13 @@ __device__ void scan_tile_sums(int* tile_sum, int ntiles) {
 }
 
 // Scan of count[0 .. *nptr] into start (exclusive), tile by tile; the last
-// tile to finish also scans the tile sums (the tile offsets k_scan_add adds).
+// tile to finish also scans the tile sums.  The readers that come before
+// k_reorder add the tile offsets themselves (TileScan), k_reorder adds them in
+// for the rest of the step.  Zeroes the counts it has read, so that they start
+// at zero in the next step without a clearing pass.
 // which: 0 the cells, 1 the block map (only in the block-sparse layout).  A
 // step whose earlier kernels raised an error is stopped here.
-__global__ void k_scan_tiles(const int* count, int* start, int* tile_sum, const int* nptr, StepScalars* S,
+__global__ void k_scan_tiles(int* count, int* start, int* tile_sum, const int* nptr, StepScalars* S,
                              int which) {
     PDL_ENTRY();
     if (S->skip || (which == 1 && !S->sparse)) return;
@@ -656,12 +659,20 @@ __global__ void k_scan_tiles(const int* count, int* start, int* tile_sum, const 
     __shared__ int sh[kScanTile];
     __shared__ int wsum[kScanThreads / 32];
     __shared__ bool last;
-    for (int k = threadIdx.x; k < kScanTile; k += kScanThreads) {
-        int g = base + k;
-        sh[k] = (g < m) ? count[g] : 0;
+    constexpr int per = kScanTile / kScanThreads;
+    int v[per];  // all loads before the stores
+#pragma unroll
+    for (int k = 0; k < per; k++) {
+        const int g = base + k * kScanThreads + threadIdx.x;
+        v[k] = (g < m) ? count[g] : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < per; k++) {
+        const int g = base + k * kScanThreads + threadIdx.x;
+        sh[k * kScanThreads + threadIdx.x] = v[k];
+        if (g < m) count[g] = 0;
     }
     __syncthreads();
-    const int per = kScanTile / kScanThreads;
     int loc[per];
     int s = 0;
     for (int k = 0; k < per; k++) { loc[k] = s; s += sh[threadIdx.x * per + k]; }
@@ -702,22 +713,9 @@ __global__ void k_scan_tiles(const int* count, int* start, int* tile_sum, const 
     if (threadIdx.x == 0) S->scan_ticket[which] = 0u;
 }
 
-__global__ void k_scan_add(int* start, const int* tile_sum, const int* nptr, const StepScalars* S, int which) {
-    PDL_ENTRY();
-    if (S->skip || S->err || (which == 1 && !S->sparse)) return;
-    int m = *nptr + 1;
-    int base = blockIdx.x * kScanTile;
-    if (base >= m) return;
-    int add = tile_sum[blockIdx.x];
-    for (int k = threadIdx.x; k < kScanTile; k += blockDim.x) {
-        int g = base + k;
-        if (g < m) start[g] += add;
-    }
-}
-
 // Scatter (grid_find :952-958): particles to start[cell] + rank (level 0
 // first, then the higher levels), out-of-domain particles behind them.
-__global__ void k_scatter(const int2* keyrank, int n, const int* start, const int* bstart, StepScalars* S, int* perm) {
+__global__ void k_scatter(const int2* keyrank, int n, TileScan start, TileScan bstart, StepScalars* S, int* perm) {
     PDL_ENTRY();
     if (S->skip) return;
     int nact = start[S->ncells];
@@ -738,41 +736,34 @@ __global__ void k_scatter(const int2* keyrank, int n, const int* start, const in
     }
 }
 
-// Orders each cell's particles by original index, so the within-cell order,
-// hence every neighbour-sum order, is independent of atomic arrival order.
-__device__ __forceinline__ void insertion_sort_by_id(int* perm, const int* id_old, int a, int b) {
-    for (int k = a + 1; k < b; k++) {
-        int pk = perm[k];
-        int key = id_old[pk];
-        int m = k - 1;
-        while (m >= a && id_old[perm[m]] > key) { perm[m + 1] = perm[m]; m--; }
-        perm[m + 1] = pk;
-    }
-}
-
-// Also zeroes the histogram it no longer needs, so the counts start at zero
-// in the next step without a clearing pass.
-__global__ void k_cell_sort(int* perm, const int* id_old, const int* start, int* count, const StepScalars* S) {
-    PDL_ENTRY();
-    if (S->skip) return;
-    int nc = S->ncells;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
-        insertion_sort_by_id(perm, id_old, start[c], start[c + 1]);
-        count[c] = 0;
-    }
-}
-
-// Gathers the state into the new (cell-sorted) order.
-// With icpwp = 3 also the pore-water pressure; with icpwp = 3 or nor_density
-// rho0, the depth RK45 keeps at its start (after the h_inf clamp of
-// Adaptive_dt_sph_SW :6540, modes 1, 2 and 10).
-__global__ void k_reorder(const PState B, int n, const int* perm, const int2* keyrank, PState A, int* cellA,
+// Gathers the state into the new (cell-sorted) order, each cell's particles
+// ordered by original index, so that the within-cell order, hence every
+// neighbour-sum order, is independent of the atomics' arrival order: a
+// particle counts the members of its cell with a smaller index (a cell holds
+// one or two).  With icpwp = 3 also the pore-water pressure; with icpwp = 3 or
+// nor_density rho0, the depth RK45 keeps at its start (after the h_inf clamp
+// of Adaptive_dt_sph_SW :6540, modes 1, 2 and 10).  Also adds the tile offsets
+// into the cell starts (to startF, since other threads still read start) and
+// the block starts.
+__global__ void k_reorder(const PState B, int n, const int* perm, const int2* keyrank, PState A,
                           float4* xhm, const StepScalars* S, Rheo c, float* rho0, int2* rcell,
-                          const unsigned char* spec_u, unsigned char* spec_a) {
+                          const unsigned char* spec_u, unsigned char* spec_a, TileScan start, int* startF, int* bstart,
+                          const int* btile) {
     PDL_ENTRY();
     if (S->skip) return;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-        int o = perm[s];
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    const int nact = S->nactive;
+    for (int s0 = tid; s0 < n; s0 += nt) {
+        const int o = perm[s0];
+        int s = s0;
+        if (s0 < nact) {
+            const int key = keyrank[o].x, a = start[key], b = start[key + 1];
+            if (b - a > 1) {
+                const int me = B.id[o];
+                s = a;
+                for (int m = a; m < b; m++) s += (B.id[perm[m]] < me) ? 1 : 0;
+            }
+        }
         float2 p = B.pos[o];
         float hs = B.hsml[o], m = B.mass[o];
         float r = B.rho[o];
@@ -787,7 +778,6 @@ __global__ void k_reorder(const PState B, int n, const int* perm, const int2* ke
         A.flag[s] = B.flag[o];
         A.id[s] = B.id[o];
         if (c.ws) spec_a[s] = spec_u[B.id[o]];
-        cellA[s] = keyrank[o].x;
         xhm[s] = make_float4(p.x, p.y, hs, m);
         if (rcell && !B.flag[o]) {  // cell of the reference's grid (:1203-1204)
             int ix = (int)((p.x - S->ref_xmin) / S->ref_delt + 1.f);
@@ -795,6 +785,9 @@ __global__ void k_reorder(const PState B, int n, const int* perm, const int2* ke
             rcell[s] = make_int2(min(ix, S->ref_ndx), min(iy, S->ref_ndy));
         }
     }
+    const int nc = S->ncells, nb = S->sparse ? S->nblocks : -1;
+    for (int k = tid; k <= nc; k += nt) startF[k] = start[k];
+    for (int k = tid; k <= nb; k += nt) bstart[k] += btile[(unsigned)k / kScanTile];
 }
 
 // Largest neighbour distance against a level whose hsml <= Hk:
