@@ -21,17 +21,17 @@ using namespace gfsph;
 namespace {
 
 enum KernelId {
-    K_PREP, K_BOUNDS, K_HIST, K_SCAN_TILES, K_SCATTER, K_REORDER, K_DENSITY, K_DENSITY_BIG, K_IFORCE, K_FORCE_BIG, K_FORCE_RK, K_XSPH, K_XSPH_BIG, K_DEM_ERODE,
+    K_PREP, K_BOUNDS, K_HIST, K_SCAN_TILES, K_SCATTER, K_REORDER, K_DENSITY, K_DENSITY_BIG, K_IFORCE, K_FORCE_RK, K_XSPH, K_DEM_ERODE,
     K_STEP_END, K_COPY, K_UNSORT, K_RASTER, K_HAZARD, K_EXPORT, K_MARK, K_BSCAN_TILES,
-    K_DENSITY_SPARSE, K_COUPLE, K_ADJOINT, K_NORM, K_NORM_BIG, K_STAGE, K_WIR,
+    K_DENSITY_SPARSE, K_COUPLE, K_ADJOINT, K_NORM, K_STAGE, K_WIR,
     K_STEPS,  // not a kernel: device time of whole gfsph_step batches (profile level 2)
     K_COUNT
 };
 const char* kKernelNames[K_COUNT] = {
-    "k_prep", "k_bounds", "k_hist", "k_scan_tiles", "k_scatter", "k_reorder", "k_density", "k_density_big", "k_iforce", "k_force_big",
-    "k_force_rk", "k_xsph", "k_xsph_big", "k_dem_erode", "k_step_end", "k_copy_state", "k_unsort",
+    "k_prep", "k_bounds", "k_hist", "k_scan_tiles", "k_scatter", "k_reorder", "k_density", "k_density_big", "k_iforce",
+    "k_force_rk", "k_xsph", "k_dem_erode", "k_step_end", "k_copy_state", "k_unsort",
     "k_raster_idw", "k_hazard", "k_export_big", "k_mark", "k_scan_tiles(blocks)",
-    "k_density(sparse)", "k_couple", "k_adjoint", "k_norm", "k_norm_big", "k_stage", "k_wir", "step_batches"};
+    "k_density(sparse)", "k_couple", "k_adjoint", "k_norm", "k_stage", "k_wir", "step_batches"};
 
 constexpr int kThreads = 128;
 static_assert(kThreads <= 32 * kScatterWarps, "erosion_scatter keeps shared terms for kScatterWarps warps");
@@ -138,7 +138,7 @@ struct gfsph_handle {
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream2 = nullptr;       // side stream used only inside graph captures
-    cudaEvent_t ev_fork[3]{}, ev_join[3]{};
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     bool capturing = false;
     gfsph_params P;
     Rheo rheo;
@@ -170,6 +170,7 @@ struct gfsph_handle {
     // staged RK45 (nor_density or ic_cosTheta = 1)
     StageCarry carry{};
     float* rhoS = nullptr;   // the five depths of a step, k-major (nor_density)
+    float* ratio = nullptr;  // m/h of the call before, two halves (nor_density)
     int2* rcell = nullptr;   // cell of the reference's grid per slot (skf 2, 3)
     float4* xsv = nullptr;   // (vx, vy, h, m) per slot after the RK update, for av_vel
     // soil and water (ic_ws_Interact = 1): material per caller index and per
@@ -324,16 +325,16 @@ void with_pair_lanes(int n, F&& f) {
 // Stage-dependent pressure: the step runs the staged RK45 kernels.
 bool staged(const gfsph_handle* h) { return h->rheo.nor_density || h->rheo.cos_theta || h->rheo.ws; }
 
-void fork(gfsph_handle* h, int k) {
+void fork(gfsph_handle* h) {
     if (!h->capturing) return;
-    cudaEventRecord(h->ev_fork[k], h->stream);
-    cudaStreamWaitEvent(h->stream2, h->ev_fork[k], 0);
+    cudaEventRecord(h->ev_fork, h->stream);
+    cudaStreamWaitEvent(h->stream2, h->ev_fork, 0);
 }
 
-void join(gfsph_handle* h, int k) {
+void join(gfsph_handle* h) {
     if (!h->capturing) return;
-    cudaEventRecord(h->ev_join[k], h->stream2);
-    cudaStreamWaitEvent(h->stream, h->ev_join[k], 0);
+    cudaEventRecord(h->ev_join, h->stream2);
+    cudaStreamWaitEvent(h->stream, h->ev_join, 0);
 }
 
 // Particles the neighbour table has room for: whole warps (tab_base).
@@ -359,11 +360,14 @@ Search make_search(gfsph_handle* h) {
     q.gzw = h->gzw;
     q.bxy = h->bxy;
     q.mass0 = h->mass0_u;
+    q.ratio[0] = h->ratio;
+    q.ratio[1] = h->ratio ? h->ratio + h->n : nullptr;
     q.kcap = h->kcap;
     return q;
 }
 
-int big_blocks(const gfsph_handle*) { return 148 * 2; }  // a block of kBigThreads per coarse-level particle; most runs have few
+// Blocks of k_iforce, k_norm and k_xsph with `lanes` lanes per particle.
+int pair_blocks(int n, int lanes) { return kBigBlocks + blocks_for((long long)n * lanes, kBigThreads); }
 
 // The cell search: bounds, grid, counting sort, reorder, neighbours+density.
 // Returns the number of kernels enqueued.
@@ -396,17 +400,17 @@ int enqueue_search(gfsph_handle* h, int advance) {
     });
     launch(h, K_SCATTER, [&] { pdl_launch(k_scatter, pb, kThreads, st, h->keyrank, n, cells, blocks, S, h->perm); });
     launch(h, K_REORDER, [&] {
-        pdl_launch(k_reorder, pb, kThreads, st, h->B, n, h->perm, h->keyrank, h->A, h->xhm, S, h->rheo, h->rho0,
+        pdl_launch(k_reorder, pb, kThreads, st, h->B, n, h->perm, h->keyrank, h->A, h->xhm, S, h->rheo, h->rho0, h->ratio,
                    h->rcell, h->spec_u, h->spec_a, cells, h->startF, h->bstart, h->btile_sum);
     });
     nk += 6;
     // the coarse-level kernels run beside the regular ones when graphs are
     // captured (side stream); serially otherwise
     cudaStream_t side = side_stream(h);
-    fork(h, 0);
+    fork(h);
     with_skf(h, [&](auto sk) {
         constexpr int SKF = decltype(sk)::value;
-        launch(h, K_DENSITY_BIG, [&] { pdl_launch(k_density_big<SKF>, big_blocks(h), kBigThreads, side, h->A, q, S, h->rheo); });
+        launch(h, K_DENSITY_BIG, [&] { pdl_launch(k_density_big<SKF>, kBigBlocks, kBigThreads, side, h->A, q, S, h->rheo); });
         // the two materials' pair types compiled in only when there are two
         with_lanes(n, [&](auto g) {
             constexpr int G = decltype(g)::value;
@@ -426,8 +430,27 @@ int enqueue_search(gfsph_handle* h, int advance) {
         });
     });
     nk += 3;
-    join(h, 0);
+    join(h);
     return nk;
+}
+
+// Call k of sum_density_Tools (k = 0 to 4) in a step with nor_density.
+void enqueue_norm(gfsph_handle* h, int k, const float* hp, float* hout, bool pdl) {
+    Search q = make_search(h);
+    const int n = h->n;
+    launch(h, K_NORM, [&] {
+        with_skf(h, [&](auto sk) {
+            with_pair_lanes(n, [&](auto g) {
+                constexpr int SKF = decltype(sk)::value, G = decltype(g)::value;
+                if (pdl)
+                    pdl_launch(k_norm<SKF, G>, pair_blocks(n, G), kBigThreads, h->stream, h->A, q, h->S, h->rheo, n, hp,
+                               k ? 1 : 0, hout, q.ratio[k & 1], q.ratio[(k + 1) & 1]);
+                else
+                    k_norm<SKF, G><<<pair_blocks(n, G), kBigThreads, 0, h->stream>>>(
+                        h->A, q, h->S, h->rheo, n, hp, k ? 1 : 0, hout, q.ratio[k & 1], q.ratio[(k + 1) & 1]);
+            });
+        });
+    });
 }
 
 // The five depths of a step with nor_density: call k of sum_density_Tools
@@ -435,32 +458,13 @@ int enqueue_search(gfsph_handle* h, int advance) {
 // the first (IntForces_SW ran in between).  Without nor_density every stage
 // uses the plain sum in A.rho.  Returns the number of kernels enqueued.
 int enqueue_norms(gfsph_handle* h, PState As[5]) {
-    const int n = h->n;
-    cudaStream_t st = h->stream;
-    const Rheo& c = h->rheo;
-    Search q = make_search(h);
-    int nk = 0;
     for (int k = 0; k < 5; k++) {
         As[k] = h->A;
-        if (c.nor_density) As[k].rho = h->rhoS + (size_t)k * n;
+        if (h->rheo.nor_density) As[k].rho = h->rhoS + (size_t)k * h->n;
     }
-    if (!c.nor_density) return 0;
-    for (int k = 0; k < 5; k++) {
-        const float* hp = k ? As[k - 1].rho : h->rho0;
-        const int clamp = k ? 1 : 0;
-        launch(h, K_NORM, [&] {
-            with_skf(h, [&](auto sk) {
-                pdl_launch(k_norm<decltype(sk)::value>, blocks_for(n), kThreads, st, h->A, q, h->S, c, n, hp, clamp, As[k].rho);
-            });
-        });
-        launch(h, K_NORM_BIG, [&] {
-            with_skf(h, [&](auto sk) {
-                pdl_launch(k_norm_big<decltype(sk)::value>, big_blocks(h), kBigThreads, st, h->A, q, h->S, c, hp, clamp, As[k].rho);
-            });
-        });
-        nk += 2;
-    }
-    return nk;
+    if (!h->rheo.nor_density) return 0;
+    for (int k = 0; k < 5; k++) enqueue_norm(h, k, k ? As[k - 1].rho : h->rho0, As[k].rho, true);
+    return 5;
 }
 
 // Pressure term of the first stage; with nor_density it takes the first
@@ -494,10 +498,7 @@ int enqueue_wir_stage(gfsph_handle* h, const PState As[5], int s) {
         pdl_launch(k_wir_nodes, blocks_for((long long)np, 256), 256, st, h->wir_acc, h->d_z, h->wir_hsz, np, S);
     });
     launch(h, K_WIR, [&] {
-        with_skf(h, [&](auto sk) {
-            pdl_launch(k_wir_press<decltype(sk)::value>, blocks_for(n), kThreads, st, h->A, q, S, c, h->dem, h->carry, s,
-                       As[s].rho, h->wir_hsz);
-        });
+        pdl_launch(k_wir_press, blocks_for(n), kThreads, st, h->A, q, S, c, h->dem, h->carry, s, As[s].rho, h->wir_hsz);
     });
     return 3;
 }
@@ -514,29 +515,20 @@ int enqueue_stages(gfsph_handle* h, PState As[5]) {
     const int pb = blocks_for(n);
     int nk = enqueue_norms(h, As);
     if (c.ws) {
-        with_skf(h, [&](auto sk) {
-            launch(h, K_WIR, [&] {
-                pdl_launch(k_wir_pairs_big<decltype(sk)::value>, big_blocks(h), kBigThreads, st, h->A, q, S, c);
-            });
-        });
-        nk += 1 + enqueue_wir_stage(h, As, 0);
+        nk += enqueue_wir_stage(h, As, 0);
     } else {
         nk += enqueue_stage_begin(h, As);
     }
     for (int s = 0; s < 4; s++) {
-        launch(h, K_FORCE_BIG, [&] {
-            with_skf(h, [&](auto sk) { pdl_launch(k_force_big<decltype(sk)::value>, big_blocks(h), kBigThreads, st, As[s], q, S, c); });
-        });
-        nk++;
         launch(h, K_IFORCE, [&] {
             with_skf(h, [&](auto sk) {
                 with_pair_lanes(n, [&](auto g) {
                     constexpr int G = decltype(g)::value;
-                    const int fb = blocks_for((long long)n * G);
-                    if (c.ws)
-                        pdl_launch(k_iforce<decltype(sk)::value, true, G>, fb, kThreads, st, As[s], q, S, c, n);
+                    const int fb = pair_blocks(n, G);
+                    if (c.ws)  // the first stage also sums the soil-water pairs
+                        pdl_launch(k_iforce<decltype(sk)::value, true, G>, fb, kBigThreads, st, As[s], q, S, c, n, s == 0 ? 1 : 0);
                     else
-                        pdl_launch(k_iforce<decltype(sk)::value, false, G>, fb, kThreads, st, As[s], q, S, c, n);
+                        pdl_launch(k_iforce<decltype(sk)::value, false, G>, fb, kBigThreads, st, As[s], q, S, c, n, 0);
                 });
             });
         });
@@ -578,6 +570,23 @@ int enqueue_step_end(gfsph_handle* h) {
     return 1;
 }
 
+// av_vel with the depths of A.
+void enqueue_xsph(gfsph_handle* h, const PState& A) {
+    Search q = make_search(h);
+    const int n = h->n;
+    launch(h, K_XSPH, [&] {
+        with_skf(h, [&](auto sk) {
+            with_pair_lanes(n, [&](auto g) {
+                constexpr int SKF = decltype(sk)::value, G = decltype(g)::value;
+                if (h->rheo.ws)
+                    pdl_launch(k_xsph<SKF, true, G>, pair_blocks(n, G), kBigThreads, h->stream, A, q, h->S, h->rheo, n, h->B);
+                else
+                    pdl_launch(k_xsph<SKF, false, G>, pair_blocks(n, G), kBigThreads, h->stream, A, q, h->S, h->rheo, n, h->B);
+            });
+        });
+    });
+}
+
 // Enqueues one step; returns the number of kernels it enqueued (not a
 // status: a failed launch surfaces through cudaGetLastError, which every
 // caller checks after the enqueue or the capture).
@@ -592,43 +601,21 @@ int enqueue_step(gfsph_handle* h) {
         PState As[5];
         nk += enqueue_stages(h, As);
         if (h->rheo.av_vel) {  // av_vel with the final depth
-            launch(h, K_XSPH_BIG, [&] {
-                with_skf(h, [&](auto sk) {
-                    pdl_launch(k_xsph_big<decltype(sk)::value>, big_blocks(h), kBigThreads, st, As[4], q, S, h->rheo, h->B);
-                });
-            });
-            launch(h, K_XSPH, [&] {
-                with_pair_lanes(n, [&](auto g) {
-                    constexpr int G = decltype(g)::value;
-                    const int fb = blocks_for((long long)n * G);
-                    if (h->rheo.ws)
-                        pdl_launch(k_xsph<true, G>, fb, kThreads, st, As[4], q, S, h->rheo, n, h->B);
-                    else
-                        pdl_launch(k_xsph<false, G>, fb, kThreads, st, As[4], q, S, h->rheo, n, h->B);
-                });
-            });
-            nk += 2;
+            enqueue_xsph(h, As[4]);
+            nk++;
         }
         nk += enqueue_step_end(h);
         return nk;
     }
-    cudaStream_t sb = side_stream(h);
-    fork(h, 1);
-    launch(h, K_FORCE_BIG, [&] {
-        with_skf(h, [&](auto sk) { pdl_launch(k_force_big<decltype(sk)::value>, big_blocks(h), kBigThreads, sb, h->A, q, S, h->rheo); });
-    });
-    nk++;
     launch(h, K_IFORCE, [&] {
         with_skf(h, [&](auto sk) {
             with_pair_lanes(n, [&](auto g) {
                 constexpr int G = decltype(g)::value;
-                pdl_launch(k_iforce<decltype(sk)::value, false, G>, blocks_for((long long)n * G), kThreads, st, h->A, q, S,
-                           h->rheo, n);
+                pdl_launch(k_iforce<decltype(sk)::value, false, G>, pair_blocks(n, G), kBigThreads, st, h->A, q, S, h->rheo, n, 0);
             });
         });
     });
     nk++;
-    join(h, 1);
     launch(h, K_FORCE_RK, [&] {
         const Rheo& c = h->rheo;
         const bool gen = !(c.nfric == 4 || (c.nfric >= 5 && c.nfric <= 8) || c.nfric == 26 || c.nfric == 27) ||
@@ -638,21 +625,8 @@ int enqueue_step(gfsph_handle* h) {
         pdl_launch(kf, pb, kThreads, st, h->A, q, S, h->rheo, h->dem, n, h->B, h->velfin, h->d_auxv, 0, nullptr);
     }); nk++;
     if (h->rheo.av_vel) {
-        fork(h, 2);
-        launch(h, K_XSPH_BIG, [&] {
-            with_skf(h, [&](auto sk) {
-                pdl_launch(k_xsph_big<decltype(sk)::value>, big_blocks(h), kBigThreads, sb, h->A, q, S, h->rheo, h->B);
-            });
-        });
+        enqueue_xsph(h, h->A);
         nk++;
-        launch(h, K_XSPH, [&] {
-            with_pair_lanes(n, [&](auto g) {
-                constexpr int G = decltype(g)::value;
-                pdl_launch(k_xsph<false, G>, blocks_for((long long)n * G), kThreads, st, h->A, q, S, h->rheo, n, h->B);
-            });
-        });
-        nk++;
-        join(h, 2);
     }
     nk += enqueue_step_end(h);
     return nk;
@@ -681,11 +655,11 @@ int build_graph(gfsph_handle* h, int steps, cudaGraphExec_t* out) {
 }
 
 int kernels_per_step(const gfsph_handle* h) {
-    // staged: 10 k_norm launches with nor_density, k_stage_begin (with soil
-    // and water: k_wir_pairs_big and per stage k_wir_scatter, k_wir_nodes,
-    // k_wir_press), four stages of (k_force_big, k_iforce, k_stage)
-    const int body = staged(h) ? (h->rheo.nor_density ? 10 : 0) + (h->rheo.ws ? 13 : 1) + 12 : 3;
-    return 10 + body + (h->rheo.av_vel ? 2 : 0) + 1;
+    // search 10; staged: 5 k_norm launches with nor_density, k_stage_begin
+    // (with soil and water per stage k_wir_scatter, k_wir_nodes, k_wir_press),
+    // four stages of (k_iforce, k_stage); else k_iforce, k_force_rk
+    const int body = staged(h) ? (h->rheo.nor_density ? 5 : 0) + (h->rheo.ws ? 12 : 1) + 8 : 2;
+    return 10 + body + (h->rheo.av_vel ? 1 : 0) + 1;
 }
 
 // The three buffer (re)allocations below drop the graphs (which hold the old
@@ -746,7 +720,7 @@ void free_particles(gfsph_handle* h) {
     dfree(h->velfin); dfree(h->pterm); dfree(h->keyrank); dfree(h->perm); dfree(h->ncount);
     dfree(h->nbr); dfree(h->f2tmp); dfree(h->xhm); dfree(h->indv); dfree(h->rho0);
     dfree(h->carry.v); dfree(h->carry.acc); dfree(h->carry.dx); dfree(h->carry.dv); dfree(h->carry.xo);
-    dfree(h->carry.out); dfree(h->carry.u); dfree(h->carry.du); dfree(h->carry.Du); dfree(h->rhoS); dfree(h->rcell); dfree(h->xsv);
+    dfree(h->carry.out); dfree(h->carry.u); dfree(h->carry.du); dfree(h->carry.Du); dfree(h->rhoS); dfree(h->ratio); dfree(h->rcell); dfree(h->xsv);
     dfree(h->spec_u); dfree(h->spec_a); dfree(h->zpw); dfree(h->gzw); dfree(h->bxy);
     dfree(h->mass0_u);
     h->kcap = 0;
@@ -1036,10 +1010,8 @@ int create_handle(const gfsph_params* p, const gfsph_dem* dem, gfsph_handle* sha
         delete h;
         return GFSPH_ERR_CUDA;
     }
-    for (int k = 0; k < 3; k++) {
-        cudaEventCreateWithFlags(&h->ev_fork[k], cudaEventDisableTiming);
-        cudaEventCreateWithFlags(&h->ev_join[k], cudaEventDisableTiming);
-    }
+    cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming);
     h->P = *p;
     Rheo& c = h->rheo;
     const float* k = p->cst;  // k[i-1] = const(i)
@@ -1205,10 +1177,8 @@ int gfsph_destroy(gfsph_handle* h) try {
         if (h->ev0[k]) cudaEventDestroy(h->ev0[k]);
         if (h->ev1[k]) cudaEventDestroy(h->ev1[k]);
     }
-    for (int k = 0; k < 3; k++) {
-        if (h->ev_fork[k]) cudaEventDestroy(h->ev_fork[k]);
-        if (h->ev_join[k]) cudaEventDestroy(h->ev_join[k]);
-    }
+    if (h->ev_fork) cudaEventDestroy(h->ev_fork);
+    if (h->ev_join) cudaEventDestroy(h->ev_join);
     if (h->stream2) cudaStreamDestroy(h->stream2);
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
     delete h;
@@ -1255,7 +1225,7 @@ int gfsph_upload(gfsph_handle* h, int n, const float* x, const float* v, const f
             st |= dalloc(&C.v, n); st |= dalloc(&C.acc, n); st |= dalloc(&C.dx, n); st |= dalloc(&C.dv, n);
             st |= dalloc(&C.xo, n); st |= dalloc(&C.out, n);
             if (h->rheo.icpwp == 1) { st |= dalloc(&C.u, n); st |= dalloc(&C.du, n); st |= dalloc(&C.Du, n); }
-            if (h->rheo.nor_density) st |= dalloc(&h->rhoS, 5 * (size_t)n);
+            if (h->rheo.nor_density) { st |= dalloc(&h->rhoS, 5 * (size_t)n); st |= dalloc(&h->ratio, 2 * (size_t)n); }
         }
         if (h->rheo.skf == 2 || h->rheo.skf == 3) st |= dalloc(&h->rcell, n);
         if (h->rheo.ws) {
@@ -1268,7 +1238,7 @@ int gfsph_upload(gfsph_handle* h, int n, const float* x, const float* v, const f
         if (st) return drop_state(h, st);
     }
     if (h->cap_cells == 0) {
-        int st = alloc_cells(h, 1 << 18);
+        int st = alloc_cells(h, (int)std::min<long long>(std::max<long long>(1 << 18, 4LL * n), kMaxCells));  // seldom outgrown
         if (st) return drop_state(h, st);
         set_field<int>(h, offsetof(StepScalars, ncells), 0);
     }
@@ -1489,19 +1459,7 @@ int gfsph_density(gfsph_handle* h, float* rho_out) try {
     if (st) return st;
     int n = h->n;
     if (h->rheo.nor_density) {  // the first call of the step: normalised with the depths held
-        Search q = make_search(h);
-        launch(h, K_NORM, [&] {
-            with_skf(h, [&](auto sk) {
-                k_norm<decltype(sk)::value><<<blocks_for(n), kThreads, 0, h->stream>>>(h->A, q, h->S, h->rheo, n, h->rho0, 0,
-                                                                                   h->rhoS);
-            });
-        });
-        launch(h, K_NORM_BIG, [&] {
-            with_skf(h, [&](auto sk) {
-                k_norm_big<decltype(sk)::value><<<big_blocks(h), kBigThreads, 0, h->stream>>>(h->A, q, h->S, h->rheo, h->rho0, 0,
-                                                                                     h->rhoS);
-            });
-        });
+        enqueue_norm(h, 0, h->rho0, h->rhoS, false);
         CK(cudaMemcpyAsync(h->A.rho, h->rhoS, (size_t)n * sizeof(float), cudaMemcpyDeviceToDevice, h->stream));
     }
     launch(h, K_COPY, [&] { k_copy_state<<<blocks_for(n), kThreads, 0, h->stream>>>(h->A, h->B, n); });
@@ -1530,13 +1488,10 @@ int gfsph_internal_forces(gfsph_handle* h, float* indvxdt) try {
     launch(h, K_IFORCE, [&] {
         with_skf(h, [&](auto sk) {
             if (h->rheo.ws)
-                k_iforce<decltype(sk)::value, true, 1><<<blocks_for(n), kThreads, 0, s>>>(As[0], q, h->S, h->rheo, n);
+                k_iforce<decltype(sk)::value, true, 1><<<pair_blocks(n, 1), kBigThreads, 0, s>>>(As[0], q, h->S, h->rheo, n, 0);
             else
-                k_iforce<decltype(sk)::value, false, 1><<<blocks_for(n), kThreads, 0, s>>>(As[0], q, h->S, h->rheo, n);
+                k_iforce<decltype(sk)::value, false, 1><<<pair_blocks(n, 1), kBigThreads, 0, s>>>(As[0], q, h->S, h->rheo, n, 0);
         });
-    });
-    launch(h, K_FORCE_BIG, [&] {
-        with_skf(h, [&](auto sk) { k_force_big<decltype(sk)::value><<<big_blocks(h), kBigThreads, 0, s>>>(As[0], q, h->S, h->rheo); });
     });
     launch(h, K_FORCE_RK, [&] {
         k_force_rk<false, true><<<blocks_for(n), kThreads, 0, s>>>(h->A, q, h->S, h->rheo, h->dem, n, h->B,
@@ -1579,7 +1534,7 @@ int gfsph_neighbours(gfsph_handle* h, int cap, int* offsets, int* idx) try {
             Search q = make_search(h);
             launch(h, K_EXPORT, [&] {
                 with_skf(h, [&](auto sk) {
-                    k_export_big<decltype(sk)::value><<<big_blocks(h), kBigThreads, 0, h->stream>>>(q, h->S, dpairs, dcount, pcap);
+                    k_export_big<decltype(sk)::value><<<kBigBlocks, kBigThreads, 0, h->stream>>>(q, h->S, dpairs, dcount, pcap);
                 });
             });
             cudaStreamSynchronize(h->stream);

@@ -132,6 +132,10 @@ struct Search {
     float2* gzw;
     float2* bxy;
     const float* mass0;  // caller index -> mass at upload (nfric 3), else null
+    // nor_density: m/h per slot with the depth of the previous
+    // sum_density_Tools call, for the next one to gather; call k reads
+    // ratio[k & 1] and writes the other
+    float* ratio[2];
     int kcap;
 };
 
@@ -746,7 +750,7 @@ __global__ void k_scatter(const int2* keyrank, int n, TileScan start, TileScan b
 // into the cell starts (to startF, since other threads still read start) and
 // the block starts.
 __global__ void k_reorder(const PState B, int n, const int* perm, const int2* keyrank, PState A,
-                          float4* xhm, const StepScalars* S, Rheo c, float* rho0, int2* rcell,
+                          float4* xhm, const StepScalars* S, Rheo c, float* rho0, float* ratio0, int2* rcell,
                           const unsigned char* spec_u, unsigned char* spec_a, TileScan start, int* startF, int* bstart,
                           const int* btile) {
     PDL_ENTRY();
@@ -773,6 +777,7 @@ __global__ void k_reorder(const PState B, int n, const int* perm, const int2* ke
         if (c.icpwp != 0) A.pwp[s] = B.pwp[o];
         if (c.icpwp != 0 || c.nor_density)
             rho0[s] = ((c.ic_adapt == 1 || c.ic_adapt == 2 || c.ic_adapt == 10) && r < c.h_inf) ? c.h_inf : r;
+        if (c.nor_density) ratio0[s] = m / rho0[s];
         A.mass[s] = m;
         A.hsml[s] = hs;
         A.flag[s] = B.flag[o];
@@ -1103,6 +1108,7 @@ __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, S
 // row's candidates.  (With one warp each, the one with the longest list took
 // 38 us of the 200k flow's step in each of the three passes.)
 constexpr int kBigThreads = 256;
+constexpr int kBigBlocks = 148;  // the first blocks of k_iforce, k_norm and k_xsph take these particles, the others the regular ones
 template <bool SPARSE, int SK, class F>
 __device__ __forceinline__ void block_rows(const Search& Q, const StepScalars* S, int i, F& f) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1206,25 +1212,52 @@ __device__ __forceinline__ void pressure_pair(const Rheo& c, float pi_, float rh
     pressure_terms(c, pi_, rhoi, pj, rhoj, mj, d0, d1, a0, a1);
 }
 
-// Internal acceleration of the coarse-level particles, one block per particle.
-template <int SKF>
-__global__ void __launch_bounds__(kBigThreads) k_force_big(PState A, Search Q, StepScalars* S, Rheo c) {
-    PDL_ENTRY();
+// One soil-water pair term of ExtForces_SW (:8502-8521) for particle i from
+// its table entry (gradient d of W_ij with x_i - x_j): a soil particle gets
+// -dens_ws g m_j grad W; a water particle, with ic_SWalg = 0, +g m_j grad W
+// of the pair taken from the soil side (-d here).
+__device__ __forceinline__ void wir_pair_term(const Rheo& c, bool water, float mj, float d0, float d1, double& b0,
+                                              double& b1) {
+    if (!water) {
+        b0 -= (double)(((c.dens_ws * c.g) * mj) * d0);
+        b1 -= (double)(((c.dens_ws * c.g) * mj) * d1);
+    } else if (c.swalg == 0) {
+        b0 += (double)(-((c.g * mj) * d0));
+        b1 += (double)(-((c.g * mj) * d1));
+    }
+}
+
+// Internal acceleration of the coarse-level particles, one block per particle:
+// the first kBigBlocks blocks of k_iforce.
+template <int SKF, bool WS>
+__device__ __forceinline__ void force_big(const PState& A, const Search& Q, const StepScalars* S, const Rheo& c,
+                                          bool cross) {
     constexpr int SK = SupportScale<SKF>::value;
-    if (S->skip) return;
     const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
-        int i = nreg + b;
+    for (int b = blockIdx.x; b < nbig; b += kBigBlocks) {
+        const int i = nreg + b;
         const float pi_ = Q.pterm[i], rhoi = A.rho[i];
-        double a0 = 0.0, a1 = 0.0;
-        const unsigned char si = c.ws ? Q.spec[i] : 0;
+        double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
+        const unsigned char si = WS ? Q.spec[i] : 0;
         block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
-            if (c.ws && Q.spec[j] != si) return;  // type 0 only (:6899)
+            if (WS && Q.spec[j] != si) {  // type 0 only (:6899)
+                if (cross) {
+                    float w, d0, d1;
+                    sph_kernel<SKF>(g.r, g.dx0, g.dx1, g.mh, w, d0, d1);
+                    wir_pair_term(c, si == 2, o.w, d0, d1, b0, b1);
+                }
+                return;
+            }
             pressure_pair<SKF>(c, pi_, rhoi, Q.pterm[j], A.rho[j], o.w, g, a0, a1);
         });
         a0 = block_sum(a0);
         a1 = block_sum(a1);
         if (threadIdx.x == 0) Q.indv[i] = make_float2((float)a0, (float)a1);
+        if (WS && cross) {
+            b0 = block_sum(b0);
+            b1 = block_sum(b1);
+            if (threadIdx.x == 0) Q.bxy[i] = make_float2((float)b0, (float)b1);
+        }
     }
 }
 
@@ -1236,18 +1269,22 @@ __global__ void __launch_bounds__(kBigThreads) k_force_big(PState A, Search Q, S
 // valid in all of them.
 template <int SKF, bool WS, int G>
 __device__ __forceinline__ void internal_force(const Search& Q, const Rheo& c, const float* rho, float hmax, int i,
-                                               int gl, float& in0, float& in1) {
+                                               int gl, bool cross, float& in0, float& in1, float2& bxy) {
     const float4 me = __ldg(&Q.xhm[i]);
     const float2 xi = make_float2(me.x, me.y);
     const bool safe = quot_safe(me.z, hmax);
     const float pi_ = __ldg(&Q.pterm[i]), rhoi = rho[i];
-    double a0 = 0.0, a1 = 0.0;
+    double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
+    const bool water = WS && Q.spec[i] == 2;
     const int cnt = Q.ncount[i];
     const size_t tab = tab_base(i, Q.kcap);
-    auto term = [&](int j, const TabGrad<SKF>& g, const float4& o, float pj) {
+    // an entry of the particle's own material (type 0, :6899) or, with cross, of the other
+    auto term = [&](int e, const TabGrad<SKF>& g, const float4& o, float pj) {
+        if (WS && e < 0 && !cross) return;
         float d0, d1;
         g.grad(xi, o, safe, d0, d1);
-        pressure_terms(c, pi_, rhoi, pj, c.pa_sph == 1 ? rho[j] : 0.f, o.w, d0, d1, a0, a1);
+        if (WS && e < 0) wir_pair_term(c, water, o.w, d0, d1, b0, b1);
+        else pressure_terms(c, pi_, rhoi, pj, c.pa_sph == 1 ? rho[e] : 0.f, o.w, d0, d1, a0, a1);
     };
     // four entries at a time, the next four on their way meanwhile
     int k = gl;
@@ -1276,22 +1313,26 @@ __device__ __forceinline__ void internal_force(const Search& Q, const Rheo& c, c
         }
         if (k + 7 * G < cnt) fetch(k + 4 * G);
 #pragma unroll
-        for (int u = 0; u < 4; u++)
-            if (!WS || je[u] >= 0) term(je[u], gg[u], o[u], pj[u]);  // type 0 only (:6899)
+        for (int u = 0; u < 4; u++) term(je[u], gg[u], o[u], pj[u]);
     }
     for (; k < cnt; k += G) {
-        const int e = __ldg(Q.nj + tab + (size_t)k * kTabStride);
-        TabGrad<SKF> g;
-        g.load(Q, tab + (size_t)k * kTabStride);
-        if (!WS || e >= 0) term(e, g, __ldg(&Q.xhm[e]), __ldg(&Q.pterm[e]));
+        const int ek = __ldg(Q.nj + tab + (size_t)k * kTabStride), j = WS ? (ek & ~kCrossBit) : ek;
+        TabGrad<SKF> gk;
+        gk.load(Q, tab + (size_t)k * kTabStride);
+        term(ek, gk, __ldg(&Q.xhm[j]), __ldg(&Q.pterm[j]));
     }
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) {
         a0 += __shfl_xor_sync(0xffffffffu, a0, o);
         a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+        if (WS && cross) {
+            b0 += __shfl_xor_sync(0xffffffffu, b0, o);
+            b1 += __shfl_xor_sync(0xffffffffu, b1, o);
+        }
     }
     in0 = (float)a0;
     in1 = (float)a1;
+    bxy = make_float2((float)b0, (float)b1);
 }
 
 // DEM node box touched by the erosion scatter, kept per thread and reduced
@@ -1458,21 +1499,28 @@ __device__ __forceinline__ void rk_finish(const PState& A, const Search& Q, Step
     }
 }
 
-// Internal acceleration of the regular particles, G lanes each.  The
+// Internal acceleration: the coarse-level particles in the first kBigBlocks
+// blocks, the regular ones, G lanes each, in the others.  The
 // warps take the particles from the last to the first: the neighbour search
 // has just written the table front to back, so its last-written part (still
 // in L2) is read first, and av_vel, which walks the table front to back after
 // this pass, starts on the part this pass read last.
+// cross (soil and water, first stage): also the sums over the soil-water
+// pairs, from the same walk.
 template <int SKF, bool WS, int G>
-__global__ void __launch_bounds__(128) k_iforce(PState A, Search Q, StepScalars* S, Rheo c, int n) {
+__global__ void __launch_bounds__(kBigThreads, 4) k_iforce(PState A, Search Q, StepScalars* S, Rheo c, int n, int cross) {
     PDL_ENTRY();
     if (S->skip) return;
+    if (blockIdx.x < kBigBlocks) {
+        force_big<SKF, WS>(A, Q, S, c, cross != 0);
+        return;
+    }
     constexpr int P = 32 / G;  // particles per warp
     const int nreg = S->nreg;
     const float hmax = o2f(S->hmax_o);
     const int nw = (nreg + P - 1) / P;
-    const int lane = threadIdx.x & 31;
-    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nw; w += (gridDim.x * blockDim.x) >> 5) {
+    const int lane = threadIdx.x & 31, bid = blockIdx.x - kBigBlocks, nb = gridDim.x - kBigBlocks;
+    for (int w = (bid * kBigThreads + threadIdx.x) >> 5; w < nw; w += (nb * kBigThreads) >> 5) {
         const int i = (nw - 1 - w) * P + lane / G;
         if (G == 1) {
             const int rows = __reduce_max_sync(0xffffffffu, Q.ncount[min(i, nreg - 1)]);
@@ -1481,8 +1529,12 @@ __global__ void __launch_bounds__(128) k_iforce(PState A, Search Q, StepScalars*
             if (lane == 1 && rows <= Q.kcap) prefetch_rows(Q.ng + (SKF == 1 ? at : 2 * at), SKF == 1 ? rows : 2 * rows);
         }
         float in0, in1;
-        internal_force<SKF, WS, G>(Q, c, A.rho, hmax, min(i, nreg - 1), lane % G, in0, in1);
-        if (i < nreg && lane % G == 0) Q.indv[i] = make_float2(in0, in1);
+        float2 b;
+        internal_force<SKF, WS, G>(Q, c, A.rho, hmax, min(i, nreg - 1), lane % G, cross != 0, in0, in1, b);
+        if (i < nreg && lane % G == 0) {
+            Q.indv[i] = make_float2(in0, in1);
+            if (WS && cross) Q.bxy[i] = b;
+        }
     }
 }
 
@@ -1643,49 +1695,75 @@ __device__ __forceinline__ float prev_depth(const Rheo& c, const float* hp, int 
     float h = __ldg(hp + j);
     return (clamp_prev && h < c.h_inf) ? c.h_inf : h;
 }
-
-// One normalised sum_density_Tools call for the regular particles, over the
-// neighbour table: h_i = num_i / (W(0,h_i) m_i/hp_i + sum_j (m_j/hp_j) W_ij),
-// num_i the plain sum of k_density (in A.rho), hp the previous call's depths.
-template <int SKF>
-__global__ void __launch_bounds__(128) k_norm(PState A, Search Q, StepScalars* S, Rheo c, int n, const float* hp,
-                                              int clamp_prev, float* hout) {
-    PDL_ENTRY();
-    if (S->skip) return;
-    const int nreg = S->nreg;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nreg; i += gridDim.x * blockDim.x) {
-        const float4 me = Q.xhm[i];
-        const float hi = me.z;
-        double den = (double)((sph_kernel_w<SKF>(0.f, hi) * me.w) / prev_depth(c, hp, i, clamp_prev));
-        const int cnt = Q.ncount[i];
-        const size_t tab = tab_base(i, Q.kcap);
-        for (int k = 0; k < cnt; k++) {
-            const int j = __ldg(Q.nj + tab + (size_t)k * kTabStride);  // read again by the next calls of the step
-            den += (double)((__ldg(&A.mass[j]) / prev_depth(c, hp, j, clamp_prev)) * __ldg(Q.nw + tab + (size_t)k * kTabStride));
-        }
-        hout[i] = A.rho[i] / (float)den;
-    }
+// The end of a normalised sum for particle i: its depth, and m/h as the next
+// call gathers it (IntForces_SW has clamped the depth by then).
+__device__ __forceinline__ void norm_store(const PState& A, const Rheo& c, int i, float mass, double den, float* hout,
+                                           float* next) {
+    const float h = A.rho[i] / (float)den;
+    hout[i] = h;
+    next[i] = mass / ((h < c.h_inf) ? c.h_inf : h);
 }
 
-// The same for the coarse-level particles, one block each.
-template <int SKF>
-__global__ void __launch_bounds__(kBigThreads) k_norm_big(PState A, Search Q, StepScalars* S, Rheo c, const float* hp,
-                                                  int clamp_prev, float* hout) {
+// One normalised sum_density_Tools call: h_i = num_i / (W(0,h_i) m_i/hp_i +
+// sum_j (m_j/hp_j) W_ij), num_i the plain sum of k_density (in A.rho), hp the
+// previous call's depths; m_j/hp_j is gathered as the quotient that call left
+// (one division per particle instead of one per pair: 23 -> 9 us a call for
+// 60k particles, with four lanes a particle).  The coarse-level particles in
+// the first kBigBlocks blocks, the regular ones over the table in the others.
+template <int SKF, int G>
+__global__ void __launch_bounds__(kBigThreads, 5) k_norm(PState A, Search Q, StepScalars* S, Rheo c, int n, const float* hp,
+                                                      int clamp_prev, float* hout, const float* ratio, float* next) {
     PDL_ENTRY();
     constexpr int SK = SupportScale<SKF>::value;
     if (S->skip) return;
     const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
-        const int i = nreg + b;
+    if (blockIdx.x < kBigBlocks) {
+        for (int b = blockIdx.x; b < nbig; b += kBigBlocks) {
+            const int i = nreg + b;
+            double den = 0.0;
+            block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
+                den += (double)(__ldg(ratio + j) * sph_kernel_w<SKF>(g.r, g.mh));
+            });
+            den = block_sum(den);
+            if (threadIdx.x == 0) {
+                const float4 me = Q.xhm[i];
+                den = (double)((sph_kernel_w<SKF>(0.f, me.z) * me.w) / prev_depth(c, hp, i, clamp_prev)) + den;
+                norm_store(A, c, i, me.w, den, hout, next);
+            }
+        }
+        return;
+    }
+    constexpr int P = 32 / G;  // particles per warp
+    const int lane = threadIdx.x & 31, gl = lane % G, bid = blockIdx.x - kBigBlocks, nb = gridDim.x - kBigBlocks;
+    const int nw = (nreg + P - 1) / P;
+    for (int wp = (bid * kBigThreads + threadIdx.x) >> 5; wp < nw; wp += (nb * kBigThreads) >> 5) {
+        const int i0 = wp * P + lane / G, i = min(i0, nreg - 1);
+        const int cnt = Q.ncount[i];
+        const size_t tab = tab_base(i, Q.kcap);
         double den = 0.0;
-        block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
-            den += (double)((o.w / prev_depth(c, hp, j, clamp_prev)) * sph_kernel_w<SKF>(g.r, g.mh));
-        });
-        den = block_sum(den);
-        if (threadIdx.x == 0) {
+        int k = gl;
+        for (; k + 3 * G < cnt; k += 4 * G) {
+            int e[4];
+            float w[4], q[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                e[u] = __ldg(Q.nj + tab + (size_t)(k + u * G) * kTabStride);
+                w[u] = __ldg(Q.nw + tab + (size_t)(k + u * G) * kTabStride);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) q[u] = __ldg(ratio + e[u]);
+#pragma unroll
+            for (int u = 0; u < 4; u++) den += (double)(q[u] * w[u]);
+        }
+        for (; k < cnt; k += G)
+            den += (double)(__ldg(ratio + __ldg(Q.nj + tab + (size_t)k * kTabStride)) *
+                            __ldg(Q.nw + tab + (size_t)k * kTabStride));
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+        if (i0 < nreg && gl == 0) {
             const float4 me = Q.xhm[i];
             den = (double)((sph_kernel_w<SKF>(0.f, me.z) * me.w) / prev_depth(c, hp, i, clamp_prev)) + den;
-            hout[i] = A.rho[i] / (float)den;
+            norm_store(A, c, i, me.w, den, hout, next);
         }
     }
 }
@@ -1774,54 +1852,19 @@ __global__ void k_wir_nodes(double2* acc, const float* z, float* hsz, int np, co
     }
 }
 
-// One soil-water pair term of ExtForces_SW (:8502-8521) for particle i from
-// its table entry (gradient d of W_ij with x_i - x_j): a soil particle gets
-// -dens_ws g m_j grad W; a water particle, with ic_SWalg = 0, +g m_j grad W
-// of the pair taken from the soil side (-d here).
-__device__ __forceinline__ void wir_pair_term(const Rheo& c, bool water, float mj, float d0, float d1, double& b0,
-                                              double& b1) {
-    if (!water) {
-        b0 -= (double)(((c.dens_ws * c.g) * mj) * d0);
-        b1 -= (double)(((c.dens_ws * c.g) * mj) * d1);
-    } else if (c.swalg == 0) {
-        b0 += (double)(-((c.g * mj) * d0));
-        b1 += (double)(-((c.g * mj) * d1));
-    }
-}
-
 // Per active particle in stage s: at a water particle Z + hs of the soil
 // and its gradient, bilinear on its DEM cell (:17869-17933; a particle on the
 // far edge of the DEM takes the last cell); then the pressure term of the
 // stage (IntForces_SW :6793-6828): g/2 (h^2 - Zp^2) for the water with
-// ic_SWalg = 1, g/2 h^2 otherwise, h clamped to h_inf.  In stage 0 also the
-// soil-water pair sum of every regular particle, from its table.
-template <int SKF>
+// ic_SWalg = 1, g/2 h^2 otherwise, h clamped to h_inf.
 __global__ void __launch_bounds__(128) k_wir_press(PState A, Search Q, StepScalars* S, Rheo c, DemView dem,
                                                    StageCarry C, int s, const float* hdep, const float* hsz) {
     PDL_ENTRY();
     if (S->skip) return;
-    const int nact = S->nactive, nreg = S->nreg;
+    const int nact = S->nactive;
     const float dt = S->dt_step;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nact; i += gridDim.x * blockDim.x) {
         const bool water = Q.spec[i] == 2;
-        if (s == 0 && i < nreg) {
-            double b0 = 0.0, b1 = 0.0;
-            const int cnt = Q.ncount[i];
-            const size_t tab = tab_base(i, Q.kcap);
-            const float4 me = Q.xhm[i];
-            const bool safe = quot_safe(me.z, o2f(S->hmax_o));
-            for (int k = 0; k < cnt; k++) {
-                const int e = Q.nj[tab + (size_t)k * kTabStride];
-                if (e >= 0) continue;
-                const float4 o = Q.xhm[e & ~kCrossBit];
-                TabGrad<SKF> g;
-                g.load(Q, tab + (size_t)k * kTabStride);
-                float d0, d1;
-                g.grad(make_float2(me.x, me.y), o, safe, d0, d1);
-                wir_pair_term(c, water, o.w, d0, d1, b0, b1);
-            }
-            Q.bxy[i] = make_float2((float)b0, (float)b1);
-        }
         float2 p;
         if (!wir_stage_pos(A, C, s, dt, i, p) || out_of_box(dem, p.x, p.y)) continue;  // keeps its term
         float zp = 0.f;
@@ -1844,29 +1887,6 @@ __global__ void __launch_bounds__(128) k_wir_press(PState A, Search Q, StepScala
         const float hc = (h < c.h_inf) ? c.h_inf : h;
         const float p_ = (water && c.swalg == 1) ? c.cgra05 * (hc * hc - zp * zp) : (c.cgra05 * hc) * hc;
         Q.pterm[i] = (c.pa_sph == 1) ? p_ : p_ / (hc * hc);
-    }
-}
-
-// The soil-water pair sums of the coarse-level particles, one block each.
-template <int SKF>
-__global__ void __launch_bounds__(kBigThreads) k_wir_pairs_big(PState A, Search Q, StepScalars* S, Rheo c) {
-    PDL_ENTRY();
-    constexpr int SK = SupportScale<SKF>::value;
-    if (S->skip) return;
-    const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
-        const int i = nreg + b;
-        const unsigned char si = Q.spec[i];
-        double b0 = 0.0, b1 = 0.0;
-        block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
-            if (Q.spec[j] == si) return;
-            float w, d0, d1;
-            sph_kernel<SKF>(g.r, g.dx0, g.dx1, g.mh, w, d0, d1);
-            wir_pair_term(c, si == 2, o.w, d0, d1, b0, b1);
-        });
-        b0 = block_sum(b0);
-        b1 = block_sum(b1);
-        if (threadIdx.x == 0) Q.bxy[i] = make_float2((float)b0, (float)b1);
     }
 }
 
@@ -2029,17 +2049,48 @@ __device__ __forceinline__ void xsph_pair(float2 vi, float rhoi, float2 vj, floa
 }
 
 // av_vel (SPH_MAIN_2019.f90:3042-3099) with the start-of-step W_ij, then
-// v += 0.3*av for particles still inside the domain (:987-993); G lanes per
-// particle as in k_iforce.
-template <bool WS, int G>
-__global__ void __launch_bounds__(128) k_xsph(PState A, Search Q, StepScalars* S, Rheo c, int n, PState B) {
+// v += 0.3*av for particles still inside the domain (:987-993); the coarse
+// particles in the first kBigBlocks blocks, the regular ones, G lanes each as
+// in k_iforce, in the others.
+template <int SKF, bool WS>
+__device__ __forceinline__ void xsph_big(const Search& Q, const StepScalars* S, const PState& B) {
+    constexpr int SK = SupportScale<SKF>::value;
+    const int nreg = S->nreg, nbig = S->nbig;
+    for (int b = blockIdx.x; b < nbig; b += kBigBlocks) {
+        const int i = nreg + b;
+        if (B.flag[i]) continue;  // uniform over the block
+        const float4 si = Q.xsv[i];
+        const float2 vi = make_float2(si.x, si.y);
+        const float rhoi = si.z;
+        double a0 = 0.0, a1 = 0.0;
+        const unsigned char own = WS ? Q.spec[i] : 0;
+        block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
+            if (WS && Q.spec[j] != own) return;  // type 0 only (SPH_MAIN_2019.f90:3071)
+            const float4 sj = Q.xsv[j];
+            xsph_pair<SKF>(vi, rhoi, make_float2(sj.x, sj.y), sj.z, sj.w, g, a0, a1);
+        });
+        a0 = block_sum(a0);
+        a1 = block_sum(a1);
+        if (threadIdx.x == 0) {
+            const float av0 = 0.3f * (float)a0, av1 = 0.3f * (float)a1;
+            B.vel[i] = make_float2(vi.x + av0, vi.y + av1);
+        }
+    }
+}
+
+template <int SKF, bool WS, int G>
+__global__ void __launch_bounds__(kBigThreads, 4) k_xsph(PState A, Search Q, StepScalars* S, Rheo c, int n, PState B) {
     PDL_ENTRY();
     if (S->skip || !c.av_vel) return;
+    if (blockIdx.x < kBigBlocks) {
+        xsph_big<SKF, WS>(Q, S, B);
+        return;
+    }
     constexpr int P = 32 / G;  // particles per warp
     const int nreg = S->nreg;
-    const int lane = threadIdx.x & 31, gl = lane % G;
+    const int lane = threadIdx.x & 31, gl = lane % G, bid = blockIdx.x - kBigBlocks, nb = gridDim.x - kBigBlocks;
     const int nw = (nreg + P - 1) / P;
-    for (int wp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; wp < nw; wp += (gridDim.x * blockDim.x) >> 5) {
+    for (int wp = (bid * kBigThreads + threadIdx.x) >> 5; wp < nw; wp += (nb * kBigThreads) >> 5) {
         const int i0 = wp * P + lane / G, i = min(i0, nreg - 1);
         const float4 si = Q.xsv[i];
         const float2 vi = make_float2(si.x, si.y);
@@ -2094,34 +2145,6 @@ __global__ void __launch_bounds__(128) k_xsph(PState A, Search Q, StepScalars* S
         }
         const float av0 = 0.3f * (float)a0, av1 = 0.3f * (float)a1;
         if (go && gl == 0) B.vel[i] = make_float2(vi.x + av0, vi.y + av1);
-    }
-}
-
-template <int SKF>
-__global__ void __launch_bounds__(kBigThreads) k_xsph_big(PState A, Search Q, StepScalars* S, Rheo c, PState B) {
-    PDL_ENTRY();
-    constexpr int SK = SupportScale<SKF>::value;
-    if (S->skip || !c.av_vel) return;
-    const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
-        int i = nreg + b;
-        if (B.flag[i]) continue;  // uniform over the block
-        const float4 si = Q.xsv[i];
-        const float2 vi = make_float2(si.x, si.y);
-        const float rhoi = si.z;
-        double a0 = 0.0, a1 = 0.0;
-        const unsigned char si_ = c.ws ? Q.spec[i] : 0;
-        block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
-            if (c.ws && Q.spec[j] != si_) return;  // type 0 only (SPH_MAIN_2019.f90:3071)
-            const float4 sj = Q.xsv[j];
-            xsph_pair<SKF>(vi, rhoi, make_float2(sj.x, sj.y), sj.z, sj.w, g, a0, a1);
-        });
-        a0 = block_sum(a0);
-        a1 = block_sum(a1);
-        if (threadIdx.x == 0) {
-            float av0 = 0.3f * (float)a0, av1 = 0.3f * (float)a1;
-            B.vel[i] = make_float2(vi.x + av0, vi.y + av1);
-        }
     }
 }
 
