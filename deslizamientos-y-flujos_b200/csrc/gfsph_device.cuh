@@ -365,6 +365,37 @@ struct Rheo {
 // x**y for a real exponent, evaluated in FP64 and rounded once.
 __device__ __forceinline__ float powr(float x, float y) { return (float)pow((double)x, (double)y); }
 
+// Manning's h**(7./3.): powr(x, 7.f/3.f) of a positive normal x, the same
+// value, without the FP64 power in all but one of 10^4 cases.  With d =
+// fl(7/3) - 7/3, x^fl(7/3) = x^3 (x^(-1/3))^2 x^d; x^(-1/3) is rcbrtf refined
+// by the third-order series of (1 - e)^(-1/3), e = 1 - x r^3, and x^d = 1 + d
+// ln x + (d ln x)^2/2 with logf, since d is 8e-8.  Ziv's rounding test (A. Ziv,
+// "Fast evaluation of elementary mathematical functions with correctly rounded
+// last bit", ACM TOMS 17, 1991) keeps it where every value within 2^-36 of it
+// rounds alike, which is far above its error (2^-40) and pow's.
+__device__ __forceinline__ float pow73(float x) {
+    const double X = x, r0 = (double)rcbrtf(x);
+    const double e = 1.0 - X * (r0 * r0 * r0);
+    const double r = r0 + r0 * (e * (1.0 / 3.0 + e * (2.0 / 9.0 + e * (14.0 / 81.0))));
+    const double t = ((double)(7.f / 3.f) - 7.0 / 3.0) * (double)logf(x);
+    const double y = ((X * X) * X) * (r * r) * (1.0 + (t + 0.5 * t * t));
+    const double lim = 1.4551915228366852e-11;  // 2^-36
+    const float lo = (float)(y - y * lim), hi = (float)(y + y * lim);
+    return (lo == hi) ? lo : powr(x, 7.f / 3.f);
+}
+
+// a/b and c/b for b > 0, sharing a reciprocal where b allows it.
+__device__ __forceinline__ void quot2(float a, float c, float b, float& qa, float& qc) {
+    if (b > 1.e-18f && b < 1.e18f) {
+        const float y = recip(b);
+        qa = quot(a, b, y);
+        qc = quot(c, b, y);
+    } else {
+        qa = a / b;
+        qc = c / b;
+    }
+}
+
 // Locals of ExtForces_SW shared with its contained routines.
 struct ExtLocal {
     float h, hu, hv, hinv, vmod, hvmod, hvmodinv, frictx, fricty, totfrict, cf5, gravx, gravy;
@@ -473,17 +504,16 @@ __device__ __forceinline__ void grav_and_friction(const Rheo& c, const DemView& 
         }
         // the Manning friction (n = const(8)) where it is larger, per component
         const float cf1 = (c.g * c.m_vexp) * c.m_vexp;
-        const float p73 = powr(hfrict, 7.f / 3.f);
-        const float fxx = ((cf1 * L.hu) * L.hvmod) / p73, fyy = ((cf1 * L.hv) * L.hvmod) / p73;
+        const float p73 = pow73(hfrict);
+        float fxx, fyy;
+        quot2((cf1 * L.hu) * L.hvmod, (cf1 * L.hv) * L.hvmod, p73, fxx, fyy);
         if (fabsf(fxx) > fabsf(L.frictx)) L.frictx = fxx;
         if (fabsf(fyy) > fabsf(L.fricty)) L.fricty = fyy;
         L.totfrict = sqrtf(L.frictx * L.frictx + L.fricty * L.fricty);
     } else if (GEN && c.nfric == 1) {  // Newtonian turbulent (Manning n = const(3)), :9426-9430
         const float cf1 = (c.g * c.xi) * c.xi;
-        const float p73 = powr(hfrict, 7.f / 3.f);
-        L.frictx = ((cf1 * L.hu) * L.hvmod) / p73;
-        L.fricty = ((cf1 * L.hv) * L.hvmod) / p73;
-        L.totfrict = sqrtf(L.frictx * L.frictx + L.fricty * L.fricty);
+        quot2((cf1 * L.hu) * L.hvmod, (cf1 * L.hv) * L.hvmod, pow73(hfrict), L.frictx, L.fricty);
+        L.totfrict = root_any(L.frictx * L.frictx + L.fricty * L.fricty);
     } else if (GEN && c.nfric == 2) {  // Newtonian laminar, :9431-9437
         const float cf2a = c.constK / (8.f * c.dens);
         L.frictx = (cf2a * L.hu) / (hfrict * hfrict);
@@ -713,10 +743,8 @@ __device__ __forceinline__ void ext_accel_wir(const Rheo& c, const DemView& d, f
         L.gravy = -(c.g * zpy);
         const float hfrict = (L.h > c.hfrict0) ? L.h : c.hfrict0;
         const float cf1 = (c.g * c.xi) * c.xi;  // cmanning = const(3)
-        const float p73 = powr(hfrict, 7.f / 3.f);
-        L.frictx = ((cf1 * L.hu) * L.hvmod) / p73;
-        L.fricty = ((cf1 * L.hv) * L.hvmod) / p73;
-        L.totfrict = sqrtf(L.frictx * L.frictx + L.fricty * L.fricty);
+        quot2((cf1 * L.hu) * L.hvmod, (cf1 * L.hv) * L.hvmod, pow73(hfrict), L.frictx, L.fricty);
+        L.totfrict = root_any(L.frictx * L.frictx + L.fricty * L.fricty);
         L.cf5 = 0.f;
     } else {
         grav_and_friction<false>(c, d, xx, yy, vx, vy, 0.f, 0.f, L);

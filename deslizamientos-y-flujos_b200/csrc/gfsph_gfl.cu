@@ -12,13 +12,15 @@
 // the reference searches every element (the same sums in the same order).
 //
 // One step, five kernels (niter + 3 launches):
-//   k_gfl_nodes   fluxes and sources at the nodes (first_step :1890-1958);
+//   k_gfl_nodes   fluxes and sources at the nodes (first_step :1890-1958), two
+//                 float4 a node: (h, hu, hv, hu hv/h), (hu hu/h + p, hv hv/h + p,
+//                 the sources of hu and hv), all that the elements read;
 //   k_gfl_elems   per element: the half-step values at the Gauss points
 //                 (first_step :1964-2048), at each of them the fluxes and
 //                 sources of second_step (:2157-2300), and the term each
 //                 Gauss point adds to each of the element's nodes (:2300-2312),
-//                 one float4 per (element, node, Gauss point);
-//   k_gfl_rhs     per node, those terms gathered over its elements in element
+//                 written to the node's own place for that element;
+//   k_gfl_rhs     per node, those terms added over its elements in element
 //                 order (Gauss points in order), then its boundary sides in side
 //                 order, as second_step adds them (:2300-2355): the right-hand
 //                 side; the wall projection of solve (:2629-2656) and its first
@@ -26,6 +28,9 @@
 //   k_gfl_mass    the further sweeps u += (rhs - M u)/ML with the wall
 //                 filter (:2660-2785), M u gathered in element order;
 //   k_gfl_update  addthem (:3199-3215) and check (:3306-3345).
+// A node's places (one per element around it) are laid out by warps of 32
+// nodes: place k of node ip at slot[ip >> 5] + 32 k + (ip & 31), so that the
+// node kernels read place k of 32 nodes as one run, whatever the mesh.
 // Every sum runs in the Fortran's order with IEEE FP32 operations (the
 // library is built without FMA contraction), so the device step equals the
 // single-precision restatement bit for bit; real powers (Manning's 7/3,
@@ -39,11 +44,14 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <new>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "../../include/gfsph.h"
+#include "gfsph_device.cuh"
 
 namespace gfsph {
 namespace gfl {
@@ -58,14 +66,16 @@ struct GflConst {
 
 struct GflDev {
     int npoin, nelem;
-    const int* elem;       // (3, nelem) 0-based
-    const float* geome;    // (7, nelem): dN/dx (3), dN/dy (3), 2 * area
-    const float* topel;    // (9, nelem)
-    const float* topol;    // (9, npoin)
-    const float* mmatl;    // lumped mass
-    const int* adj_ptr;    // node -> (element, local node) entries, element order
-    const int2* adj;
-    const int* bside_ptr;  // node -> (boundary side, position in it), side order
+    const int4* el_nodes;    // element -> its nodes (0-based), and node 0's place for it
+    const int2* el_places;   // the places of nodes 1 and 2
+    const float4* el_geo;    // two per element: (dN/dx (3), dN/dy of node 0), (dN/dy of nodes 1 and 2, 2 * area, 0)
+    const float* topel;      // 9 rows of nelem
+    const float* topol;      // 9 rows of npoin
+    const float* mmatl;      // lumped mass
+    const int* slot;         // first place of each warp of nodes
+    const int* deg;          // elements around each node
+    const int4* place;       // place -> the element's nodes and the bits of 2 * area / 24
+    const int* bside_ptr;    // node -> (boundary side, position in it), side order
     const int2* bside;
     const int2* side_nodes;   // boundary side -> its two nodes
     const float4* side_geom;  // cosx, cosy, length
@@ -74,11 +84,11 @@ struct GflDev {
     const float* hs_w;        // WIR: soil depth at the nodes (or null)
     const float2* gradhs_w;   // WIR: its nodal gradient
     float* unkno;             // (3, npoin) h, hu, hv
-    float* fnode;             // (9, npoin): fluxp(3), fluyp(3), gpoin(3)
-    float4* gt;               // per element, local node and Gauss point (3 x 3 float4): the rhs terms of
-                              // second_step for h, hu, hv (w unused)
-    float* rhs1;              // (3, npoin)
-    float* rhs0[2];           // (3, npoin), double buffer of the sweeps
+    float4* fnode;            // two per node (see above)
+    float4 *gt0, *gt1;        // per place: the rhs terms of second_step for h, hu, hv, Gauss points in order:
+    float* gt2;               // nine floats as 4 + 4 + 1
+    float4* rhs1;             // per node: h, hu, hv
+    float4* rhs0[2];          // double buffer of the sweeps
 };
 
 // frictlaws (GFL_MAIN_2019.f90:3801-3990) with pwp = 0 and no wind or
@@ -87,22 +97,20 @@ __device__ __forceinline__ void frictlaws(const GflConst& c, float tanfi, const 
                                           float HH, float& frictx, float& fricty, float& slopx, float& slopy,
                                           float& correx, float& correy) {
     const float gtanfi = c.cgra * tanfi, gtanfi8 = c.cgra * c.tanfi8;
-    const double c73 = (double)(7.f / 3.f);
     float hinv = 0.f;
-    if (h > 0.f) hinv = 1.f / h;
+    if (h > 1.e-30f) hinv = recip(h);
+    else if (h > 0.f) hinv = 1.f / h;
     const float hfrict = fmaxf(h, c.hfrict0);
-    const float hvmod = sqrtf(hu * hu + hv * hv);
+    const float hvmod = root_any(hu * hu + hv * hv);
     const float vmod = hvmod * hinv;
     float hvmodinv = 0.f;
-    if (hvmod >= 1.e-5f) hvmodinv = 1.f / hvmod;
+    if (hvmod >= 1.e-5f) hvmodinv = recip(hvmod);
     const float pwp = 0.f;
     frictx = 0.f;
     fricty = 0.f;
     if (c.nfric == 1) {
         const float cf1 = (c.cgra * c.cmanning) * c.cmanning;
-        const float p = (float)pow((double)hfrict, c73);
-        frictx = ((cf1 * hu) * hvmod) / p;
-        fricty = ((cf1 * hv) * hvmod) / p;
+        quot2((cf1 * hu) * hvmod, (cf1 * hv) * hvmod, pow73(hfrict), frictx, fricty);
     } else if (c.nfric == 2) {
         const float cf2a = c.constK / (8.f * c.dens);
         frictx = (cf2a * hu) / (hfrict * hfrict);
@@ -158,9 +166,10 @@ __device__ __forceinline__ void frictlaws(const GflConst& c, float tanfi, const 
     }
     if (c.cmanning != 0.f && c.nfric != 1) {
         const float cf1 = (c.cgra * c.cmanning) * c.cmanning;
-        const float p = (float)pow((double)hfrict, c73);
-        frictx = frictx + ((cf1 * hu) * hvmod) / p;
-        fricty = fricty + ((cf1 * hv) * hvmod) / p;
+        float fx, fy;
+        quot2((cf1 * hu) * hvmod, (cf1 * hv) * hvmod, pow73(hfrict), fx, fy);
+        frictx = frictx + fx;
+        fricty = fricty + fy;
     }
     slopx = -((c.cgra * (h - HH)) * mt[1]);
     slopy = -((c.cgra * (h - HH)) * mt[2]);
@@ -180,37 +189,63 @@ __device__ __forceinline__ void sources(const GflConst& c, float frx, float fry,
     }
 }
 
-__global__ void k_gfl_nodes(GflDev d, GflConst c, float tanfi) {
+// The kernels of the steps run one after another in one stream; each waits
+// for the one before it and lets the next be set up meanwhile (programmatic
+// dependent launch).
+#define GFL_ENTRY()                                              \
+    do {                                                         \
+        asm volatile("griddepcontrol.wait;" ::: "memory");       \
+        asm volatile("griddepcontrol.launch_dependents;" :::);   \
+    } while (0)
+
+// Rows 1 to 8 of the topography of a node or element as frictlaws reads them:
+// the slopes only under a still-water level (sources drops the slope term
+// over a dry bed), the others only in the v^2/R laws.
+__device__ __forceinline__ void topo_rows(const GflConst& c, const float* rows, size_t stride, size_t i, float mt[9]) {
+#pragma unroll
+    for (int k = 0; k < 9; k++) mt[k] = 0.f;
+    if (c.ntype == 2) {
+        mt[1] = rows[stride + i];
+        mt[2] = rows[2 * stride + i];
+    }
+    if (c.nfric == 7 || c.nfric == 8) {
+#pragma unroll
+        for (int k = 3; k < 9; k++) mt[k] = rows[k * stride + i];
+    }
+}
+
+__global__ void __launch_bounds__(kGflThreads) k_gfl_nodes(GflDev d, GflConst c, float tanfi) {
+    GFL_ENTRY();
     for (int ip = blockIdx.x * blockDim.x + threadIdx.x; ip < d.npoin; ip += gridDim.x * blockDim.x) {
-        const float h = d.unkno[3 * ip], hu = d.unkno[3 * ip + 1], hv = d.unkno[3 * ip + 2];
+        const float h = d.unkno[3 * (size_t)ip], hu = d.unkno[3 * (size_t)ip + 1], hv = d.unkno[3 * (size_t)ip + 2];
         float hinv = 0.f;
-        if (h >= c.comp) hinv = 1.f / h;
+        if (h >= c.comp) hinv = (h > 1.e-30f) ? recip(h) : 1.f / h;
         float HH, pres;
         if (c.ntype == 2) {
-            HH = c.swl - d.topol[9 * ip];
+            HH = c.swl - d.topol[ip];
             if (d.hs_w) HH = HH - d.hs_w[ip];
             pres = (0.5f * c.cgra) * (h * h - HH * HH);
         } else {
             HH = 0.f;
             pres = ((0.5f * c.cgra) * h) * h;
         }
-        float* f = d.fnode + 9 * (size_t)ip;
-        f[0] = hu; f[1] = (hu * hu) * hinv + pres; f[2] = (hu * hv) * hinv;
-        f[3] = hv; f[4] = (hu * hv) * hinv; f[5] = (hv * hv) * hinv + pres;
         float mt[9];
-        for (int k = 0; k < 9; k++) mt[k] = d.topol[9 * (size_t)ip + k];
+        topo_rows(c, d.topol, d.npoin, ip, mt);
         if (d.hs_w) { mt[1] = mt[1] + d.gradhs_w[ip].x; mt[2] = mt[2] + d.gradhs_w[ip].y; }
-        float frx, fry, slx, sly, cx, cy;
+        float frx, fry, slx, sly, cx, cy, src[3];
         frictlaws(c, tanfi, mt, h, hu, hv, HH, frx, fry, slx, sly, cx, cy);
-        sources(c, frx, fry, slx, sly, cx, cy, hu, hv, f + 6);
+        sources(c, frx, fry, slx, sly, cx, cy, hu, hv, src);
+        d.fnode[2 * (size_t)ip] = make_float4(h, hu, hv, (hu * hv) * hinv);
+        d.fnode[2 * (size_t)ip + 1] = make_float4((hu * hu) * hinv + pres, (hv * hv) * hinv + pres, src[1], src[2]);
     }
 }
 
-__device__ __forceinline__ void gauss_point(int ngaus, int ig, float sh[3]) {
-    if (ngaus == 3) {
-        const float p1[3] = {1.0f / 6.0f, 4.0f / 6.0f, 1.0f / 6.0f}, p2[3] = {1.0f / 6.0f, 1.0f / 6.0f, 4.0f / 6.0f};
-        sh[0] = p1[ig];
-        sh[1] = p2[ig];
+// Shape functions at Gauss point ig of NG.
+template <int NG>
+__device__ __forceinline__ void gauss_point(int ig, float sh[3]) {
+    if (NG == 3) {
+        sh[0] = (ig == 1) ? 4.0f / 6.0f : 1.0f / 6.0f;
+        sh[1] = (ig == 2) ? 4.0f / 6.0f : 1.0f / 6.0f;
     } else {
         sh[0] = 1.0f / 3.0f;
         sh[1] = 1.0f / 3.0f;
@@ -218,56 +253,76 @@ __device__ __forceinline__ void gauss_point(int ngaus, int ig, float sh[3]) {
     sh[2] = (1.0f - sh[0]) - sh[1];
 }
 
-__global__ void k_gfl_elems(GflDev d, GflConst c, float tanfi, float dt) {
+// Bound by the FP64 power of Manning's law (three a triangle) and by L2: per
+// element 56 B of its own, three gathers of 32 B, three places of 36 B written.
+template <int NG>
+__global__ void __launch_bounds__(kGflThreads) k_gfl_elems(GflDev d, GflConst c, float tanfi, float dt) {
+    GFL_ENTRY();
     const float delt2 = 0.5f * dt;
     const float cgra05 = c.cgra * 0.5f;
     for (int ie = blockIdx.x * blockDim.x + threadIdx.x; ie < d.nelem; ie += gridDim.x * blockDim.x) {
-        int nd[3];
-        float gx[3], gy[3];
+        const int4 en = d.el_nodes[ie];
+        const int2 ep = d.el_places[ie];
+        const int nd[3] = {en.x, en.y, en.z}, pl[3] = {en.w, ep.x, ep.y};
+        const float4 ga = d.el_geo[2 * (size_t)ie], gb = d.el_geo[2 * (size_t)ie + 1];
+        const float gx[3] = {ga.x, ga.y, ga.z}, gy[3] = {ga.w, gb.x, gb.y};
+        float4 na[3], nb[3];
+#pragma unroll
         for (int k = 0; k < 3; k++) {
-            nd[k] = d.elem[3 * (size_t)ie + k];
-            gx[k] = d.geome[7 * (size_t)ie + k];
-            gy[k] = d.geome[7 * (size_t)ie + 3 + k];
+            na[k] = d.fnode[2 * (size_t)nd[k]];
+            nb[k] = d.fnode[2 * (size_t)nd[k] + 1];
         }
+        // na = (h, hu, hv, hu hv/h), nb = (fx of hu, fy of hv, source of hu, source of hv)
         float div[3] = {0.f, 0.f, 0.f};
+#pragma unroll
         for (int k = 0; k < 3; k++) {
-            const float* f = d.fnode + 9 * (size_t)nd[k];
-            for (int ia = 0; ia < 3; ia++) div[ia] = (div[ia] + gx[k] * f[ia]) + gy[k] * f[3 + ia];
+            div[0] = (div[0] + gx[k] * na[k].y) + gy[k] * na[k].z;
+            div[1] = (div[1] + gx[k] * nb[k].x) + gy[k] * na[k].w;
+            div[2] = (div[2] + gx[k] * na[k].w) + gy[k] * nb[k].y;
         }
         // element gradient of the WIR soil depth (get_gradhs_w :469-481)
-        float gw0 = 0.f, gw1 = 0.f;
+        float gw0 = 0.f, gw1 = 0.f, hw[3] = {0.f, 0.f, 0.f};
         if (d.hs_w)
+#pragma unroll
             for (int k = 0; k < 3; k++) {
-                gw0 = gw0 + d.hs_w[nd[k]] * gx[k];
-                gw1 = gw1 + d.hs_w[nd[k]] * gy[k];
+                hw[k] = d.hs_w[nd[k]];
+                gw0 = gw0 + hw[k] * gx[k];
+                gw1 = gw1 + hw[k] * gy[k];
             }
         float mt[9];
-        for (int k = 0; k < 9; k++) mt[k] = d.topel[9 * (size_t)ie + k];
+        topo_rows(c, d.topel, d.nelem, ie, mt);
         if (d.hs_w) { mt[1] = mt[1] + gw0; mt[2] = mt[2] + gw1; }
-        for (int ig = 0; ig < c.ngaus; ig++) {
+        float zn[3] = {0.f, 0.f, 0.f};
+        if (c.ntype == 2)
+#pragma unroll
+            for (int k = 0; k < 3; k++) zn[k] = d.topol[nd[k]];
+        float t[3][9];  // the terms of each node: Gauss points x (h, hu, hv)
+#pragma unroll
+        for (int ig = 0; ig < NG; ig++) {
             float sh[3];
-            gauss_point(c.ngaus, ig, sh);
+            gauss_point<NG>(ig, sh);
             float src[3] = {0.f, 0.f, 0.f}, var[3] = {0.f, 0.f, 0.f};
+#pragma unroll
             for (int k = 0; k < 3; k++) {
-                const float* f = d.fnode + 9 * (size_t)nd[k];
-                const float* u = d.unkno + 3 * (size_t)nd[k];
-                for (int ia = 0; ia < 3; ia++) {
-                    src[ia] = src[ia] + sh[k] * f[6 + ia];
-                    var[ia] = var[ia] + sh[k] * u[ia];
-                }
+                src[0] = src[0] + sh[k] * 0.f;
+                src[1] = src[1] + sh[k] * nb[k].z;
+                src[2] = src[2] + sh[k] * nb[k].w;
+                var[0] = var[0] + sh[k] * na[k].x;
+                var[1] = var[1] + sh[k] * na[k].y;
+                var[2] = var[2] + sh[k] * na[k].z;
             }
-            float ue[3];
-            for (int ia = 0; ia < 3; ia++) ue[ia] = var[ia] + delt2 * (src[ia] - div[ia]);
             // second_step at this Gauss point
-            const float h = ue[0], hu = ue[1], hv = ue[2];
+            const float h = var[0] + delt2 * (src[0] - div[0]), hu = var[1] + delt2 * (src[1] - div[1]),
+                        hv = var[2] + delt2 * (src[2] - div[2]);
             float hinv = 0.f;
-            if (h >= c.comp) hinv = 1.f / h;
+            if (h >= c.comp) hinv = (h > 1.e-30f) ? recip(h) : 1.f / h;
             float HH, pres;
             if (c.ntype == 2) {
                 HH = 0.f;
+#pragma unroll
                 for (int k = 0; k < 3; k++) {
-                    HH = HH + sh[k] * d.topol[9 * (size_t)nd[k]];
-                    if (d.hs_w) HH = HH + sh[k] * d.hs_w[nd[k]];
+                    HH = HH + sh[k] * zn[k];
+                    if (d.hs_w) HH = HH + sh[k] * hw[k];
                 }
                 HH = c.swl - HH;
                 pres = cgra05 * (h * h - HH * HH);
@@ -282,12 +337,21 @@ __global__ void k_gfl_elems(GflDev d, GflConst c, float tanfi, float dt) {
             frictlaws(c, tanfi, mt, h, hu, hv, HH, frx, fry, slx, sly, cx, cy);
             sources(c, frx, fry, slx, sly, cx, cy, hu, hv, o + 6);
             // the terms this Gauss point adds to each node's rhs (:2300-2312)
-            const float dvolu = d.geome[7 * (size_t)ie + 6] / (float)(2 * c.ngaus);
-            for (int in = 0; in < 3; in++) {
-                float t[3];
+            const float dvolu = gb.z / (float)(2 * NG);
+#pragma unroll
+            for (int in = 0; in < 3; in++)
+#pragma unroll
                 for (int ia = 0; ia < 3; ia++)
-                    t[ia] = (((gx[in] * o[ia] + gy[in] * o[3 + ia]) + sh[in] * o[6 + ia]) * dvolu) * dt;
-                d.gt[3 * (3 * (size_t)ie + in) + ig] = make_float4(t[0], t[1], t[2], 0.f);
+                    t[in][3 * ig + ia] = (((gx[in] * o[ia] + gy[in] * o[3 + ia]) + sh[in] * o[6 + ia]) * dvolu) * dt;
+        }
+#pragma unroll
+        for (int in = 0; in < 3; in++) {
+            if (NG == 3) {
+                d.gt0[pl[in]] = make_float4(t[in][0], t[in][1], t[in][2], t[in][3]);
+                d.gt1[pl[in]] = make_float4(t[in][4], t[in][5], t[in][6], t[in][7]);
+                d.gt2[pl[in]] = t[in][8];
+            } else {
+                d.gt0[pl[in]] = make_float4(t[in][0], t[in][1], t[in][2], 0.f);
             }
         }
     }
@@ -301,81 +365,117 @@ __device__ __forceinline__ void wall(float2 t, float* r) {
     r[2] = r[2] - rn * any;
 }
 
-__global__ void k_gfl_rhs(GflDev d, GflConst c, float dt) {
-    const float mmatb[2][2] = {{2.f, 1.f}, {1.f, 2.f}};
+template <int NG>
+__global__ void __launch_bounds__(kGflThreads) k_gfl_rhs(GflDev d, GflConst c, float dt) {
+    GFL_ENTRY();
     for (int ip = blockIdx.x * blockDim.x + threadIdx.x; ip < d.npoin; ip += gridDim.x * blockDim.x) {
         float r[3] = {0.f, 0.f, 0.f};
-        for (int q = d.adj_ptr[ip]; q < d.adj_ptr[ip + 1]; q++) {
-            const int2 a = d.adj[q];  // element, local node: its terms in Gauss point order
-            const float4* row = d.gt + 3 * (3 * (size_t)a.x + a.y);
-            for (int ig = 0; ig < c.ngaus; ig++) {
-                const float4 t = row[ig];
-                r[0] = r[0] + t.x; r[1] = r[1] + t.y; r[2] = r[2] + t.z;
+        const int p0 = d.slot[ip >> 5] + (ip & 31), n = d.deg[ip];
+        for (int q0 = 0; q0 < n; q0 += 3) {  // element order; an element's terms in Gauss point order
+            float4 a[3], b[3];
+            float e[3];
+#pragma unroll
+            for (int u = 0; u < 3; u++) {  // three elements' loads at once
+                const int at = p0 + 32 * min(q0 + u, n - 1);
+                a[u] = __ldcs(d.gt0 + at);
+                if (NG == 3) {
+                    b[u] = __ldcs(d.gt1 + at);
+                    e[u] = __ldcs(d.gt2 + at);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 3; u++) {
+                if (q0 + u >= n) break;
+                r[0] = r[0] + a[u].x; r[1] = r[1] + a[u].y; r[2] = r[2] + a[u].z;
+                if (NG == 3) {
+                    r[0] = r[0] + a[u].w; r[1] = r[1] + b[u].x; r[2] = r[2] + b[u].y;
+                    r[0] = r[0] + b[u].z; r[1] = r[1] + b[u].w; r[2] = r[2] + e[u];
+                }
             }
         }
-        for (int q = d.bside_ptr[ip]; q < d.bside_ptr[ip + 1]; q++) {
+        const int bn = d.bnode[ip];
+        for (int q = d.bside_ptr[ip], qe = d.bside_ptr[ip + 1]; q < qe; q++) {
             const int2 b = d.bside[q];  // side, position of this node in it
             const int2 nn = d.side_nodes[b.x];
             const float4 g = d.side_geom[b.x];
             const float coe = g.z / 6.f;
             for (int j = 0; j < 2; j++) {
                 const int jn = j ? nn.y : nn.x;
-                const float cm = (mmatb[b.y][j] * coe) * dt;
-                const float* f = d.fnode + 9 * (size_t)jn;
-                for (int ia = 0; ia < 3; ia++) r[ia] = r[ia] - cm * (f[ia] * g.x + f[3 + ia] * g.y);
+                const float cm = ((j == b.y ? 2.f : 1.f) * coe) * dt;
+                const float4 fa = d.fnode[2 * (size_t)jn], fb = d.fnode[2 * (size_t)jn + 1];
+                r[0] = r[0] - cm * (fa.y * g.x + fa.z * g.y);
+                r[1] = r[1] - cm * (fb.x * g.x + fa.w * g.y);
+                r[2] = r[2] - cm * (fa.w * g.x + fb.y * g.y);
             }
         }
-        const int bn = d.bnode[ip];
         if (bn >= 0) wall(d.rtang[bn], r);
         const float cm = d.mmatl[ip];
+        d.rhs1[ip] = make_float4(r[0], r[1], r[2], 0.f);
         float r0[3];
-        for (int ia = 0; ia < 3; ia++) {
-            d.rhs1[3 * (size_t)ip + ia] = r[ia];
-            r0[ia] = r[ia] / cm;
-        }
+        for (int ia = 0; ia < 3; ia++) r0[ia] = r[ia] / cm;
         if (bn >= 0) {
             const float2 t = d.rtang[bn];
             if (!(fabsf(t.x) + fabsf(t.y) < 1.e-06f)) wall(t, r0);
         }
-        for (int ia = 0; ia < 3; ia++) d.rhs0[0][3 * (size_t)ip + ia] = r0[ia];
+        d.rhs0[0][ip] = make_float4(r0[0], r0[1], r0[2], 0.f);
     }
 }
 
-__global__ void k_gfl_mass(GflDev d, int src) {
-    const float mm[3][3] = {{2.f, 1.f, 1.f}, {1.f, 2.f, 1.f}, {1.f, 1.f, 2.f}};
-    const float* __restrict__ in = src ? d.rhs0[1] : d.rhs0[0];
-    float* __restrict__ out = src ? d.rhs0[0] : d.rhs0[1];
+__global__ void __launch_bounds__(kGflThreads) k_gfl_mass(GflDev d, int src) {
+    GFL_ENTRY();
+    const float4* __restrict__ in = src ? d.rhs0[1] : d.rhs0[0];
+    float4* __restrict__ out = src ? d.rhs0[0] : d.rhs0[1];
     for (int ip = blockIdx.x * blockDim.x + threadIdx.x; ip < d.npoin; ip += gridDim.x * blockDim.x) {
         float r2[3] = {0.f, 0.f, 0.f};
-        for (int q = d.adj_ptr[ip]; q < d.adj_ptr[ip + 1]; q++) {
-            const int2 a = d.adj[q];
-            const float coe = d.geome[7 * (size_t)a.x + 6] / 24.f;
-            for (int jn = 0; jn < 3; jn++) {
-                const int jp = d.elem[3 * (size_t)a.x + jn];
-                const float cm = mm[a.y][jn];
-                for (int ia = 0; ia < 3; ia++) r2[ia] = r2[ia] + (cm * coe) * in[3 * (size_t)jp + ia];
+        const int p0 = d.slot[ip >> 5] + (ip & 31), n = d.deg[ip];
+        for (int q0 = 0; q0 < n; q0 += 3) {  // three elements' gathers at once
+            int4 e[3];
+            float4 v[3][3];
+#pragma unroll
+            for (int u = 0; u < 3; u++) e[u] = d.place[p0 + 32 * min(q0 + u, n - 1)];
+#pragma unroll
+            for (int u = 0; u < 3; u++) {
+                v[u][0] = in[e[u].x];
+                v[u][1] = in[e[u].y];
+                v[u][2] = in[e[u].z];
+            }
+#pragma unroll
+            for (int u = 0; u < 3; u++) {
+                if (q0 + u >= n) break;
+                const float coe = __int_as_float(e[u].w);
+                const int jp[3] = {e[u].x, e[u].y, e[u].z};
+#pragma unroll
+                for (int jn = 0; jn < 3; jn++) {
+                    const float cm = (jp[jn] == ip ? 2.f : 1.f) * coe;
+                    r2[0] = r2[0] + cm * v[u][jn].x;
+                    r2[1] = r2[1] + cm * v[u][jn].y;
+                    r2[2] = r2[2] + cm * v[u][jn].z;
+                }
             }
         }
         const float ml = d.mmatl[ip];
-        float r0[3];
-        for (int ia = 0; ia < 3; ia++) r0[ia] = in[3 * (size_t)ip + ia] + (d.rhs1[3 * (size_t)ip + ia] - r2[ia]) / ml;
+        const float4 u = in[ip], b = d.rhs1[ip];
+        float r0[3] = {u.x + (b.x - r2[0]) / ml, u.y + (b.y - r2[1]) / ml, u.z + (b.z - r2[2]) / ml};
         const int bn = d.bnode[ip];
         if (bn >= 0) {
             const float2 t = d.rtang[bn];
             if (!(fabsf(t.x) + fabsf(t.y) < 1.e-06f)) wall(t, r0);
         }
-        for (int ia = 0; ia < 3; ia++) out[3 * (size_t)ip + ia] = r0[ia];
+        out[ip] = make_float4(r0[0], r0[1], r0[2], 0.f);
     }
 }
 
-__global__ void k_gfl_update(GflDev d, GflConst c, int src) {
-    const float* __restrict__ du = src ? d.rhs0[1] : d.rhs0[0];
+__global__ void __launch_bounds__(kGflThreads) k_gfl_update(GflDev d, GflConst c, int src) {
+    GFL_ENTRY();
+    const float4* __restrict__ du = src ? d.rhs0[1] : d.rhs0[0];
     for (int ip = blockIdx.x * blockDim.x + threadIdx.x; ip < d.npoin; ip += gridDim.x * blockDim.x) {
         float* u = d.unkno + 3 * (size_t)ip;
-        for (int ia = 0; ia < 3; ia++) u[ia] = u[ia] + du[3 * (size_t)ip + ia];
-        if (u[0] < c.comp) {  // check: ff = 0 without prescribed values, unkno = ff * unkno
-            u[0] = 0.f * u[0]; u[1] = 0.f * u[1]; u[2] = 0.f * u[2];
+        const float4 a = du[ip];
+        float h = u[0] + a.x, hu = u[1] + a.y, hv = u[2] + a.z;
+        if (h < c.comp) {  // check: ff = 0 without prescribed values, unkno = ff * unkno
+            h = 0.f * h; hu = 0.f * hu; hv = 0.f * hv;
         }
+        u[0] = h; u[1] = hu; u[2] = hv;
     }
 }
 
@@ -390,6 +490,21 @@ int blocks(long long n) {
     return (int)std::min<long long>(std::max<long long>(b, 1), 148LL * 32);
 }
 
+// One thread per node or element, with programmatic stream serialisation.
+template <typename... KArgs, typename... Args>
+void gfl_launch(void (*kernel)(KArgs...), long long n, cudaStream_t s, Args&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)blocks(n));
+    cfg.blockDim = dim3(kGflThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
 }  // namespace gfl
 }  // namespace gfsph
 
@@ -402,13 +517,15 @@ struct gfsph_gfl {
     cudaStream_t stream = nullptr;
     double time = 0.0;
     std::vector<float> topol, topel;  // host copies (gfsph_gfl_topol)
-    int *elem = nullptr, *adj_ptr = nullptr, *bside_ptr = nullptr, *bnode = nullptr;
-    int2 *adj = nullptr, *bside = nullptr, *side_nodes = nullptr;
-    float *geome = nullptr, *d_topel = nullptr, *d_topol = nullptr, *mmatl = nullptr, *hs_w = nullptr;
-    float4* side_geom = nullptr;
+    int *slot = nullptr, *deg = nullptr, *bside_ptr = nullptr, *bnode = nullptr;
+    int4 *el_nodes = nullptr, *place = nullptr;
+    int2 *el_places = nullptr, *bside = nullptr, *side_nodes = nullptr;
+    float *d_topel = nullptr, *d_topol = nullptr, *mmatl = nullptr, *hs_w = nullptr;
+    float4 *el_geo = nullptr, *side_geom = nullptr;
     float2 *rtang = nullptr, *gradhs_w = nullptr;
-    float4* gt = nullptr;
-    float *unkno = nullptr, *fnode = nullptr, *rhs1 = nullptr, *rhs0a = nullptr, *rhs0b = nullptr;
+    float4 *gt0 = nullptr, *gt1 = nullptr;
+    float *gt2 = nullptr, *unkno = nullptr;
+    float4 *fnode = nullptr, *rhs1 = nullptr, *rhs0a = nullptr, *rhs0b = nullptr;
     bool wir = false;
     long long launches = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // around the last gfsph_gfl_step
@@ -418,9 +535,9 @@ struct gfsph_gfl {
 namespace {
 
 void gfl_free(gfsph_gfl* g) {
-    void* ptrs[] = {g->elem, g->adj_ptr, g->bside_ptr, g->bnode, g->adj, g->bside, g->side_nodes, g->geome,
-                    g->d_topel, g->d_topol, g->mmatl, g->hs_w, g->side_geom, g->rtang, g->gradhs_w, g->unkno,
-                    g->fnode, g->gt, g->rhs1, g->rhs0a, g->rhs0b};
+    void* ptrs[] = {g->slot, g->deg, g->bside_ptr, g->bnode, g->el_nodes, g->place, g->el_places, g->bside,
+                    g->side_nodes, g->d_topel, g->d_topol, g->mmatl, g->hs_w, g->el_geo, g->side_geom, g->rtang,
+                    g->gradhs_w, g->gt0, g->gt1, g->gt2, g->unkno, g->fnode, g->rhs1, g->rhs0a, g->rhs0b};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (g->ev0) cudaEventDestroy(g->ev0);
@@ -430,11 +547,14 @@ void gfl_free(gfsph_gfl* g) {
 
 GflDev view(gfsph_gfl* g) {
     GflDev d;
-    d.npoin = g->npoin; d.nelem = g->nelem; d.elem = g->elem; d.geome = g->geome; d.topel = g->d_topel;
-    d.topol = g->d_topol; d.mmatl = g->mmatl; d.adj_ptr = g->adj_ptr; d.adj = g->adj; d.bside_ptr = g->bside_ptr;
+    d.npoin = g->npoin; d.nelem = g->nelem;
+    d.el_nodes = g->el_nodes; d.el_places = g->el_places; d.el_geo = g->el_geo;
+    d.topel = g->d_topel; d.topol = g->d_topol; d.mmatl = g->mmatl;
+    d.slot = g->slot; d.deg = g->deg; d.place = g->place; d.bside_ptr = g->bside_ptr;
     d.bside = g->bside; d.side_nodes = g->side_nodes; d.side_geom = g->side_geom; d.bnode = g->bnode;
     d.rtang = g->rtang; d.hs_w = g->wir ? g->hs_w : nullptr; d.gradhs_w = g->gradhs_w; d.unkno = g->unkno;
-    d.fnode = g->fnode; d.gt = g->gt; d.rhs1 = g->rhs1; d.rhs0[0] = g->rhs0a; d.rhs0[1] = g->rhs0b;
+    d.fnode = g->fnode; d.gt0 = g->gt0; d.gt1 = g->gt1; d.gt2 = g->gt2;
+    d.rhs1 = g->rhs1; d.rhs0[0] = g->rhs0a; d.rhs0[1] = g->rhs0b;
     return d;
 }
 
@@ -630,9 +750,45 @@ int gfsph_gfl_create(const gfsph_gfl_params* p, int npoin, int nelem, const floa
             bside[fill[side_nodes[b].y]++] = make_int2((int)b, 1);
         }
     }
-    std::vector<int> elem(3 * ne);
+    // the nodes' places: warps of 32 nodes, each as long as its node with most elements
+    const size_t nwarp = (np + 31) / 32;
+    std::vector<int> slot(nwarp), ndeg(np);
+    size_t nplace = 0;
+    for (size_t w = 0; w < nwarp; w++) {
+        int most = 0;
+        for (size_t ip = 32 * w; ip < std::min(np, 32 * w + 32); ip++) {
+            ndeg[ip] = deg[ip + 1] - deg[ip];
+            most = std::max(most, ndeg[ip]);
+        }
+        if (nplace + 32 * (size_t)most > 0x7fffffffULL) return GFSPH_ERR_CAPACITY;
+        slot[w] = (int)nplace;
+        nplace += 32 * (size_t)most;
+    }
+    std::vector<int4> el_nodes(ne), place(nplace, make_int4(0, 0, 0, 0));
+    std::vector<int2> el_places(ne);
+    std::vector<float4> el_geo(2 * ne);
+    for (size_t ie = 0; ie < ne; ie++) {
+        el_nodes[ie] = make_int4(IM(0, ie), IM(1, ie), IM(2, ie), 0);
+        el_geo[2 * ie] = make_float4(G(0, ie), G(1, ie), G(2, ie), G(3, ie));
+        el_geo[2 * ie + 1] = make_float4(G(4, ie), G(5, ie), G(6, ie), 0.f);
+    }
+    for (size_t ip = 0; ip < np; ip++)
+        for (int q = deg[ip]; q < deg[ip + 1]; q++) {
+            const int2 a = adj[q];  // element, local node
+            const int at = slot[ip >> 5] + 32 * (q - deg[ip]) + (int)(ip & 31);
+            const float coe = G(6, a.x) / 24.f;
+            int bits;
+            std::memcpy(&bits, &coe, 4);
+            place[at] = make_int4(IM(0, a.x), IM(1, a.x), IM(2, a.x), bits);
+            if (a.y == 0) el_nodes[a.x].w = at;
+            else if (a.y == 1) el_places[a.x].x = at;
+            else el_places[a.x].y = at;
+        }
+    std::vector<float> topolT(9 * np), topelT(9 * ne);  // by rows
+    for (size_t ip = 0; ip < np; ip++)
+        for (int r = 0; r < 9; r++) topolT[r * np + ip] = topol[9 * ip + r];
     for (size_t ie = 0; ie < ne; ie++)
-        for (int in = 0; in < 3; in++) elem[3 * ie + in] = IM(in, ie);
+        for (int r = 0; r < 9; r++) topelT[r * ne + ie] = topel[9 * ie + r];
 
     gfsph_gfl* g = new (std::nothrow) gfsph_gfl();
     if (!g) return GFSPH_ERR_HOST;
@@ -646,22 +802,27 @@ int gfsph_gfl_create(const gfsph_gfl_params* p, int npoin, int nelem, const floa
     g->topel = topel;
     const size_t nb = std::max<size_t>(rtang.size(), 1), ns = std::max<size_t>(side_nodes.size(), 1);
     int st = 0;
-    st |= dal(&g->elem, 3 * ne); st |= dal(&g->adj_ptr, np + 1); st |= dal(&g->adj, 3 * ne);
+    st |= dal(&g->el_nodes, ne); st |= dal(&g->el_places, ne); st |= dal(&g->el_geo, 2 * ne);
+    st |= dal(&g->slot, nwarp); st |= dal(&g->deg, np); st |= dal(&g->place, nplace);
     st |= dal(&g->bside_ptr, np + 1); st |= dal(&g->bside, bside.size()); st |= dal(&g->side_nodes, ns);
     st |= dal(&g->side_geom, ns); st |= dal(&g->bnode, np); st |= dal(&g->rtang, nb);
-    st |= dal(&g->geome, 7 * ne); st |= dal(&g->d_topel, 9 * ne); st |= dal(&g->d_topol, 9 * np);
+    st |= dal(&g->d_topel, 9 * ne); st |= dal(&g->d_topol, 9 * np);
     st |= dal(&g->mmatl, np); st |= dal(&g->hs_w, np); st |= dal(&g->gradhs_w, np);
-    st |= dal(&g->unkno, 3 * np); st |= dal(&g->fnode, 9 * np); st |= dal(&g->gt, 9 * ne);
-    st |= dal(&g->rhs1, 3 * np); st |= dal(&g->rhs0a, 3 * np); st |= dal(&g->rhs0b, 3 * np);
+    st |= dal(&g->unkno, 3 * np); st |= dal(&g->fnode, 2 * np); st |= dal(&g->gt0, nplace);
+    if (p->ngaus == 3) { st |= dal(&g->gt1, nplace); st |= dal(&g->gt2, nplace); }
+    st |= dal(&g->rhs1, np); st |= dal(&g->rhs0a, np); st |= dal(&g->rhs0b, np);
     if (st || cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&g->ev0) != cudaSuccess || cudaEventCreate(&g->ev1) != cudaSuccess) {
         gfl_free(g);
         delete g;
         return GFSPH_ERR_CUDA;
     }
-    cudaMemcpy(g->elem, elem.data(), elem.size() * sizeof(int), cudaMemcpyHostToDevice);
-    cudaMemcpy(g->adj_ptr, deg.data(), deg.size() * sizeof(int), cudaMemcpyHostToDevice);
-    cudaMemcpy(g->adj, adj.data(), adj.size() * sizeof(int2), cudaMemcpyHostToDevice);
+    cudaMemcpy(g->el_nodes, el_nodes.data(), ne * sizeof(int4), cudaMemcpyHostToDevice);
+    cudaMemcpy(g->el_places, el_places.data(), ne * sizeof(int2), cudaMemcpyHostToDevice);
+    cudaMemcpy(g->el_geo, el_geo.data(), 2 * ne * sizeof(float4), cudaMemcpyHostToDevice);
+    cudaMemcpy(g->slot, slot.data(), nwarp * sizeof(int), cudaMemcpyHostToDevice);
+    cudaMemcpy(g->deg, ndeg.data(), np * sizeof(int), cudaMemcpyHostToDevice);
+    cudaMemcpy(g->place, place.data(), nplace * sizeof(int4), cudaMemcpyHostToDevice);
     cudaMemcpy(g->bside_ptr, bptr.data(), bptr.size() * sizeof(int), cudaMemcpyHostToDevice);
     cudaMemcpy(g->bside, bside.data(), bside.size() * sizeof(int2), cudaMemcpyHostToDevice);
     if (!side_nodes.empty()) {
@@ -670,9 +831,8 @@ int gfsph_gfl_create(const gfsph_gfl_params* p, int npoin, int nelem, const floa
     }
     cudaMemcpy(g->bnode, bnode.data(), np * sizeof(int), cudaMemcpyHostToDevice);
     if (!rtang.empty()) cudaMemcpy(g->rtang, rtang.data(), rtang.size() * sizeof(float2), cudaMemcpyHostToDevice);
-    cudaMemcpy(g->geome, geome.data(), geome.size() * sizeof(float), cudaMemcpyHostToDevice);
-    cudaMemcpy(g->d_topel, topel.data(), topel.size() * sizeof(float), cudaMemcpyHostToDevice);
-    cudaMemcpy(g->d_topol, topol.data(), topol.size() * sizeof(float), cudaMemcpyHostToDevice);
+    cudaMemcpy(g->d_topel, topelT.data(), topelT.size() * sizeof(float), cudaMemcpyHostToDevice);
+    cudaMemcpy(g->d_topol, topolT.data(), topolT.size() * sizeof(float), cudaMemcpyHostToDevice);
     cudaMemcpy(g->mmatl, mmatl.data(), np * sizeof(float), cudaMemcpyHostToDevice);
     cudaMemset(g->unkno, 0, 3 * np * sizeof(float));
     if (cudaGetLastError() != cudaSuccess) { gfl_free(g); delete g; return GFSPH_ERR_CUDA; }
@@ -742,15 +902,20 @@ int gfsph_gfl_step(gfsph_gfl* g, int nsteps, float dt) try {
         float tanfi = c.tanfi8;
         if (c.bfact >= 1.e-6f)
             tanfi = c.tanfi8 + (c.tanfi0 - c.tanfi8) * (float)exp((double)(-((float)g->time / c.bfact)));
-        k_gfl_nodes<<<blocks(g->npoin), kGflThreads, 0, s>>>(d, c, tanfi);
-        k_gfl_elems<<<blocks(g->nelem), kGflThreads, 0, s>>>(d, c, tanfi, dt);
-        k_gfl_rhs<<<blocks(g->npoin), kGflThreads, 0, s>>>(d, c, dt);
+        gfl_launch(k_gfl_nodes, g->npoin, s, d, c, tanfi);
+        if (c.ngaus == 3) {
+            gfl_launch(k_gfl_elems<3>, g->nelem, s, d, c, tanfi, dt);
+            gfl_launch(k_gfl_rhs<3>, g->npoin, s, d, c, dt);
+        } else {
+            gfl_launch(k_gfl_elems<1>, g->nelem, s, d, c, tanfi, dt);
+            gfl_launch(k_gfl_rhs<1>, g->npoin, s, d, c, dt);
+        }
         int src = 0;
         for (int it = 2; it <= g->P.niter; it++) {
-            k_gfl_mass<<<blocks(g->npoin), kGflThreads, 0, s>>>(d, src);
+            gfl_launch(k_gfl_mass, g->npoin, s, d, src);
             src ^= 1;
         }
-        k_gfl_update<<<blocks(g->npoin), kGflThreads, 0, s>>>(d, c, src);
+        gfl_launch(k_gfl_update, g->npoin, s, d, c, src);
         g->launches += 3 + (g->P.niter - 1) + 1;
         g->time = g->time + (double)dt;
     }

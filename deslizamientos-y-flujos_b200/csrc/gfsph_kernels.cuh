@@ -2022,21 +2022,13 @@ __global__ void __launch_bounds__(128) k_stage_final(PState A, Search Q, StepSca
 }
 
 // One pair term of av_vel (SPH_MAIN_2019.f90:3072-3080) for particle i with
-// the pair's kernel value w.  The two quotients share a reciprocal (quot) while
-// the depths are within 1e-18 .. 1e18.
+// the pair's kernel value w.
 __device__ __forceinline__ void xsph_terms(float2 vi, float rhoi, float2 vj, float rhoj, float mj, float w, double& a0,
                                            double& a1) {
     const float den = rhoi + rhoj;
     const float n0 = (2.f * mj) * (vi.x - vj.x), n1 = (2.f * mj) * (vi.y - vj.y);
     float q0, q1;
-    if (den > 1.e-18f && den < 1.e18f) {
-        const float y = recip(den);
-        q0 = quot(n0, den, y);
-        q1 = quot(n1, den, y);
-    } else {
-        q0 = n0 / den;
-        q1 = n1 / den;
-    }
+    quot2(n0, n1, den, q0, q1);
     a0 -= (double)(q0 * w);
     a1 -= (double)(q1 * w);
 }

@@ -59,3 +59,39 @@ def test_recip_root_quot_round_correctly(tmp_path):
     out = (C.c_ulonglong * 3)()
     assert C.CDLL(str(so)).check(out) == 0
     assert list(out) == [0, 0, 0]
+
+
+POW = r"""
+#include "gfsph_device.cuh"
+using namespace gfsph;
+__global__ void k_check(unsigned long long* bad) {
+    const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    const int ex[7] = {-60, -24, -7, -1, 0, 3, 14};
+    unsigned long long b0 = 0;
+    for (unsigned m = tid; m < (1u << 23); m += nt)
+        for (int e = 0; e < 7; e++) {
+            const float x = __uint_as_float(((unsigned)(127 + ex[e]) << 23) | m);
+            if (pow73(x) != powr(x, 7.f / 3.f)) b0++;
+        }
+    if (b0) atomicAdd(bad, b0);
+}
+extern "C" int check(unsigned long long* out) {
+    unsigned long long* d = nullptr;
+    if (cudaMalloc((void**)&d, 24) != cudaSuccess || cudaMemset(d, 0, 24) != cudaSuccess) return 1;
+    k_check<<<148 * 8, 256>>>(d);
+    const int st = cudaMemcpy(out, d, 24, cudaMemcpyDeviceToHost) != cudaSuccess;
+    cudaFree(d);
+    return st;
+}
+"""
+
+
+def test_manning_power_equals_the_fp64_power(tmp_path):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    src, so = tmp_path / "pow.cu", tmp_path / "pow.so"
+    src.write_text(POW)
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "--fmad=false", "-I", CSRC,
+                    "-shared", "-Xcompiler", "-fPIC", str(src), "-o", str(so)], check=True, capture_output=True)
+    out = (C.c_ulonglong * 3)()
+    assert C.CDLL(str(so)).check(out) == 0
+    assert out[0] == 0
