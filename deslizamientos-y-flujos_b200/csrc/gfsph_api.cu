@@ -918,6 +918,8 @@ int validate(const gfsph_params* p) {
 
 }  // namespace
 
+int cg_solve_on_device(gfsph_cg* c, const float* rhs, float* x, float tol, cudaStream_t st);  // gfsph_cg.cu
+
 extern "C" int gfsph_dem_topol(int mode, int nx, int ny, float dx, float dy, float* topol);
 
 extern "C" {
@@ -2327,15 +2329,9 @@ int gfsph_gradhs(gfsph_handle* h, int ix0, int iy0, int nwx, int nwy, int niter,
         if (s2) return s2;
         std::memcpy(h->cw_key, key, sizeof(key));
     }
-    std::vector<float> rhs(2 * (size_t)nn), fixed(2 * (size_t)nn, 0.f), sol(2 * (size_t)nn, 0.f);
-    std::vector<int> iffix(2 * (size_t)nn, 0);
-    CK(cudaMemcpyAsync(rhs.data(), h->cw_rhs, (size_t)nn * sizeof(float2), cudaMemcpyDeviceToHost, st));
     if (hs_w) CK(cudaMemcpyAsync(hs_w, h->cw_hs, (size_t)nn * sizeof(float), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    int iters = 0;
-    int s3 = gfsph_cg_solve(h->cw_cg, iffix.data(), fixed.data(), rhs.data(), sol.data(), tol, &iters);
+    const int s3 = cg_solve_on_device(h->cw_cg, reinterpret_cast<const float*>(h->cw_rhs), gradhs_w, tol, st);
     if (s3 < 0) return s3;
-    if (gradhs_w) std::memcpy(gradhs_w, sol.data(), sol.size() * sizeof(float));
     return GFSPH_OK;
 } catch (...) {  // a C++ exception never crosses the C ABI
     return GFSPH_ERR_HOST;
