@@ -15,7 +15,7 @@
 //
 // Every kernel is a gather over the step's neighbour table in the step's
 // cell-sorted order and writes only its own particle, so no atomics are
-// needed except for the two parameter sums.
+// needed except for the parameter sums.
 #pragma once
 #include "gfsph_kernels.cuh"
 
@@ -23,27 +23,48 @@ namespace gfsph {
 
 // Hessian of the kernel at separation d (r = |d|, smoothing length mh):
 // d(grad W)/dd = ca * dhat dhat^T + cb * I.
-__device__ __forceinline__ void sph_kernel_hess(int skf, float r, float mh, float& ca, float& cb) {
-    float q = r / mh;
+// safe: mh within kQuotMin .. kQuotMax, where the quotients by one
+// denominator share its reciprocal (the same values).
+__device__ __forceinline__ float div_by(float a, float b, float y, bool safe) { return safe ? quot(a, b, y) : a / b; }
+__device__ __forceinline__ void sph_kernel_hess(int skf, float r, float mh, bool safe, float& ca, float& cb) {
+    const float ym = safe ? recip(mh) : 0.f;
+    float q = div_by(r, mh, ym, safe);
     ca = 0.f; cb = 0.f;
+    const float m2 = mh * mh, y2 = safe ? recip(m2) : 0.f;
     if (skf == 1) {
-        float s = (15.f / (((7.f * kPi) * mh) * mh)) / (mh * mh);
+        const float fd = ((7.f * kPi) * mh) * mh;
+        float s = div_by(div_by(15.f, fd, safe ? recip(fd) : 0.f, safe), m2, y2, safe);
         if (q <= 1.f) {
             ca = s * (1.5f * q);
             cb = s * (-2.f + 1.5f * q);
         } else if (q <= 2.f) {
             float u = 2.f - q;
-            ca = s * (u + (u * u) / (2.f * q));
-            cb = s * (-(u * u) / (2.f * q));
+            const float q2 = 2.f * q, e = div_by(u * u, q2, safe ? recip(q2) : 0.f, safe);
+            ca = s * (u + e);
+            cb = s * -e;
         }
     } else {
-        float s = (7.f / (((4.f * kPi) * mh) * mh)) / (mh * mh);
+        const float fd = ((4.f * kPi) * mh) * mh;
+        float s = div_by(div_by(7.f, fd, safe ? recip(fd) : 0.f, safe), m2, y2, safe);
         if (q <= 2.f) {
             float a = 1.f - q / 2.f;
             ca = s * ((7.5f * q) * (a * a));
             cb = s * (-(5.f * ((a * a) * a)));
         }
     }
+}
+
+// 1/b in FP64 from the FP32 reciprocal by two Newton-Raphson steps, for b
+// within FP32's range; within an ulp.
+__device__ __forceinline__ double recip64(double b) {
+    if (!(b > 1.e-30 && b < 1.e30)) return 1.0 / b;
+    double y = (double)recip((float)b);
+    y = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+    return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+}
+__device__ __forceinline__ double lanes_sum(double v, int lanes) {
+    for (int o = lanes / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
 // Derivatives of the kernel with respect to its smoothing length mh at
@@ -260,43 +281,53 @@ __global__ void k_adj_seed(const PState A, int n, const float2* lx_o, const floa
 }
 
 // The gradient of table entry `at` (skf 1 and 4, the adjoint's kernels).
-__device__ __forceinline__ void adj_grad(const Search& Q, int skf, size_t at, float2 xk, float4 o, float& d0, float& d1) {
+__device__ __forceinline__ void adj_grad(const Search& Q, int skf, size_t at, float2 xk, float4 o, bool safe, float& d0,
+                                         float& d1) {
     if (skf == 1) {
         TabGrad<1> g;
         g.load(Q, at);
-        g.grad(xk, o, false, d0, d1);
+        g.grad(xk, o, safe, d0, d1);
     } else {
         TabGrad<4> g;
         g.load(Q, at);
-        g.grad(xk, o, false, d0, d1);
+        g.grad(xk, o, safe, d0, d1);
     }
+}
+// Whether the pair (hi, hj) takes the shared reciprocals.
+__device__ __forceinline__ bool adj_safe(float hi, float hj) {
+    return hi >= 2.f * kQuotMin && hi <= kQuotMax && hj >= 0.f && hj <= kQuotMax;
 }
 
 // Adjoint of av_vel: v''_k = v'_k + eps sum_j c_kj (v'_j - v'_k),
 // c_kj = 2 m_j W_kj / (h_k + h_j), W at the start-of-step geometry.
+// G lanes a particle, as in k_iforce.
+template <int G>
 __global__ void __launch_bounds__(128) k_adj_xsph(PState A, Search Q, Rheo c, int n, const float2* velfin,
                                                   const float2* lv2, float2* lvp, float* lh, double* lm,
                                                   double2* lxacc, double* lhsacc) {
     const float eps = 0.3f;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const int gl = threadIdx.x % G;
+    constexpr int P = 128 / G;  // particles per block
+    for (int base = blockIdx.x * P; base < n; base += gridDim.x * P) {
+        const int k0 = base + threadIdx.x / G, k = min(k0, n - 1);
         const float4 me = Q.xhm[k];
         const float2 xk = make_float2(me.x, me.y), vk = velfin[k], lk = lv2[k];
         const float hk = A.rho[k], mk = me.w;
         const int cnt = Q.ncount[k];
         double s = 0.0, a0 = 0.0, a1 = 0.0, dm = 0.0, dh = 0.0, dx0 = 0.0, dx1 = 0.0, dhs = 0.0;
-        for (int q = 0; q < cnt; q++) {
+        for (int q = gl; q < cnt; q += G) {
             // the pair's W and grad W as the replayed step's search stored them
             const size_t at = tab_base(k, Q.kcap) + (size_t)q * kTabStride;
             const int j = Q.nj[at];
             const float w = Q.nw[at];
             const float4 o = Q.xhm[j];
             float d0, d1;
-            adj_grad(Q, c.skf, at, xk, o, d0, d1);
+            adj_grad(Q, c.skf, at, xk, o, adj_safe(me.z, o.z), d0, d1);
             // the pair terms in FP64: their sums over the neighbours cancel
             // strongly (antisymmetric in k, j)
             const float2 vj = velfin[j], lj = lv2[j];
             const double den = (double)hk + (double)A.rho[j], mj = o.w, wd = w;
-            const double rden = 1.0 / den;
+            const double rden = recip64(den);
             const double ckj = (2.0 * mj * wd) * rden, cjk = (2.0 * (double)mk * wd) * rden;
             const double D0 = (double)vj.x - vk.x, D1 = (double)vj.y - vk.y;
             const double pk = lk.x * D0 + lk.y * D1;     // lambda_k . (v_j - v_k)
@@ -317,6 +348,15 @@ __global__ void __launch_bounds__(128) k_adj_xsph(PState A, Search Q, Rheo c, in
                 dhs += 0.5 * lw * dwdh;
             }
         }
+        s = lanes_sum(s, G);
+        a0 = lanes_sum(a0, G);
+        a1 = lanes_sum(a1, G);
+        dm = lanes_sum(dm, G);
+        dh = lanes_sum(dh, G);
+        dx0 = lanes_sum(dx0, G);
+        dx1 = lanes_sum(dx1, G);
+        if (lhsacc) dhs = lanes_sum(dhs, G);
+        if (gl != 0 || k0 >= n) continue;
         if (lhsacc) lhsacc[k] += eps * dhs;
         lvp[k] = make_float2((float)(lk.x * (1.0 - eps * s) + eps * a0), (float)(lk.y * (1.0 - eps * s) + eps * a1));
         lh[k] += (float)(eps * dh);
@@ -329,7 +369,8 @@ __global__ void __launch_bounds__(128) k_adj_xsph(PState A, Search Q, Rheo c, in
 // Adjoint of the fused RK4 of k_force_rk (stages recomputed in registers):
 // from dL/dx', dL/dv' to dL/dx0, dL/dv0, dL/d(internal acceleration), dL/dh
 // and the parameter sums.
-__global__ void __launch_bounds__(128) k_adj_rk(PState A, Search Q, const StepScalars* S, Rheo c, DemView dem, int n,
+constexpr int kAdjRkThreads = 64;  // small blocks: 150 registers and a long serial chain, balanced over the SMs
+__global__ void __launch_bounds__(kAdjRkThreads) k_adj_rk(PState A, Search Q, const StepScalars* S, Rheo c, DemView dem, int n,
                                                 const float2* lx1, const float2* lvp, float* lh, float2* lin,
                                                 double2* lxacc, float2* lv0, double* lpar) {
     const float dt = S->dt_step;
@@ -394,43 +435,54 @@ __global__ void __launch_bounds__(128) k_adj_rk(PState A, Search Q, const StepSc
         sxi += g.xi;
         sty += g.tauy;
     }
-    smu = warp_sum(smu);
-    sxi = warp_sum(sxi);
-    sty = warp_sum(sty);
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&lpar[0], smu);
-        atomicAdd(&lpar[1], sxi);
-        atomicAdd(&lpar[2], sty);
+    // one atomic per block and parameter, none for a parameter without a share
+    __shared__ double part[3][kAdjRkThreads / 32];
+    const double v[3] = {warp_sum(smu), warp_sum(sxi), warp_sum(sty)};
+    if ((threadIdx.x & 31) == 0)
+        for (int r = 0; r < 3; r++) part[r][threadIdx.x >> 5] = v[r];
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        double t = 0.0;
+        for (int w = 0; w < kAdjRkThreads / 32; w++) t += part[threadIdx.x][w];
+        if (t != 0.0) atomicAdd(&lpar[threadIdx.x], t);
     }
 }
 
 // Adjoint of the summation density h_k = W0 m_k + sum_j m_j W_kj and of the
 // internal force a_k = -sum_j m_j (P_k + P_j) grad W_kj, gathered at k.
+// G lanes a particle, as in k_iforce.
+template <int G>
 __global__ void __launch_bounds__(128) k_adj_gather(PState A, Search Q, Rheo c, int n, const float2* lin,
                                                     const float* lh, double* lm, double2* lxacc, double* lhsacc) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const int gl = threadIdx.x % G;
+    constexpr int P = 128 / G;  // particles per block
+    for (int base = blockIdx.x * P; base < n; base += gridDim.x * P) {
+        const int k0 = base + threadIdx.x / G, k = min(k0, n - 1);
         const float4 me = Q.xhm[k];
         const float2 xk = make_float2(me.x, me.y);
         const float mk = me.w, pk = Q.pterm[k], lhk = lh[k];
         const float2 lak = lin[k];
         const int cnt = Q.ncount[k];
         const float w0 = sph_kernel_w(c.skf, 0.f, me.z);
-        double dm = (double)(lhk * w0);
+        double dm = 0.0;
         double dx0 = 0.0, dx1 = 0.0;
-        // the self term W(0, hs_k) m_k: dW/dh = -2 W/h
-        double dhs = lhsacc ? (double)lhk * (double)mk * (-2.0 * (double)w0 / (double)me.z) : 0.0;
-        for (int q = 0; q < cnt; q++) {
+        double dhs = 0.0;
+        for (int q = gl; q < cnt; q += G) {
             // the pair's W and grad W as the replayed step's search stored them
             const size_t at = tab_base(k, Q.kcap) + (size_t)q * kTabStride;
             const int j = Q.nj[at];
             const float w = Q.nw[at];
             const float4 o = Q.xhm[j];
             float d0, d1;
-            adj_grad(Q, c.skf, at, xk, o, d0, d1);
-            PairGeom g;
-            pair_test(xk, make_float2(o.x, o.y), me.z, o.z, g);
+            const bool safe = adj_safe(me.z, o.z);
+            adj_grad(Q, c.skf, at, xk, o, safe, d0, d1);
+            PairGeom g;  // pair_test, the square root by root_any
+            g.dx0 = xk.x - o.x;
+            g.dx1 = xk.y - o.y;
+            g.mh = (me.z + o.z) / 2.f;
+            g.r = root_any(g.dx0 * g.dx0 + g.dx1 * g.dx1);
             float ca, cb;
-            sph_kernel_hess(c.skf, g.r, g.mh, ca, cb);
+            sph_kernel_hess(c.skf, g.r, g.mh, safe, ca, cb);
             // the pair terms in FP64: their sums over the neighbours cancel
             // strongly (the kernel gradient is antisymmetric in k, j)
             const double mj = o.w, pj = Q.pterm[j], lhj = lh[j];
@@ -442,7 +494,7 @@ __global__ void __launch_bounds__(128) k_adj_gather(PState A, Search Q, Rheo c, 
             dx1 += fd * d1;
             // (P_k + P_j) H(d_kj) (m_k lambda_j - m_j lambda_k), H = ca dhat dhat^T + cb I
             const double u0 = (double)mk * laj.x - mj * lak.x, u1 = (double)mk * laj.y - mj * lak.y;
-            const double ir = 1.0 / (double)g.r;
+            const double ir = recip64((double)g.r);
             const double dh0 = (double)g.dx0 * ir, dh1 = (double)g.dx1 * ir;
             const double du = dh0 * u0 + dh1 * u1;
             dx0 += cp * ((double)ca * dh0 * du + (double)cb * u0);
@@ -454,7 +506,14 @@ __global__ void __launch_bounds__(128) k_adj_gather(PState A, Search Q, Rheo c, 
                 dhs += 0.5 * cp * dgdh * ((double)g.dx0 * u0 + (double)g.dx1 * u1);
             }
         }
-        if (lhsacc) lhsacc[k] += dhs;
+        dm = lanes_sum(dm, G);
+        dx0 = lanes_sum(dx0, G);
+        dx1 = lanes_sum(dx1, G);
+        if (lhsacc) dhs = lanes_sum(dhs, G);
+        if (gl != 0 || k0 >= n) continue;
+        dm += (double)(lhk * w0);
+        // the self term W(0, hs_k) m_k: dW/dh = -2 W/h
+        if (lhsacc) lhsacc[k] += dhs + (double)lhk * (double)mk * (-2.0 * (double)w0 / (double)me.z);
         lm[k] += dm;
         double2 ax = lxacc[k];
         lxacc[k] = make_double2(ax.x + dx0, ax.y + dx1);

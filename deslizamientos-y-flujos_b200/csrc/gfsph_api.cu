@@ -1892,6 +1892,7 @@ constexpr int kAdjParams = 3;  // dL/d tanfi, dL/d xi, dL/d Bingham yield stress
 
 struct gfsph_adjoint {
     gfsph_handle* h = nullptr;
+    char* arena = nullptr;  // one allocation: every array below lies in it
     int n = 0, nsteps = 0, every = 1, nck = 0;
     double t0 = 0.0;
     float dt0 = 0.f;
@@ -1936,7 +1937,7 @@ int adj_capture(gfsph_adjoint* a, float2* x, float2* v, bool fields, float* hs =
 }
 
 int adj_restore(gfsph_adjoint* a, const float2* x, const float2* v, const float* rho = nullptr,
-                const float* hs = nullptr, bool clear_err = true) {
+                const float* hs = nullptr, bool clear_err = true, bool set_dt = true) {
     gfsph_handle* h = a->h;
     if (h->n != a->n) return GFSPH_ERR_STATE;  // the handle's buffers were dropped or resized
     launch(h, K_ADJOINT, [&] {
@@ -1944,7 +1945,7 @@ int adj_restore(gfsph_adjoint* a, const float2* x, const float2* v, const float*
                                                                     hs ? hs : a->hsml0);
     });
     CK(cudaGetLastError());
-    set_field<float>(h, offsetof(StepScalars, dt), a->dt0);
+    if (set_dt) set_field<float>(h, offsetof(StepScalars, dt), a->dt0);
     if (clear_err) set_field<int>(h, offsetof(StepScalars, err), 0);
     h->has_state = true;
     return 0;
@@ -1960,32 +1961,59 @@ int adj_segment_check(gfsph_handle* h) {
     int st = read_scalars(h);
     if (st) return st;
     if (h->hS->err) return GFSPH_ERR_CAPACITY;
-    if (h->hS->nactive != h->n || h->hS->nreg != h->hS->nactive) return GFSPH_ERR_UNSUPPORTED;
+    if (h->hS->irregular) return GFSPH_ERR_UNSUPPORTED;
     return 0;
 }
 
-// One step of the handle from its current buffers; fails unless it ran.
-int adj_one_step(gfsph_handle* h) {
+// One more step of a replay, behind the chunk that has prepared the scalars:
+// the step before it has left them ready, and dt is fixed.
+int adj_replay_step(gfsph_handle* h) {
+    if (h->profile || !h->g1) return enqueue_chunk(h, 1, 1e300);
+    CK(cudaGraphLaunch(h->g1, h->stream));
+    h->launches += kernels_per_step(h);
+    return 0;
+}
+
+// `count` steps of the handle from its current buffers; fails unless they all
+// ran with every particle active and regular.
+int adj_steps(gfsph_handle* h, int count) {
     int done = 0, guard = 0;
-    for (;;) {
-        int st = enqueue_chunk(h, 1, 1e300);
+    set_field<int>(h, offsetof(StepScalars, irregular), 0);
+    while (done < count) {
+        const int chunk = std::min(kChunkSteps, count - done);
+        int st = enqueue_chunk(h, chunk, 1e300);
         if (st) return st;
-        st = finish_chunk(h, 1, 1e300, done, guard);
+        st = finish_chunk(h, chunk, 1e300, done, guard);
         if (st < 0) return st;
-        if (done >= 1) break;
+        if (h->hS->irregular) return GFSPH_ERR_UNSUPPORTED;
     }
-    // every particle active and regular (nbig and nout are cleared when a step ends)
-    if (h->hS->nactive != h->n || h->hS->nreg != h->hS->nactive) return GFSPH_ERR_UNSUPPORTED;
     return 0;
 }
 
-void adj_free(gfsph_adjoint* a) {
-    dfree(a->ckx); dfree(a->ckv); dfree(a->segx); dfree(a->segv); dfree(a->rho0); dfree(a->mass0); dfree(a->hsml0);
-    dfree(a->rhoN);
-    dfree(a->lx); dfree(a->lv); dfree(a->lm); dfree(a->lpar); dfree(a->gh); dfree(a->lx1); dfree(a->lv2);
-    dfree(a->lvp); dfree(a->lin); dfree(a->lv0); dfree(a->lh); dfree(a->lxacc); dfree(a->lms);
-    dfree(a->ckh); dfree(a->segh); dfree(a->lhs); dfree(a->lhsacc);
+// Lays the record's arrays out in one allocation.
+int adj_alloc(gfsph_adjoint* a) {
+    const size_t n = (size_t)a->n;
+    size_t off = 0;
+    auto lay = [&](auto*& p, size_t count) {
+        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(a->arena + off);  // an offset while arena is null
+        off += (count * sizeof(*p) + 255) / 256 * 256;
+    };
+    for (int pass = 0; pass < 2; pass++) {
+        off = 0;
+        lay(a->ckx, n * a->nck); lay(a->ckv, n * a->nck);
+        lay(a->segx, n * a->every); lay(a->segv, n * a->every);
+        lay(a->rho0, n); lay(a->mass0, n); lay(a->hsml0, n); lay(a->rhoN, n);
+        lay(a->lx, n); lay(a->lv, n); lay(a->lm, n); lay(a->lpar, kAdjParams);
+        lay(a->gh, n); lay(a->lx1, n); lay(a->lv2, n); lay(a->lvp, n);
+        lay(a->lin, n); lay(a->lv0, n); lay(a->lh, n); lay(a->lxacc, n);
+        lay(a->lms, n);
+        if (a->sle) { lay(a->ckh, n * a->nck); lay(a->segh, n * a->every); lay(a->lhs, n); lay(a->lhsacc, n); }
+        if (pass == 0 && dalloc(&a->arena, off)) return GFSPH_ERR_CUDA;
+    }
+    return 0;
 }
+
+void adj_free(gfsph_adjoint* a) { dfree(a->arena); }
 
 }  // namespace
 
@@ -2099,19 +2127,8 @@ int gfsph_adjoint_forward(gfsph_handle* h, int nsteps, int every, gfsph_adjoint*
     a->h = h; a->n = h->n; a->nsteps = nsteps; a->every = std::min(every, nsteps);
     a->nck = (nsteps + a->every - 1) / a->every + 1;
     const size_t n = (size_t)h->n;
-    int st = 0;
-    st |= dalloc(&a->ckx, n * a->nck); st |= dalloc(&a->ckv, n * a->nck);
-    st |= dalloc(&a->segx, n * a->every); st |= dalloc(&a->segv, n * a->every);
-    st |= dalloc(&a->rho0, n); st |= dalloc(&a->mass0, n); st |= dalloc(&a->hsml0, n); st |= dalloc(&a->rhoN, n);
-    st |= dalloc(&a->lx, n); st |= dalloc(&a->lv, n); st |= dalloc(&a->lm, n); st |= dalloc(&a->lpar, kAdjParams);
-    st |= dalloc(&a->gh, n); st |= dalloc(&a->lx1, n); st |= dalloc(&a->lv2, n); st |= dalloc(&a->lvp, n);
-    st |= dalloc(&a->lin, n); st |= dalloc(&a->lv0, n); st |= dalloc(&a->lh, n); st |= dalloc(&a->lxacc, n);
-    st |= dalloc(&a->lms, n);
     a->sle = (c.sle == 1);
-    if (a->sle) {
-        st |= dalloc(&a->ckh, n * a->nck); st |= dalloc(&a->segh, n * a->every);
-        st |= dalloc(&a->lhs, n); st |= dalloc(&a->lhsacc, n);
-    }
+    int st = adj_alloc(a);
     if (st) { adj_free(a); delete a; return GFSPH_ERR_CUDA; }
     st = read_scalars(h);
     if (st) { adj_free(a); delete a; return st; }
@@ -2120,7 +2137,7 @@ int gfsph_adjoint_forward(gfsph_handle* h, int nsteps, int every, gfsph_adjoint*
     st = adj_capture(a, a->ckx, a->ckv, true, a->sle ? a->ckh : nullptr);
     for (int t = 0, k = 1; !st && t < nsteps; k++) {
         int chunk = std::min(a->every, nsteps - t);
-        for (int q = 0; q < chunk && !st; q++) st = adj_one_step(h);
+        st = adj_steps(h, chunk);
         t += chunk;
         if (!st) st = adj_capture(a, a->ckx + n * k, a->ckv + n * k, false, a->sle ? a->ckh + n * k : nullptr);
     }
@@ -2171,9 +2188,15 @@ int gfsph_adjoint_backward(gfsph_adjoint* a, const float* gx, const float* gv, c
         if (a->sle) CK(cudaMemcpyAsync(a->segh, a->ckh + un * sg, un * sizeof(float), cudaMemcpyDeviceToDevice, st));
         auto seg_h = [&](int q) -> float* { return a->sle ? a->segh + un * q : nullptr; };
         set_field<int>(h, offsetof(StepScalars, err), 0);
-        for (int q = 1; q < len; q++) {
-            int r = adj_restore(a, a->segx + un * (q - 1), a->segv + un * (q - 1), nullptr, seg_h(q - 1), false);
-            if (!r) r = enqueue_chunk(h, 1, 1e300);
+        set_field<int>(h, offsetof(StepScalars, irregular), 0);
+        for (int q = 1; q < len; q++) {  // the segment's states, one step after the other from its checkpoint
+            int r = 0;
+            if (q == 1) {
+                r = adj_restore(a, a->segx, a->segv, nullptr, seg_h(0), false);
+                if (!r) r = enqueue_chunk(h, 1, 1e300);
+            } else {
+                r = adj_replay_step(h);
+            }
             if (!r) r = adj_capture(a, a->segx + un * q, a->segv + un * q, false, seg_h(q));
             if (r) return r;
         }
@@ -2183,8 +2206,9 @@ int gfsph_adjoint_backward(gfsph_adjoint* a, const float* gx, const float* gv, c
         }
         for (int q = len - 1; q >= 0; q--) {
             const bool last = (t0 + q == a->nsteps - 1);
-            int r = adj_restore(a, a->segx + un * q, a->segv + un * q, nullptr, seg_h(q), false);
-            if (!r) r = enqueue_chunk(h, 1, 1e300);  // neighbour table, density, forces of this step
+            // neighbour table, density, forces of this step
+            int r = adj_restore(a, a->segx + un * q, a->segv + un * q, nullptr, seg_h(q), false, q == len - 1);
+            if (!r) r = (q == len - 1) ? enqueue_chunk(h, 1, 1e300) : adj_replay_step(h);
             if (r) return r;
             Search Q = make_search(h);
             const int pb = blocks_for(n);
@@ -2195,18 +2219,25 @@ int gfsph_adjoint_backward(gfsph_adjoint* a, const float* gx, const float* gv, c
             });
             if (h->rheo.av_vel) {
                 launch(h, K_ADJOINT, [&] {
-                    k_adj_xsph<<<pb, kThreads, 0, st>>>(h->A, Q, h->rheo, n, h->velfin, a->lv2, a->lvp, a->lh,
-                                                        a->lms, a->lxacc, a->lhsacc);
+                    with_pair_lanes(n, [&](auto g) {
+                        constexpr int G = decltype(g)::value;
+                        k_adj_xsph<G><<<blocks_for((long long)n * G), 128, 0, st>>>(
+                            h->A, Q, h->rheo, n, h->velfin, a->lv2, a->lvp, a->lh, a->lms, a->lxacc, a->lhsacc);
+                    });
                 });
             } else {
                 CK(cudaMemcpyAsync(a->lvp, a->lv2, un * sizeof(float2), cudaMemcpyDeviceToDevice, st));
             }
             launch(h, K_ADJOINT, [&] {
-                k_adj_rk<<<pb, kThreads, 0, st>>>(h->A, Q, h->S, h->rheo, h->dem, n, a->lx1, a->lvp, a->lh, a->lin,
+                k_adj_rk<<<blocks_for(n, kAdjRkThreads), kAdjRkThreads, 0, st>>>(h->A, Q, h->S, h->rheo, h->dem, n, a->lx1, a->lvp, a->lh, a->lin,
                                                   a->lxacc, a->lv0, a->lpar);
             });
             launch(h, K_ADJOINT, [&] {
-                k_adj_gather<<<pb, kThreads, 0, st>>>(h->A, Q, h->rheo, n, a->lin, a->lh, a->lms, a->lxacc, a->lhsacc);
+                with_pair_lanes(n, [&](auto g) {
+                    constexpr int G = decltype(g)::value;
+                    k_adj_gather<G><<<blocks_for((long long)n * G), 128, 0, st>>>(h->A, Q, h->rheo, n, a->lin, a->lh, a->lms,
+                                                                                 a->lxacc, a->lhsacc);
+                });
             });
             launch(h, K_ADJOINT, [&] {
                 k_adj_scatter<<<pb, kThreads, 0, st>>>(h->A, n, a->lxacc, a->lv0, a->lms, a->lx, a->lv, a->lm,

@@ -76,6 +76,7 @@ struct StepScalars {
     float ref_xmin, ref_ymin, ref_delt;
     int ref_ndx, ref_ndy;
     int advance;      // 1 inside gfsph_step, 0 for search-only passes
+    int irregular;    // some step since the host cleared it had a particle outside the DEM or on a coarse level
 };
 
 // Particle state, structure of arrays, one buffer set per ordering.
@@ -737,6 +738,7 @@ __global__ void k_scatter(const int2* keyrank, int n, TileScan start, TileScan b
         S->nreg = nreg;
         S->nbig = nact - nreg;
         S->nactive = nact;
+        if (nreg != n) S->irregular = 1;
     }
 }
 
