@@ -21,14 +21,14 @@ using namespace gfsph;
 namespace {
 
 enum KernelId {
-    K_PREP, K_BOUNDS, K_HIST, K_SCAN_TILES, K_SCATTER, K_REORDER, K_DENSITY, K_DENSITY_BIG, K_IFORCE, K_FORCE_RK, K_XSPH, K_DEM_ERODE,
+    K_PREP, K_BOUNDS, K_GRID, K_HIST, K_SCAN_TILES, K_SCATTER, K_REORDER, K_DENSITY, K_IFORCE, K_FORCE_RK, K_XSPH, K_DEM_ERODE,
     K_STEP_END, K_COPY, K_UNSORT, K_RASTER, K_HAZARD, K_EXPORT, K_MARK, K_BSCAN_TILES,
     K_DENSITY_SPARSE, K_COUPLE, K_ADJOINT, K_NORM, K_STAGE, K_WIR,
     K_STEPS,  // not a kernel: device time of whole gfsph_step batches (profile level 2)
     K_COUNT
 };
 const char* kKernelNames[K_COUNT] = {
-    "k_prep", "k_bounds", "k_hist", "k_scan_tiles", "k_scatter", "k_reorder", "k_density", "k_density_big", "k_iforce",
+    "k_prep", "k_bounds", "k_grid", "k_hist", "k_scan_tiles", "k_scatter", "k_reorder", "k_density", "k_iforce",
     "k_force_rk", "k_xsph", "k_dem_erode", "k_step_end", "k_copy_state", "k_unsort",
     "k_raster_idw", "k_hazard", "k_export_big", "k_mark", "k_scan_tiles(blocks)",
     "k_density(sparse)", "k_couple", "k_adjoint", "k_norm", "k_stage", "k_wir", "step_batches"};
@@ -137,9 +137,6 @@ struct gfsph_handle {
     int dev = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;
-    cudaStream_t stream2 = nullptr;       // side stream used only inside graph captures
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    bool capturing = false;
     gfsph_params P;
     Rheo rheo;
     // DEM
@@ -281,9 +278,6 @@ int profile_collect(gfsph_handle* h) {
     return 0;
 }
 
-// Side stream for the coarse-level kernels while a graph is captured.
-cudaStream_t side_stream(gfsph_handle* h) { return h->capturing ? h->stream2 : h->stream; }
-
 // Calls f with std::integral_constant<int, skf>: the neighbour kernels are
 // compiled per SPH kernel function (skf 1 to 4).
 template <class F>
@@ -324,18 +318,6 @@ void with_pair_lanes(int n, F&& f) {
 
 // Stage-dependent pressure: the step runs the staged RK45 kernels.
 bool staged(const gfsph_handle* h) { return h->rheo.nor_density || h->rheo.cos_theta || h->rheo.ws; }
-
-void fork(gfsph_handle* h) {
-    if (!h->capturing) return;
-    cudaEventRecord(h->ev_fork, h->stream);
-    cudaStreamWaitEvent(h->stream2, h->ev_fork, 0);
-}
-
-void join(gfsph_handle* h) {
-    if (!h->capturing) return;
-    cudaEventRecord(h->ev_join, h->stream2);
-    cudaStreamWaitEvent(h->stream, h->ev_join, 0);
-}
 
 // Particles the neighbour table has room for: whole warps (tab_base).
 size_t tab_rows(const gfsph_handle* h) { return ((size_t)std::max(h->n, 1) + 31) / 32 * 32; }
@@ -384,9 +366,10 @@ int enqueue_search(gfsph_handle* h, int advance) {
     const int* ncel = reinterpret_cast<const int*>(reinterpret_cast<const char*>(S) + offsetof(StepScalars, ncells));
     if (!advance) { launch(h, K_PREP, [&] { pdl_launch(k_prep, 1, 32, st, S, advance); }); nk++; }
     const GridArgs ga{h->cap_blocks, h->cap_cells, kMaxCells, h->level_factor, h->cell_div, h->reg_levels};
-    launch(h, K_BOUNDS, [&] {
-        pdl_launch(k_bounds, std::min(kBoundsBlocks, blocks_for(n, kThreadsBounds)), kThreadsBounds, st, h->B, n, h->rheo, h->dem, S, h->bparts, ga);
-    }); nk++;
+    const int bb = std::min(kBoundsBlocks, blocks_for(n, kThreadsBounds));
+    launch(h, K_BOUNDS, [&] { pdl_launch(k_bounds, bb, kThreadsBounds, st, h->B, n, h->rheo, h->dem, S, h->bparts); });
+    launch(h, K_GRID, [&] { pdl_launch(k_grid, 1, kThreadsBounds, st, h->rheo, S, h->bparts, bb, ga); });
+    nk += 2;
     const TileScan cells{h->start, h->tile_sum}, blocks{h->bstart, h->btile_sum};
     launch(h, K_MARK, [&] { pdl_launch(k_mark, pb, kThreads, st, h->B, n, h->dem, S, h->bmark); });
     launch(h, K_BSCAN_TILES, [&] {
@@ -404,19 +387,14 @@ int enqueue_search(gfsph_handle* h, int advance) {
                    h->rcell, h->spec_u, h->spec_a, cells, h->startF, h->bstart, h->btile_sum);
     });
     nk += 6;
-    // the coarse-level kernels run beside the regular ones when graphs are
-    // captured (side stream); serially otherwise
-    cudaStream_t side = side_stream(h);
-    fork(h);
     with_skf(h, [&](auto sk) {
         constexpr int SKF = decltype(sk)::value;
-        launch(h, K_DENSITY_BIG, [&] { pdl_launch(k_density_big<SKF>, kBigBlocks, kBigThreads, side, h->A, q, S, h->rheo); });
         // the two materials' pair types compiled in only when there are two
         with_lanes(n, [&](auto g) {
             constexpr int G = decltype(g)::value;
             // the launch of the layout not in use returns at once: one block per SM, also where it is used after all
-            const int full = std::min(blocks_for((long long)n * G, kDenThreads), 148 * kDenBlocks * 3);
-            const int idle = std::min(full, 148);
+            const int full = kBigBlocks + std::min(blocks_for((long long)n * G, kDenThreads), 148 * kDenBlocks * 3);
+            const int idle = std::min(full, kBigBlocks + 148);
             const int db = h->sparse_seen ? idle : full, sb = h->sparse_seen ? full : idle;
             if (h->rheo.ws) {
                 launch(h, K_DENSITY, [&] { pdl_launch(k_density<false, SKF, true, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
@@ -429,8 +407,7 @@ int enqueue_search(gfsph_handle* h, int advance) {
             }
         });
     });
-    nk += 3;
-    join(h);
+    nk += 2;
     return nk;
 }
 
@@ -563,7 +540,7 @@ int enqueue_step_end(gfsph_handle* h) {
     StepScalars* S = h->S;
     if (h->rheo.erosion)
         launch(h, K_DEM_ERODE, [&] {
-            pdl_launch(k_dem_erode, 148 * 2, 256, h->stream, h->d_auxv, h->d_z, h->d_eroded, h->d_avail, h->nx, S);
+            pdl_launch(k_dem_erode, 148, 256, h->stream, h->d_auxv, h->d_z, h->d_eroded, h->d_avail, h->nx, S);
         });
     else
         launch(h, K_STEP_END, [&] { pdl_launch(k_step_end, 1, 32, h->stream, S); });
@@ -636,9 +613,7 @@ int build_graph(gfsph_handle* h, int steps, cudaGraphExec_t* out) {
     cudaGraph_t g = nullptr;
     long long before = h->launches;
     CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    h->capturing = true;
     for (int s = 0; s < steps; s++) enqueue_step(h);
-    h->capturing = false;
     // a launch that failed during the capture (bad configuration) is reported
     // after the capture has been ended, so the stream leaves capture mode
     const cudaError_t le = cudaGetLastError();
@@ -1007,13 +982,6 @@ int create_handle(const gfsph_params* p, const gfsph_dem* dem, gfsph_handle* sha
         return GFSPH_ERR_CUDA;
     }
     h->stream = h->own_stream;
-    if (cudaStreamCreateWithFlags(&h->stream2, cudaStreamNonBlocking) != cudaSuccess) {
-        cudaStreamDestroy(h->own_stream);
-        delete h;
-        return GFSPH_ERR_CUDA;
-    }
-    cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming);
-    cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming);
     h->P = *p;
     Rheo& c = h->rheo;
     const float* k = p->cst;  // k[i-1] = const(i)
@@ -1179,9 +1147,6 @@ int gfsph_destroy(gfsph_handle* h) try {
         if (h->ev0[k]) cudaEventDestroy(h->ev0[k]);
         if (h->ev1[k]) cudaEventDestroy(h->ev1[k]);
     }
-    if (h->ev_fork) cudaEventDestroy(h->ev_fork);
-    if (h->ev_join) cudaEventDestroy(h->ev_join);
-    if (h->stream2) cudaStreamDestroy(h->stream2);
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
     delete h;
     return GFSPH_OK;

@@ -33,7 +33,7 @@ constexpr int kBlkY = 8;            // cells per block along y
 constexpr int kBlockCells = kBlkX * kBlkY;
 constexpr long long kDenseCells = 1LL << 22;  // dense-mode budget (or 8 cells per particle)
 constexpr int kThreadsBounds = 256;
-constexpr int kBoundsBlocks = 148 * 4;  // at most; the last block reduces their partials
+constexpr int kBoundsBlocks = 148 * 4;  // at most; k_grid reduces their partials
 
 // error bits in StepScalars::err
 constexpr int kErrCells = 1;
@@ -68,7 +68,6 @@ struct StepScalars {
     int nreg, nbig, nactive, nout;
     int need_cells, need_nbr, need_big, need_blocks;
     int ex0, ex1, ey0, ey1;  // DEM node box touched by erosion this step
-    unsigned int bounds_ticket;  // blocks of k_bounds done (the last one resets it)
     unsigned int scan_ticket[2];  // tiles of k_scan_tiles done: cells, block map
     unsigned int end_ticket;      // blocks of k_dem_erode done
     int reg_levels;   // levels 0 .. reg_levels-1 are regular (thread + neighbour table)
@@ -268,8 +267,8 @@ __device__ __forceinline__ int warp_sum(int v) {
 // flagged; then the Check_Out_Domain at the start of time_integration_sph
 // (SPH_MAIN_2019.f90:232, :1764-1788) and, over the particles still inside,
 // the bounds, max and mean of hsml for the cell grid.
-// One launch: the per-particle part, block partials, and in the last block
-// the global bounds and grid_setup.
+// k_bounds: the per-particle part and block partials; k_grid, one block: the
+// global bounds and grid_setup.
 struct BoundsPart {
     float xmn, xmx, ymn, ymx, hmx, dtm;
     double hsum;
@@ -292,8 +291,8 @@ struct GridArgs {
 
 __device__ void grid_setup(const Rheo& c, StepScalars* S, const GridArgs ga);
 
-__global__ void __launch_bounds__(kThreadsBounds) k_bounds(PState B, int n, Rheo c, DemView dem, StepScalars* S,
-                                                           BoundsPart* part, GridArgs ga) {
+__global__ void __launch_bounds__(kThreadsBounds) k_bounds(PState B, int n, Rheo c, DemView dem, const StepScalars* S,
+                                                           BoundsPart* part) {
     PDL_ENTRY();
     if (step_skipped(S)) return;
     float xmn = 3.4e38f, xmx = -3.4e38f, ymn = 3.4e38f, ymx = -3.4e38f, hmx = 0.f, dtm = 1.e10f;
@@ -333,48 +332,40 @@ __global__ void __launch_bounds__(kThreadsBounds) k_bounds(PState B, int n, Rheo
                 dtm = fminf(dtm, sqrtf(dem.dx * dem.dx + dem.dy * dem.dy) / vv);
         }
     }
-    // block partials, then the last block to finish reduces them in block
-    // order (deterministic FP64 sum, no same-address atomics) and sets up
-    // the grids
     __shared__ BoundsPart wp[kThreadsBounds / 32];
-    __shared__ bool last;
     BoundsPart q{warp_min(xmn), warp_max(xmx), warp_min(ymn), warp_max(ymx), warp_max(hmx), warp_min(dtm),
                  warp_sum(hs_sum), warp_sum(hs_cnt), __any_sync(0xffffffffu, bad) ? 1 : 0};
     if ((threadIdx.x & 31) == 0) wp[threadIdx.x >> 5] = q;
     __syncthreads();
     if (threadIdx.x == 0) {
         BoundsPart b = wp[0];
-        for (int k = 1; k < (int)(blockDim.x >> 5); k++) bounds_merge(b, wp[k]);
+        for (int k = 1; k < kThreadsBounds / 32; k++) bounds_merge(b, wp[k]);
         part[blockIdx.x] = b;
-        __threadfence();
-        last = (atomicAdd(&S->bounds_ticket, 1u) == gridDim.x - 1);
     }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
+}
+
+// The partials in a fixed order (deterministic FP64 sum, no same-address
+// atomics), then the grids.
+__global__ void __launch_bounds__(kThreadsBounds) k_grid(Rheo c, StepScalars* S, const BoundsPart* part, int nparts,
+                                                         GridArgs ga) {
+    PDL_ENTRY();
+    if (step_skipped(S)) return;
+    __shared__ BoundsPart wp[kThreadsBounds / 32];
+    StepScalars* L = scalars_to_smem(S);
     BoundsPart b{3.4e38f, -3.4e38f, 3.4e38f, -3.4e38f, 0.f, 1.e10f, 0.0, 0, 0};
-    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
-        BoundsPart o;
-        const volatile BoundsPart* vp = part + k;
-        o.xmn = vp->xmn; o.xmx = vp->xmx; o.ymn = vp->ymn; o.ymx = vp->ymx; o.hmx = vp->hmx; o.dtm = vp->dtm;
-        o.hsum = vp->hsum; o.hcnt = vp->hcnt; o.bad = vp->bad;
-        bounds_merge(b, o);
-    }
+    for (int k = threadIdx.x; k < nparts; k += kThreadsBounds) bounds_merge(b, part[k]);
     b.xmn = warp_min(b.xmn); b.xmx = warp_max(b.xmx); b.ymn = warp_min(b.ymn); b.ymx = warp_max(b.ymx);
     b.hmx = warp_max(b.hmx); b.dtm = warp_min(b.dtm); b.hsum = warp_sum(b.hsum); b.hcnt = warp_sum(b.hcnt);
     b.bad = __any_sync(0xffffffffu, b.bad) ? 1 : 0;
-    __syncthreads();
     if ((threadIdx.x & 31) == 0) wp[threadIdx.x >> 5] = b;
     __syncthreads();
-    StepScalars* L = scalars_to_smem(S);
     if (threadIdx.x < 32) {
         BoundsPart t = wp[0];
-        for (int k = 1; k < (int)(blockDim.x >> 5); k++) bounds_merge(t, wp[k]);
+        for (int k = 1; k < kThreadsBounds / 32; k++) bounds_merge(t, wp[k]);
         if (threadIdx.x == 0) {
             L->xmin_o = f2o(t.xmn); L->xmax_o = f2o(t.xmx); L->ymin_o = f2o(t.ymn); L->ymax_o = f2o(t.ymx);
             L->hmax_o = f2o(t.hmx); L->dtmin_o = f2o(t.dtm);
             L->hsum = t.hsum; L->hcount = t.hcnt; L->bad = t.bad;
-            L->bounds_ticket = 0u;
         }
         __syncwarp();
         grid_setup(c, L, ga);
@@ -707,6 +698,10 @@ __global__ void k_scan_tiles(int* count, int* start, int* tile_sum, const int* n
         int g = base + k;
         if (g < m) start[g] = sh[k];
     }
+    if (ntiles == 1) {
+        if (threadIdx.x == 0) tile_sum[0] = 0;
+        return;
+    }
     if (threadIdx.x == 0) {
         __threadfence();
         last = (atomicAdd(&S->scan_ticket[which], 1u) == (unsigned)ntiles - 1u);
@@ -912,6 +907,86 @@ struct LevelRows {
     }
 };
 
+// A coarse-level particle, few but with up to every particle in its support,
+// takes a block (of kBigThreads, in k_density of kDenThreads): its warps share the rows of a level's stencil,
+// the lanes fetch the slot ranges of up to 32 rows at once, then share each
+// row's candidates.  (With one warp each, the one with the longest list took
+// 38 us of the 200k flow's step in each of the three passes.)
+constexpr int kBigThreads = 256;
+constexpr int kBigBlocks = 148;  // the first blocks of the pair kernels take these particles, the others the regular ones
+template <int T, bool SPARSE, int SK, class F>
+__device__ __forceinline__ void block_rows(const Search& Q, const StepScalars* S, int i, F& f) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    constexpr int W = T / 32;
+    const float4 me = Q.xhm[i];
+    const float2 xi = make_float2(me.x, me.y);
+    const float hi = me.z;
+    const int2 ci = (SK == 2) ? make_int2(0, 0) : Q.rcell[i];
+    for (int k = 0; k < S->nlev; k++) {
+        LevelRows<SPARSE> rows;
+        if (!rows.template open<SK>(S, k, xi, hi)) continue;
+        for (int rb = 0; rb < rows.nrow; rb += T) {
+            const int row = rb + W * lane + wid;
+            int ja = 0, jb = 0;
+            if (row < rows.nrow) rows.range(Q, row, ja, jb);
+            const int nr = min(32, (rows.nrow - rb - wid + W - 1) / W);
+            for (int r = 0; r < nr; r++) {
+                const int a = __shfl_sync(0xffffffffu, ja, r), e = __shfl_sync(0xffffffffu, jb, r);
+                for (int j = a + lane; j < e; j += 32) {
+                    if (j == i) continue;
+                    const float4 o = Q.xhm[j];
+                    PairGeom g;
+                    if (pair_search<SK>(xi, make_float2(o.x, o.y), hi, o.z, g) && ref_adjacent<SK>(Q, ci, j))
+                        f(j, o, g);
+                }
+            }
+        }
+    }
+}
+template <int SK, int T = kBigThreads, class F>
+__device__ __forceinline__ void block_neighbours(const Search& Q, const StepScalars* S, int i, F&& f) {
+    if (S->sparse) block_rows<T, true, SK>(Q, S, i, f);
+    else block_rows<T, false, SK>(Q, S, i, f);
+}
+// Sum over the block in a fixed order, in thread 0; every thread calls it.
+__device__ __forceinline__ double block_sum(double v) {
+    __shared__ double part[kBigThreads / 32];
+    v = warp_sum(v);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += part[w];
+    return t;
+}
+
+// Summation density of the coarse-level particles, one block per particle:
+// the first kBigBlocks blocks of k_density.
+template <int SKF, bool WS>
+__device__ __forceinline__ void density_big(const PState& A, const Search& Q, const StepScalars* S, const Rheo& c) {
+    constexpr int SK = SupportScale<SKF>::value;
+    const int nreg = S->nreg, nbig = S->nbig;
+    for (int b = blockIdx.x; b < nbig; b += kBigBlocks) {
+        const int i = nreg + b;
+        double acc = 0.0;
+        const unsigned char si = WS ? Q.spec[i] : 0;
+        block_neighbours<SK, kDenThreads>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
+            if (WS && Q.spec[j] != si) return;  // type 1: not in the density (:1829)
+            acc += (double)(o.w * sph_kernel_w<SKF>(g.r, g.mh));
+        });
+        acc = block_sum(acc);
+        if (threadIdx.x == 0) {
+            float4 me = Q.xhm[i];
+            float h = (float)((double)(sph_kernel_w<SKF>(0.f, me.z) * me.w) + acc);
+            A.rho[i] = h;
+            float hc = (h < c.h_inf) ? c.h_inf : h;
+            float p = (c.cgra05 * hc) * hc;
+            Q.pterm[i] = (c.pa_sph == 1) ? p : p / (hc * hc);
+        }
+    }
+}
+
 // Bound by FP32 issue and the latency of the gathers: 200k particles (release,
 // two lanes) 89 us a launch where one thread per particle, evaluating each
 // pair as it was found, took 115; the flow with coarse levels 106 against 190;
@@ -922,6 +997,10 @@ __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, S
     PDL_ENTRY();
     if ((S->sparse != 0) != SPARSE) return;
     if (__syncthreads_or(S->skip)) return;  // another block may set it meanwhile: one decision per block
+    if (blockIdx.x < kBigBlocks) {
+        density_big<SKF, WS>(A, Q, S, c);
+        return;
+    }
     constexpr int SK = SupportScale<SKF>::value;
     constexpr int L = DenList<G>::value, P = kDenThreads / G;
     constexpr unsigned full = 0xffffffffu;
@@ -935,7 +1014,8 @@ __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, S
     const bool scan_big = nbig > 0 && nbig <= kBigScan;
     const int nlev = (nbig > 0 && !scan_big) ? S->nlev : min(S->nlev, S->reg_levels);
     const float hmax = o2f(S->hmax_o);
-    for (int base = blockIdx.x * P; base < nreg; base += gridDim.x * P) {  // the same trips for the whole block
+    const int bid = blockIdx.x - kBigBlocks, nb = gridDim.x - kBigBlocks;
+    for (int base = bid * P; base < nreg; base += nb * P) {  // the same trips for the whole block
         const int i = base + tid / G;
         const bool act = i < nreg;
         const float4 me = Q.xhm[act ? i : base];
@@ -1103,89 +1183,6 @@ __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, S
         if (scan_big) __syncthreads();  // the box is rewritten
     }
 }
-
-// A coarse-level particle, few but with up to every particle in its support,
-// takes a block of kBigThreads: its warps share the rows of a level's stencil,
-// the lanes fetch the slot ranges of up to 32 rows at once, then share each
-// row's candidates.  (With one warp each, the one with the longest list took
-// 38 us of the 200k flow's step in each of the three passes.)
-constexpr int kBigThreads = 256;
-constexpr int kBigBlocks = 148;  // the first blocks of k_iforce, k_norm and k_xsph take these particles, the others the regular ones
-template <bool SPARSE, int SK, class F>
-__device__ __forceinline__ void block_rows(const Search& Q, const StepScalars* S, int i, F& f) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    constexpr int W = kBigThreads / 32;
-    const float4 me = Q.xhm[i];
-    const float2 xi = make_float2(me.x, me.y);
-    const float hi = me.z;
-    const int2 ci = (SK == 2) ? make_int2(0, 0) : Q.rcell[i];
-    for (int k = 0; k < S->nlev; k++) {
-        LevelRows<SPARSE> rows;
-        if (!rows.template open<SK>(S, k, xi, hi)) continue;
-        for (int rb = 0; rb < rows.nrow; rb += kBigThreads) {
-            const int row = rb + W * lane + wid;
-            int ja = 0, jb = 0;
-            if (row < rows.nrow) rows.range(Q, row, ja, jb);
-            const int nr = min(32, (rows.nrow - rb - wid + W - 1) / W);
-            for (int r = 0; r < nr; r++) {
-                const int a = __shfl_sync(0xffffffffu, ja, r), e = __shfl_sync(0xffffffffu, jb, r);
-                for (int j = a + lane; j < e; j += 32) {
-                    if (j == i) continue;
-                    const float4 o = Q.xhm[j];
-                    PairGeom g;
-                    if (pair_search<SK>(xi, make_float2(o.x, o.y), hi, o.z, g) && ref_adjacent<SK>(Q, ci, j))
-                        f(j, o, g);
-                }
-            }
-        }
-    }
-}
-template <int SK, class F>
-__device__ __forceinline__ void block_neighbours(const Search& Q, const StepScalars* S, int i, F&& f) {
-    if (S->sparse) block_rows<true, SK>(Q, S, i, f);
-    else block_rows<false, SK>(Q, S, i, f);
-}
-// Sum over the block in a fixed order, in thread 0; every thread calls it.
-__device__ __forceinline__ double block_sum(double v) {
-    __shared__ double part[kBigThreads / 32];
-    v = warp_sum(v);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double t = 0.0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < kBigThreads / 32; w++) t += part[w];
-    return t;
-}
-
-// Summation density of the coarse-level particles, one block per particle.
-template <int SKF>
-__global__ void __launch_bounds__(kBigThreads) k_density_big(PState A, Search Q, StepScalars* S, Rheo c) {
-    PDL_ENTRY();
-    constexpr int SK = SupportScale<SKF>::value;
-    if (S->skip) return;
-    const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
-        int i = nreg + b;
-        double acc = 0.0;
-        const unsigned char si = c.ws ? Q.spec[i] : 0;
-        block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
-            if (c.ws && Q.spec[j] != si) return;  // type 1: not in the density (:1829)
-            acc += (double)(o.w * sph_kernel_w<SKF>(g.r, g.mh));
-        });
-        acc = block_sum(acc);
-        if (threadIdx.x == 0) {
-            float4 me = Q.xhm[i];
-            float h = (float)((double)(sph_kernel_w<SKF>(0.f, me.z) * me.w) + acc);
-            A.rho[i] = h;
-            float hc = (h < c.h_inf) ? c.h_inf : h;
-            float p = (c.cgra05 * hc) * hc;
-            const float pt = (c.pa_sph == 1) ? p : p / (hc * hc);
-            Q.pterm[i] = pt;
-        }
-    }
-}
-
 // One pair term of IntForces_SW (SPH_SW_2019.f90:6905-6920) for particle i,
 // from the pair's kernel gradient (d0, d1).
 __device__ __forceinline__ void pressure_terms(const Rheo& c, float pi_, float rhoi, float pj, float rhoj, float mj,
