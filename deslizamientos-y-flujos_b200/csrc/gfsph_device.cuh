@@ -46,6 +46,68 @@ __device__ __forceinline__ float quot(float a, float b, float y) {
     const float q = a * y;
     return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
 }
+// Two FP32 values in one register pair, with Blackwell's two-wide operations:
+// each half rounds as the scalar operation does, for one instruction issued
+// instead of two.  The pair kernels are bound by instruction issue.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2(float a) { return f2(a, a); }
+__device__ __forceinline__ void split(F2 a, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v)); }
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) {
+    F2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+// The product as a b + 0, rounded once: a two-wide mul.rn followed by add.rn was
+// contracted into one rounding here, which no flag or qualifier prevented.
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(0ULL));
+    return r;
+}
+__device__ __forceinline__ F2 pick(bool a0, bool a1, F2 a, F2 b) {  // per half: a where set, else b
+    float x0, x1, y0, y1;
+    split(a, x0, x1);
+    split(b, y0, y1);
+    return f2(a0 ? x0 : y0, a1 ? x1 : y1);
+}
+// recip, root and quot on both halves; nb = -b.
+__device__ __forceinline__ F2 recip(F2 b, F2 nb) {
+    float x, y;
+    split(b, x, y);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(x) : "f"(x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(y));
+    const F2 r = f2(x, y);
+    return fma2(fma2(nb, r, f2(1.f)), r, r);
+}
+__device__ __forceinline__ F2 root(F2 d) {
+    float x, y;
+    split(d, x, y);
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(x) : "f"(x));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(y));
+    const F2 r = f2(x, y), g = d * r;
+    return fma2(fma2(g * f2(-1.f), g, d), r * f2(0.5f), g);
+}
+__device__ __forceinline__ F2 quot(F2 a, F2 nb, F2 y) {
+    const F2 q = a * y;
+    return fma2(fma2(q, nb, a), y, q);
+}
 // The square root of any value: root() within its range, else the operator.
 __device__ __forceinline__ float root_any(float d) { return (d >= 1.e-30f && d <= 1.e37f) ? root(d) : sqrtf(d); }
 // Smoothing lengths for which every product and quotient of a pair's kernel
@@ -154,6 +216,25 @@ __device__ __forceinline__ void spline_pair(float dr, float hs, bool safe, float
         w = ((factor * 1.f) / 6.f) * ((u * u) * u);
         t = ((((factor * 1.f) / 6.f) * 3.f) * (u * u)) / hs;
     }
+}
+// spline_pair of two pairs at once (safe).
+__device__ __forceinline__ void spline_pair2(F2 dr, F2 hs, F2& w, F2& t) {
+    float r0, r1;
+    split(dr, r0, r1);
+    const F2 r = root(f2(fmaxf(r0, 1.e-36f), fmaxf(r1, 1.e-36f)));
+    const F2 nh = hs * f2(-1.f), yh = recip(hs, nh), q = quot(r, nh, yh);
+    const F2 fd = (f2(7.f * kPi) * hs) * hs, nf = fd * f2(-1.f);
+    const F2 factor = quot(f2(15.f), nf, recip(fd, nf));
+    const F2 f6 = quot(factor, f2(-6.f), f2(1.f / 6.f));
+    float q0, q1;
+    split(q, q0, q1);
+    const bool in0 = q0 <= 1.f, in1 = q1 <= 1.f;
+    const F2 u = f2(2.f) - q, u2 = u * u, h2 = hs * hs, nh2 = h2 * f2(-1.f), qq = q * q;
+    const F2 wi = factor * ((f2(kTwoThirds) - qq) + (qq * q) * f2(0.5f));
+    const F2 wo = f6 * (u2 * u);
+    const F2 ti = factor * (f2(-2.f) + f2(1.5f) * q), to = (f6 * f2(3.f)) * u2;
+    w = pick(in0, in1, wi, wo);
+    t = quot(pick(in0, in1, ti, to), pick(in0, in1, nh2, nh), pick(in0, in1, recip(h2, nh2), yh));
 }
 // grad W from t and the separation dx.
 __device__ __forceinline__ void spline_grad(float t, float dx0, float dx1, bool safe, float& d0, float& d1) {

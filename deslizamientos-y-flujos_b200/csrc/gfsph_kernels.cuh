@@ -1132,13 +1132,7 @@ __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, S
                     if (t >= from[o]) { own = o; f = from[o]; }
                 return list[(t - f) * kDenThreads + tid - gl + own];
             };
-            auto pair = [&](int t, int j, const float4& o) {
-                const float dx0 = xi.x - o.x, dx1 = xi.y - o.y;
-                const float dr = dx0 * dx0 + dx1 * dx1;
-                const float mh = (hi + o.z) / 2.f;
-                float w, d0, d1;
-                if (SKF == 1) spline_pair(dr, mh, safe, w, d0);
-                else sph_kernel<SKF>(sqrtf(dr), dx0, dx1, mh, w, d0, d1);
+            auto store = [&](int t, int j, const float4& o, float w, float d0, float d1) {
                 const bool cross = WS && Q.spec[j] != si;
                 if (found + t < Q.kcap) {
                     const size_t to = tab + (size_t)(found + t) * kTabStride;
@@ -1149,12 +1143,35 @@ __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, S
                 }
                 if (!cross) acc += (double)(o.w * w);
             };
+            auto pair = [&](int t, int j, const float4& o) {
+                const float dx0 = xi.x - o.x, dx1 = xi.y - o.y;
+                const float dr = dx0 * dx0 + dx1 * dx1;
+                const float mh = (hi + o.z) / 2.f;
+                float w, d0, d1 = 0.f;
+                if (SKF == 1) spline_pair(dr, mh, safe, w, d0);
+                else sph_kernel<SKF>(sqrtf(dr), dx0, dx1, mh, w, d0, d1);
+                store(t, j, o, w, d0, d1);
+            };
             int t = gl;
             for (; t + G < tot; t += 2 * G) {  // two independent pairs at a time
                 const int ja = entry(t), jb = entry(t + G);
                 const float4 oa = Q.xhm[ja], ob = Q.xhm[jb];
-                pair(t, ja, oa);
-                pair(t + G, jb, ob);
+                if (SKF == 1 && safe) {
+                    const F2 da = f2(xi.x, xi.y) - f2(oa.x, oa.y), db = f2(xi.x, xi.y) - f2(ob.x, ob.y);
+                    float a0, a1, b0, b1;
+                    split(da * da, a0, a1);
+                    split(db * db, b0, b1);
+                    F2 w, g;
+                    spline_pair2(f2(a0 + a1, b0 + b1), (f2(hi) + f2(oa.z, ob.z)) * f2(0.5f), w, g);
+                    float wa, wb, ga, gb;
+                    split(w, wa, wb);
+                    split(g, ga, gb);
+                    store(t, ja, oa, wa, ga, 0.f);
+                    store(t + G, jb, ob, wb, gb, 0.f);
+                } else {
+                    pair(t, ja, oa);
+                    pair(t + G, jb, ob);
+                }
             }
             if (t < tot) {
                 const int j = entry(t);
