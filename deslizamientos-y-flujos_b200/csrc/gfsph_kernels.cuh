@@ -1384,19 +1384,15 @@ __device__ __forceinline__ void flush_node_box(StepScalars* S, NodeBox b) {
 // adds base/dist and 1/dist to the 4x4 DEM nodes around its DEM cell.
 // Consecutive particles of the cell-sorted order mostly share a DEM cell, so
 // within a warp the lanes form runs of equal DEM cell.  Each lane writes its
-// 32 FP32 terms (16 nodes x {base/dist, 1/dist}) to shared memory; then lane t
-// adds up term t over each run of lanes, in lane order and in FP64, and
-// issues that run's atomic for it.  The run boundaries are the same for every
-// lane, so the summing loop does not diverge.  Lanes with part == false take
-// no part; every lane of the warp must call this, in blocks of at most
-// kScatterWarps warps.
-constexpr int kScatterWarps = 4;
+// 32 FP32 terms (16 nodes x {base/dist, 1/dist}) to shared memory, and
+// add_node_runs sums them.  Lanes with part == false take no part; every lane
+// of the warp must call this, in blocks of at most kScatterWarps warps.
 __device__ __forceinline__ void erosion_scatter(const DemView& dem, float xx, float xy, float base, bool part,
                                                 double2* auxv, NodeBox& box) {
-    __shared__ float sterm[kScatterWarps][32][33];  // [term][lane], padded against bank conflicts
-    __shared__ int skey[kScatterWarps][33], spx[kScatterWarps][32], spy[kScatterWarps][32];
+    __shared__ NodeRuns runs[kScatterWarps];
     const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    NodeRuns& R = runs[threadIdx.x >> 5];
     int ipx = 0, ipy = 0, key = -1 - lane;  // non-participants: singleton runs with zero terms
     if (part) {
         ipx = dem_node_x(dem, xx);
@@ -1404,7 +1400,6 @@ __device__ __forceinline__ void erosion_scatter(const DemView& dem, float xx, fl
         key = ipy * (dem.nx + 2) + ipx;
     }
     if (!__any_sync(full, part)) return;
-    float(*T)[33] = sterm[wid];
     // the 4x4 nodes (ipx-1..ipx+2) x (ipy-1..ipy+2); nodes outside the DEM add zero
     float dx2[4], dy2[4];
 #pragma unroll
@@ -1420,33 +1415,10 @@ __device__ __forceinline__ void erosion_scatter(const DemView& dem, float xx, fl
         // max(1e-6, distance); the root is kept off 0
         const float dist = fmaxf(root(fmaxf(dx2[o >> 2] + dy2[o & 3], 1.e-30f)), 1.e-6f);
         const float y = recip(dist);
-        T[o][lane] = inside ? quot(base, dist, y) : 0.f;
-        T[16 + o][lane] = inside ? y : 0.f;
+        R.term[o][lane] = inside ? quot(base, dist, y) : 0.f;
+        R.term[16 + o][lane] = inside ? y : 0.f;
     }
-    skey[wid][lane] = key;
-    if (lane == 0) skey[wid][32] = INT_MIN;  // no key: closes the last run
-    spx[wid][lane] = ipx;
-    spy[wid][lane] = ipy;
-    __syncwarp();
-    const int o = lane & 15, ox = (o >> 2) - 1, oy = (o & 3) - 1;
-    double acc = 0.0;
-    int kr = skey[wid][0];
-    for (int r = 0; r < 32; r++) {
-        acc += (double)T[lane][r];
-        const int kn = skey[wid][r + 1];
-        if (kn != kr) {  // run ends at lane r (the same r for every lane)
-            if (kr >= 0) {
-                const int ix = spx[wid][r] + ox, iy = spy[wid][r] + oy;
-                if (ix >= 1 && ix <= dem.nx && iy >= 1 && iy <= dem.ny) {
-                    double* dst = &auxv[(iy - 1) * dem.nx + (ix - 1)].x;
-                    atomicAdd(dst + (lane >> 4), acc);  // .x for base/dist, .y for 1/dist
-                }
-            }
-            acc = 0.0;
-            kr = kn;
-        }
-    }
-    __syncwarp();  // the terms are rewritten by the next call
+    add_node_runs(R, lane, key, ipx, ipy, dem.nx, dem.ny, auxv);
     if (part) {
         box.x0 = min(box.x0, max(1, ipx - 1)); box.x1 = max(box.x1, min(dem.nx, ipx + 2));
         box.y0 = min(box.y0, max(1, ipy - 1)); box.y1 = max(box.y1, min(dem.ny, ipy + 2));
@@ -2244,28 +2216,14 @@ __global__ void k_export_big(Search Q, StepScalars* S, int2* pairs, int* npairs,
 
 // Depth raster: IDW of h onto the 4x4 DEM nodes around each particle
 // (SPH_SW_2019.f90:14310-14400, auxv(1)/auxv(5)).
-__global__ void k_raster_idw(const PState B, int n, DemView dem, double2* acc) {
-    float distg = sqrtf(dem.dx * dem.dx + dem.dy * dem.dy);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (B.flag[i]) continue;
-        float2 p = B.pos[i];
-        float h = B.rho[i];
-        int ipx = (int)((p.x - dem.xmin) / dem.dx + 1.f);
-        int ipy = (int)((p.y - dem.ymin) / dem.dy + 1.f);
-        int ix0 = max(1, ipx - 1), iy0 = max(1, ipy - 1), ix1 = min(dem.nx, ipx + 2), iy1 = min(dem.ny, ipy + 2);
-        for (int ix = ix0; ix <= ix1; ix++)
-            for (int iy = iy0; iy <= iy1; iy++) {
-                int ip = (iy - 1) * dem.nx + (ix - 1);
-                float ddx = p.x - (dem.xmin + (float)(ix - 1) * dem.dx);
-                ddx = ddx * ddx;
-                float ddy = p.y - (dem.ymin + (float)(iy - 1) * dem.dy);
-                ddy = ddy * ddy;
-                float dist = sqrtf(ddx + ddy);
-                dist = (1.e-6f > dist) ? 1.e-6f : dist;
-                dist = dist / distg;
-                atomicAdd(&acc[ip].x, (double)(h / dist));
-                atomicAdd(&acc[ip].y, (double)(1.f / dist));
-            }
+__global__ void __launch_bounds__(32 * kScatterWarps) k_raster_idw(const PState B, int n, DemView dem, double2* acc) {
+    const float distg = sqrtf(dem.dx * dem.dx + dem.dy * dem.dy);
+    // block-uniform trip count: every lane of a warp reaches idw_scatter
+    for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
+        const int i = i0 + threadIdx.x;
+        const bool part = i < n && !B.flag[i];
+        idw_scatter(dem.nx, dem.ny, dem.xmin, dem.ymin, dem.dx, dem.dy, distg, part ? B.pos[i] : make_float2(0.f, 0.f),
+                    part ? B.rho[i] : 0.f, part, acc);
     }
 }
 

@@ -34,30 +34,18 @@ __global__ void k_noalloc_clear(double2* acc, int np) {
         acc[k] = make_double2(0.0, 0.0);
 }
 
-// Same arithmetic as the handle's IDW raster (SPH_SW_2019.f90:14310-14400).
-__global__ void k_noalloc_idw(const float2* pos, const float* rho, const int* flag, int n, int nx, int ny, float xmin,
-                              float ymin, float dx, float dy, double2* acc) {
-    float distg = sqrtf(dx * dx + dy * dy);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (flag && flag[i]) continue;
-        float2 p = pos[i];
-        float h = rho[i];
-        int ipx = (int)((p.x - xmin) / dx + 1.f);
-        int ipy = (int)((p.y - ymin) / dy + 1.f);
-        int ix0 = max(1, ipx - 1), iy0 = max(1, ipy - 1), ix1 = min(nx, ipx + 2), iy1 = min(ny, ipy + 2);
-        for (int ix = ix0; ix <= ix1; ix++)
-            for (int iy = iy0; iy <= iy1; iy++) {
-                int ip = (iy - 1) * nx + (ix - 1);
-                float ddx = p.x - (xmin + (float)(ix - 1) * dx);
-                ddx = ddx * ddx;
-                float ddy = p.y - (ymin + (float)(iy - 1) * dy);
-                ddy = ddy * ddy;
-                float dist = sqrtf(ddx + ddy);
-                dist = (1.e-6f > dist) ? 1.e-6f : dist;
-                dist = dist / distg;
-                atomicAdd(&acc[ip].x, (double)(h / dist));
-                atomicAdd(&acc[ip].y, (double)(1.f / dist));
-            }
+// The terms of the handle's IDW raster (SPH_SW_2019.f90:14310-14400).
+__global__ void __launch_bounds__(32 * gfsph::kScatterWarps) k_noalloc_idw(const float2* pos, const float* rho,
+                                                                             const int* flag, int n, int nx, int ny,
+                                                                             float xmin, float ymin, float dx,
+                                                                             float dy, double2* acc) {
+    const float distg = sqrtf(dx * dx + dy * dy);
+    // block-uniform trip count: every lane of a warp reaches idw_scatter
+    for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
+        const int i = i0 + threadIdx.x;
+        const bool part = i < n && !(flag && flag[i]);
+        gfsph::idw_scatter(nx, ny, xmin, ymin, dx, dy, distg, part ? pos[i] : make_float2(0.f, 0.f),
+                           part ? rho[i] : 0.f, part, acc);
     }
 }
 
