@@ -1,5 +1,6 @@
 // C ABI of the SPH step (include/gfsph.h): handle, device memory, the
 // per-step launch sequence, CUDA-graph replay and capacity growth.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -56,10 +57,45 @@ __global__ void k_unsort(PState B, int n, PState U) {
     }
 }
 
-// Uaux(1,:) = pwp0rel * rho * alphas at input (Input_SW, SPH_SW_2019.f90:1829-1852).
-__global__ void k_pwp_init(float* pwp, const float* rho, int n, float pwp0rel, float alfs) {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
-        pwp[s] = pwp0rel * (rho[s] * alfs);
+// The state of a new run in caller order: the arrays given, read where the
+// caller has them (null: they are in B already), out-of-domain flags of 0
+// where none are given, the identity order, and u or Uaux(1) at the start,
+// pwp0rel * rho * alphas (Input_SW, SPH_SW_2019.f90:1829-1852).
+struct NewState {
+    const float2 *x, *v;
+    const float *rho, *mass, *hsml;
+    const int* flag;
+    int keep_flag;       // the flags are in B already
+    float* mass0;        // nfric 3: the mass at the start of the run (Input_SW :1995), or null
+    int pwp;             // icpwp of the run
+    float pwp0rel, alfs;
+};
+
+__global__ void k_take(NewState a, int n, PState B) {
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+        const float rho = a.x ? a.rho[s] : B.rho[s], mass = a.x ? a.mass[s] : B.mass[s];
+        if (a.x) {
+            const float2 x = a.x[s], v = a.v[s];
+            const float hs = a.hsml[s];
+            B.pos[s] = x; B.vel[s] = v; B.rho[s] = rho; B.mass[s] = mass; B.hsml[s] = hs;
+        }
+        if (!a.keep_flag) B.flag[s] = a.flag ? a.flag[s] : 0;
+        B.id[s] = s;
+        B.pwp[s] = a.pwp ? a.pwp0rel * (rho * a.alfs) : 0.f;
+        if (a.mass0) a.mass0[s] = mass;
+    }
+}
+
+// The caller-order state to arrays of the caller (null: not wanted).
+__global__ void k_give(PState U, int n, float2* x, float2* v, float* rho, float* mass, float* hsml, int* flag) {
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
+        if (x) x[s] = U.pos[s];
+        if (v) v[s] = U.vel[s];
+        if (rho) rho[s] = U.rho[s];
+        if (mass) mass[s] = U.mass[s];
+        if (hsml) hsml[s] = U.hsml[s];
+        if (flag) flag[s] = U.flag[s];
+    }
 }
 
 // dst[s] = src[id[s]]: a caller array in the original order into slot order.
@@ -71,8 +107,12 @@ __global__ void k_unsort_f2(const float2* src, const int* id, int n, float2* dst
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) dst[id[s]] = src[s];
 }
 
-__global__ void k_iota(int* id, int n) {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) id[s] = s;
+// One launch instead of five memsets and their gaps.
+__global__ void k_hazard_clear(double* sum_h, double* sum_v, unsigned int* max_h, unsigned int* max_v, int* cnt, int np) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < np; k += gridDim.x * blockDim.x) {
+        sum_h[k] = 0.0; sum_v[k] = 0.0;
+        max_h[k] = 0u; max_v[k] = 0u; cnt[k] = 0;
+    }
 }
 
 __global__ void k_hazard_finish(const unsigned int* mo, float* out, int np) {
@@ -364,7 +404,7 @@ int enqueue_search(gfsph_handle* h, int advance) {
     int nbscan = (h->cap_blocks + kScanTile - 1) / kScanTile;
     const int* nblk = reinterpret_cast<const int*>(reinterpret_cast<const char*>(S) + offsetof(StepScalars, nblocks));
     const int* ncel = reinterpret_cast<const int*>(reinterpret_cast<const char*>(S) + offsetof(StepScalars, ncells));
-    if (!advance) { launch(h, K_PREP, [&] { pdl_launch(k_prep, 1, 32, st, S, advance); }); nk++; }
+    if (!advance) { launch(h, K_PREP, [&] { pdl_launch(k_prep, 1, 32, st, S, 0, 0.0); }); nk++; }
     const GridArgs ga{h->cap_blocks, h->cap_cells, kMaxCells, h->level_factor, h->cell_div, h->reg_levels};
     const int bb = std::min(kBoundsBlocks, blocks_for(n, kThreadsBounds));
     launch(h, K_BOUNDS, [&] { pdl_launch(k_bounds, bb, kThreadsBounds, st, h->B, n, h->rheo, h->dem, S, h->bparts); });
@@ -737,6 +777,60 @@ int set_field(gfsph_handle* h, size_t off, T value) {
     *host = value;
     CK(cudaMemcpyAsync(reinterpret_cast<char*>(h->S) + off, host, sizeof(T), cudaMemcpyHostToDevice, h->stream));
     return 0;
+}
+
+struct Span {  // n elements of an array of the caller; null: not given
+    const void* p;
+    size_t elem;
+};
+
+// Whether a kernel may read (write: or write) the caller's host arrays where
+// they are: all of them page-locked, mapped into this device's address space
+// over their whole length, and aligned to their elements.  A call has up to
+// six arrays and each copy costs the host and the stream a few us whatever
+// its size; one kernel over the bus costs one launch.  us with copies and in
+// place, upload with set_time / download: 850 particles 57 / 48 and 30 / 33,
+// 23k 68 / 64 and 42 / 47, 100k 108 / 107 and 84 / 95, 200k 163 / 164 and 139 /
+// 157, 500k 314 / 339 and 305 / 342, 1M 571 / 627 and 574 / 652: from ~300k on
+// the bus is what counts and the copy engine uses it a little better.
+constexpr size_t kInPlaceBytes = 8 << 20;
+bool in_place(const Span* a, int count, size_t n, bool write) {
+    using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Query query = [] {  // looked up once: libcuda is not linked
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 7000, cudaEnableDefault, &r) != cudaSuccess ||
+            r != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<Query>(f);
+    }();
+    if (!query) return false;
+    size_t bytes = 0;
+    for (int k = 0; k < count; k++)
+        if (a[k].p) bytes += n * a[k].elem;
+    if (bytes > kInPlaceBytes) return false;
+    for (int k = 0; k < count; k++) {
+        if (!a[k].p) continue;
+        const uintptr_t p = reinterpret_cast<uintptr_t>(a[k].p);
+        if (p % a[k].elem) return false;
+        unsigned type = 0, managed = 1;
+        CUdeviceptr dev = 0, start = 0;
+        size_t size = 0;
+        CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                      CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                      CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+        void* to[] = {&type, &managed, &dev, &start, &size};
+        if (query(5, what, to, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
+        if (type != CU_MEMORYTYPE_HOST || managed || dev != p) return false;
+        if (p < start || p + n * a[k].elem > start + size) return false;
+        unsigned flags = 0;
+        if (write && (cudaHostGetFlags(&flags, const_cast<void*>(a[k].p)) != cudaSuccess ||
+                      (flags & cudaHostRegisterReadOnly))) {
+            cudaGetLastError();
+            return false;
+        }
+    }
+    return true;
 }
 
 // After a step batch stopped on a capacity error: grow and clear the error.
@@ -1214,16 +1308,26 @@ int gfsph_upload(gfsph_handle* h, int n, const float* x, const float* v, const f
         if (st) return drop_state(h, st);
     }
     cudaStream_t st = h->stream;
-    CK(cudaMemcpyAsync(h->B.pos, x, (size_t)n * sizeof(float2), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(h->B.vel, v, (size_t)n * sizeof(float2), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(h->B.rho, rho, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(h->B.mass, mass, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, st));
-    // mass0 = mass at the start of the run (Input_SW SPH_SW_2019.f90:1995)
-    if (h->rheo.nfric == 3) CK(cudaMemcpyAsync(h->mass0_u, mass, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(h->B.hsml, hsml, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, st));
-    if (out_flag) CK(cudaMemcpyAsync(h->B.flag, out_flag, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, st));
-    else CK(cudaMemsetAsync(h->B.flag, 0, (size_t)n * sizeof(int), st));
-    launch(h, K_UNSORT, [&] { k_iota<<<blocks_for(n), kThreads, 0, st>>>(h->B.id, n); });
+    const Span in[] = {{x, 8}, {v, 8}, {rho, 4}, {mass, 4}, {hsml, 4}, {out_flag, 4}};
+    NewState a{};
+    if (in_place(in, 6, n, false)) {
+        a.x = reinterpret_cast<const float2*>(x);
+        a.v = reinterpret_cast<const float2*>(v);
+        a.rho = rho; a.mass = mass; a.hsml = hsml; a.flag = out_flag;
+    } else {
+        CK(cudaMemcpyAsync(h->B.pos, x, (size_t)n * sizeof(float2), cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(h->B.vel, v, (size_t)n * sizeof(float2), cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(h->B.rho, rho, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(h->B.mass, mass, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(h->B.hsml, hsml, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, st));
+        if (out_flag) CK(cudaMemcpyAsync(h->B.flag, out_flag, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, st));
+        a.keep_flag = out_flag != nullptr;
+    }
+    if (h->rheo.nfric == 3) a.mass0 = h->mass0_u;
+    a.pwp = h->rheo.icpwp;
+    a.pwp0rel = h->P.pwp0rel;
+    a.alfs = h->P.cst[13];
+    launch(h, K_UNSORT, [&] { k_take<<<blocks_for(n), kThreads, 0, st>>>(a, n, h->B); });
     if (h->rheo.ws) {  // the material of each particle, in caller order
         std::vector<unsigned char> sp((size_t)n, 1);
         if (itype)
@@ -1231,12 +1335,6 @@ int gfsph_upload(gfsph_handle* h, int n, const float* x, const float* v, const f
         CK(cudaMemcpyAsync(h->spec_u, sp.data(), (size_t)n, cudaMemcpyHostToDevice, st));
         CK(cudaStreamSynchronize(st));  // sp is a local
     }
-    if (h->rheo.icpwp != 0)  // u (icpwp 1) or Uaux(1) (icpwp 3): the same start, :1724-1737, 1829-1852
-        launch(h, K_UNSORT, [&] {
-            k_pwp_init<<<blocks_for(n), kThreads, 0, st>>>(h->B.pwp, h->B.rho, n, h->P.pwp0rel, h->P.cst[13]);
-        });
-    else
-        CK(cudaMemsetAsync(h->B.pwp, 0, (size_t)n * sizeof(float), st));
     CK(cudaGetLastError());
     h->has_state = true;
     h->searched = false;
@@ -1251,12 +1349,21 @@ int gfsph_download(gfsph_handle* h, float* x, float* v, float* rho, float* mass,
     int n = h->n;
     cudaStream_t st = h->stream;
     launch(h, K_UNSORT, [&] { k_unsort<<<blocks_for(n), kThreads, 0, st>>>(h->B, n, h->U); });
-    if (x) CK(cudaMemcpyAsync(x, h->U.pos, (size_t)n * sizeof(float2), cudaMemcpyDeviceToHost, st));
-    if (v) CK(cudaMemcpyAsync(v, h->U.vel, (size_t)n * sizeof(float2), cudaMemcpyDeviceToHost, st));
-    if (rho) CK(cudaMemcpyAsync(rho, h->U.rho, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, st));
-    if (mass) CK(cudaMemcpyAsync(mass, h->U.mass, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, st));
-    if (hsml) CK(cudaMemcpyAsync(hsml, h->U.hsml, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, st));
-    if (out_flag) CK(cudaMemcpyAsync(out_flag, h->U.flag, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, st));
+    const Span out[] = {{x, 8}, {v, 8}, {rho, 4}, {mass, 4}, {hsml, 4}, {out_flag, 4}};
+    if (in_place(out, 6, n, true)) {
+        launch(h, K_UNSORT, [&] {
+            k_give<<<blocks_for(n), kThreads, 0, st>>>(h->U, n, reinterpret_cast<float2*>(x), reinterpret_cast<float2*>(v),
+                                                       rho, mass, hsml, out_flag);
+        });
+        CK(cudaGetLastError());
+    } else {
+        if (x) CK(cudaMemcpyAsync(x, h->U.pos, (size_t)n * sizeof(float2), cudaMemcpyDeviceToHost, st));
+        if (v) CK(cudaMemcpyAsync(v, h->U.vel, (size_t)n * sizeof(float2), cudaMemcpyDeviceToHost, st));
+        if (rho) CK(cudaMemcpyAsync(rho, h->U.rho, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, st));
+        if (mass) CK(cudaMemcpyAsync(mass, h->U.mass, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, st));
+        if (hsml) CK(cudaMemcpyAsync(hsml, h->U.hsml, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, st));
+        if (out_flag) CK(cudaMemcpyAsync(out_flag, h->U.flag, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost, st));
+    }
     CK(cudaStreamSynchronize(st));
     return GFSPH_OK;
 } catch (...) {  // a C++ exception never crosses the C ABI
@@ -1302,8 +1409,10 @@ int gfsph_get_time(gfsph_handle* h, double* t, float* dt) try {
 
 int gfsph_set_time(gfsph_handle* h, double t, float dt) try {
     if (!h || !(dt > 0.f)) return GFSPH_ERR_ARG;
-    set_field<double>(h, offsetof(StepScalars, time), t);
-    set_field<float>(h, offsetof(StepScalars, dt), dt);
+    h->hS->time = t;
+    h->hS->dt = dt;
+    k_set_time<<<1, 1, 0, h->stream>>>(h->S, t, dt);
+    CK(cudaGetLastError());
     CK(cudaStreamSynchronize(h->stream));
     return GFSPH_OK;
 } catch (...) {  // a C++ exception never crosses the C ABI
@@ -1316,9 +1425,7 @@ namespace {
 
 // Enqueues one chunk of steps (no host synchronisation).
 int enqueue_chunk(gfsph_handle* h, int chunk, double t_end) {
-    set_field<double>(h, offsetof(StepScalars, t_end), t_end);
-    set_field<int>(h, offsetof(StepScalars, steps_done), 0);
-    launch(h, K_PREP, [&] { k_prep<<<1, 32, 0, h->stream>>>(h->S, 1); });
+    launch(h, K_PREP, [&] { k_prep<<<1, 32, 0, h->stream>>>(h->S, 1, t_end); });
     if (h->profile) {
         for (int s = 0; s < chunk; s++) {
             enqueue_step(h);
@@ -1628,11 +1735,11 @@ int gfsph_hazard_reset(gfsph_handle* h) try {
         }
     }
     cudaStream_t s = h->stream;
-    CK(cudaMemsetAsync(h->haz_sum_h, 0, (size_t)np * sizeof(double), s));
-    CK(cudaMemsetAsync(h->haz_sum_v, 0, (size_t)np * sizeof(double), s));
-    CK(cudaMemsetAsync(h->haz_max_h, 0, (size_t)np * sizeof(unsigned int), s));
-    CK(cudaMemsetAsync(h->haz_max_v, 0, (size_t)np * sizeof(unsigned int), s));
-    CK(cudaMemsetAsync(h->haz_cnt, 0, (size_t)np * sizeof(int), s));
+    launch(h, K_HAZARD, [&] {
+        k_hazard_clear<<<blocks_for(np, 256), 256, 0, s>>>(h->haz_sum_h, h->haz_sum_v, h->haz_max_h, h->haz_max_v,
+                                                           h->haz_cnt, np);
+    });
+    CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s));
     return GFSPH_OK;
 } catch (...) {  // a C++ exception never crosses the C ABI

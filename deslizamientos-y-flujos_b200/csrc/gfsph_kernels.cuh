@@ -238,11 +238,20 @@ __device__ __forceinline__ void prepare_step(StepScalars* S, int advance) {
     for (int k = 0; k < kMaxLevels; k++) S->lev_hmax_o[k] = 0u;
 }
 
-__global__ void k_prep(StepScalars* S, int advance) {
+// advance: the start of a batch of steps up to t_end.
+__global__ void k_prep(StepScalars* S, int advance, double t_end) {
     PDL_ENTRY();
     StepScalars* L = scalars_to_smem(S);
-    if (threadIdx.x == 0) prepare_step(L, advance);
+    if (threadIdx.x == 0) {
+        if (advance) { L->t_end = t_end; L->steps_done = 0; }
+        prepare_step(L, advance);
+    }
     scalars_from_smem(S, L);
+}
+
+__global__ void k_set_time(StepScalars* S, double t, float dt) {
+    S->time = t;
+    S->dt = dt;
 }
 
 __device__ __forceinline__ float warp_min(float v) {
