@@ -250,7 +250,8 @@ struct gfsph_handle {
     long long prof_cnt[K_COUNT]{};
     long long launches = 0;
     bool has_state = false, searched = false;
-    bool sparse_seen = false;  // a step has used the block-sparse layout: its launches get the full grids
+    bool sparse_seen = false;  // the latest steps used the block-sparse layout: its launches get the full grids
+    int dense_chunks = 0;      // chunks in a row that ended in the dense layout since
     // outputs
     double2* d_racc = nullptr;
     float* d_rout = nullptr;
@@ -333,25 +334,30 @@ void with_skf(const gfsph_handle* h, F&& f) {
 // Calls f with std::integral_constant<int, lanes per particle> of k_density
 // for n particles.  Few particles leave the chip idle and the step waits for
 // the longest chain of one lane: more lanes shorten it (850 particles: 57 us a
-// launch with one, 11 with 8; 23k: 4 and 8 lanes equal, 3.29 and 3.32 ms per 25
-// steps).  From ~100k on the chip is full and the lanes' uneven rows and
-// shuffles count (200k particles, 20 steps with their copies: 6.4, 6.0, 6.4 ms
+// launch with one, 9 with 8; 23k: 4 and 8 lanes equal, 3.29 and 3.32 ms per 25
+// steps).  Then the chip is full and the lanes' uneven rows and shuffles count:
+// us a launch with 4 and 2 lanes 20k 23 and 25, 30k 26 and 26, 45k 34 and 27.5,
+// 60k 38.5 and 32 (200k particles, 20 steps with their copies: 6.4, 6.0, 6.4 ms
 // for 1, 2, 4 lanes; 1M, 10 steps: 10.2, 9.7, 10.6 ms).
 template <class F>
 void with_lanes(int n, F&& f) {
     if (n < 12000) f(std::integral_constant<int, 8>{});
-    else if (n < 100000) f(std::integral_constant<int, 4>{});
+    else if (n < 45000) f(std::integral_constant<int, 4>{});
     else f(std::integral_constant<int, 2>{});
 }
 
-// The same for k_iforce and k_xsph, which wait for their gathers: us a launch
-// (k_iforce / k_xsph) for 850 particles 13 / 10 with one lane, 5 / 5 with 4,
-// 4 / 3 with 8; 23k 16 / 13, 7 / 5, 9 / 7; 200k 33 / 30 with one, 33 / 27 with 2,
-// 41 / 32 with 4; 1M 130 / 107 with one, 150 / 120 with 2.
+// The same for the kernels over the neighbour table, which wait for their
+// gathers.  k_iforce and k_xsph, us a launch with 8 / 4 / 2 / 1 lanes: 850
+// particles 4 and 3 with 8, 5 and 5 with 4; 23k 9 and 7, 7 and 5; 200k - , 41
+// and 32, 33 and 27, 33 and 30; 1M -, -, 150 and 120, 130 and 107.  Between 4 and 2
+// (the whole step): 30k 85 and 98, 45k 95 and 92.5, 60k 108 and 101, 80k 121 and
+// 120.  four: up to where 4 lanes (the adjoint kernels, with more work a pair,
+// gain from them longer: 18 us a launch against 24 for 50k).
+constexpr int kAdjFourLanes = 100000;
 template <class F>
-void with_pair_lanes(int n, F&& f) {
+void with_pair_lanes(int n, F&& f, int four = 45000) {
     if (n < 12000) f(std::integral_constant<int, 8>{});
-    else if (n < 100000) f(std::integral_constant<int, 4>{});
+    else if (n < four) f(std::integral_constant<int, 4>{});
     else if (n < 500000) f(std::integral_constant<int, 2>{});
     else f(std::integral_constant<int, 1>{});
 }
@@ -1467,9 +1473,16 @@ int finish_chunk(gfsph_handle* h, int chunk, double t_end, int& done, int& guard
     if (st) return st;
     done += h->hS->steps_done;
     h->searched = true;
-    if (h->hS->sparse && !h->sparse_seen) {
-        h->sparse_seen = true;
-        drop_graphs(h);
+    // the launches of the layout not in use are small (sparse_seen); back to the dense one only after it has lasted
+    // some chunks, for the graphs are captured anew
+    if (!h->hS->sparse != !h->sparse_seen) {
+        if (h->hS->sparse || ++h->dense_chunks == 4) {
+            h->sparse_seen = h->hS->sparse != 0;
+            h->dense_chunks = 0;
+            drop_graphs(h);
+        }
+    } else {
+        h->dense_chunks = 0;
     }
     if (h->hS->err) {
         if (++guard > 16) return GFSPH_ERR_CAPACITY;
@@ -2295,7 +2308,7 @@ int gfsph_adjoint_backward(gfsph_adjoint* a, const float* gx, const float* gv, c
                         constexpr int G = decltype(g)::value;
                         k_adj_xsph<G><<<blocks_for((long long)n * G), 128, 0, st>>>(
                             h->A, Q, h->rheo, n, h->velfin, a->lv2, a->lvp, a->lh, a->lms, a->lxacc, a->lhsacc);
-                    });
+                    }, kAdjFourLanes);
                 });
             } else {
                 CK(cudaMemcpyAsync(a->lvp, a->lv2, un * sizeof(float2), cudaMemcpyDeviceToDevice, st));
@@ -2309,7 +2322,7 @@ int gfsph_adjoint_backward(gfsph_adjoint* a, const float* gx, const float* gv, c
                     constexpr int G = decltype(g)::value;
                     k_adj_gather<G><<<blocks_for((long long)n * G), 128, 0, st>>>(h->A, Q, h->rheo, n, a->lin, a->lh, a->lms,
                                                                                  a->lxacc, a->lhsacc);
-                });
+                }, kAdjFourLanes);
             });
             launch(h, K_ADJOINT, [&] {
                 k_adj_scatter<<<pb, kThreads, 0, st>>>(h->A, n, a->lxacc, a->lv0, a->lms, a->lx, a->lv, a->lm,

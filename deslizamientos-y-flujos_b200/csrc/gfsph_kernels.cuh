@@ -1286,6 +1286,18 @@ __device__ __forceinline__ void force_big(const PState& A, const Search& Q, cons
     }
 }
 
+// With 4 or 8 lanes a particle a lane has some 6 to 12 entries and the one by
+// one rest of a loop over fours is up to half of its chain of loads: there
+// the rest goes together, with the registers of fewer resident blocks (the
+// few particles leave room).  us with ~6 of the event, k_iforce / k_xsph: 850
+// particles 10.6 / 10.5 -> 8.9 / 8.6; a step of 13k 79 -> 75, of 23k 91 -> 88.
+// With 1 or 2 lanes occupancy hides the rest and the registers spill (1M
+// particles 142 -> 210).
+template <int G>
+constexpr bool kFewPerLane = G >= 4;
+template <int G>
+constexpr int kPairBlocks = G == 8 ? 2 : G == 4 ? 3 : 4;
+
 // Internal acceleration of a regular particle over its neighbour table, by G
 // lanes: lane gl takes every G-th entry.  Per entry the stored gradient and
 // the gathers of (x, m) and the pressure term of the neighbour (its depth too
@@ -1312,17 +1324,19 @@ __device__ __forceinline__ void internal_force(const Search& Q, const Rheo& c, c
         else pressure_terms(c, pi_, rhoi, pj, c.pa_sph == 1 ? rho[e] : 0.f, o.w, d0, d1, a0, a1);
     };
     // four entries at a time, the next four on their way meanwhile
+    constexpr bool few = kFewPerLane<G>;  // the last ones, up to three, together as well
     int k = gl;
     int e[4];
     TabGrad<SKF> g[4];
     auto fetch = [&](int k0) {
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            e[u] = __ldg(Q.nj + tab + (size_t)(k0 + u * G) * kTabStride);
-            g[u].load(Q, tab + (size_t)(k0 + u * G) * kTabStride);
-        }
+        for (int u = 0; u < 4; u++)
+            if (!few || k0 + u * G < cnt) {
+                e[u] = __ldg(Q.nj + tab + (size_t)(k0 + u * G) * kTabStride);
+                g[u].load(Q, tab + (size_t)(k0 + u * G) * kTabStride);
+            }
     };
-    if (k + 3 * G < cnt) fetch(k);
+    if (few || k + 3 * G < cnt) fetch(k);
     for (; k + 3 * G < cnt; k += 4 * G) {
         int je[4];
         TabGrad<SKF> gg[4];
@@ -1336,11 +1350,25 @@ __device__ __forceinline__ void internal_force(const Search& Q, const Rheo& c, c
             o[u] = __ldg(&Q.xhm[j]);
             pj[u] = __ldg(&Q.pterm[j]);
         }
-        if (k + 7 * G < cnt) fetch(k + 4 * G);
+        if (few || k + 7 * G < cnt) fetch(k + 4 * G);
 #pragma unroll
         for (int u = 0; u < 4; u++) term(je[u], gg[u], o[u], pj[u]);
     }
-    for (; k < cnt; k += G) {
+    if (few) {
+        float4 o[3];
+        float pj[3];
+#pragma unroll
+        for (int u = 0; u < 3; u++)
+            if (k + u * G < cnt) {
+                const int j = WS ? (e[u] & ~kCrossBit) : e[u];
+                o[u] = __ldg(&Q.xhm[j]);
+                pj[u] = __ldg(&Q.pterm[j]);
+            }
+#pragma unroll
+        for (int u = 0; u < 3; u++)
+            if (k + u * G < cnt) term(e[u], g[u], o[u], pj[u]);
+    }
+    for (; !few && k < cnt; k += G) {
         const int ek = __ldg(Q.nj + tab + (size_t)k * kTabStride), j = WS ? (ek & ~kCrossBit) : ek;
         TabGrad<SKF> gk;
         gk.load(Q, tab + (size_t)k * kTabStride);
@@ -1505,7 +1533,7 @@ __device__ __forceinline__ void rk_finish(const PState& A, const Search& Q, Step
 // cross (soil and water, first stage): also the sums over the soil-water
 // pairs, from the same walk.
 template <int SKF, bool WS, int G>
-__global__ void __launch_bounds__(kBigThreads, 4) k_iforce(PState A, Search Q, StepScalars* S, Rheo c, int n, int cross) {
+__global__ void __launch_bounds__(kBigThreads, kPairBlocks<G>) k_iforce(PState A, Search Q, StepScalars* S, Rheo c, int n, int cross) {
     PDL_ENTRY();
     if (S->skip) return;
     if (blockIdx.x < kBigBlocks) {
@@ -2068,14 +2096,15 @@ __device__ __forceinline__ void xsph_big(const Search& Q, const StepScalars* S, 
 }
 
 template <int SKF, bool WS, int G>
-__global__ void __launch_bounds__(kBigThreads, 4) k_xsph(PState A, Search Q, StepScalars* S, Rheo c, int n, PState B) {
+__global__ void __launch_bounds__(kBigThreads, kPairBlocks<G>) k_xsph(PState A, Search Q, StepScalars* S, Rheo c, int n, PState B) {
     PDL_ENTRY();
     if (S->skip || !c.av_vel) return;
     if (blockIdx.x < kBigBlocks) {
         xsph_big<SKF, WS>(Q, S, B);
         return;
     }
-    constexpr int P = 32 / G;  // particles per warp
+    constexpr int P = 32 / G;     // particles per warp
+    constexpr bool few = kFewPerLane<G>;
     const int nreg = S->nreg;
     const int lane = threadIdx.x & 31, gl = lane % G, bid = blockIdx.x - kBigBlocks, nb = gridDim.x - kBigBlocks;
     const int nw = (nreg + P - 1) / P;
@@ -2099,12 +2128,13 @@ __global__ void __launch_bounds__(kBigThreads, 4) k_xsph(PState A, Search Q, Ste
         float w[4];
         auto fetch = [&](int k0) {
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                e[u] = __ldcs(Q.nj + tab + (size_t)(k0 + u * G) * kTabStride);
-                w[u] = __ldcs(Q.nw + tab + (size_t)(k0 + u * G) * kTabStride);
-            }
+            for (int u = 0; u < 4; u++)
+                if (!few || k0 + u * G < cnt) {
+                    e[u] = __ldcs(Q.nj + tab + (size_t)(k0 + u * G) * kTabStride);
+                    w[u] = __ldcs(Q.nw + tab + (size_t)(k0 + u * G) * kTabStride);
+                }
         };
-        if (k + 3 * G < cnt) fetch(k);
+        if (few || k + 3 * G < cnt) fetch(k);
         for (; k + 3 * G < cnt; k += 4 * G) {
             int je[4];
             float ww[4];
@@ -2115,13 +2145,23 @@ __global__ void __launch_bounds__(kBigThreads, 4) k_xsph(PState A, Search Q, Ste
                 ww[u] = w[u];
                 sj[u] = Q.xsv[WS ? (e[u] & ~kCrossBit) : e[u]];
             }
-            if (k + 7 * G < cnt) fetch(k + 4 * G);
+            if (few || k + 7 * G < cnt) fetch(k + 4 * G);
 #pragma unroll
             for (int u = 0; u < 4; u++)
                 if (!WS || je[u] >= 0)  // type 0 only (SPH_MAIN_2019.f90:3071)
                     xsph_terms(vi, rhoi, make_float2(sj[u].x, sj[u].y), sj[u].z, sj[u].w, ww[u], a0, a1);
         }
-        for (; k < cnt; k += G) {
+        if (few) {
+            float4 sj[3];
+#pragma unroll
+            for (int u = 0; u < 3; u++)
+                if (k + u * G < cnt) sj[u] = Q.xsv[WS ? (e[u] & ~kCrossBit) : e[u]];
+#pragma unroll
+            for (int u = 0; u < 3; u++)
+                if (k + u * G < cnt && (!WS || e[u] >= 0))
+                    xsph_terms(vi, rhoi, make_float2(sj[u].x, sj[u].y), sj[u].z, sj[u].w, w[u], a0, a1);
+        }
+        for (; !few && k < cnt; k += G) {
             const int e = __ldcs(Q.nj + tab + (size_t)k * kTabStride);
             const float w = __ldcs(Q.nw + tab + (size_t)k * kTabStride);
             const float4 sj = Q.xsv[WS ? (e & ~kCrossBit) : e];

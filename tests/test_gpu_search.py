@@ -84,3 +84,9 @@ def test_coarse_particles_by_direct_scan(gfsph_lib, oracle_mod, far, hs):
 def test_more_coarse_particles_than_the_direct_scan(gfsph_lib, oracle_mod):
     x, h = cloud(60000, 7, 1100.0, 1.0, 4500, 7.0)
     check(oracle_mod, x, h, forces=False)
+
+
+@pytest.mark.parametrize("n", [44999, 45001])
+def test_sets_and_forces_where_lanes_change(gfsph_lib, oracle_mod, n):
+    x, h = cloud(n, n, 500.0, 1.8)
+    check(oracle_mod, x, h)
