@@ -33,8 +33,9 @@
 // node kernels read place k of 32 nodes as one run, whatever the mesh.
 // Every sum runs in the Fortran's order with IEEE FP32 operations (the
 // library is built without FMA contraction), so the device step equals the
-// single-precision restatement bit for bit; real powers (Manning's 7/3,
-// Coussot's) and the exp of the tanfi decay are taken in FP64 and rounded once.
+// single-precision restatement bit for bit; real powers (Coussot's; Manning's
+// 7/3 by pow73, which rounds as the FP64 power does) and the exp of the tanfi
+// decay are taken in FP64 and rounded once.
 //
 // Scope: nsour 1, itens 0, icpwpF 0, no prescribed, absorbing or loaded
 // boundary nodes (every boundary node is a wall), no atmospheric pressure or
@@ -253,8 +254,10 @@ __device__ __forceinline__ void gauss_point(int ig, float sh[3]) {
     sh[2] = (1.0f - sh[0]) - sh[1];
 }
 
-// Bound by the FP64 power of Manning's law (three a triangle) and by L2: per
+// Bound by issue and by L2 at 20 warps an SM (96 registers; held to 80 it
+// spills and is no faster): three evaluations of Manning's law a triangle; per
 // element 56 B of its own, three gathers of 32 B, three places of 36 B written.
+// 498k triangles: 46 us with the FP64 pow and fields apart, 36 so.
 template <int NG>
 __global__ void __launch_bounds__(kGflThreads) k_gfl_elems(GflDev d, GflConst c, float tanfi, float dt) {
     GFL_ENTRY();

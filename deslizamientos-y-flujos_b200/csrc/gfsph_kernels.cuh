@@ -997,9 +997,10 @@ __device__ __forceinline__ void density_big(const PState& A, const Search& Q, co
 }
 
 // Bound by FP32 issue and the latency of the gathers: 200k particles (release,
-// two lanes) 89 us a launch where one thread per particle, evaluating each
-// pair as it was found, took 115; the flow with coarse levels 106 against 190;
-// 1M particles 390 against 480.  Instantiated for both cell layouts; the
+// two lanes) 78 us a launch (89 before the pairs were evaluated two at a time)
+// where one thread per particle, evaluating each pair as it was found, took
+// 115; the flow with coarse levels 94 (106) against 190; 1M particles 350 (390)
+// against 480.  Instantiated for both cell layouts; the
 // launch whose layout this step does not use returns at once.
 template <bool SPARSE, int SKF, bool WS, int G>
 __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, Search Q, StepScalars* S, Rheo c, int n) {
@@ -1564,8 +1565,7 @@ __global__ void __launch_bounds__(kBigThreads, kPairBlocks<G>) k_iforce(PState A
 }
 
 // The RK45 body for each active particle, entirely in registers: the
-// internal acceleration (stage-invariant, see below; from k_iforce or
-// k_force_big), four stages of
+// internal acceleration (stage-invariant, see below; from k_iforce), four stages of
 // x = x0 + c_i dt v, v = v0 + c_i dt (ex + in) with ExtForces_SW(0) at each
 // stage (SPH_MAIN_2019.f90:808-906), the final update (:908-922), the
 // out-of-domain freeze (Check_Out_Domain), Hungr erosion of mass and the DEM
