@@ -369,10 +369,15 @@ __global__ void __launch_bounds__(128) k_adj_xsph(PState A, Search Q, Rheo c, in
 // Adjoint of the fused RK4 of k_force_rk (stages recomputed in registers):
 // from dL/dx', dL/dv' to dL/dx0, dL/dv0, dL/d(internal acceleration), dL/dh
 // and the parameter sums.
-constexpr int kAdjRkThreads = 64;  // small blocks: 150 registers and a long serial chain, balanced over the SMs
-__global__ void __launch_bounds__(kAdjRkThreads) k_adj_rk(PState A, Search Q, const StepScalars* S, Rheo c, DemView dem, int n,
+// One copy of the stage's code in either direction, the stages' states in shared
+// memory: unrolled, 196 registers and a body beyond the instruction cache took
+// 47 us a launch for 50k particles (a third of a warp's time without an
+// instruction), so 15.
+constexpr int kAdjRkThreads = 64;  // small blocks: many registers and a long serial chain, balanced over the SMs
+__global__ void __launch_bounds__(kAdjRkThreads, 8) k_adj_rk(PState A, Search Q, const StepScalars* S, Rheo c, DemView dem, int n,
                                                 const float2* lx1, const float2* lvp, float* lh, float2* lin,
                                                 double2* lxacc, float2* lv0, double* lpar) {
+    __shared__ float4 stage[4][kAdjRkThreads];  // (x, y, vx, vy) of the thread's own particle
     const float dt = S->dt_step;
     double smu = 0.0, sxi = 0.0, sty = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -381,15 +386,14 @@ __global__ void __launch_bounds__(kAdjRkThreads) k_adj_rk(PState A, Search Q, co
         const float h = A.rho[i];
         const float hc = (h < c.h_inf) ? c.h_inf : h;
         const float2 x0 = A.pos[i], v0 = A.vel[i];
-        float xs[4], ys[4], us[4], ws[4];
         float vx = v0.x, vy = v0.y, ex0 = 0.f, ex1 = 0.f;
-#pragma unroll
+#pragma unroll 1
         for (int s = 0; s < 4; s++) {
             const float f1 = (s == 0) ? 0.f : (s == 3 ? 1.f : 0.5f);
             float fdt = f1 * dt;
             float nxx = x0.x + fdt * vx, nxy = x0.y + fdt * vy;
             float nvx = v0.x + fdt * (ex0 + in0), nvy = v0.y + fdt * (ex1 + in1);
-            xs[s] = nxx; ys[s] = nxy; us[s] = nvx; ws[s] = nvy;
+            stage[s][threadIdx.x] = make_float4(nxx, nxy, nvx, nvy);
             vx = nvx; vy = nvy;
             // the adjoint's scope (nfric 4-6, no erosion) needs only the common laws
             ext_accel<false, false>(c, dem, dt, nxx, nxy, nvx, nvy, hc, 0.f, 0.f, in0, in1, ex0, ex1);
@@ -397,33 +401,27 @@ __global__ void __launch_bounds__(kAdjRkThreads) k_adj_rk(PState A, Search Q, co
         const float2 lx = lx1[i], lv = lvp[i];
         const float dt6 = dt / 6.f;
         ExtGrad g{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.0, 0.0, 0.0};
-        float lxs0[4], lxs1[4], lvs0[4], lvs1[4], lex0[4], lex1[4];
-#pragma unroll
-        for (int s = 0; s < 4; s++) {
-            const float f2 = (s == 0 || s == 3) ? 1.f : 2.f;
-            lxs0[s] = 0.f; lxs1[s] = 0.f;
-            lvs0[s] = dt6 * f2 * lx.x; lvs1[s] = dt6 * f2 * lx.y;
-            lex0[s] = dt6 * f2 * lv.x; lex1[s] = dt6 * f2 * lv.y;
-        }
         float lx00 = lx.x, lx01 = lx.y, lv00 = lv.x, lv01 = lv.y;
         float li0 = dt * lv.x, li1 = dt * lv.y;
-#pragma unroll
+        // what stage s hands to stage s - 1: its shares of dL/dv and dL/d(ex)
+        float cv0 = 0.f, cv1 = 0.f, ce0 = 0.f, ce1 = 0.f;
+#pragma unroll 1
         for (int s = 3; s >= 0; s--) {
+            const float f2 = (s == 0 || s == 3) ? 1.f : 2.f;
+            float lvs0 = dt6 * f2 * lx.x, lvs1 = dt6 * f2 * lx.y, lex0 = dt6 * f2 * lv.x, lex1 = dt6 * f2 * lv.y;
+            if (s < 3) { lvs0 += cv0; lvs1 += cv1; lex0 += ce0; lex1 += ce1; }
             g.x = 0.f; g.y = 0.f; g.vx = 0.f; g.vy = 0.f; g.in0 = 0.f; g.in1 = 0.f;
-            ext_vjp(c, dem, dt, xs[s], ys[s], us[s], ws[s], hc, in0, in1, lex0[s], lex1[s], g);
-            lxs0[s] += g.x; lxs1[s] += g.y;
-            lvs0[s] += g.vx; lvs1[s] += g.vy;
+            const float4 at = stage[s][threadIdx.x];
+            ext_vjp(c, dem, dt, at.x, at.y, at.z, at.w, hc, in0, in1, lex0, lex1, g);
+            lvs0 += g.vx; lvs1 += g.vy;
             li0 += g.in0; li1 += g.in1;
+            lx00 += g.x; lx01 += g.y;
+            lv00 += lvs0; lv01 += lvs1;
             if (s > 0) {
                 const float f1 = (s == 3) ? 1.f : 0.5f;
-                lx00 += lxs0[s]; lx01 += lxs1[s];
-                lvs0[s - 1] += f1 * dt * lxs0[s]; lvs1[s - 1] += f1 * dt * lxs1[s];
-                lv00 += lvs0[s]; lv01 += lvs1[s];
-                lex0[s - 1] += f1 * dt * lvs0[s]; lex1[s - 1] += f1 * dt * lvs1[s];
-                li0 += f1 * dt * lvs0[s]; li1 += f1 * dt * lvs1[s];
-            } else {
-                lx00 += lxs0[0]; lx01 += lxs1[0];
-                lv00 += lvs0[0]; lv01 += lvs1[0];
+                cv0 = f1 * dt * g.x; cv1 = f1 * dt * g.y;
+                ce0 = f1 * dt * lvs0; ce1 = f1 * dt * lvs1;
+                li0 += ce0; li1 += ce1;
             }
         }
         double2 ax = lxacc[i];
