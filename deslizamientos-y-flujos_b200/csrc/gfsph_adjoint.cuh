@@ -300,7 +300,10 @@ __device__ __forceinline__ bool adj_safe(float hi, float hj) {
 
 // Adjoint of av_vel: v''_k = v'_k + eps sum_j c_kj (v'_j - v'_k),
 // c_kj = 2 m_j W_kj / (h_k + h_j), W at the start-of-step geometry.
-// G lanes a particle, as in k_iforce.
+// G lanes a particle, as in k_iforce.  Bound by the latency of the gathers: the
+// next pair's j and W are on their way while a pair is evaluated (50k
+// particles: 39.5 -> 31.7 us a launch; k_adj_gather 62 -> 52).  Held to the
+// registers of 7 or 8 blocks an SM it spills and is no faster.
 template <int G>
 __global__ void __launch_bounds__(128) k_adj_xsph(PState A, Search Q, Rheo c, int n, const float2* velfin,
                                                   const float2* lv2, float2* lvp, float* lh, double* lm,
@@ -315,11 +318,16 @@ __global__ void __launch_bounds__(128) k_adj_xsph(PState A, Search Q, Rheo c, in
         const float hk = A.rho[k], mk = me.w;
         const int cnt = Q.ncount[k];
         double s = 0.0, a0 = 0.0, a1 = 0.0, dm = 0.0, dh = 0.0, dx0 = 0.0, dx1 = 0.0, dhs = 0.0;
+        const size_t tab = tab_base(k, Q.kcap);
+        int jn = 0;
+        float wn = 0.f;
+        if (gl < cnt) { jn = Q.nj[tab + (size_t)gl * kTabStride]; wn = Q.nw[tab + (size_t)gl * kTabStride]; }
         for (int q = gl; q < cnt; q += G) {
-            // the pair's W and grad W as the replayed step's search stored them
-            const size_t at = tab_base(k, Q.kcap) + (size_t)q * kTabStride;
-            const int j = Q.nj[at];
-            const float w = Q.nw[at];
+            // the pair's W and grad W as the replayed step's search stored them, j and W fetched a pair ahead
+            const size_t at = tab + (size_t)q * kTabStride;
+            const int j = jn;
+            const float w = wn;
+            if (q + G < cnt) { jn = Q.nj[at + G * kTabStride]; wn = Q.nw[at + G * kTabStride]; }
             const float4 o = Q.xhm[j];
             float d0, d1;
             adj_grad(Q, c.skf, at, xk, o, adj_safe(me.z, o.z), d0, d1);
@@ -448,7 +456,7 @@ __global__ void __launch_bounds__(kAdjRkThreads, 8) k_adj_rk(PState A, Search Q,
 
 // Adjoint of the summation density h_k = W0 m_k + sum_j m_j W_kj and of the
 // internal force a_k = -sum_j m_j (P_k + P_j) grad W_kj, gathered at k.
-// G lanes a particle, as in k_iforce.
+// G lanes a particle, the next pair's j and W ahead, as in k_adj_xsph.
 template <int G>
 __global__ void __launch_bounds__(128) k_adj_gather(PState A, Search Q, Rheo c, int n, const float2* lin,
                                                     const float* lh, double* lm, double2* lxacc, double* lhsacc) {
@@ -465,11 +473,16 @@ __global__ void __launch_bounds__(128) k_adj_gather(PState A, Search Q, Rheo c, 
         double dm = 0.0;
         double dx0 = 0.0, dx1 = 0.0;
         double dhs = 0.0;
+        const size_t tab = tab_base(k, Q.kcap);
+        int jn = 0;
+        float wn = 0.f;
+        if (gl < cnt) { jn = Q.nj[tab + (size_t)gl * kTabStride]; wn = Q.nw[tab + (size_t)gl * kTabStride]; }
         for (int q = gl; q < cnt; q += G) {
-            // the pair's W and grad W as the replayed step's search stored them
-            const size_t at = tab_base(k, Q.kcap) + (size_t)q * kTabStride;
-            const int j = Q.nj[at];
-            const float w = Q.nw[at];
+            // the pair's W and grad W as the replayed step's search stored them, j and W fetched a pair ahead
+            const size_t at = tab + (size_t)q * kTabStride;
+            const int j = jn;
+            const float w = wn;
+            if (q + G < cnt) { jn = Q.nj[at + G * kTabStride]; wn = Q.nw[at + G * kTabStride]; }
             const float4 o = Q.xhm[j];
             float d0, d1;
             const bool safe = adj_safe(me.z, o.z);
