@@ -252,15 +252,24 @@ __device__ __forceinline__ void ext_vjp(const Rheo& c, const DemView& dem, float
     }
 }
 
+// Whether the replayed step of this sweep is void: it stopped on a capacity
+// (the handle's buffers are not those of the recorded run) or split the
+// particles otherwise than the recorded step did (other search tunables), so
+// that the sorted state, the neighbour counts or the table are not this step's
+// and must not be followed.  The sweep's kernels then do nothing; the host reads
+// the same two words at the end of the segment and returns the error.
+__device__ __forceinline__ bool replay_void(const StepScalars* S) { return (S->err | S->irregular) != 0; }
+
 // Seeds the step's adjoints in sorted order from the caller-order ones:
 // lx1 = dL/dx', lv2 = dL/dv'' (after XSPH), lh = dL/dh (final depth, last
 // step only); clears the accumulators.
 // With sle 1, lhs_o = dL/d hsml' of the next step (caller order, zero after
 // the last) goes back through h_upgrade, hsml' = 2 sqrt(m/h):
 // d hsml'/dh = -hsml'/(2h), d hsml'/dm = hsml'/(2m).
-__global__ void k_adj_seed(const PState A, int n, const float2* lx_o, const float2* lv_o, const float* gh_o,
-                           float2* lx1, float2* lv2, float* lh, double2* lxacc, double* lm, const float* lhs_o,
-                           double* lhsacc) {
+__global__ void k_adj_seed(const PState A, const StepScalars* S, int n, const float2* lx_o, const float2* lv_o,
+                           const float* gh_o, float2* lx1, float2* lv2, float* lh, double2* lxacc, double* lm,
+                           const float* lhs_o, double* lhsacc) {
+    if (replay_void(S)) return;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         int o = A.id[s];
         lx1[s] = lx_o[o];
@@ -305,9 +314,10 @@ __device__ __forceinline__ bool adj_safe(float hi, float hj) {
 // particles: 39.5 -> 31.7 us a launch; k_adj_gather 62 -> 52).  Held to the
 // registers of 7 or 8 blocks an SM it spills and is no faster.
 template <int G>
-__global__ void __launch_bounds__(128) k_adj_xsph(PState A, Search Q, Rheo c, int n, const float2* velfin,
-                                                  const float2* lv2, float2* lvp, float* lh, double* lm,
-                                                  double2* lxacc, double* lhsacc) {
+__global__ void __launch_bounds__(128) k_adj_xsph(PState A, Search Q, const StepScalars* S, Rheo c, int n,
+                                                  const float2* velfin, const float2* lv2, float2* lvp, float* lh,
+                                                  double* lm, double2* lxacc, double* lhsacc) {
+    if (replay_void(S)) return;
     const float eps = 0.3f;
     const int gl = threadIdx.x % G;
     constexpr int P = 128 / G;  // particles per block
@@ -385,6 +395,7 @@ constexpr int kAdjRkThreads = 64;  // small blocks: many registers and a long se
 __global__ void __launch_bounds__(kAdjRkThreads, 8) k_adj_rk(PState A, Search Q, const StepScalars* S, Rheo c, DemView dem, int n,
                                                 const float2* lx1, const float2* lvp, float* lh, float2* lin,
                                                 double2* lxacc, float2* lv0, double* lpar) {
+    if (replay_void(S)) return;
     __shared__ float4 stage[4][kAdjRkThreads];  // (x, y, vx, vy) of the thread's own particle
     const float dt = S->dt_step;
     double smu = 0.0, sxi = 0.0, sty = 0.0;
@@ -458,8 +469,10 @@ __global__ void __launch_bounds__(kAdjRkThreads, 8) k_adj_rk(PState A, Search Q,
 // internal force a_k = -sum_j m_j (P_k + P_j) grad W_kj, gathered at k.
 // G lanes a particle, the next pair's j and W ahead, as in k_adj_xsph.
 template <int G>
-__global__ void __launch_bounds__(128) k_adj_gather(PState A, Search Q, Rheo c, int n, const float2* lin,
-                                                    const float* lh, double* lm, double2* lxacc, double* lhsacc) {
+__global__ void __launch_bounds__(128) k_adj_gather(PState A, Search Q, const StepScalars* S, Rheo c, int n,
+                                                    const float2* lin, const float* lh, double* lm, double2* lxacc,
+                                                    double* lhsacc) {
+    if (replay_void(S)) return;
     const int gl = threadIdx.x % G;
     constexpr int P = 128 / G;  // particles per block
     for (int base = blockIdx.x * P; base < n; base += gridDim.x * P) {
@@ -533,8 +546,10 @@ __global__ void __launch_bounds__(128) k_adj_gather(PState A, Search Q, Rheo c, 
 
 // The step's input adjoints back to the caller's order; volumes accumulate
 // over the steps.
-__global__ void k_adj_scatter(const PState A, int n, const double2* lxacc, const float2* lv0, const double* lm,
-                              float2* lx_o, float2* lv_o, double* lm_o, const double* lhsacc, float* lhs_o) {
+__global__ void k_adj_scatter(const PState A, const StepScalars* S, int n, const double2* lxacc, const float2* lv0,
+                              const double* lm, float2* lx_o, float2* lv_o, double* lm_o, const double* lhsacc,
+                              float* lhs_o) {
+    if (replay_void(S)) return;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         int o = A.id[s];
         double2 a = lxacc[s];

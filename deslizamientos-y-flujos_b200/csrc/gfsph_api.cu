@@ -2039,9 +2039,11 @@ int adj_restore(gfsph_adjoint* a, const float2* x, const float2* v, const float*
 // The backward sweep replays steps that the recording run has taken from
 // the same states with the same deterministic kernels, so their capacity and
 // their particle counts (every particle active and regular) were checked
-// then: within a segment the steps are enqueued without waiting, the error
-// word left set by any failed step (which also makes every later step skip),
-// and checked once at the segment's end.
+// then: within a segment the steps are enqueued without waiting and checked
+// once at the segment's end.  A step can still fail here, if the handle has been
+// uploaded anew (its table is as narrow as at the start again) or has other
+// search tunables than the recording run: the error word stays set and makes
+// every later step skip, and the sweep's kernels look at it (replay_void).
 int adj_segment_check(gfsph_handle* h) {
     int st = read_scalars(h);
     if (st) return st;
@@ -2298,7 +2300,7 @@ int gfsph_adjoint_backward(gfsph_adjoint* a, const float* gx, const float* gv, c
             Search Q = make_search(h);
             const int pb = blocks_for(n);
             launch(h, K_ADJOINT, [&] {
-                k_adj_seed<<<pb, kThreads, 0, st>>>(h->A, n, a->lx, a->lv, (last && gh) ? a->gh : nullptr, a->lx1,
+                k_adj_seed<<<pb, kThreads, 0, st>>>(h->A, h->S, n, a->lx, a->lv, (last && gh) ? a->gh : nullptr, a->lx1,
                                                     a->lv2, a->lh, a->lxacc, a->lms, a->sle ? a->lhs : nullptr,
                                                     a->lhsacc);
             });
@@ -2307,7 +2309,7 @@ int gfsph_adjoint_backward(gfsph_adjoint* a, const float* gx, const float* gv, c
                     with_pair_lanes(n, [&](auto g) {
                         constexpr int G = decltype(g)::value;
                         k_adj_xsph<G><<<blocks_for((long long)n * G), 128, 0, st>>>(
-                            h->A, Q, h->rheo, n, h->velfin, a->lv2, a->lvp, a->lh, a->lms, a->lxacc, a->lhsacc);
+                            h->A, Q, h->S, h->rheo, n, h->velfin, a->lv2, a->lvp, a->lh, a->lms, a->lxacc, a->lhsacc);
                     }, kAdjFourLanes);
                 });
             } else {
@@ -2320,12 +2322,12 @@ int gfsph_adjoint_backward(gfsph_adjoint* a, const float* gx, const float* gv, c
             launch(h, K_ADJOINT, [&] {
                 with_pair_lanes(n, [&](auto g) {
                     constexpr int G = decltype(g)::value;
-                    k_adj_gather<G><<<blocks_for((long long)n * G), 128, 0, st>>>(h->A, Q, h->rheo, n, a->lin, a->lh, a->lms,
-                                                                                 a->lxacc, a->lhsacc);
+                    k_adj_gather<G><<<blocks_for((long long)n * G), 128, 0, st>>>(h->A, Q, h->S, h->rheo, n, a->lin, a->lh,
+                                                                                 a->lms, a->lxacc, a->lhsacc);
                 }, kAdjFourLanes);
             });
             launch(h, K_ADJOINT, [&] {
-                k_adj_scatter<<<pb, kThreads, 0, st>>>(h->A, n, a->lxacc, a->lv0, a->lms, a->lx, a->lv, a->lm,
+                k_adj_scatter<<<pb, kThreads, 0, st>>>(h->A, h->S, n, a->lxacc, a->lv0, a->lms, a->lx, a->lv, a->lm,
                                                        a->lhsacc, a->lhs);
             });
             CK(cudaGetLastError());
