@@ -250,8 +250,6 @@ struct gfsph_handle {
     long long prof_cnt[K_COUNT]{};
     long long launches = 0;
     bool has_state = false, searched = false;
-    bool sparse_seen = false;  // the latest steps used the block-sparse layout: its launches get the full grids
-    int dense_chunks = 0;      // chunks in a row that ended in the dense layout since
     // outputs
     double2* d_racc = nullptr;
     float* d_rout = nullptr;
@@ -438,18 +436,20 @@ int enqueue_search(gfsph_handle* h, int advance) {
         // the two materials' pair types compiled in only when there are two
         with_lanes(n, [&](auto g) {
             constexpr int G = decltype(g)::value;
-            // the launch of the layout not in use returns at once: one block per SM, also where it is used after all
-            const int full = kBigBlocks + std::min(blocks_for((long long)n * G, kDenThreads), 148 * kDenBlocks * 3);
-            const int idle = std::min(full, kBigBlocks + 148);
-            const int db = h->sparse_seen ? idle : full, sb = h->sparse_seen ? full : idle;
+            // Only the device knows which layout a step uses, and the launch for the other returns at once: both have
+            // the same grid, two rounds of resident blocks.  One block per SM for the layout the last batch did not
+            // use is right only until the layout changes: us a step, 60k 96 and 228 where it changed, 200k 211 and
+            // 655, 1M 867 and 2910.  One, two and three rounds for both: 60k 97 each, 200k 217, 211 and 214.5, its
+            // flow 250, 241.5 and 242.5, 1M 884, 867 and 883.
+            const int db = kBigBlocks + std::min(blocks_for((long long)n * G, kDenThreads), 148 * kDenBlocks * 2);
             if (h->rheo.ws) {
                 launch(h, K_DENSITY, [&] { pdl_launch(k_density<false, SKF, true, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
                 launch(h, K_DENSITY_SPARSE,
-                       [&] { pdl_launch(k_density<true, SKF, true, G>, sb, kDenThreads, st, h->A, q, S, h->rheo, n); });
+                       [&] { pdl_launch(k_density<true, SKF, true, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
             } else {
                 launch(h, K_DENSITY, [&] { pdl_launch(k_density<false, SKF, false, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
                 launch(h, K_DENSITY_SPARSE,
-                       [&] { pdl_launch(k_density<true, SKF, false, G>, sb, kDenThreads, st, h->A, q, S, h->rheo, n); });
+                       [&] { pdl_launch(k_density<true, SKF, false, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
             }
         });
     });
@@ -1473,17 +1473,6 @@ int finish_chunk(gfsph_handle* h, int chunk, double t_end, int& done, int& guard
     if (st) return st;
     done += h->hS->steps_done;
     h->searched = true;
-    // the launches of the layout not in use are small (sparse_seen); back to the dense one only after it has lasted
-    // some chunks, for the graphs are captured anew
-    if (!h->hS->sparse != !h->sparse_seen) {
-        if (h->hS->sparse || ++h->dense_chunks == 4) {
-            h->sparse_seen = h->hS->sparse != 0;
-            h->dense_chunks = 0;
-            drop_graphs(h);
-        }
-    } else {
-        h->dense_chunks = 0;
-    }
     if (h->hS->err) {
         if (++guard > 16) return GFSPH_ERR_CAPACITY;
         st = grow_after_error(h);
