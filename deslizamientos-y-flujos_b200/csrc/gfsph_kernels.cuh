@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kThreadsBounds) k_grid(Rheo c, StepScalars* S,
 // Hc*2^k/cell_div over the same box, and one cell-key space covers all
 // levels.  The particles of the first reg_levels levels ("regular") take a
 // thread each and the neighbour table; those of the coarser levels, few and
-// with long neighbour lists, a warp each.  A particle
+// with long neighbour lists, a block or a warp each.  A particle
 // searches each level within hsml_i + (that level's hsml bound), so the
 // neighbour set is the reference's {j : r_ij < 2*(h_i+h_j)/2} exactly.
 // level_factor and cell_div are the search's tunables (gfsph_set_search):
@@ -844,9 +844,11 @@ constexpr int kScanStep = 4;  // candidates loaded at a time
 template <int G> struct DenList { static constexpr int value = (G == 2) ? 40 : (G == 4 ? 24 : 16); };  // ~1.5x a lane's share of 50
 // The particles of the coarse levels, few, are not searched through their
 // mostly empty grids: each block picks those that reach its particles' box
-// and its lanes test these alone.  Beyond kBigScan of them the grids are
-// walked as well.
-constexpr int kBigScan = 4096;
+// and its lanes test these alone.  Beyond kBigScan of them, when every block
+// reads as many more, the grids are walked as well: us a launch for 200k
+// particles, direct and walked, 1000 coarse ones 107 and 96, 3000 172 and 128,
+// 4000 214 and 146 (300: 86 direct).
+constexpr int kBigScan = 512;
 
 // The rows of level k's cells that the support of particle i (position xi,
 // smoothing length hi) can touch: every j of the level has hsml_j <= Hk (the
@@ -916,17 +918,36 @@ struct LevelRows {
     }
 };
 
-// A coarse-level particle, few but with up to every particle in its support,
-// takes a block (of kBigThreads, in k_density of kDenThreads): its warps share the rows of a level's stencil,
-// the lanes fetch the slot ranges of up to 32 rows at once, then share each
-// row's candidates.  (With one warp each, the one with the longest list took
-// 38 us of the 200k flow's step in each of the three passes.)
+// The coarse-level particles, with up to every particle in their support, are
+// shared out over all blocks of the pair kernels (of kBigThreads, k_density of
+// kDenThreads); the first kBigBlocks blocks take nothing else, so that the usual
+// few do not hold up regular ones.  All warps of a block share a particle (with
+// one warp each, the one with the longest list took 38 us of the 200k flow's
+// step in each of the three passes), until there are more than four a block:
+// then a warp takes a particle, since there are warps enough and the block's
+// barriers and short rows count (20,000: 844 us a step, 1084 with blocks).  us a
+// step of 200k particles with 300, 1000, 5000 and 20,000 coarse ones of 8 times
+// the smoothing length: 208, 237, 423 and 844; with the first kBigBlocks blocks
+// alone 207, 255, 760 and 2790; without coarse ones 180.
 constexpr int kBigThreads = 256;
-constexpr int kBigBlocks = 148;  // the first blocks of the pair kernels take these particles, the others the regular ones
-template <int T, bool SPARSE, int SK, class F>
-__device__ __forceinline__ void block_rows(const Search& Q, const StepScalars* S, int i, F& f) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    constexpr int W = T / 32;
+constexpr int kBigBlocks = 148;
+// Calls f(i, lw) for this block's or warp's coarse particles; 1 << lw warps share one.
+template <int T, class F>
+__device__ __forceinline__ void coarse_particles(const StepScalars* S, F&& f) {
+    constexpr int LW = T == 256 ? 3 : 2;
+    static_assert(T == 32 << LW, "T is 128 or 256");
+    const int nreg = S->nreg, nbig = S->nbig;
+    const bool alone = nbig > 4 * (int)gridDim.x;
+    const int lw = alone ? 0 : LW, step = (int)gridDim.x << (LW - lw);
+    for (int b = alone ? (blockIdx.x << LW) + (threadIdx.x >> 5) : blockIdx.x; b < nbig; b += step) f(nreg + b, lw);
+}
+
+// The neighbours of coarse particle i: the sharing warps take the rows of a
+// level's stencil in turn, the lanes fetch the slot ranges of up to 32 rows at
+// once, then share each row's candidates.
+template <bool SPARSE, int SK, class F>
+__device__ __forceinline__ void coarse_rows(const Search& Q, const StepScalars* S, int i, int lw, F& f) {
+    const int lane = threadIdx.x & 31, wid = (threadIdx.x >> 5) & ((1 << lw) - 1);
     const float4 me = Q.xhm[i];
     const float2 xi = make_float2(me.x, me.y);
     const float hi = me.z;
@@ -934,11 +955,11 @@ __device__ __forceinline__ void block_rows(const Search& Q, const StepScalars* S
     for (int k = 0; k < S->nlev; k++) {
         LevelRows<SPARSE> rows;
         if (!rows.template open<SK>(S, k, xi, hi)) continue;
-        for (int rb = 0; rb < rows.nrow; rb += T) {
-            const int row = rb + W * lane + wid;
+        for (int rb = 0; rb < rows.nrow; rb += 32 << lw) {
+            const int row = rb + (lane << lw) + wid;
             int ja = 0, jb = 0;
             if (row < rows.nrow) rows.range(Q, row, ja, jb);
-            const int nr = min(32, (rows.nrow - rb - wid + W - 1) / W);
+            const int nr = min(32, (rows.nrow - rb - wid + (1 << lw) - 1) >> lw);
             for (int r = 0; r < nr; r++) {
                 const int a = __shfl_sync(0xffffffffu, ja, r), e = __shfl_sync(0xffffffffu, jb, r);
                 for (int j = a + lane; j < e; j += 32) {
@@ -952,15 +973,17 @@ __device__ __forceinline__ void block_rows(const Search& Q, const StepScalars* S
         }
     }
 }
-template <int SK, int T = kBigThreads, class F>
-__device__ __forceinline__ void block_neighbours(const Search& Q, const StepScalars* S, int i, F&& f) {
-    if (S->sparse) block_rows<T, true, SK>(Q, S, i, f);
-    else block_rows<T, false, SK>(Q, S, i, f);
+template <int SK, class F>
+__device__ __forceinline__ void coarse_neighbours(const Search& Q, const StepScalars* S, int i, int lw, F&& f) {
+    if (S->sparse) coarse_rows<true, SK>(Q, S, i, lw, f);
+    else coarse_rows<false, SK>(Q, S, i, lw, f);
 }
-// Sum over the block in a fixed order, in thread 0; every thread calls it.
-__device__ __forceinline__ double block_sum(double v) {
-    __shared__ double part[kBigThreads / 32];
+// Sum over the warps that share a particle, in a fixed order, in the first lane
+// of the first; every thread of them calls it.
+__device__ __forceinline__ double coarse_sum(double v, int lw) {
     v = warp_sum(v);
+    if (lw == 0) return v;
+    __shared__ double part[kBigThreads / 32];
     __syncthreads();
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
     __syncthreads();
@@ -969,23 +992,21 @@ __device__ __forceinline__ double block_sum(double v) {
         for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += part[w];
     return t;
 }
+__device__ __forceinline__ bool coarse_first(int lw) { return (threadIdx.x & (lw ? ~0u : 31u)) == 0; }
 
-// Summation density of the coarse-level particles, one block per particle:
-// the first kBigBlocks blocks of k_density.
+// Summation density of the coarse-level particles.
 template <int SKF, bool WS>
 __device__ __forceinline__ void density_big(const PState& A, const Search& Q, const StepScalars* S, const Rheo& c) {
     constexpr int SK = SupportScale<SKF>::value;
-    const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = blockIdx.x; b < nbig; b += kBigBlocks) {
-        const int i = nreg + b;
+    coarse_particles<kDenThreads>(S, [&](int i, int lw) {
         double acc = 0.0;
         const unsigned char si = WS ? Q.spec[i] : 0;
-        block_neighbours<SK, kDenThreads>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
+        coarse_neighbours<SK>(Q, S, i, lw, [&](int j, float4 o, const PairGeom& g) {
             if (WS && Q.spec[j] != si) return;  // type 1: not in the density (:1829)
             acc += (double)(o.w * sph_kernel_w<SKF>(g.r, g.mh));
         });
-        acc = block_sum(acc);
-        if (threadIdx.x == 0) {
+        acc = coarse_sum(acc, lw);
+        if (coarse_first(lw)) {
             float4 me = Q.xhm[i];
             float h = (float)((double)(sph_kernel_w<SKF>(0.f, me.z) * me.w) + acc);
             A.rho[i] = h;
@@ -993,7 +1014,7 @@ __device__ __forceinline__ void density_big(const PState& A, const Search& Q, co
             float p = (c.cgra05 * hc) * hc;
             Q.pterm[i] = (c.pa_sph == 1) ? p : p / (hc * hc);
         }
-    }
+    });
 }
 
 // Bound by FP32 issue and the latency of the gathers: 200k particles (release,
@@ -1007,10 +1028,8 @@ __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, S
     PDL_ENTRY();
     if ((S->sparse != 0) != SPARSE) return;
     if (__syncthreads_or(S->skip)) return;  // another block may set it meanwhile: one decision per block
-    if (blockIdx.x < kBigBlocks) {
-        density_big<SKF, WS>(A, Q, S, c);
-        return;
-    }
+    density_big<SKF, WS>(A, Q, S, c);
+    if (blockIdx.x < kBigBlocks) return;
     constexpr int SK = SupportScale<SKF>::value;
     constexpr int L = DenList<G>::value, P = kDenThreads / G;
     constexpr unsigned full = 0xffffffffu;
@@ -1253,19 +1272,16 @@ __device__ __forceinline__ void wir_pair_term(const Rheo& c, bool water, float m
     }
 }
 
-// Internal acceleration of the coarse-level particles, one block per particle:
-// the first kBigBlocks blocks of k_iforce.
+// Internal acceleration of the coarse-level particles.
 template <int SKF, bool WS>
 __device__ __forceinline__ void force_big(const PState& A, const Search& Q, const StepScalars* S, const Rheo& c,
                                           bool cross) {
     constexpr int SK = SupportScale<SKF>::value;
-    const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = blockIdx.x; b < nbig; b += kBigBlocks) {
-        const int i = nreg + b;
+    coarse_particles<kBigThreads>(S, [&](int i, int lw) {
         const float pi_ = Q.pterm[i], rhoi = A.rho[i];
         double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
         const unsigned char si = WS ? Q.spec[i] : 0;
-        block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
+        coarse_neighbours<SK>(Q, S, i, lw, [&](int j, float4 o, const PairGeom& g) {
             if (WS && Q.spec[j] != si) {  // type 0 only (:6899)
                 if (cross) {
                     float w, d0, d1;
@@ -1276,15 +1292,15 @@ __device__ __forceinline__ void force_big(const PState& A, const Search& Q, cons
             }
             pressure_pair<SKF>(c, pi_, rhoi, Q.pterm[j], A.rho[j], o.w, g, a0, a1);
         });
-        a0 = block_sum(a0);
-        a1 = block_sum(a1);
-        if (threadIdx.x == 0) Q.indv[i] = make_float2((float)a0, (float)a1);
+        a0 = coarse_sum(a0, lw);
+        a1 = coarse_sum(a1, lw);
+        if (coarse_first(lw)) Q.indv[i] = make_float2((float)a0, (float)a1);
         if (WS && cross) {
-            b0 = block_sum(b0);
-            b1 = block_sum(b1);
-            if (threadIdx.x == 0) Q.bxy[i] = make_float2((float)b0, (float)b1);
+            b0 = coarse_sum(b0, lw);
+            b1 = coarse_sum(b1, lw);
+            if (coarse_first(lw)) Q.bxy[i] = make_float2((float)b0, (float)b1);
         }
-    }
+    });
 }
 
 // With 4 or 8 lanes a particle a lane has some 6 to 12 entries and the one by
@@ -1525,8 +1541,8 @@ __device__ __forceinline__ void rk_finish(const PState& A, const Search& Q, Step
     }
 }
 
-// Internal acceleration: the coarse-level particles in the first kBigBlocks
-// blocks, the regular ones, G lanes each, in the others.  The
+// Internal acceleration: the coarse-level particles in all blocks, the regular
+// ones, G lanes each, in those from kBigBlocks on.  The
 // warps take the particles from the last to the first: the neighbour search
 // has just written the table front to back, so its last-written part (still
 // in L2) is read first, and av_vel, which walks the table front to back after
@@ -1537,10 +1553,8 @@ template <int SKF, bool WS, int G>
 __global__ void __launch_bounds__(kBigThreads, kPairBlocks<G>) k_iforce(PState A, Search Q, StepScalars* S, Rheo c, int n, int cross) {
     PDL_ENTRY();
     if (S->skip) return;
-    if (blockIdx.x < kBigBlocks) {
-        force_big<SKF, WS>(A, Q, S, c, cross != 0);
-        return;
-    }
+    force_big<SKF, WS>(A, Q, S, c, cross != 0);
+    if (blockIdx.x < kBigBlocks) return;
     constexpr int P = 32 / G;  // particles per warp
     const int nreg = S->nreg;
     const float hmax = o2f(S->hmax_o);
@@ -1729,35 +1743,40 @@ __device__ __forceinline__ void norm_store(const PState& A, const Rheo& c, int i
     next[i] = mass / ((h < c.h_inf) ? c.h_inf : h);
 }
 
+// A normalised sum of the coarse-level particles.
+template <int SKF>
+__device__ __forceinline__ void norm_big(const PState& A, const Search& Q, const StepScalars* S, const Rheo& c,
+                                         const float* hp, int clamp_prev, float* hout, const float* ratio,
+                                         float* next) {
+    constexpr int SK = SupportScale<SKF>::value;
+    coarse_particles<kBigThreads>(S, [&](int i, int lw) {
+        double den = 0.0;
+        coarse_neighbours<SK>(Q, S, i, lw, [&](int j, float4 o, const PairGeom& g) {
+            den += (double)(__ldg(ratio + j) * sph_kernel_w<SKF>(g.r, g.mh));
+        });
+        den = coarse_sum(den, lw);
+        if (coarse_first(lw)) {
+            const float4 me = Q.xhm[i];
+            den = (double)((sph_kernel_w<SKF>(0.f, me.z) * me.w) / prev_depth(c, hp, i, clamp_prev)) + den;
+            norm_store(A, c, i, me.w, den, hout, next);
+        }
+    });
+}
+
 // One normalised sum_density_Tools call: h_i = num_i / (W(0,h_i) m_i/hp_i +
 // sum_j (m_j/hp_j) W_ij), num_i the plain sum of k_density (in A.rho), hp the
 // previous call's depths; m_j/hp_j is gathered as the quotient that call left
 // (one division per particle instead of one per pair: 23 -> 9 us a call for
 // 60k particles, with four lanes a particle).  The coarse-level particles in
-// the first kBigBlocks blocks, the regular ones over the table in the others.
+// all blocks, the regular ones over the table in those from kBigBlocks on.
 template <int SKF, int G>
 __global__ void __launch_bounds__(kBigThreads, 5) k_norm(PState A, Search Q, StepScalars* S, Rheo c, int n, const float* hp,
                                                       int clamp_prev, float* hout, const float* ratio, float* next) {
     PDL_ENTRY();
-    constexpr int SK = SupportScale<SKF>::value;
     if (S->skip) return;
-    const int nreg = S->nreg, nbig = S->nbig;
-    if (blockIdx.x < kBigBlocks) {
-        for (int b = blockIdx.x; b < nbig; b += kBigBlocks) {
-            const int i = nreg + b;
-            double den = 0.0;
-            block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
-                den += (double)(__ldg(ratio + j) * sph_kernel_w<SKF>(g.r, g.mh));
-            });
-            den = block_sum(den);
-            if (threadIdx.x == 0) {
-                const float4 me = Q.xhm[i];
-                den = (double)((sph_kernel_w<SKF>(0.f, me.z) * me.w) / prev_depth(c, hp, i, clamp_prev)) + den;
-                norm_store(A, c, i, me.w, den, hout, next);
-            }
-        }
-        return;
-    }
+    const int nreg = S->nreg;
+    norm_big<SKF>(A, Q, S, c, hp, clamp_prev, hout, ratio, next);
+    if (blockIdx.x < kBigBlocks) return;
     constexpr int P = 32 / G;  // particles per warp
     const int lane = threadIdx.x & 31, gl = lane % G, bid = blockIdx.x - kBigBlocks, nb = gridDim.x - kBigBlocks;
     const int nw = (nreg + P - 1) / P;
@@ -2067,42 +2086,38 @@ __device__ __forceinline__ void xsph_pair(float2 vi, float rhoi, float2 vj, floa
 
 // av_vel (SPH_MAIN_2019.f90:3042-3099) with the start-of-step W_ij, then
 // v += 0.3*av for particles still inside the domain (:987-993); the coarse
-// particles in the first kBigBlocks blocks, the regular ones, G lanes each as
-// in k_iforce, in the others.
+// particles in all blocks, the regular ones, G lanes each as in k_iforce, in
+// those from kBigBlocks on.
 template <int SKF, bool WS>
 __device__ __forceinline__ void xsph_big(const Search& Q, const StepScalars* S, const PState& B) {
     constexpr int SK = SupportScale<SKF>::value;
-    const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = blockIdx.x; b < nbig; b += kBigBlocks) {
-        const int i = nreg + b;
-        if (B.flag[i]) continue;  // uniform over the block
+    coarse_particles<kBigThreads>(S, [&](int i, int lw) {
+        if (B.flag[i]) return;  // uniform over the warps that share i
         const float4 si = Q.xsv[i];
         const float2 vi = make_float2(si.x, si.y);
         const float rhoi = si.z;
         double a0 = 0.0, a1 = 0.0;
         const unsigned char own = WS ? Q.spec[i] : 0;
-        block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
+        coarse_neighbours<SK>(Q, S, i, lw, [&](int j, float4 o, const PairGeom& g) {
             if (WS && Q.spec[j] != own) return;  // type 0 only (SPH_MAIN_2019.f90:3071)
             const float4 sj = Q.xsv[j];
             xsph_pair<SKF>(vi, rhoi, make_float2(sj.x, sj.y), sj.z, sj.w, g, a0, a1);
         });
-        a0 = block_sum(a0);
-        a1 = block_sum(a1);
-        if (threadIdx.x == 0) {
+        a0 = coarse_sum(a0, lw);
+        a1 = coarse_sum(a1, lw);
+        if (coarse_first(lw)) {
             const float av0 = 0.3f * (float)a0, av1 = 0.3f * (float)a1;
             B.vel[i] = make_float2(vi.x + av0, vi.y + av1);
         }
-    }
+    });
 }
 
 template <int SKF, bool WS, int G>
 __global__ void __launch_bounds__(kBigThreads, kPairBlocks<G>) k_xsph(PState A, Search Q, StepScalars* S, Rheo c, int n, PState B) {
     PDL_ENTRY();
     if (S->skip || !c.av_vel) return;
-    if (blockIdx.x < kBigBlocks) {
-        xsph_big<SKF, WS>(Q, S, B);
-        return;
-    }
+    xsph_big<SKF, WS>(Q, S, B);
+    if (blockIdx.x < kBigBlocks) return;
     constexpr int P = 32 / G;     // particles per warp
     constexpr bool few = kFewPerLane<G>;
     const int nreg = S->nreg;
@@ -2251,14 +2266,12 @@ __global__ void k_dem_erode(double2* auxv, float* z, float* eroded, float* avail
 template <int SKF>
 __global__ void k_export_big(Search Q, StepScalars* S, int2* pairs, int* npairs, int cap) {
     constexpr int SK = SupportScale<SKF>::value;
-    const int nreg = S->nreg, nbig = S->nbig;
-    for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
-        int i = nreg + b;
-        block_neighbours<SK>(Q, S, i, [&](int j, float4 o, const PairGeom& g) {
+    coarse_particles<kBigThreads>(S, [&](int i, int lw) {
+        coarse_neighbours<SK>(Q, S, i, lw, [&](int j, float4 o, const PairGeom& g) {
             int k = atomicAdd(npairs, 1);
             if (k < cap) pairs[k] = make_int2(i, j);
         });
-    }
+    });
 }
 
 // ---------------------------------------------------------------- outputs

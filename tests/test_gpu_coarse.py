@@ -1,0 +1,92 @@
+"""The coarse-level particles of the pair kernels where their sharing changes: around the number that the density's
+direct scan takes (512), around one per block, and beyond four per block, where a warp takes a particle (9000 particles:
+430 blocks in the force and velocity passes, 711 in the density).  Sets are exact; densities and forces are FP64 sums of
+the oracle's FP32 terms in another order, so one rounding to FP32 separates them (1e-6)."""
+import numpy as np
+import pytest
+
+import gfsph
+import workloads
+
+pytestmark = pytest.mark.gpu
+N = 9000
+
+
+def cloud(far):
+    rng = np.random.default_rng(far)
+    x = rng.uniform(20.0, 170.0, (N, 2)).astype(np.float32)
+    hs = rng.uniform(0.8, 1.25, N).astype(np.float32)
+    hs[rng.choice(N, far, replace=False)] *= np.float32(8.0)
+    rho = rng.uniform(0.5, 1.5, N).astype(np.float32)
+    return x, rng.normal(0.0, 0.5, (N, 2)).astype(np.float32), rho, (rho * hs * hs * np.float32(0.25)), hs
+
+
+def handle(**opts):
+    z = np.zeros((64, 64), np.float32)
+    p = gfsph.make_params(workloads.voellmy_const(0.2, 500.0), pa_sph=2, nnps=2, sle=1, average_velocity=1, ic_adapt=0,
+                          h_inf=0.01, dt=1e-3, dem_deriv=1, **opts)
+    sim = gfsph.Sim(p, z, dx=5.0, dy=5.0)
+    sim.set_search(1.0, 3.0)  # coarse beyond twice the mean, so that up to 40 % of the particles can be
+    return sim, p, z
+
+
+@pytest.mark.parametrize("skf", [1, 3])
+@pytest.mark.parametrize("far", [148, 149, 430, 431, 512, 513, 1720, 1721, 2100])
+def test_sets_density_and_forces(gfsph_lib, oracle_mod, far, skf):
+    x, v, rho, mass, hs = cloud(far)
+    sim, p, _ = handle(skf=skf)
+    sim.upload(x, v, rho, mass, hs)
+    dens = sim.density()
+    assert sim.stats()["coarse"] == far
+    off, idx = sim.neighbours()
+    ref = oracle_mod.pairs(oracle_mod.MODE_FP32_DACC, p, x, hs, mass=mass, rho=rho, want_rho=True, want_force=True)
+    assert np.array_equal(off, ref["offsets"]) and np.array_equal(idx, ref["idx"])
+    assert np.max(np.abs(dens - ref["rho"]) / np.abs(ref["rho"])) <= 1e-6
+    f = sim.internal_forces()
+    assert np.abs(f - ref["force"]).max() <= 1e-6 * np.abs(ref["force"]).max()
+    sim.close()
+
+
+@pytest.mark.parametrize("opts", [{}, {"nor_density": 1}])
+@pytest.mark.parametrize("far", [431, 2100])
+def test_one_step(gfsph_lib, oracle_mod, far, opts):
+    """av_vel and the normalised density with coarse particles in every block, whole blocks and single warps."""
+    x, v, rho, mass, hs = cloud(far)
+    sim, p, z = handle(**opts)
+    sim.upload(x, v, rho, mass, hs)
+    sim.step(1)
+    g = sim.download()
+    sim.close()
+    topol = oracle_mod.initial_topol(z, 5.0, 5.0, {}, deriv=1, mode=oracle_mod.MODE_FP32_DACC)
+    st = oracle_mod.State(x, v, rho, mass, hs, topol, dt=p.dt)
+    oracle_mod.run(oracle_mod.MODE_FP32_DACC, p, 64, 64, 5.0, 5.0, st, 1)
+    assert np.array_equal(g["flag"], st.flag)
+    for key, ref in (("x", st.x), ("v", st.v), ("rho", st.rho), ("hsml", st.hsml)):
+        err = np.abs(g[key].astype(np.float64) - ref) / np.maximum(np.abs(ref), 1e-3)
+        assert err.max() <= 1e-6, (key, err.max())
+
+
+def test_many_coarse_particles_use_the_whole_chip(gfsph_lib):
+    """A tenth of 200,000 particles coarse, some five times the pairs: by a fixed 148 blocks the step took 15 times the
+    one without them, shared out over all blocks 4.7 times."""
+    w = workloads.fractal_channel(n_target=200_000, dem_k=10, cell=5.0, seed=3, erosion=None)
+    rng = np.random.default_rng(4)
+    best = []
+    for far in (0, 20_000):
+        x, hs = w.x.copy(), w.hsml.copy()
+        at = rng.choice(w.n, far, replace=False)
+        x[at] = rng.uniform(x.min(0), x.max(0), (far, 2))
+        hs[at] = np.float32(8.0 * np.median(w.hsml))
+        sim = gfsph.Sim(workloads.make_params(w, gfsph, sle=0, ic_adapt=0, dt=1e-4), w.z, dx=w.dx, dy=w.dy)
+        sim.upload(x, w.v, w.rho, w.mass, hs)
+        sim.step(10)
+        ms = []
+        for _ in range(3):
+            sim.profile(2)
+            sim.step(8)
+            ms.append(sim.profile_read()["step_batches"][0])
+            sim.profile(0)
+        assert sim.stats()["coarse"] == far
+        sim.close()
+        best.append(min(ms))
+    assert best[1] <= 8.0 * best[0], best
