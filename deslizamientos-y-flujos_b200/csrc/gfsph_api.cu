@@ -436,20 +436,22 @@ int enqueue_search(gfsph_handle* h, int advance) {
         // the two materials' pair types compiled in only when there are two
         with_lanes(n, [&](auto g) {
             constexpr int G = decltype(g)::value;
-            // Only the device knows which layout a step uses, and the launch for the other returns at once: both have
-            // the same grid, two rounds of resident blocks.  One block per SM for the layout the last batch did not
-            // use is right only until the layout changes: us a step, 60k 96 and 228 where it changed, 200k 211 and
-            // 655, 1M 867 and 2910.  One, two and three rounds for both: 60k 97 each, 200k 217, 211 and 214.5, its
-            // flow 250, 241.5 and 242.5, 1M 884, 867 and 883.
-            const int db = kBigBlocks + std::min(blocks_for((long long)n * G, kDenThreads), 148 * kDenBlocks * 2);
+            // Only the device knows which layout a step uses, and the launch for the other returns at once: their grids,
+            // two rounds of resident blocks and one, are right in either.  One block per SM for the layout the last
+            // batch did not use is right only until it changes: us a step, 60k 96 and 228 where it changed, 200k 211
+            // and 655, 1M 867 and 2910.  Rounds for the dense and the sparse layout, 3 and 3, 2 and 2, 2 and 1, 1 and
+            // 1: dense, 200k 215, 212, 211 and 217, its flow 242.5, 242, 241 and 255, 1M 885, 868, 867 and 886; sparse,
+            // 200k 215, 208, 211 and 210, 1M 726, 717, 712 and 712.
+            const int need = blocks_for((long long)n * G, kDenThreads), round = 148 * kDenBlocks;
+            const int db = kBigBlocks + std::min(need, 2 * round), sb = kBigBlocks + std::min(need, round);
             if (h->rheo.ws) {
                 launch(h, K_DENSITY, [&] { pdl_launch(k_density<false, SKF, true, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
                 launch(h, K_DENSITY_SPARSE,
-                       [&] { pdl_launch(k_density<true, SKF, true, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
+                       [&] { pdl_launch(k_density<true, SKF, true, G>, sb, kDenThreads, st, h->A, q, S, h->rheo, n); });
             } else {
                 launch(h, K_DENSITY, [&] { pdl_launch(k_density<false, SKF, false, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
                 launch(h, K_DENSITY_SPARSE,
-                       [&] { pdl_launch(k_density<true, SKF, false, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
+                       [&] { pdl_launch(k_density<true, SKF, false, G>, sb, kDenThreads, st, h->A, q, S, h->rheo, n); });
             }
         });
     });

@@ -918,28 +918,43 @@ struct LevelRows {
     }
 };
 
-// The coarse-level particles, with up to every particle in their support, are
-// shared out over all blocks of the pair kernels (of kBigThreads, k_density of
-// kDenThreads); the first kBigBlocks blocks take nothing else, so that the usual
-// few do not hold up regular ones.  All warps of a block share a particle (with
-// one warp each, the one with the longest list took 38 us of the 200k flow's
-// step in each of the three passes), until there are more than four a block:
-// then a warp takes a particle, since there are warps enough and the block's
-// barriers and short rows count (20,000: 844 us a step, 1084 with blocks).  us a
-// step of 200k particles with 300, 1000, 5000 and 20,000 coarse ones of 8 times
-// the smoothing length: 208, 237, 423 and 844; with the first kBigBlocks blocks
-// alone 207, 255, 760 and 2790; without coarse ones 180.
+// The coarse-level particles, with up to every particle in their support, have
+// blocks of their own in the pair kernels (of kBigThreads, k_density of
+// kDenThreads): the first kBigBlocks, which take the usual few, up to kBigRounds
+// each, beside the regular ones, and with more of them also the last half of the
+// others.  All warps of a block share a particle (with one warp each, the one
+// with the longest list took 38 us of the 200k flow's step in each of the three
+// passes), until there are more than four a block: then a warp takes a particle,
+// since there are warps enough and the block's barriers and short rows count.
+// us a step of 200k particles with 0, 300, 1000, 5000 and 20,000 coarse ones of
+// 8 times the smoothing length: 181, 208, 230, 374 and 870; with the first
+// kBigBlocks blocks alone 180, 207, 255, 760 and 2790; with one warp each and the
+// kernels of a thread per particle 246, 321, 342, 432 and 1000.  (Blocks that
+// take regular and coarse particles in turn, or more blocks behind the regular
+// ones, cost every step 1 to 3 %.)
 constexpr int kBigThreads = 256;
 constexpr int kBigBlocks = 148;
-// Calls f(i, lw) for this block's or warp's coarse particles; 1 << lw warps share one.
+constexpr int kBigRounds = 4;
+// What the pair kernels read of the scalars first, in one trip to memory, and
+// the blocks of the coarse particles: the first kBigBlocks and those from tail on.
+struct PairWork {
+    int skip, nreg, nbig, tail;
+    __device__ __forceinline__ explicit PairWork(const StepScalars* S) : skip(S->skip), nreg(S->nreg), nbig(S->nbig) {
+        const int grid = (int)gridDim.x;
+        tail = nbig > kBigRounds * kBigBlocks ? kBigBlocks + (grid - kBigBlocks + 1) / 2 : grid;
+    }
+    __device__ __forceinline__ bool coarse() const { return blockIdx.x < kBigBlocks || (int)blockIdx.x >= tail; }
+};
+// Calls f(i, lw) for the coarse particles of this block or warp; 1 << lw warps share one.
 template <int T, class F>
-__device__ __forceinline__ void coarse_particles(const StepScalars* S, F&& f) {
+__device__ __forceinline__ void coarse_particles(int nreg, int nbig, int tail, F&& f) {
     constexpr int LW = T == 256 ? 3 : 2;
     static_assert(T == 32 << LW, "T is 128 or 256");
-    const int nreg = S->nreg, nbig = S->nbig;
-    const bool alone = nbig > 4 * (int)gridDim.x;
-    const int lw = alone ? 0 : LW, step = (int)gridDim.x << (LW - lw);
-    for (int b = alone ? (blockIdx.x << LW) + (threadIdx.x >> 5) : blockIdx.x; b < nbig; b += step) f(nreg + b, lw);
+    const int nc = kBigBlocks + (int)gridDim.x - tail;
+    const int cb = blockIdx.x < kBigBlocks ? blockIdx.x : kBigBlocks + (int)blockIdx.x - tail;
+    const bool alone = nbig > 4 * nc;
+    const int lw = alone ? 0 : LW, step = nc << (LW - lw);
+    for (int b = alone ? (cb << LW) + (threadIdx.x >> 5) : cb; b < nbig; b += step) f(nreg + b, lw);
 }
 
 // The neighbours of coarse particle i: the sharing warps take the rows of a
@@ -996,9 +1011,9 @@ __device__ __forceinline__ bool coarse_first(int lw) { return (threadIdx.x & (lw
 
 // Summation density of the coarse-level particles.
 template <int SKF, bool WS>
-__device__ __forceinline__ void density_big(const PState& A, const Search& Q, const StepScalars* S, const Rheo& c) {
+__device__ __forceinline__ void density_big(const PState& A, const Search& Q, const StepScalars* S, const Rheo& c, const PairWork& pw) {
     constexpr int SK = SupportScale<SKF>::value;
-    coarse_particles<kDenThreads>(S, [&](int i, int lw) {
+    coarse_particles<kDenThreads>(pw.nreg, pw.nbig, pw.tail, [&](int i, int lw) {
         double acc = 0.0;
         const unsigned char si = WS ? Q.spec[i] : 0;
         coarse_neighbours<SK>(Q, S, i, lw, [&](int j, float4 o, const PairGeom& g) {
@@ -1027,9 +1042,12 @@ template <bool SPARSE, int SKF, bool WS, int G>
 __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, Search Q, StepScalars* S, Rheo c, int n) {
     PDL_ENTRY();
     if ((S->sparse != 0) != SPARSE) return;
-    if (__syncthreads_or(S->skip)) return;  // another block may set it meanwhile: one decision per block
-    density_big<SKF, WS>(A, Q, S, c);
-    if (blockIdx.x < kBigBlocks) return;
+    const PairWork pw(S);
+    if (__syncthreads_or(pw.skip)) return;  // another block may set it meanwhile: one decision per block
+    if (pw.coarse()) {
+        density_big<SKF, WS>(A, Q, S, c, pw);
+        return;
+    }
     constexpr int SK = SupportScale<SKF>::value;
     constexpr int L = DenList<G>::value, P = kDenThreads / G;
     constexpr unsigned full = 0xffffffffu;
@@ -1039,11 +1057,11 @@ __global__ void __launch_bounds__(kDenThreads, kDenBlocks) k_density(PState A, S
     __shared__ float wbox[kDenThreads / 32][5];
     __shared__ int wcnt[kDenThreads / 32];
     const int tid = threadIdx.x, gl = tid % G, lane = tid & 31, wid = tid >> 5;
-    const int nreg = S->nreg, nbig = S->nbig;
+    const int nreg = pw.nreg, nbig = pw.nbig;
     const bool scan_big = nbig > 0 && nbig <= kBigScan;
     const int nlev = (nbig > 0 && !scan_big) ? S->nlev : min(S->nlev, S->reg_levels);
     const float hmax = o2f(S->hmax_o);
-    const int bid = blockIdx.x - kBigBlocks, nb = gridDim.x - kBigBlocks;
+    const int bid = blockIdx.x - kBigBlocks, nb = pw.tail - kBigBlocks;
     for (int base = bid * P; base < nreg; base += nb * P) {  // the same trips for the whole block
         const int i = base + tid / G;
         const bool act = i < nreg;
@@ -1275,9 +1293,9 @@ __device__ __forceinline__ void wir_pair_term(const Rheo& c, bool water, float m
 // Internal acceleration of the coarse-level particles.
 template <int SKF, bool WS>
 __device__ __forceinline__ void force_big(const PState& A, const Search& Q, const StepScalars* S, const Rheo& c,
-                                          bool cross) {
+                                          bool cross, const PairWork& pw) {
     constexpr int SK = SupportScale<SKF>::value;
-    coarse_particles<kBigThreads>(S, [&](int i, int lw) {
+    coarse_particles<kBigThreads>(pw.nreg, pw.nbig, pw.tail, [&](int i, int lw) {
         const float pi_ = Q.pterm[i], rhoi = A.rho[i];
         double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
         const unsigned char si = WS ? Q.spec[i] : 0;
@@ -1541,8 +1559,8 @@ __device__ __forceinline__ void rk_finish(const PState& A, const Search& Q, Step
     }
 }
 
-// Internal acceleration: the coarse-level particles in all blocks, the regular
-// ones, G lanes each, in those from kBigBlocks on.  The
+// Internal acceleration: the coarse-level particles in their own blocks, the
+// regular ones, G lanes each, in the others.  The
 // warps take the particles from the last to the first: the neighbour search
 // has just written the table front to back, so its last-written part (still
 // in L2) is read first, and av_vel, which walks the table front to back after
@@ -1552,14 +1570,17 @@ __device__ __forceinline__ void rk_finish(const PState& A, const Search& Q, Step
 template <int SKF, bool WS, int G>
 __global__ void __launch_bounds__(kBigThreads, kPairBlocks<G>) k_iforce(PState A, Search Q, StepScalars* S, Rheo c, int n, int cross) {
     PDL_ENTRY();
-    if (S->skip) return;
-    force_big<SKF, WS>(A, Q, S, c, cross != 0);
-    if (blockIdx.x < kBigBlocks) return;
+    const PairWork pw(S);
+    if (pw.skip) return;
+    if (pw.coarse()) {
+        force_big<SKF, WS>(A, Q, S, c, cross != 0, pw);
+        return;
+    }
     constexpr int P = 32 / G;  // particles per warp
-    const int nreg = S->nreg;
+    const int nreg = pw.nreg;
     const float hmax = o2f(S->hmax_o);
     const int nw = (nreg + P - 1) / P;
-    const int lane = threadIdx.x & 31, bid = blockIdx.x - kBigBlocks, nb = gridDim.x - kBigBlocks;
+    const int lane = threadIdx.x & 31, bid = blockIdx.x - kBigBlocks, nb = pw.tail - kBigBlocks;
     for (int w = (bid * kBigThreads + threadIdx.x) >> 5; w < nw; w += (nb * kBigThreads) >> 5) {
         const int i = (nw - 1 - w) * P + lane / G;
         if (G == 1) {
@@ -1747,9 +1768,9 @@ __device__ __forceinline__ void norm_store(const PState& A, const Rheo& c, int i
 template <int SKF>
 __device__ __forceinline__ void norm_big(const PState& A, const Search& Q, const StepScalars* S, const Rheo& c,
                                          const float* hp, int clamp_prev, float* hout, const float* ratio,
-                                         float* next) {
+                                         float* next, const PairWork& pw) {
     constexpr int SK = SupportScale<SKF>::value;
-    coarse_particles<kBigThreads>(S, [&](int i, int lw) {
+    coarse_particles<kBigThreads>(pw.nreg, pw.nbig, pw.tail, [&](int i, int lw) {
         double den = 0.0;
         coarse_neighbours<SK>(Q, S, i, lw, [&](int j, float4 o, const PairGeom& g) {
             den += (double)(__ldg(ratio + j) * sph_kernel_w<SKF>(g.r, g.mh));
@@ -1768,17 +1789,20 @@ __device__ __forceinline__ void norm_big(const PState& A, const Search& Q, const
 // previous call's depths; m_j/hp_j is gathered as the quotient that call left
 // (one division per particle instead of one per pair: 23 -> 9 us a call for
 // 60k particles, with four lanes a particle).  The coarse-level particles in
-// all blocks, the regular ones over the table in those from kBigBlocks on.
+// their own blocks, the regular ones over the table in the others.
 template <int SKF, int G>
 __global__ void __launch_bounds__(kBigThreads, 5) k_norm(PState A, Search Q, StepScalars* S, Rheo c, int n, const float* hp,
                                                       int clamp_prev, float* hout, const float* ratio, float* next) {
     PDL_ENTRY();
-    if (S->skip) return;
-    const int nreg = S->nreg;
-    norm_big<SKF>(A, Q, S, c, hp, clamp_prev, hout, ratio, next);
-    if (blockIdx.x < kBigBlocks) return;
+    const PairWork pw(S);
+    if (pw.skip) return;
+    const int nreg = pw.nreg;
+    if (pw.coarse()) {
+        norm_big<SKF>(A, Q, S, c, hp, clamp_prev, hout, ratio, next, pw);
+        return;
+    }
     constexpr int P = 32 / G;  // particles per warp
-    const int lane = threadIdx.x & 31, gl = lane % G, bid = blockIdx.x - kBigBlocks, nb = gridDim.x - kBigBlocks;
+    const int lane = threadIdx.x & 31, gl = lane % G, bid = blockIdx.x - kBigBlocks, nb = pw.tail - kBigBlocks;
     const int nw = (nreg + P - 1) / P;
     for (int wp = (bid * kBigThreads + threadIdx.x) >> 5; wp < nw; wp += (nb * kBigThreads) >> 5) {
         const int i0 = wp * P + lane / G, i = min(i0, nreg - 1);
@@ -2086,12 +2110,12 @@ __device__ __forceinline__ void xsph_pair(float2 vi, float rhoi, float2 vj, floa
 
 // av_vel (SPH_MAIN_2019.f90:3042-3099) with the start-of-step W_ij, then
 // v += 0.3*av for particles still inside the domain (:987-993); the coarse
-// particles in all blocks, the regular ones, G lanes each as in k_iforce, in
-// those from kBigBlocks on.
+// particles in their own blocks, the regular ones, G lanes each as in k_iforce,
+// in the others.
 template <int SKF, bool WS>
-__device__ __forceinline__ void xsph_big(const Search& Q, const StepScalars* S, const PState& B) {
+__device__ __forceinline__ void xsph_big(const Search& Q, const StepScalars* S, const PState& B, const PairWork& pw) {
     constexpr int SK = SupportScale<SKF>::value;
-    coarse_particles<kBigThreads>(S, [&](int i, int lw) {
+    coarse_particles<kBigThreads>(pw.nreg, pw.nbig, pw.tail, [&](int i, int lw) {
         if (B.flag[i]) return;  // uniform over the warps that share i
         const float4 si = Q.xsv[i];
         const float2 vi = make_float2(si.x, si.y);
@@ -2115,13 +2139,16 @@ __device__ __forceinline__ void xsph_big(const Search& Q, const StepScalars* S, 
 template <int SKF, bool WS, int G>
 __global__ void __launch_bounds__(kBigThreads, kPairBlocks<G>) k_xsph(PState A, Search Q, StepScalars* S, Rheo c, int n, PState B) {
     PDL_ENTRY();
-    if (S->skip || !c.av_vel) return;
-    xsph_big<SKF, WS>(Q, S, B);
-    if (blockIdx.x < kBigBlocks) return;
+    const PairWork pw(S);
+    if (pw.skip || !c.av_vel) return;
+    if (pw.coarse()) {
+        xsph_big<SKF, WS>(Q, S, B, pw);
+        return;
+    }
     constexpr int P = 32 / G;     // particles per warp
     constexpr bool few = kFewPerLane<G>;
-    const int nreg = S->nreg;
-    const int lane = threadIdx.x & 31, gl = lane % G, bid = blockIdx.x - kBigBlocks, nb = gridDim.x - kBigBlocks;
+    const int nreg = pw.nreg;
+    const int lane = threadIdx.x & 31, gl = lane % G, bid = blockIdx.x - kBigBlocks, nb = pw.tail - kBigBlocks;
     const int nw = (nreg + P - 1) / P;
     for (int wp = (bid * kBigThreads + threadIdx.x) >> 5; wp < nw; wp += (nb * kBigThreads) >> 5) {
         const int i0 = wp * P + lane / G, i = min(i0, nreg - 1);
@@ -2266,7 +2293,7 @@ __global__ void k_dem_erode(double2* auxv, float* z, float* eroded, float* avail
 template <int SKF>
 __global__ void k_export_big(Search Q, StepScalars* S, int2* pairs, int* npairs, int cap) {
     constexpr int SK = SupportScale<SKF>::value;
-    coarse_particles<kBigThreads>(S, [&](int i, int lw) {
+    coarse_particles<kBigThreads>(S->nreg, S->nbig, kBigBlocks, [&](int i, int lw) {
         coarse_neighbours<SK>(Q, S, i, lw, [&](int j, float4 o, const PairGeom& g) {
             int k = atomicAdd(npairs, 1);
             if (k < cap) pairs[k] = make_int2(i, j);
