@@ -1346,6 +1346,12 @@ int gfsph_upload(gfsph_handle* h, int n, const float* x, const float* v, const f
     CK(cudaGetLastError());
     h->has_state = true;
     h->searched = false;
+    // The caller's arrays are its own again on return, whatever memory they are in: page-locked ones are read by the
+    // kernel or the copies above while this call would already have returned.  (A stream that is being captured only
+    // records the reads and cannot be waited for.)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &capture));
+    if (capture == cudaStreamCaptureStatusNone) CK(cudaStreamSynchronize(st));
     return GFSPH_OK;
 } catch (...) {  // a C++ exception never crosses the C ABI
     return GFSPH_ERR_HOST;
@@ -1419,9 +1425,9 @@ int gfsph_set_time(gfsph_handle* h, double t, float dt) try {
     if (!h || !(dt > 0.f)) return GFSPH_ERR_ARG;
     h->hS->time = t;
     h->hS->dt = dt;
+    // t and dt are arguments of the kernel: nothing of the caller is read later, and there is nothing to wait for
     k_set_time<<<1, 1, 0, h->stream>>>(h->S, t, dt);
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(h->stream));
     return GFSPH_OK;
 } catch (...) {  // a C++ exception never crosses the C ABI
     return GFSPH_ERR_HOST;

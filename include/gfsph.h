@@ -155,7 +155,10 @@ int gfsph_destroy(gfsph_handle* h);
  * bed, with sw_alg 1, is the soil surface Z + hs (Get_hs_at_w_SW
  * :17789-17938, IntForces_SW :6809-6828, Get_Grav_Ext_SW :9322-9331).  That
  * option runs the staged RK45 (the soil surface of every stage); it excludes
- * erosion, pore pressure, nor_density and ic_cosTheta = 1, and the adjoint. */
+ * erosion, pore pressure, nor_density and ic_cosTheta = 1, and the adjoint.
+ * The arrays have been read when the call returns, page-locked ones too
+ * (unless the handle's stream is being captured, when nothing can wait: they
+ * are then read each time the graph runs). */
 int gfsph_upload(gfsph_handle* h, int n, const float* x, const float* v, const float* rho,
                  const float* mass, const float* hsml, const int* itype, const int* out_flag);
 
