@@ -21,17 +21,25 @@ __device__ __forceinline__ float ipow5(float x) {
 }
 
 // Correctly rounded reciprocal, square root and quotient from the hardware's
-// approximations, for operands that the caller bounds (kQuotMin .. kQuotMax
-// below), so that no range check and no slow path is compiled in:
+// approximations, for operands that the caller bounds, so that no range check
+// and no slow path is compiled in:
 // - recip: one Newton-Raphson step in FMA on the approximate reciprocal;
 // - root: Markstein's square root step (P. Markstein, "Computation of
 //   elementary functions on the IBM RISC System/6000 processor", 1990) on the
 //   approximate reciprocal root: g = d y, then g + (d - g g) y/2;
-// - quot: his division step with y = RN(1/b): q = RN(a y), the exact
-//   remainder r = a - q b, RN(q + r y) = RN(a/b); several quotients by one
-//   denominator share the reciprocal.
+// - quot: his division step with y = RN(1/b): q = RN(a y), the remainder
+//   r = a - q b, RN(q + r y) = RN(a/b); several quotients by one denominator
+//   share the reciprocal.  r has to be exact and q normal: with b within 1e-18
+//   .. 1e18, a 0 (the quotient is then +0) or within 2^-60 .. 2^61 (quot_fits;
+//   ulp(q) ulp(b) is then 2^-107 or more, and q between 2^-121 and 2^122).
 // The first two equal the IEEE operators for every mantissa, the third in
-// 1.8e10 random quotients (tests/test_gpu_rounding.py repeats the check).
+// 1.2e9 quotients of random operands and of dividends next to the midpoints
+// between two floats (tests/test_gpu_rounding.py).  recip_any, root_any and
+// quot2 take any operand.  The step's pair terms and basal laws use quot as it
+// is: their numerators leave its range only where a velocity or a friction is
+// infinite (the quotient is NaN where the operator gives an infinity, and the
+// next step stops with either) or below 1e-18, where a last bit of the quotient
+// is far below every sum it enters.
 __device__ __forceinline__ float recip(float b) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
@@ -47,6 +55,11 @@ __device__ __forceinline__ float quot(float a, float b, float y) {
     const float q = a * y;
     return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
 }
+__device__ __forceinline__ bool quot_fits(float a) {
+    const unsigned u = __float_as_uint(a) << 1;  // without the sign: exponent 67 .. 187
+    return u - 0x43000000u < 0x79000000u || u == 0u;
+}
+__device__ __forceinline__ float recip_any(float b) { return (b > 1.e-30f && b < 1.e30f) ? recip(b) : 1.f / b; }
 // Two FP32 values in one register pair, with Blackwell's two-wide operations:
 // each half rounds as the scalar operation does, for one instruction issued
 // instead of two.  The pair kernels are bound by instruction issue.
@@ -111,8 +124,9 @@ __device__ __forceinline__ F2 quot(F2 a, F2 nb, F2 y) {
 }
 // The square root of any value: root() within its range, else the operator.
 __device__ __forceinline__ float root_any(float d) { return (d >= 1.e-30f && d <= 1.e37f) ? root(d) : sqrtf(d); }
-// Smoothing lengths for which every product and quotient of a pair's kernel
-// stays far from overflow and underflow.
+// Smoothing lengths for which a pair's kernel is the operators' value: no
+// remainder is inexact, the smallest quotients (next to the edge of the support
+// (2 - q)^2 times about 1/h^3) included.
 constexpr float kQuotMin = 1.e-6f, kQuotMax = 1.e9f;
 
 // kernel_TOOLS, My_SPH_Tools_2019.f90:2062-2180 (2-D; skf 1 cubic spline,
@@ -367,7 +381,8 @@ struct DemView {
 };
 
 // The DEM node (1-based) at or below a point of the box, as
-// int((x - xmin)/dx + 1).
+// int((x - xmin)/dx + 1).  (In the box quot's numerators are 0, or so small that
+// nothing of the quotient reaches the sum, or within its range.)
 __device__ __forceinline__ int dem_node_x(const DemView& d, float xx) {
     return (int)(quot(xx - d.xmin, d.dx, d.rdx) + 1.f);
 }
@@ -466,12 +481,22 @@ __device__ __forceinline__ float pow73(float x) {
     return (lo == hi) ? lo : powr(x, 7.f / 3.f);
 }
 
-// a/b and c/b for b > 0, sharing a reciprocal where b allows it.
-__device__ __forceinline__ void quot2(float a, float c, float b, float& qa, float& qc) {
+// a/b and c/b for b > 0, sharing a reciprocal where b allows it, a and c as for
+// quot.
+__device__ __forceinline__ void quot2_in(float a, float c, float b, float& qa, float& qc) {
     if (b > 1.e-18f && b < 1.e18f) {
         const float y = recip(b);
         qa = quot(a, b, y);
         qc = quot(c, b, y);
+    } else {
+        qa = a / b;
+        qc = c / b;
+    }
+}
+// The same for any a and c.
+__device__ __forceinline__ void quot2(float a, float c, float b, float& qa, float& qc) {
+    if (quot_fits(a) && quot_fits(c)) {
+        quot2_in(a, c, b, qa, qc);
     } else {
         qa = a / b;
         qc = c / b;

@@ -99,13 +99,12 @@ __device__ __forceinline__ void frictlaws(const GflConst& c, float tanfi, const 
                                           float& correx, float& correy) {
     const float gtanfi = c.cgra * tanfi, gtanfi8 = c.cgra * c.tanfi8;
     float hinv = 0.f;
-    if (h > 1.e-30f) hinv = recip(h);
-    else if (h > 0.f) hinv = 1.f / h;
+    if (h > 0.f) hinv = recip_any(h);
     const float hfrict = fmaxf(h, c.hfrict0);
     const float hvmod = root_any(hu * hu + hv * hv);
     const float vmod = hvmod * hinv;
     float hvmodinv = 0.f;
-    if (hvmod >= 1.e-5f) hvmodinv = recip(hvmod);
+    if (hvmod >= 1.e-5f) hvmodinv = recip_any(hvmod);
     const float pwp = 0.f;
     frictx = 0.f;
     fricty = 0.f;
@@ -220,7 +219,7 @@ __global__ void __launch_bounds__(kGflThreads) k_gfl_nodes(GflDev d, GflConst c,
     for (int ip = blockIdx.x * blockDim.x + threadIdx.x; ip < d.npoin; ip += gridDim.x * blockDim.x) {
         const float h = d.unkno[3 * (size_t)ip], hu = d.unkno[3 * (size_t)ip + 1], hv = d.unkno[3 * (size_t)ip + 2];
         float hinv = 0.f;
-        if (h >= c.comp) hinv = (h > 1.e-30f) ? recip(h) : 1.f / h;
+        if (h >= c.comp) hinv = recip_any(h);
         float HH, pres;
         if (c.ntype == 2) {
             HH = c.swl - d.topol[ip];
@@ -318,7 +317,7 @@ __global__ void __launch_bounds__(kGflThreads) k_gfl_elems(GflDev d, GflConst c,
             const float h = var[0] + delt2 * (src[0] - div[0]), hu = var[1] + delt2 * (src[1] - div[1]),
                         hv = var[2] + delt2 * (src[2] - div[2]);
             float hinv = 0.f;
-            if (h >= c.comp) hinv = (h > 1.e-30f) ? recip(h) : 1.f / h;
+            if (h >= c.comp) hinv = recip_any(h);
             float HH, pres;
             if (c.ntype == 2) {
                 HH = 0.f;

@@ -1490,6 +1490,15 @@ __device__ __forceinline__ void erosion_scatter(const DemView& dem, float xx, fl
         R.term[o][lane] = inside ? quot(base, dist, y) : 0.f;
         R.term[16 + o][lane] = inside ? y : 0.f;
     }
+    if (part && !quot_fits(base)) {  // beyond quot: an infinite rate, or next to none
+#pragma unroll 1
+        for (int o = 0; o < 16; o++) {
+            const int ix = ipx + (o >> 2) - 1, iy = ipy + (o & 3) - 1;
+            const float ddx = xx - (dem.xmin + (float)(ix - 1) * dem.dx), ddy = xy - (dem.ymin + (float)(iy - 1) * dem.dy);
+            if (ix >= 1 && ix <= dem.nx && iy >= 1 && iy <= dem.ny)
+                R.term[o][lane] = base / fmaxf(sqrtf(ddx * ddx + ddy * ddy), 1.e-6f);
+        }
+    }
     add_node_runs(R, lane, key, ipx, ipy, dem.nx, dem.ny, auxv);
     if (part) {
         box.x0 = min(box.x0, max(1, ipx - 1)); box.x1 = max(box.x1, min(dem.nx, ipx + 2));
@@ -2096,7 +2105,7 @@ __device__ __forceinline__ void xsph_terms(float2 vi, float rhoi, float2 vj, flo
     const float den = rhoi + rhoj;
     const float n0 = (2.f * mj) * (vi.x - vj.x), n1 = (2.f * mj) * (vi.y - vj.y);
     float q0, q1;
-    quot2(n0, n1, den, q0, q1);
+    quot2_in(n0, n1, den, q0, q1);
     a0 -= (double)(q0 * w);
     a1 -= (double)(q1 * w);
 }
