@@ -1571,10 +1571,12 @@ int gfsph_internal_forces(gfsph_handle* h, float* indvxdt) try {
     }
     launch(h, K_IFORCE, [&] {
         with_skf(h, [&](auto sk) {
-            if (h->rheo.ws)
-                k_iforce<decltype(sk)::value, true, 1><<<pair_blocks(n, 1), kBigThreads, 0, s>>>(As[0], q, h->S, h->rheo, n, 0);
-            else
-                k_iforce<decltype(sk)::value, false, 1><<<pair_blocks(n, 1), kBigThreads, 0, s>>>(As[0], q, h->S, h->rheo, n, 0);
+            with_pair_lanes(n, [&](auto g) {  // the step's own kernel for this many particles
+                constexpr int SKF = decltype(sk)::value, G = decltype(g)::value;
+                const int fb = pair_blocks(n, G);
+                if (h->rheo.ws) k_iforce<SKF, true, G><<<fb, kBigThreads, 0, s>>>(As[0], q, h->S, h->rheo, n, 0);
+                else k_iforce<SKF, false, G><<<fb, kBigThreads, 0, s>>>(As[0], q, h->S, h->rheo, n, 0);
+            });
         });
     });
     launch(h, K_FORCE_RK, [&] {
