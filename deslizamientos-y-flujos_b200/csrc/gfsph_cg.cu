@@ -94,9 +94,10 @@ __device__ __forceinline__ double sum_partials(const double* part, int nb) {
     return warp_sum(v);
 }
 
-// Polls of a barrier wait before it gives up (about a second; a barrier of
-// co-resident blocks takes microseconds).
-constexpr long long kBarrierPolls = 1LL << 23;
+// Polls of a barrier wait before it gives up: two reads of L2 and a pause each,
+// about a microsecond, so about a second in all (a barrier of co-resident blocks
+// takes microseconds).
+constexpr long long kBarrierPolls = 1LL << 20;
 
 // Grid barrier over the co-resident blocks of a cooperative launch, with a
 // reduction: thread 0 holds the block's nr sums in mine; they go to part[r*nb +
@@ -567,7 +568,6 @@ int gfsph_cg_create(int npoin, int nelem, int nnode, int ndofn, const int* intma
     if (c->regs) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_iterate<kCgRows>, kCgIterThreads, 0);
     else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_iterate<0>, kCgIterThreads, 0);
     c->coop_blocks = std::max(1, std::min(want, nsm * std::max(per_sm, 1)));
-    if (c->regs && (long long)c->coop_blocks * kCgIterThreads * kCgRows < n) c->regs = false;
     cudaMemcpy(c->first, first.data(), nwarp * sizeof(int), cudaMemcpyHostToDevice);
     cudaMemcpy(c->len, len.data(), n * sizeof(int), cudaMemcpyHostToDevice);
     cudaMemcpy(c->col, col.data(), total * sizeof(int), cudaMemcpyHostToDevice);
