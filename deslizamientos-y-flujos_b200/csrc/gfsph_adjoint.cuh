@@ -55,7 +55,8 @@ __device__ __forceinline__ void sph_kernel_hess(int skf, float r, float mh, bool
 }
 
 // 1/b in FP64 from the FP32 reciprocal by two Newton-Raphson steps, for b
-// within FP32's range; within an ulp.
+// within FP32's range: the correctly rounded value unless b's mantissa is 53
+// ones, which neither an FP32 value nor the sum of two has (48 set bits at most).
 __device__ __forceinline__ double recip64(double b) {
     if (!(b > 1.e-30 && b < 1.e30)) return 1.0 / b;
     double y = (double)recip((float)b);

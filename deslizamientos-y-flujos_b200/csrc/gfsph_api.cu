@@ -332,11 +332,10 @@ void with_skf(const gfsph_handle* h, F&& f) {
 // Calls f with std::integral_constant<int, lanes per particle> of k_density
 // for n particles.  Few particles leave the chip idle and the step waits for
 // the longest chain of one lane: more lanes shorten it (850 particles: 57 us a
-// launch with one, 9 with 8; 23k: 4 and 8 lanes equal, 3.29 and 3.32 ms per 25
-// steps).  Then the chip is full and the lanes' uneven rows and shuffles count:
-// us a launch with 4 and 2 lanes 20k 23 and 25, 30k 26 and 26, 45k 34 and 27.5,
-// 60k 38.5 and 32 (200k particles, 20 steps with their copies: 6.4, 6.0, 6.4 ms
-// for 1, 2, 4 lanes; 1M, 10 steps: 10.2, 9.7, 10.6 ms).
+// launch with one, 9 with 8).  Then the chip is full and the lanes' uneven rows
+// and shuffles count.  us a step of a flow with 8 and 4 lanes: 6k 76 and 74.5, 9k
+// 78 and 76.5, 12k 81 and 80, 16k 88 and 88 (850: the launch 9 and 12); with 4 and
+// 2: 30k 94 and 102, 45k 104 and 104, 60k 118 and 113.5.
 template <class F>
 void with_lanes(int n, F&& f) {
     if (n < 12000) f(std::integral_constant<int, 8>{});
@@ -345,12 +344,14 @@ void with_lanes(int n, F&& f) {
 }
 
 // The same for the kernels over the neighbour table, which wait for their
-// gathers.  k_iforce and k_xsph, us a launch with 8 / 4 / 2 / 1 lanes: 850
-// particles 4 and 3 with 8, 5 and 5 with 4; 23k 9 and 7, 7 and 5; 200k - , 41
-// and 32, 33 and 27, 33 and 30; 1M -, -, 150 and 120, 130 and 107.  Between 4 and 2
-// (the whole step): 30k 85 and 98, 45k 95 and 92.5, 60k 108 and 101, 80k 121 and
-// 120.  four: up to where 4 lanes (the adjoint kernels, with more work a pair,
-// gain from them longer: 18 us a launch against 24 for 50k).
+// gathers.  us a step of a flow with k_iforce and k_xsph of 8 and 4 lanes: 6k 76
+// and 72, 9k 78 and 80, 12k 81 and 83, 16k 89 and 88 (850: the launches 4 and 3
+// with 8, 5 and 5 with 4); with 4 and 2: 30k 93 and 92, 45k 105 and 104, 60k 117
+// and 112; with 2 and 1: 200k 241.5 and 249, 350k 398 and 397, 500k 533 and 527,
+// 700k 802 and 781.  four: up to where 4 lanes.  The adjoint kernels, with more
+// work a pair, gain from them longer; us a step of the sweep with 8, 4 and 2: 6k
+// 170, 181, 195, 12k 193, 195, 212, 60k 321, 314, 321, 100k 481, 467, 475, 150k 655,
+// 627, 634: beyond the line 4 lanes would still be 1 % ahead.
 constexpr int kAdjFourLanes = 100000;
 template <class F>
 void with_pair_lanes(int n, F&& f, int four = 45000) {

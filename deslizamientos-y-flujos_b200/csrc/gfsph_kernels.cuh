@@ -598,9 +598,6 @@ __global__ void k_hist(const PState B, int n, DemView dem, StepScalars* S, TileS
         if (lmax[k]) atomicMax(&S->lev_hmax_o[k], lmax[k]);
 }
 
-// Exclusive scan of the histogram, tile pass: each block scans kScanTile
-// cells and writes its tile total.
-// only_sparse: the block-map scan, which dense steps skip.
 // Exclusive prefix of the tile sums, by one block (1 <= ntiles <= kScanTops *
 // blockDim.x): tile_sum[t] becomes the first index of tile t.
 constexpr int kScanTops = 32;
@@ -1327,7 +1324,9 @@ __device__ __forceinline__ void force_big(const PState& A, const Search& Q, cons
 // few particles leave room).  us with ~6 of the event, k_iforce / k_xsph: 850
 // particles 10.6 / 10.5 -> 8.9 / 8.6; a step of 13k 79 -> 75, of 23k 91 -> 88.
 // With 1 or 2 lanes occupancy hides the rest and the registers spill (1M
-// particles 142 -> 210).
+// particles 142 -> 210).  Soil and water with 2 lanes spill 52 B at 4 blocks and
+// nothing at 3, a step of 60k 263 and 254 us, but of 120k 334 and 344, of 250k 608
+// and 629 (1 lane, 560k: equal).
 template <int G>
 constexpr bool kFewPerLane = G >= 4;
 template <int G>
