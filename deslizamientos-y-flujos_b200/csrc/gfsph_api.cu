@@ -438,13 +438,17 @@ int enqueue_search(gfsph_handle* h, int advance) {
         with_lanes(n, [&](auto g) {
             constexpr int G = decltype(g)::value;
             // Only the device knows which layout a step uses, and the launch for the other returns at once: their grids,
-            // two rounds of resident blocks and one, are right in either.  One block per SM for the layout the last
-            // batch did not use is right only until it changes: us a step, 60k 96 and 228 where it changed, 200k 211
+            // two rounds of resident blocks and one, or eight, are right in either.  One block per SM for the layout the
+            // last batch did not use is right only until it changes: us a step, 60k 96 and 228 where it changed, 200k 211
             // and 655, 1M 867 and 2910.  Rounds for the dense and the sparse layout, 3 and 3, 2 and 2, 2 and 1, 1 and
             // 1: dense, 200k 215, 212, 211 and 217, its flow 242.5, 242, 241 and 255, 1M 885, 868, 867 and 886; sparse,
-            // 200k 215, 208, 211 and 210, 1M 726, 717, 712 and 712.
+            // 200k 215, 208, 211 and 210, 1M 726, 717, 712 and 712.  Beyond 24 rounds' work the
+            // blocks' shares differ by more than a round takes, and more, shorter blocks even them out: us a step with 2 and 1 rounds, 4 and 4, 8 and 8: dense, 1.3M 1045, 1042, 1046, 1.7M 1329,
+            // 1329, 1327, 2.4M 1875, 1854, 1823, 4M 3096, 3036, 2961; sparse, 4M 3097, 2984, 2932.
             const int need = blocks_for((long long)n * G, kDenThreads), round = 148 * kDenBlocks;
-            const int db = kBigBlocks + std::min(need, 2 * round), sb = kBigBlocks + std::min(need, round);
+            const bool many = (long long)n * G > 24LL * round * kDenThreads;
+            const int db = kBigBlocks + std::min(need, (many ? 8 : 2) * round);
+            const int sb = kBigBlocks + std::min(need, (many ? 8 : 1) * round);
             if (h->rheo.ws) {
                 launch(h, K_DENSITY, [&] { pdl_launch(k_density<false, SKF, true, G>, db, kDenThreads, st, h->A, q, S, h->rheo, n); });
                 launch(h, K_DENSITY_SPARSE,
