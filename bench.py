@@ -45,7 +45,7 @@ B_ALG = {"k_density": 24, "k_iforce": 24, "k_force_rk": 48, "k_xsph": 44, "k_his
 # The issue-bound figure is printed only when the run times those same steps,
 # since the neighbour work per step grows as the flow spreads.
 NCU_STEPS = (6, 25)
-NCU_PER_PARTICLE = {"k_density": {"warp_inst": 53.89e6 / 200011, "dram_bytes": 61.77e6 / 200011}}
+NCU_PER_PARTICLE = {"k_density": {"warp_inst": 54.55e6 / 200011, "dram_bytes": 61.73e6 / 200011}}
 NCU_SOURCE = "profiles/neighbour_kernels_fractal_channel_200k.md (ncu, cold caches, steps 6/16/25), scaled by active particles"
 ISSUE_PEAK = 148 * 4 * 1.965e9  # warp instructions/s: SMs x schedulers x max SM clock
 
