@@ -1332,7 +1332,7 @@ __device__ __forceinline__ void force_big(const PState& A, const Search& Q, cons
 // few particles leave room).  us with ~6 of the event, k_iforce / k_xsph: 850
 // particles 10.6 / 10.5 -> 8.9 / 8.6; a step of 13k 79 -> 75, of 23k 91 -> 88.
 // With 1 or 2 lanes occupancy hides the rest and the registers spill (1M
-// particles 142 -> 210).  Soil and water with 2 lanes spill 56 B at 4 blocks and
+// particles 142 -> 210).  Soil and water with 2 lanes spill 52 B at 4 blocks and
 // nothing at 3, a step of 60k 263 and 254 us, but of 120k 334 and 344, of 250k 608
 // and 629 (1 lane, 560k: equal).
 template <int G>
@@ -1597,9 +1597,8 @@ __global__ void __launch_bounds__(kBigThreads, kPairBlocks<G>) k_iforce(PState A
     const float hmax = o2f(S->hmax_o);
     const int nw = (nreg + P - 1) / P;
     const int lane = threadIdx.x & 31, bid = blockIdx.x - kBigBlocks, nb = pw.tail - kBigBlocks;
-    // counted down: with both ends of the count kept, two lanes spill 20 B
-    for (int w = nw - 1 - ((bid * kBigThreads + threadIdx.x) >> 5); w >= 0; w -= (nb * kBigThreads) >> 5) {
-        const int i = w * P + lane / G;
+    for (int w = (bid * kBigThreads + threadIdx.x) >> 5; w < nw; w += (nb * kBigThreads) >> 5) {
+        const int i = (nw - 1 - w) * P + lane / G;
         if (G == 1) {
             const int rows = __reduce_max_sync(0xffffffffu, Q.ncount[min(i, nreg - 1)]);
             const size_t at = tab_base(i - lane, Q.kcap);
