@@ -1334,7 +1334,9 @@ __device__ __forceinline__ void force_big(const PState& A, const Search& Q, cons
 // With 1 or 2 lanes occupancy hides the rest and the registers spill (1M
 // particles 142 -> 210).  Soil and water with 2 lanes spill 52 B at 4 blocks and
 // nothing at 3, a step of 60k 263 and 254 us, but of 120k 334 and 344, of 250k 608
-// and 629 (1 lane, 560k: equal).
+// and 629 (1 lane, 560k: equal).  k_iforce for one material with 2 lanes spills
+// 20 B; its warps counted down instead spill nothing and are slower, 200k
+// particles 43 and 45 us.
 template <int G>
 constexpr bool kFewPerLane = G >= 4;
 template <int G>
